@@ -275,7 +275,7 @@ def measure_tf32_peak(device_index: int):
 
 def tf32_slots(kernel_name: str) -> float:
     """TF32-instruction-equivalents of tensor-core time per fp32 product of a kernel's arithmetic."""
-    return 2.0 if "tf32_bf16x2" in kernel_name else 3.0
+    return 1.5 if "f16x3" in kernel_name else (2.0 if "tf32_bf16x2" in kernel_name else 3.0)
 
 
 def kernel_table(trace, precision: str, peaks, tf32_peak):

@@ -70,6 +70,10 @@ struct Node {
     bool xchg = false, xchg_replicate_x = false;
     int xchg_res = -1, xchg_x = -1, xchg_y = -1, xchg_gamma = -1, xchg_beta = -1;
     float xchg_eps = 0.f;
+    // the node leaves its output in split form (runtime.hpp): scales and row maxima of it, and how many maxima per row
+    bool splits = false;
+    size_t split_off = 0;
+    int split_parts = 1;
 };
 
 }  // namespace
@@ -108,6 +112,8 @@ struct fxf_engine {
     size_t p2p_off = 0;
     PeerMap peers;
     bool peers_mapped = false;
+    std::vector<SplitMat> splits;      // by tensor id: activations kept in split form in their arena slots
+    std::vector<uint32_t> split_root;  // by tensor id: the tensor whose storage it shares
     // decode that evaluates the final Linear only at the position whose logits are read
     int tail_node = -1;                // index of that Linear (the last node), -1 when the graph does not end in one
     size_t lastrow_off = 0, lastrow_bytes = 0;  // its [B,V] output
@@ -157,7 +163,20 @@ int run_node(fxf_engine* e, size_t i) {
         e->ctx.xchg.eps = n.xchg_eps;
         e->ctx.xchg.replicate_x = n.xchg_replicate_x;
     }
+    e->ctx.split_out = SplitOut{};
+    if (n.splits) {
+        const int64_t rows = n.plan->split_rows;
+        SplitOut& so = e->ctx.split_out;
+        so.planes = static_cast<uint16_t*>(e->reg[n.out[0]].ptr);
+        so.plane = rows * n.plan->split_cols;
+        so.inv = reinterpret_cast<float*>(e->base + n.split_off);
+        so.amax = so.inv + rows;
+        so.parts_out = &n.split_parts;
+    }
     if (n.fn(e->reg, n.in, n.out, n.params, n.plan.get(), e->ctx)) return 1;
+    if (n.splits)
+        for (size_t id = 0; id < e->splits.size(); id++)
+            if (e->split_root[id] == e->split_root[n.out[0]]) e->splits[id].parts = n.split_parts;
     if (n.fuse_out >= 0) {
         FXF_CHECK(e->ctx.fuse.consumed, "node %zu (%s): the folded residual Add was not performed by the kernel", i, op_entry(n.op).name);
         e->ctx.fuse = EpilogueFusion{};
@@ -426,6 +445,13 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             }
         }
     }
+    // scales and row maxima of the activations that may be kept in split form (decided below, once the fusions are known)
+    for (auto& n : e->nodes)
+        if (n.plan->makes_split) {
+            const int parts = n.op == FXF_OP_LINEAR || n.op == FXF_OP_LINEAR_RELU ? gemm_f16_split_parts(n.plan->split_cols) : 1;
+            n.split_off = cursor;
+            cursor = round_up(cursor + size_t(n.plan->split_rows) * sizeof(float) * size_t(1 + parts), kAlign);
+        }
     e->total_bytes = cursor;
 
     // ---- the one device allocation -----------------------------------------------------------
@@ -648,6 +674,38 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             A.fuse_relu = B.op == FXF_OP_ADD_RELU;
             B.folded = true;
         }
+
+        // -- an activation that only feeds products of the f16 GEMM is written in that GEMM's operand form by the node that
+        // produces it (same bytes, same arena slot): no conversion pass, and the GEMM has nothing to convert.
+        e->split_root.resize(n_tensors);
+        for (uint32_t id = 0; id < n_tensors; id++) e->split_root[id] = root(id);
+        e->splits.assign(n_tensors, SplitMat{});
+        for (size_t pi = 0; pi < e->nodes.size() && e->opts.tp_size == 1; pi++) {
+            Node& P = e->nodes[pi];
+            if (!P.plan->makes_split || P.folded || P.xchg || P.fuse_out >= 0 || P.out.size() != 1) continue;
+            const uint32_t t = root(P.out[0]);
+            int64_t lo = 0, hi = 0;
+            if (escapes[t] || meta[t].kind != kActivation || producer[t] != int(pi) || n_readers[t] == 0 || !arena_range(t, &lo, &hi)) continue;
+            if (numel(e->reg[P.out[0]]) != P.plan->split_rows * P.plan->split_cols || e->reg[P.out[0]].dtype != FXF_F32 || !is_contiguous(e->reg[P.out[0]])) continue;
+            bool ok = true;
+            for (size_t ri = 0; ri < e->nodes.size() && ok; ri++)
+                for (size_t k = 0; k < e->nodes[ri].in.size(); k++) {
+                    const uint32_t id = e->nodes[ri].in[k];
+                    if (root(id) != t) continue;
+                    const FxfTensor& x = e->reg[id];
+                    ok = ok && ri > pi && k < 32 && ((e->nodes[ri].plan->takes_split >> k) & 1u) && x.rank >= 1 && x.shape[x.rank - 1] == P.plan->split_cols;
+                }
+            if (!ok) continue;
+            P.splits = true;
+            SplitMat m;
+            m.planes = reinterpret_cast<const uint16_t*>(e->base + meta[t].offset);
+            m.plane = P.plan->split_rows * P.plan->split_cols;
+            m.inv = reinterpret_cast<const float*>(e->base + P.split_off);
+            m.amax = m.inv + P.plan->split_rows;
+            for (uint32_t id = 0; id < n_tensors; id++)
+                if (root(id) == t) e->splits[id] = m;
+        }
+        e->ctx.splits = &e->splits;
     }
 
     // ---- registry binding, in file order (an alias binds to an already-built source) --------
@@ -700,6 +758,7 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
         if (n.plan->prepare(e->reg, n.in, n.out, n.params, e->ctx)) return 1;
     }
     FXF_CUDA(cudaDeviceSynchronize());
+    e->ctx.weights_settled = true;   // prepared and waited for: later kernels may read weights before their predecessors end
 
     // ---- warm-up run (validates every node's arguments), then capture ------------------------
     FXF_CUDA(cudaStreamCreateWithFlags(&e->capture_stream, cudaStreamNonBlocking));
@@ -906,6 +965,7 @@ int fxf_engine_describe(const fxf_engine* e, char* out, size_t out_bytes) {
         if (n.xchg)
             os << " +exchange(residual " << n.xchg_res << ") -> x " << n.xchg_x << (n.xchg_x >= 0 ? (n.xchg_replicate_x ? " [all rows on every rank]" : " [own rows]") : "")
                << " y " << n.xchg_y;
+        if (n.splits) os << " output in split form";
         if (n.folded) os << " folded into an earlier node";
         os << "\n";
     }
@@ -1215,7 +1275,19 @@ static int last_row_head(fxf_engine* e, int64_t* tokens, int cur, ExecCtx& ctx) 
     ctx.status = e->ctx.status;
     ctx.gemm_ws = e->ctx.gemm_ws; ctx.gemm_ws_bytes = e->ctx.gemm_ws_bytes;
     ctx.gemm_flags = e->ctx.gemm_flags; ctx.gemm_flag_count = e->ctx.gemm_flag_count;
-    if (linear_on_rows(t.plan.get(), static_cast<const float*>(x.ptr) + int64_t(cur - 1) * D, B, int64_t(T) * D, rows, V, ctx)) return 1;
+    ctx.scratch = e->ctx.scratch; ctx.scratch_bytes = e->ctx.scratch_bytes;
+    ctx.weights_settled = e->ctx.weights_settled;
+    SplitMat split_rows;
+    const SplitMat* sx = split_of(e->ctx, t.in[0]);
+    if (sx != nullptr) {   // row cur-1 of every sequence, in split form
+        split_rows = *sx;
+        split_rows.planes += int64_t(cur - 1) * D;
+        split_rows.ld = int64_t(T) * D;
+        split_rows.inv += cur - 1;
+        split_rows.amax += int64_t(cur - 1) * split_rows.parts;
+        split_rows.inv_stride = T;
+    }
+    if (linear_on_rows(t.plan.get(), static_cast<const float*>(x.ptr) + int64_t(cur - 1) * D, sx ? &split_rows : nullptr, B, int64_t(T) * D, rows, V, ctx)) return 1;
     if (!e->head_sharded) return decode_argmax_scatter_rows(rows, V, 0, tokens, B, T, V, cur, ctx);
     char* cand = reinterpret_cast<char*>(e->base + e->cand_off);
     return decode_argmax_scatter_sharded_rows(rows, V, 0, tokens, B, T, V, cur, col0, ncols, cand, cand + size_t(B) * 16, ctx);

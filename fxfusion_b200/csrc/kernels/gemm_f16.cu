@@ -1,0 +1,848 @@
+// Tensor-core GEMM for sm_100a on operands that are ALREADY in tensor-core form:
+//     out[M,N] = act(x[M,K] · w[N,K]^T + bias[N])
+// with fp32-grade results from three fp16 products per fp32 product ("f16x3"), or one bf16 product in the bf16 mode.
+//
+// Split form.  A row r of an fp32 matrix is stored as two fp16 planes and one power of two:
+//     x[r,k] * s_r = hi[r,k] + lo[r,k],   s_r a power of two with max_k |x[r,k]| * s_r <= 2^15,
+// hi = fp16(x * s_r), lo = fp16(x * s_r - hi): 22 significant bits for every element down to 2^-17 of the row's bound and an
+// absolute error of 2^-40 of that bound below it.  An fp16 significand has the 11 bits of TF32, so
+//     x·w = (hi·hi + hi·lo + lo·hi) / (s_x s_w)
+// drops the same 2^-22 term as three TF32 products (and less than one TF32 product + two bf16 corrections, whose corrections
+// are rounded at 2^-19), but a kind::f16 instruction covers K = 16 where a kind::tf32 instruction covers 8: three
+// instructions per 16 K-elements instead of four or six, and 4 instead of 8 bytes per weight element.  The scales are powers
+// of two, so multiplying by 1 / (s_x s_w) in the epilogue is exact.
+// Both planes of [rows, K] take the bytes of the fp32 matrix: a tensor of the engine keeps its arena slot in either form.
+//
+// Who splits.  Weights: once per engine (split_rows_kernel).  Activations: the kernel that produces them, where it knows a
+// bound of each row: LayerNorm holds the row, and this kernel's own epilogue bounds its output rows by
+//     |y[r,j]| <= amax_r * max_j ||w_j||_1 + max_j |b_j|
+// (amax_r = max_k |x[r,k]|, kept beside the planes).  Anything else goes through split_rows_kernel first.
+//
+// Structure: persistent, 384 threads, one CTA per SM.  Warps 0-7 epilogue, warp 8 TMA producer, warp 9 MMA issuer (10 and 11
+// complete the warpgroup that setmaxnreg takes registers from: a wide tile's epilogue holds 128 running sums); nothing
+// touches an operand between TMA and the tensor core, so K-slabs are 64 deep (128-byte rows, one 3-D TMA load brings both
+// planes of a tile).  PAIR: two CTAs of a cluster share a 256-row tile (cta_group::2), each staging half of the weight tile.
+// Accumulation runs in chains of `chunk_slabs` K-slabs into one of two TMEM accumulators; the epilogue warps drain finished
+// chains into fp32 registers (the tensor core adds with truncation: chains bound that error, see kChunkKDense).
+// Launches are programmatic dependents: weight tiles of the first stages are requested before the previous kernel has
+// finished, everything else waits for it.
+// Every mbarrier wait is bounded; on expiry the CTA records an error in the status word and leaves.
+//
+// Bound: tensor pipe.  A 128 x 256 x 16 instruction takes 128 cycles, so a pair's 64-deep slab is 12 x 128 = 1536 cycles of
+// tensor time against 64 KB of TMA writes and 144 KB of operand reads per SM (1625 cycles at 128 B per clock); the measured
+// slab takes 1520.  Times on B200, before (one TF32 product + two bf16 corrections, operands split inside the kernel) and now:
+// 8192 x 3072 x 768 133 -> 80 us (481 TFLOP/s; three times that is the library's bf16 rate under the power cap),
+// 8192 x 768 x 768 57 -> 24 us, 1500 x 512 x 512 18 -> 7.8 us, 512 x 256 x 256 11 -> 4.5 us.
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <mutex>
+
+#include "../runtime.hpp"
+#include "sm100.cuh"
+
+namespace fxf {
+namespace {
+
+using namespace sm100;
+
+constexpr int BM = 128, BK = 64;
+constexpr int kEpiWarps = 8, kTmaWarp = 8, kMmaWarp = 9, kThreads = 384;
+constexpr int ACC = 2;
+enum : int { kErrWaitFull = 131, kErrWaitEmpty = 133, kErrWaitAcc = 134, kErrWaitAccEmpty = 135, kErrWaitPartial = 136 };
+
+// output staging buffers per epilogue warp: two where the operand ring leaves room, so that a store may still be reading one
+constexpr int staging_buffers(int bn, int bnb, int stages, int npl) {
+    return stages * npl * (BM + bnb) * BK * 2 + 2 * kEpiWarps * 2048 + kEpiWarps * bn * 4 <= 225 * 1024 ? 2 : 1;
+}
+
+// BNB = weight rows held by this CTA; NPL = planes per operand (2: f16x3, 1: bf16)
+template <int BN, int BNB, int STAGES, int NPL, int NSTG>
+struct alignas(1024) F16Smem {
+    uint16_t a[STAGES][NPL][BM * BK];
+    uint16_t b[STAGES][NPL][BNB * BK];
+    float stage_out[kEpiWarps][NSTG][32 * 16];       // 32 rows x 16 columns per epilogue warp (64-byte rows, 64-byte swizzle)
+    float col_inv[kEpiWarps][BN / 2], col_bias[kEpiWarps][BN / 2];   // 1 / scale and bias of a warp's columns
+    uint64_t full[STAGES];
+    uint64_t empty[STAGES];
+    uint64_t acc_full[ACC];
+    uint64_t acc_empty[ACC];
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+struct F16Params {
+    const float* bias;
+    const float* residual;        // optional, addressed like `out`
+    const float *x_inv, *w_inv;   // 1 / scale per row of x and per row of w (NULL in bf16 mode)
+    int64_t x_inv_stride;         // entries of x_inv between the rows of this product
+    float* out;                   // NULL when the result leaves in split form
+    int64_t M, N, K, ldo;
+    int relu;
+    int tma_out;                  // the result leaves through map_o (16-byte aligned rows): fp32 [M, N] or both planes of the split form
+    int tiles_m, tiles_n, m_fastest;
+    int full_tiles, tail_tiles, tail_split;   // tiles of the last round are cut along K into tail_split parts
+    int chunk_slabs;
+    int early_w;                  // weight tiles may be requested before the previous kernel has finished
+    float* ws;
+    int* flags;
+    int* status;
+    // split-form output [M, N]: planes (hi at 0, lo at so_plane), 1 / scale per row, and per row `so_parts` partial maxima
+    // of |y| (one per column half of a tile); bounds of the row come from x_amax (x_parts per row) and w_bound = {max_j ||w_j||_1, max_j |b_j|}
+    uint16_t* so;
+    int64_t so_plane;
+    float *so_inv, *so_amax;
+    int so_parts;
+    const float *x_amax, *w_bound;
+    int x_parts;
+    // transposed column range (GemmArgs::vt_*)
+    float* vt_out;
+    unsigned char* vt_flags;
+    int64_t vt_col0;
+    int vt_T, vt_heads, vt_n32;
+};
+
+struct Unit { int tile, k0, k1, part, nparts, u; };
+__device__ __forceinline__ Unit get_unit(const F16Params& p, int unit, int num_k) {
+    Unit r;
+    if (unit < p.full_tiles) {
+        r.tile = unit; r.k0 = 0; r.k1 = num_k; r.part = 0; r.nparts = 1; r.u = 0;
+    } else {
+        r.u = unit - p.full_tiles;
+        r.nparts = p.tail_split;
+        r.tile = p.full_tiles + r.u / r.nparts;
+        r.part = r.u % r.nparts;
+        r.k0 = int(int64_t(num_k) * r.part / r.nparts);
+        r.k1 = int(int64_t(num_k) * (r.part + 1) / r.nparts);
+    }
+    return r;
+}
+__device__ __forceinline__ void tile_coords(const F16Params& p, int tile, int& tm, int& tn) {
+    if (p.m_fastest) {
+        tm = tile % p.tiles_m;
+        tn = tile / p.tiles_m;
+    } else {
+        tn = tile % p.tiles_n;
+        tm = tile / p.tiles_n;
+    }
+}
+// a wait counts only if it succeeded for every lane, so that a warp gives up as a whole
+__device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
+__device__ __forceinline__ float relu_keep_nan(float v) { return v > 0.f ? v : (v != v ? v : 0.f); }
+
+template <int HALF>
+__device__ __forceinline__ void drain_chunk(uint32_t tacc, float (&sum)[HALF]) {
+#pragma unroll
+    for (int c = 0; c < HALF; c += 16) {
+        uint32_t r[16];
+        tmem_ld16(tacc + uint32_t(c), r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; j++) sum[c + j] += __uint_as_float(r[j]);
+    }
+}
+
+template <int BN, int STAGES, bool PAIR, int NPL>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_o, F16Params p) {
+    extern __shared__ unsigned char smem_raw[];
+    constexpr int BNB = PAIR ? BN / 2 : BN;
+    using Smem = F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL)>;
+    Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    constexpr uint32_t kABytes = NPL * BM * BK * 2, kBBytes = NPL * BNB * BK * 2;
+    constexpr uint32_t kIdesc = NPL == 2 ? umma_idesc_f16(PAIR ? 2 * BM : BM, BN) : umma_idesc_bf16(PAIR ? 2 * BM : BM, BN);
+    constexpr uint32_t kTmemCols = ACC * BN <= 64 ? 64 : (ACC * BN <= 128 ? 128 : (ACC * BN <= 256 ? 256 : 512));
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int num_k = int((p.K + BK - 1) / BK);
+    const int num_units = p.full_tiles + p.tail_tiles * p.tail_split;
+    const int chunk = p.chunk_slabs > 0 ? p.chunk_slabs : num_k;
+    const int rank = PAIR ? int(cluster_ctarank()) : 0;
+    const int sched_id = PAIR ? int(blockIdx.x >> 1) : int(blockIdx.x), sched_n = PAIR ? int(gridDim.x >> 1) : int(gridDim.x);
+    volatile int* abort_flag = &s.abort_flag;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < STAGES; i++) {
+            mbar_init(&s.full[i], 1);
+            mbar_init(&s.empty[i], 1);
+        }
+        for (int i = 0; i < ACC; i++) {
+            mbar_init(&s.acc_full[i], 1);
+            mbar_init(&s.acc_empty[i], PAIR ? 2 * kEpiWarps : kEpiWarps);
+        }
+        s.abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kTmaWarp && lane == 0) {
+        prefetch_tensormap(&map_x);
+        prefetch_tensormap(&map_w);
+        if (p.tma_out) prefetch_tensormap(&map_o);
+    }
+    if (warp == kMmaWarp) {
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem_base)), "r"(kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem_base)), "r"(kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (PAIR) cluster_sync_all();   // the other CTA's barriers exist before anything of this CTA signals them
+    tc_fence_after();
+    const uint32_t tmem_base = s.tmem_base;
+    grid_dep_launch();
+
+    // 384 x 168 registers at launch = 256 x 208 + 128 x 88
+    if (warp >= kEpiWarps) {
+      if (BN >= 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+      if (warp == kTmaWarp) {
+        // ---------------- TMA producer ----------------
+        if (lane == 0) {
+            auto load_x = [&](int st, int k, int tm) {
+                if (PAIR) tma_load_3d_pair(s.a[st], &map_x, k * BK, tm * BM, 0, &s.full[st]);
+                else tma_load_3d(s.a[st], &map_x, k * BK, tm * BM, 0, &s.full[st]);
+            };
+            auto load_w = [&](int st, int k, int tn) {   // also announces the bytes of the whole stage (of both CTAs: the leader's barrier)
+                if (PAIR) {
+                    if (rank == 0) mbar_expect_tx(&s.full[st], 2 * (kABytes + kBBytes));
+                    tma_load_3d_pair(s.b[st], &map_w, k * BK, tn * BN + rank * BNB, 0, &s.full[st]);
+                } else {
+                    mbar_expect_tx(&s.full[st], kABytes + kBBytes);
+                    tma_load_3d(s.b[st], &map_w, k * BK, tn * BN, 0, &s.full[st]);
+                }
+            };
+            uint32_t it = 0;
+            bool first = true;
+            for (int unit = sched_id; unit < num_units; unit += sched_n) {
+                const Unit un = get_unit(p, unit, num_k);
+                int tm, tn;
+                tile_coords(p, un.tile, tm, tn);
+                if (PAIR) tm = tm * 2 + rank;
+                int k = un.k0;
+                if (first) {   // the ring is empty: fill it without waiting, the weights ahead of the previous kernel's end
+                    const int pre = min(STAGES, un.k1 - un.k0);
+                    if (!p.early_w) grid_dep_wait();
+                    for (int i = 0; i < pre; i++) load_w(i, un.k0 + i, tn);
+                    if (p.early_w) grid_dep_wait();
+                    for (int i = 0; i < pre; i++) load_x(i, un.k0 + i, tm);
+                    k += pre;
+                    it += pre;
+                    first = false;
+                }
+                for (; k < un.k1; k++, it++) {
+                    const int st = it % STAGES;
+                    if (it >= uint32_t(STAGES) && !mbar_wait(&s.empty[st], ((it / STAGES) - 1) & 1, abort_flag)) {
+                        give_up(abort_flag, p.status, kErrWaitEmpty);
+                        goto producer_done;
+                    }
+                    load_w(st, k, tn);
+                    load_x(st, k, tm);
+                }
+            }
+        producer_done:
+            if (first) grid_dep_wait();
+        }
+      } else if (warp == kMmaWarp) {
+        // ---------------- MMA issuer ----------------
+        // The whole warp walks the loop, so the descriptors stay in uniform registers; one elected lane issues.
+        if (rank == 0) {
+            const uint32_t leader = elect_one();
+            const uint64_t a0 = umma_desc_k_major_bytes<128>(smem_u32(s.a[0][0])), b0 = umma_desc_k_major_bytes<128>(smem_u32(s.b[0][0]));
+            constexpr uint64_t kALo = (NPL - 1) * (BM * BK * 2 / 16), kBLo = (NPL - 1) * (BNB * BK * 2 / 16);   // lo plane, 16-byte units
+            uint32_t st = 0, par = 0, ccount = 0;
+            for (int unit = sched_id; unit < num_units; unit += sched_n) {
+                const Unit un = get_unit(p, unit, num_k);
+                for (int kc0 = un.k0; kc0 < un.k1; kc0 += chunk, ccount++) {
+                    const int kc1 = min(kc0 + chunk, un.k1);
+                    const uint32_t buf = ccount % ACC;
+                    if (ccount >= uint32_t(ACC) &&
+                        !warp_all(PAIR ? mbar_wait_cluster(&s.acc_empty[buf], ((ccount / ACC) - 1) & 1, abort_flag) : mbar_wait(&s.acc_empty[buf], ((ccount / ACC) - 1) & 1, abort_flag))) {
+                        give_up(abort_flag, p.status, kErrWaitAccEmpty);
+                        goto mma_done;
+                    }
+                    tc_fence_after();
+                    const uint32_t acc = tmem_base + buf * uint32_t(BN);
+                    for (int k = kc0; k < kc1; k++) {
+                        if (!warp_all(mbar_wait(&s.full[st], par, abort_flag))) {
+                            give_up(abort_flag, p.status, kErrWaitFull);
+                            goto mma_done;
+                        }
+                        tc_fence_after();
+                        if (leader) {
+                            const uint64_t a = a0 + st * (kABytes / 16), b = b0 + st * (kBBytes / 16);
+#pragma unroll
+                            for (int kk = 0; kk < BK / 16; kk++) {   // 16 elements = 32 bytes per instruction inside the swizzle row
+                                const uint64_t adv = uint64_t((kk * 32) >> 4);
+                                const uint32_t acc_on = (k > kc0 || kk > 0) ? 1u : 0u;
+                                if (NPL == 2) {
+                                    umma_f16_ss<PAIR>(acc, a + kALo + adv, b + adv, kIdesc, acc_on);
+                                    umma_f16_ss<PAIR>(acc, a + adv, b + kBLo + adv, kIdesc, 1u);
+                                    umma_f16_ss<PAIR>(acc, a + adv, b + adv, kIdesc, 1u);
+                                } else {
+                                    umma_f16_ss<PAIR>(acc, a + adv, b + adv, kIdesc, acc_on);
+                                }
+                            }
+                            if (PAIR) umma_commit_pair(&s.empty[st]);
+                            else umma_commit(&s.empty[st]);
+                            if (k + 1 == kc1) {
+                                if (PAIR) umma_commit_pair(&s.acc_full[buf]);
+                                else umma_commit(&s.acc_full[buf]);
+                            }
+                        }
+                        if (++st == STAGES) { st = 0; par ^= 1; }
+                    }
+                }
+            }
+        mma_done:;
+        }
+      }
+    } else {
+        if (BN >= 128) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+        // ---------------- epilogue (warp w owns TMEM lanes 32*(w%4).. and column half w/4) ----------------
+        // One thread owns one row of its warp's 32 x HALF block.  The group loop stays rolled (only picking a group's sixteen
+        // running sums is spelled out): unrolled, its code missed the instruction cache at every group.  A group leaves as one
+        // TMA store from a swizzled staging block; row-contiguous stores by the LSU, with the lanes re-arranged through shared
+        // memory, took 250 instructions and 1900 cycles per group and bound every product of K <= 1024.
+        constexpr int HALF = BN / 2, NSTG = staging_buffers(BN, BNB, STAGES, NPL);
+        const int q = warp & 3, chalf = warp >> 2;
+        const uint32_t lane_base = uint32_t(q * 32) << 16;
+        float *cinv = s.col_inv[warp], *cbias = s.col_bias[warp];
+        uint32_t ccount = 0, sbuf = 0;
+        grid_dep_wait();
+        for (int unit = sched_id; unit < num_units; unit += sched_n) {
+            const Unit un = get_unit(p, unit, num_k);
+            int tm, tn;
+            tile_coords(p, un.tile, tm, tn);
+            if (PAIR) tm = tm * 2 + rank;
+            const bool writes_partial = un.nparts > 1 && un.part > 0;
+            const bool adds_partials = un.nparts > 1 && un.part == 0;
+            const int slot = PAIR ? un.u * 2 + rank : un.u, pstep = PAIR ? 2 : 1;
+            // partial tiles: [column half][row quarter][4-column group][lane] float4, so that every access is coalesced
+            float4* ws_mine = reinterpret_cast<float4*>(p.ws + size_t(slot) * size_t(BM * BN)) + warp * (HALF / 4) * 32 + lane;
+            const int64_t trow = int64_t(tm) * BM + q * 32, grow = trow + lane;   // first row of this warp, row of this thread
+            const bool row_ok = grow < p.M;
+            const int64_t col_base = int64_t(tn) * BN + chalf * HALF;
+            // constants of the row and of the columns, fetched while the tensor core works
+            const float ri = (row_ok && p.x_inv != nullptr) ? __ldg(p.x_inv + grow * p.x_inv_stride) : 1.f;
+            float rscale = 1.f, rmax = 0.f;
+            if (NPL == 2 && p.so != nullptr && !writes_partial && row_ok) {
+                float am = 0.f, inv;
+                for (int j = 0; j < p.x_parts; j++) am = fmaxf(am, __ldg(p.x_amax + grow * p.x_inv_stride * p.x_parts + j));
+                split_scale(fmaf(am, __ldg(p.w_bound), __ldg(p.w_bound + 1)), rscale, inv);
+                if (chalf == 0 && tn == 0) p.so_inv[grow] = inv;
+            }
+            __syncwarp();
+            for (int j = lane; j < HALF; j += 32) {
+                const int64_t c = col_base + j;
+                cinv[j] = (p.w_inv && c < p.N) ? __ldg(p.w_inv + c) : 1.f;
+                cbias[j] = (p.bias && c < p.N) ? __ldg(p.bias + c) : 0.f;
+            }
+            __syncwarp();
+            float sum[HALF];
+#pragma unroll
+            for (int j = 0; j < HALF; j++) sum[j] = 0.f;
+            bool alive = true;
+            for (int kc0 = un.k0; kc0 < un.k1; kc0 += chunk, ccount++) {
+                const uint32_t buf = ccount % ACC;
+                if (!warp_all(mbar_wait(&s.acc_full[buf], (ccount / ACC) & 1, abort_flag))) {
+                    give_up(abort_flag, p.status, kErrWaitAcc);
+                    alive = false;
+                    break;
+                }
+                tc_fence_after();
+                drain_chunk<HALF>(tmem_base + buf * uint32_t(BN) + lane_base + uint32_t(chalf * HALF), sum);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (PAIR) mbar_arrive_leader(&s.acc_empty[buf]);
+                    else mbar_arrive(&s.acc_empty[buf]);
+                }
+            }
+            if (!alive) break;
+            if (adds_partials) {
+                int ok = 1;
+                if (lane == 0)
+                    for (int pp = 1; pp < un.nparts && ok; pp++) ok = flag_wait(p.flags + (slot + pp * pstep) * kEpiWarps + warp, abort_flag) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok) {
+                    give_up(abort_flag, p.status, kErrWaitPartial);
+                    break;
+                }
+            }
+            const bool transposes = p.vt_out != nullptr && col_base >= p.vt_col0;
+            // rows that do not start on 16-byte boundaries (a pitch like the 50257-column vocabulary): row r starts `shift` floats
+            // past one and is stored as aligned 16-byte pieces, 16 columns lagging by `shift`
+            float* orow = p.out + grow * p.ldo + col_base;
+            const int shift = int((reinterpret_cast<uintptr_t>(orow) >> 2) & 3);
+            float c0 = 0.f, c1 = 0.f, c2 = 0.f;   // the last three columns of the previous group
+#pragma unroll 1
+            for (int g = 0; g < HALF / 16; g++) {
+                const int64_t col = col_base + g * 16;
+                if (col >= p.N && !writes_partial) break;   // warp-uniform
+                float v[16];
+#pragma unroll
+                for (int gg = 0; gg < HALF / 16; gg++)
+                    if (gg == g) {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) v[j] = sum[gg * 16 + j];
+                    }
+                if (writes_partial) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) ws_mine[(g * 4 + j) * 32] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    continue;
+                }
+                if (adds_partials) {
+#pragma unroll 1
+                    for (int pp = 1; pp < un.nparts; pp++) {
+                        const float4* src = ws_mine + size_t(pp * pstep) * size_t(BM * BN / 4) + g * 4 * 32;
+                        float4 w[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) w[j] = __ldcg(src + j * 32);
+#pragma unroll
+                        for (int j = 0; j < 4; j++) { v[4 * j] += w[j].x; v[4 * j + 1] += w[j].y; v[4 * j + 2] += w[j].z; v[4 * j + 3] += w[j].w; }
+                    }
+                }
+                float4 r4[4];
+                if (p.residual != nullptr && p.tma_out) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        r4[j] = (row_ok && col + 4 * j < p.N) ? *reinterpret_cast<const float4*>(p.residual + grow * p.ldo + col + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) {
+                    const float4 ci = *reinterpret_cast<const float4*>(cinv + g * 16 + j), cb = *reinterpret_cast<const float4*>(cbias + g * 16 + j);
+                    // both factors are powers of two; the weight's goes first: the product of the two may leave the range of fp32
+                    v[j] = fmaf(v[j] * ci.x, ri, cb.x); v[j + 1] = fmaf(v[j + 1] * ci.y, ri, cb.y);
+                    v[j + 2] = fmaf(v[j + 2] * ci.z, ri, cb.z); v[j + 3] = fmaf(v[j + 3] * ci.w, ri, cb.w);
+                }
+                if (transposes) {
+                    // V third of a packed QKV projection, transposed per head: the 32 lanes write 32 consecutive keys of a V^T row
+                    const int64_t b = grow / p.vt_T, t = grow - b * p.vt_T, v0 = col - p.vt_col0, h = v0 >> 6;
+                    const int d0 = int(v0 & 63);
+                    float* dst = p.vt_out + ((b * p.vt_heads + h) * 64 + d0) * int64_t(p.vt_T) + t;
+                    bool bad = false;
+#pragma unroll
+                    for (int d = 0; d < 16; d++) {
+                        bad = bad || (v[d] - v[d] != 0.f);   // NaN or infinity
+                        if (row_ok) dst[int64_t(d) * p.vt_T] = v[d];
+                    }
+                    const unsigned any_bad = __ballot_sync(0xffffffffu, row_ok && bad);
+                    if (lane == 0 && row_ok) {
+                        unsigned char* fl = p.vt_flags + ((b * p.vt_heads + h) * 2 + (d0 >> 5)) * p.vt_n32 + (t >> 5);
+                        *fl = (any_bad != 0 || ((d0 & 16) && *fl != 0)) ? 1 : 0;   // two groups share a flag, in this order
+                    }
+                    continue;
+                }
+                if (p.residual != nullptr) {
+                    if (p.tma_out) {
+#pragma unroll
+                        for (int j = 0; j < 4; j++) { v[4 * j] += r4[j].x; v[4 * j + 1] += r4[j].y; v[4 * j + 2] += r4[j].z; v[4 * j + 3] += r4[j].w; }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            if (row_ok && col + j < p.N) v[j] += p.residual[grow * p.ldo + col + j];
+                    }
+                }
+                if (p.relu) {
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] = relu_keep_nan(v[j]);
+                }
+                char* stage = reinterpret_cast<char*>(s.stage_out[warp][NSTG > 1 ? sbuf : 0]);
+                if (p.tma_out) {
+                    if (lane == 0) bulk_wait_read<NSTG - 1>();   // the store that used this buffer has read it
+                    __syncwarp();
+                    if (p.so == nullptr) {
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            *reinterpret_cast<float4*>(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    } else if (NPL == 1) {
+#pragma unroll
+                        for (int j = 0; j < 2; j++)
+                            *reinterpret_cast<uint4*>(stage + lane * 32 + ((j ^ ((lane >> 2) & 1)) << 4)) =
+                                make_uint4(pack_bf16x2(v[8 * j], v[8 * j + 1]), pack_bf16x2(v[8 * j + 2], v[8 * j + 3]), pack_bf16x2(v[8 * j + 4], v[8 * j + 5]), pack_bf16x2(v[8 * j + 6], v[8 * j + 7]));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 2; j++) {
+                            uint4 hi, lo;
+                            uint32_t* hp = &hi.x;
+                            uint32_t* lp = &lo.x;
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                const float x = v[8 * j + 2 * e], y = v[8 * j + 2 * e + 1];
+                                rmax = fmaxf(rmax, fmaxf(fabsf(x), fabsf(y)));
+                                split_f16x2(x * rscale, y * rscale, hp[e], lp[e]);
+                            }
+                            const int at = lane * 32 + ((j ^ ((lane >> 2) & 1)) << 4);
+                            *reinterpret_cast<uint4*>(stage + at) = hi;
+                            *reinterpret_cast<uint4*>(stage + 1024 + at) = lo;
+                        }
+                    }
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (trow < p.M) tma_store_3d(&map_o, stage, int(col), int(trow), 0);
+                        bulk_commit();
+                    }
+                    sbuf ^= 1;
+                    continue;
+                }
+                // ---- unaligned rows: out[k] = column 16g - shift + k of the row, by two select steps over {previous three, v} ----
+                float u[18], w[16];
+                {
+                    const bool s1 = shift & 1, s2 = shift & 2;
+                    u[0] = s1 ? c0 : c1; u[1] = s1 ? c1 : c2; u[2] = s1 ? c2 : v[0];
+#pragma unroll
+                    for (int k = 3; k < 18; k++) u[k] = s1 ? v[k - 3] : v[k - 2];
+#pragma unroll
+                    for (int k = 0; k < 16; k++) w[k] = s2 ? u[k] : u[k + 2];
+                }
+                if (row_ok && shift > 0) {   // the 4 - shift leading and the shift trailing columns of this block's row segment
+                    if (g == 0) {
+                        if (col < p.N) orow[0] = v[0];
+                        if (shift < 3 && col + 1 < p.N) orow[1] = v[1];
+                        if (shift < 2 && col + 2 < p.N) orow[2] = v[2];
+                    }
+                    if (g + 1 == HALF / 16 || col + 16 >= p.N) {
+                        if (col + 15 < p.N) orow[g * 16 + 15] = v[15];
+                        if (shift > 1 && col + 14 < p.N) orow[g * 16 + 14] = v[14];
+                        if (shift > 2 && col + 13 < p.N) orow[g * 16 + 13] = v[13];
+                    }
+                }
+                c0 = v[13]; c1 = v[14]; c2 = v[15];
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    *reinterpret_cast<float4*>(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = make_float4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+                __syncwarp();
+                const int piece = lane & 3;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {   // 4 lanes cover a row's 64 bytes, 8 rows per instruction
+                    const int rr = i * 8 + (lane >> 2);
+                    const int64_t gr = trow + rr;
+                    float* rp = p.out + gr * p.ldo + col;
+                    const int a = int((reinterpret_cast<uintptr_t>(rp) >> 2) & 3), c = piece * 4 - a;
+                    const float4 x = *reinterpret_cast<const float4*>(stage + rr * 64 + ((piece ^ ((rr >> 1) & 3)) << 4));
+                    if (gr >= p.M || (g == 0 && c < 0)) continue;   // the piece left of the block belongs to the neighbour
+                    if (col + c + 3 < p.N) {
+                        *reinterpret_cast<float4*>(rp + c) = x;
+                    } else {
+                        if (col + c < p.N) rp[c] = x.x;
+                        if (col + c + 1 < p.N) rp[c + 1] = x.y;
+                        if (col + c + 2 < p.N) rp[c + 2] = x.z;
+                    }
+                }
+            }
+            if (NPL == 2 && p.so != nullptr && !writes_partial && row_ok) p.so_amax[grow * p.so_parts + tn * 2 + chalf] = rmax;
+            if (writes_partial) {
+                __threadfence();
+                __syncwarp();
+                if (lane == 0) flag_set(p.flags + slot * kEpiWarps + warp, 1);
+            } else if (adds_partials) {
+                __syncwarp();
+                if (lane == 0)
+                    for (int pp = 1; pp < un.nparts; pp++) flag_set(p.flags + (slot + pp * pstep) * kEpiWarps + warp, 0);
+            }
+        }
+        if (p.tma_out && lane == 0) bulk_wait_all();
+    }
+    // ---------------- teardown ----------------
+    tc_fence_before();
+    __syncthreads();
+    if (PAIR) cluster_sync_all();
+    if (warp == kMmaWarp) {
+        tc_fence_after();
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+    }
+}
+
+// ---- fp32 rows -> split form ---------------------------------------------------------------------------
+// One block per row (rows are hundreds to thousands of floats): maximum, then the two planes from the row's second read,
+// which hits L1 / L2.  bound != NULL also raises bound[0] to the largest L1 norm of a row (weights; one atomic per row).
+// MODE 0: f16 planes; 1: bf16 plane only.
+template <int MODE>
+__global__ void __launch_bounds__(128) split_rows_kernel(const float* __restrict__ x, int64_t ld, uint16_t* __restrict__ planes, int64_t plane, float* __restrict__ inv_out,
+                                                         float* __restrict__ amax_out, float* __restrict__ bound, int64_t M, int K) {
+    __shared__ float red[8];
+    grid_dep_launch();
+    grid_dep_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int64_t r = blockIdx.x; r < M; r += gridDim.x) {
+        const float* xr = x + r * ld;
+        uint16_t* hr = planes + r * K;
+        const bool vec = (reinterpret_cast<uintptr_t>(xr) & 15) == 0;
+        auto load = [&](int k) {
+            return vec ? *reinterpret_cast<const float4*>(xr + k) : make_float4(xr[k], xr[k + 1], xr[k + 2], xr[k + 3]);
+        };
+        if (MODE == 1) {
+            for (int k = threadIdx.x * 4; k < K; k += 512) {
+                const float4 v = load(k);
+                *reinterpret_cast<uint2*>(hr + k) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+            }
+            continue;
+        }
+        float m = 0.f, l1 = 0.f;
+        for (int k = threadIdx.x * 4; k < K; k += 512) {
+            const float4 v = load(k);
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+            l1 += (fabsf(v.x) + fabsf(v.y)) + (fabsf(v.z) + fabsf(v.w));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+        }
+        __syncthreads();
+        if (lane == 0) { red[warp] = m; red[4 + warp] = l1; }
+        __syncthreads();
+        m = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+        float scale, inv;
+        split_scale(m, scale, inv);
+        if (threadIdx.x == 0) {
+            inv_out[r] = inv;
+            if (amax_out) amax_out[r] = m;
+            if (bound) atomicMax(reinterpret_cast<int*>(bound), __float_as_int((red[4] + red[5] + red[6] + red[7]) * 1.0001f));   // non-negative floats order like ints
+        }
+        for (int k = threadIdx.x * 4; k < K; k += 512) {
+            uint2 hi, lo;
+            split_f16x4(load(k), scale, hi, lo);
+            *reinterpret_cast<uint2*>(hr + k) = hi;
+            *reinterpret_cast<uint2*>(hr + plane + k) = lo;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) bias_bound_kernel(const float* __restrict__ b, int64_t n, float* __restrict__ bound) {
+    float m = 0.f;
+    if (b != nullptr)
+        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) m = fmaxf(m, fabsf(b[i]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(bound + 1), __float_as_int(m));
+}
+
+// ---- host side -------------------------------------------------------------------------------------
+using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_fn() {
+    static EncodeTiledFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            return reinterpret_cast<EncodeTiledFn>(p);
+        return EncodeTiledFn(nullptr);
+    }();
+    return fn;
+}
+// [planes][rows][cols] 16-bit elements, `ld` elements between rows and `plane` between planes; box = 64 columns x box_rows x all planes
+int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int64_t plane, int planes, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
+    cuuint64_t dims[3] = {cuuint64_t(cols), cuuint64_t(rows), cuuint64_t(planes)};
+    cuuint64_t strides[2] = {cuuint64_t(ld) * 2, cuuint64_t(planes > 1 ? plane : rows * ld) * 2};
+    cuuint32_t box[3] = {cuuint32_t(BK), cuuint32_t(box_rows), cuuint32_t(planes)};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    FXF_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (f16) failed with code %d (rows %lld cols %lld planes %d)", int(r), (long long)rows, (long long)cols, planes);
+    return 0;
+}
+
+// the result as the epilogue stores it: boxes of 32 rows x 16 columns, fp32 (64-byte rows) or split form (32-byte rows, all planes)
+int make_out_map(CUtensorMap* map, const F16GemmArgs& a, int planes) {
+    EncodeTiledFn fn = encode_fn();
+    FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
+    const bool split = a.split_out.planes != nullptr;
+    const cuuint64_t esz = split ? 2 : 4, pitch = cuuint64_t(split ? a.N : a.ldo) * esz;
+    cuuint64_t dims[3] = {cuuint64_t(a.N), cuuint64_t(a.M), cuuint64_t(split ? planes : 1)};
+    cuuint64_t strides[2] = {pitch, split && planes > 1 ? cuuint64_t(a.split_out.plane) * 2 : pitch * cuuint64_t(a.M)};
+    cuuint32_t box[3] = {16, 32, cuuint32_t(split ? planes : 1)};
+    cuuint32_t estr[3] = {1, 1, 1};
+    void* base = split ? static_cast<void*>(a.split_out.planes) : static_cast<void*>(a.out);
+    CUresult r = fn(map, split ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    split ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    FXF_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (f16 output) failed with code %d", int(r));
+    return 0;
+}
+
+constexpr int kChunkKDense = 1024, kChunkKConv = 64;
+
+// Times in microseconds as measured on B200 inside a chain of launches: `slab` per 64-deep K-slab of a tile, `gap` what every
+// tile adds (its epilogue runs under the next tile's products), `drain` the exposed epilogue of the last one.
+struct Variant { bool pair; int bn; double slab, gap, drain; };
+const Variant kVariants[] = {
+    {true, 256, 0.88, 1.5, 6.8}, {true, 192, 0.78, 0.6, 4.9}, {true, 128, 0.54, 0.4, 2.8}, {true, 64, 0.37, 0.2, 1.5},
+    {false, 128, 0.64, 0.3, 2.0}, {false, 64, 0.47, 0.3, 1.0}, {false, 32, 0.39, 0.2, 0.3},
+};
+struct TailSplit { int64_t full, tail; int parts; double us; };
+// Whole tiles first, then the remainder R = tiles % workers cut along K into s parts each (see F16Params).
+TailSplit plan_tail(int64_t tiles, int num_k, const Variant& v, int workers, bool allowed) {
+    const double tile_us = num_k * v.slab + v.gap;
+    const int64_t R = tiles % workers, rounds = tiles / workers;
+    TailSplit best{tiles, 0, 1, double(rounds + (R ? 1 : 0)) * tile_us + v.drain};
+    if (!allowed || R == 0) return best;
+    const int64_t smax = std::min<int64_t>(std::min<int64_t>(workers / R, num_k / 2), 8);
+    for (int64_t s = 2; s <= smax; s++) {   // writing, fetching and adding partial tiles: 2 us and another one per part
+        const double us = double(rounds) * tile_us + double((num_k + s - 1) / s) * v.slab + v.gap + v.drain + 1.0 + 1.0 * double(s);
+        if (us < best.us) best = TailSplit{tiles - R, R, int(s), us};
+    }
+    return best;
+}
+
+template <int BN, int STAGES, bool PAIR, int NPL>
+int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int workers, ExecCtx& ctx) {
+    constexpr int BNB = PAIR ? BN / 2 : BN;
+    CUtensorMap mx, mw, mo;
+    if (make_map(&mx, a.x.planes, a.M, a.K, a.x.ld ? a.x.ld : a.K, a.x.plane, NPL, BM)) return 1;
+    if (make_map(&mw, a.w.planes, a.N, a.K, a.K, a.w.plane, NPL, BNB)) return 1;
+    mo = mx;
+    if (p.tma_out && make_out_map(&mo, a, NPL)) return 1;
+    const size_t smem = sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL)>) + 1024;
+    static_assert(sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL)>) + 1024 <= 227 * 1024, "shared memory of a CTA");
+    auto kernel = gemm_f16_kernel<BN, STAGES, PAIR, NPL>;
+    static bool configured[64] = {};
+    int dev = 0;
+    FXF_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        FXF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    const int64_t units = ts.full + ts.tail * ts.parts;
+    const int grid = int(std::min<int64_t>(units, workers)) * (PAIR ? 2 : 1);
+    FXF_CUDA(launch_dependent(kernel, dim3(unsigned(grid)), dim3(kThreads), smem, ctx.stream, PAIR ? 2 : 1, mx, mw, mo, p));
+    FXF_LAUNCHED(ctx);
+    return 0;
+}
+
+}  // namespace
+
+bool gemm_f16_shape_ok(int64_t M, int64_t N, int64_t K) {
+    return M >= 1 && N >= 1 && K >= 16 && K % 8 == 0 && M < (int64_t(1) << 31) && N < (int64_t(1) << 31) && K < (int64_t(1) << 31);
+}
+
+int gemm_f16_split_parts(int64_t N) { return int((N + 31) / 32) * 2; }
+
+int launch_split_rows(const float* x, int64_t ld, int64_t M, int64_t K, bool bf16, const SplitOut& out, float* bound, ExecCtx& ctx) {
+    if (M == 0) return 0;
+    FXF_CHECK(K % 8 == 0 && out.planes != nullptr, "split rows: K must be a multiple of 8");
+    const int grid = int(std::min<int64_t>(M, int64_t(ctx.sm_count) * 16));
+    tag_launch(ctx, bf16 ? "split_rows_bf16" : "split_rows_f16", 0, (bf16 ? 6.0 : 8.0) * double(M) * double(K));
+    if (bf16) FXF_CUDA(launch_dependent(split_rows_kernel<1>, dim3(grid), dim3(128), 0, ctx.stream, 1, x, ld, out.planes, out.plane, out.inv, out.amax, bound, M, int(K)));
+    else FXF_CUDA(launch_dependent(split_rows_kernel<0>, dim3(grid), dim3(128), 0, ctx.stream, 1, x, ld, out.planes, out.plane, out.inv, out.amax, bound, M, int(K)));
+    FXF_LAUNCHED(ctx);
+    return 0;
+}
+
+int launch_bias_bound(const float* bias, int64_t n, float* bound, ExecCtx& ctx) {
+    tag_launch(ctx, "bias_bound", 0, 4.0 * double(n));
+    bias_bound_kernel<<<1, 256, 0, ctx.stream>>>(bias, n, bound);
+    FXF_LAUNCHED(ctx);
+    return 0;
+}
+
+// The variant with the least modelled time.  Wide pair tiles win once they fill the machine; smaller problems take narrower
+// tiles until every SM has one.  `force` >= 0 picks an entry of kVariants.
+static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pairs, bool k_split, bool vt, int64_t vt_col0, TailSplit* out_ts, int* out_workers, int force) {
+    const int num_k = int((K + BK - 1) / BK);
+    int best = -1;
+    double best_us = 0;
+    for (int i = 0; i < int(sizeof(kVariants) / sizeof(kVariants[0])); i++) {
+        const Variant& v = kVariants[i];
+        if (force >= 0 && i != force) continue;
+        if (v.pair && (!pairs || M <= BM || sm_count < 2)) continue;
+        if (vt && ((v.bn / 2) % 32 != 0 || vt_col0 % (v.bn / 2) != 0)) continue;   // a warp's columns: whole halves of a head
+        const int rows = v.pair ? 2 * BM : BM, workers = v.pair ? sm_count / 2 : sm_count;
+        const int64_t tiles = ((M + rows - 1) / rows) * ((N + v.bn - 1) / v.bn);
+        const TailSplit ts = plan_tail(tiles, num_k, v, workers, k_split && !vt);
+        if (best < 0 || ts.us < best_us) {
+            best = i;
+            best_us = ts.us;
+            if (out_ts) *out_ts = ts;
+            if (out_workers) *out_workers = workers;
+        }
+    }
+    return best;
+}
+
+std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, int sm_count) {
+    const int v = pick_variant(M, N, K, sm_count, true, true, false, 0, nullptr, nullptr, -1);
+    if (v < 0) return "none";
+    return strfmt("%s-%dx%d%s", bf16 ? "bf16" : "f16x3", kVariants[v].pair ? 256 : 128, kVariants[v].bn, kVariants[v].pair ? "-pair" : "");
+}
+
+bool gemm_f16_vt_ok(const F16GemmArgs& a, const ExecCtx& ctx) {
+    if (a.vt_out == nullptr || a.vt_flags == nullptr || a.residual != nullptr || a.relu || a.split_out.planes != nullptr) return false;
+    if (a.vt_T <= 0 || a.vt_T % 32 != 0 || a.M % a.vt_T != 0 || (a.N - a.vt_col0) != int64_t(a.vt_heads) * 64) return false;
+    return pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, false, true, a.vt_col0, nullptr, nullptr, -1) >= 0;
+}
+
+int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx) {
+    if (a.M == 0 || a.N == 0) return 0;
+    FXF_CHECK(gemm_f16_shape_ok(a.M, a.N, a.K) && a.x.planes && a.w.planes && aligned16(a.x.planes) && aligned16(a.w.planes) && (a.x.plane * 2) % 16 == 0,
+              "f16 GEMM: unsupported operands (M=%lld N=%lld K=%lld)", (long long)a.M, (long long)a.N, (long long)a.K);
+    const bool split = a.split_out.planes != nullptr;
+    FXF_CHECK(split || a.out != nullptr, "f16 GEMM: no output");
+    FXF_CHECK(!split || (a.N % 8 == 0 && a.residual == nullptr && a.vt_out == nullptr), "f16 GEMM: a split output needs N %% 8 == 0 and no residual");
+    TailSplit ts{};
+    int workers = 0;
+    const bool ks = ctx.gemm_ws != nullptr && ctx.gemm_flags != nullptr;
+    const int v = pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, ks, a.vt_out != nullptr, a.vt_col0, &ts, &workers, ctx.f16_variant);
+    FXF_CHECK(v >= 0, "f16 GEMM: no kernel variant for M=%lld N=%lld K=%lld", (long long)a.M, (long long)a.N, (long long)a.K);
+    const Variant& var = kVariants[v];
+    const int rows = var.pair ? 2 * BM : BM, per_unit = var.pair ? 2 : 1;
+    F16Params p{};
+    p.bias = a.bias; p.residual = a.residual; p.out = a.out;
+    p.x_inv = a.bf16 ? nullptr : a.x.inv; p.w_inv = a.bf16 ? nullptr : a.w.inv;
+    p.x_inv_stride = a.x.inv_stride;
+    p.M = a.M; p.N = a.N; p.K = a.K; p.ldo = split ? a.N : a.ldo;
+    p.relu = a.relu ? 1 : 0;
+    p.tma_out = (split || (a.ldo % 4 == 0 && aligned16(a.out) && (a.residual == nullptr || aligned16(a.residual)))) ? 1 : 0;
+    p.tiles_m = int((a.M + rows - 1) / rows);
+    p.tiles_n = int((a.N + var.bn - 1) / var.bn);
+    p.m_fastest = a.N > a.M ? 1 : 0;
+    p.status = ctx.status;
+    if (ts.parts > 1 && (size_t(ts.tail) * ts.parts * per_unit * size_t(BM) * var.bn * sizeof(float) > ctx.gemm_ws_bytes ||
+                         ts.tail * ts.parts * per_unit * kEpiWarps > ctx.gemm_flag_count))
+        ts = TailSplit{int64_t(p.tiles_m) * p.tiles_n, 0, 1, 0.0};
+    p.full_tiles = int(ts.full); p.tail_tiles = int(ts.tail); p.tail_split = ts.parts;
+    p.chunk_slabs = std::max(1, (ctx.tc_chunk_k > 0 ? ctx.tc_chunk_k : (a.conv_chain ? kChunkKConv : kChunkKDense)) / BK);
+    p.ws = ctx.gemm_ws; p.flags = ctx.gemm_flags;
+    p.early_w = ctx.weights_settled ? 1 : 0;
+    if (split) {
+        p.so = a.split_out.planes; p.so_plane = a.split_out.plane; p.so_inv = a.split_out.inv; p.so_amax = a.split_out.amax;
+        p.so_parts = 2 * p.tiles_n;
+        if (a.split_out.parts_out) *a.split_out.parts_out = p.so_parts;
+        p.x_amax = a.x.amax; p.x_parts = a.x.parts; p.w_bound = a.w.bound;
+        FXF_CHECK(a.bf16 || (p.so_inv && p.so_amax && p.x_amax && p.w_bound), "f16 GEMM: a split output needs the row bounds of x and w");
+    }
+    if (a.vt_out != nullptr) {
+        p.vt_out = a.vt_out; p.vt_flags = a.vt_flags; p.vt_col0 = a.vt_col0; p.vt_T = a.vt_T; p.vt_heads = a.vt_heads; p.vt_n32 = a.vt_n32;
+    }
+    tag_launch(ctx, a.bf16 ? "gemm_bf16_tcgen05" : "gemm_f16x3_tcgen05", 2.0 * double(a.M) * double(a.N) * double(a.K),
+               4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.N) + double(a.M) * a.N));
+    if (a.bf16) {
+        switch (v) {
+            case 0: return launch_variant<256, 6, true, 1>(a, p, ts, workers, ctx);
+            case 1: return launch_variant<192, 6, true, 1>(a, p, ts, workers, ctx);
+            case 2: return launch_variant<128, 6, true, 1>(a, p, ts, workers, ctx);
+            case 3: return launch_variant<64, 6, true, 1>(a, p, ts, workers, ctx);
+            case 4: return launch_variant<128, 6, false, 1>(a, p, ts, workers, ctx);
+            case 5: return launch_variant<64, 8, false, 1>(a, p, ts, workers, ctx);
+            default: return launch_variant<32, 8, false, 1>(a, p, ts, workers, ctx);
+        }
+    }
+    switch (v) {
+        case 0: return launch_variant<256, 3, true, 2>(a, p, ts, workers, ctx);
+        case 1: return launch_variant<192, 3, true, 2>(a, p, ts, workers, ctx);
+        case 2: return launch_variant<128, 4, true, 2>(a, p, ts, workers, ctx);
+        case 3: return launch_variant<64, 4, true, 2>(a, p, ts, workers, ctx);
+        case 4: return launch_variant<128, 3, false, 2>(a, p, ts, workers, ctx);
+        case 5: return launch_variant<64, 4, false, 2>(a, p, ts, workers, ctx);
+        default: return launch_variant<32, 4, false, 2>(a, p, ts, workers, ctx);
+    }
+}
+
+}  // namespace fxf

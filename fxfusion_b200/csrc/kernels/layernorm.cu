@@ -11,6 +11,7 @@
 // strides over rows.  Rows wider than 32 lanes x 8 float4 (N > 1024) or not 16-byte aligned
 // use a block-per-row kernel that re-reads the row from L2 instead.
 #include "../runtime.hpp"
+#include "sm100.cuh"
 
 namespace fxf {
 namespace {
@@ -23,10 +24,15 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-template <int NV, bool ADD>
+// Where the rows go: fp32, the split form of the f16 GEMM (the whole row is in registers: its maximum gives the scale), or bf16.
+enum RowForm { kF32 = 0, kSplitF16 = 1, kBf16 = 2 };
+
+template <int NV, bool ADD, int FORM>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) layernorm_warp_kernel(const float4* __restrict__ x, const float4* __restrict__ z,
                                                                              const float4* __restrict__ w, const float4* __restrict__ b,
-                                                                             float4* __restrict__ out, int64_t M, int n4, float inv_n, float eps) {
+                                                                             float4* __restrict__ out, SplitOut so, int64_t M, int n4, float inv_n, float eps) {
+    sm100::grid_dep_launch();
+    sm100::grid_dep_wait();
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int64_t row_stride = int64_t(gridDim.x) * kWarpsPerBlock;
     for (int64_t row = int64_t(blockIdx.x) * kWarpsPerBlock + warp; row < M; row += row_stride) {
@@ -61,7 +67,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) layernorm_warp_kernel(con
         float var = warp_sum(q) * inv_n;
         float rstd = 1.0f / sqrtf(var + eps);
         float shift = -rstd * mean;
-        float4* orow = out + row * n4;
+        float m = 0.f;
 #pragma unroll
         for (int i = 0; i < NV; i++) {
             int c = lane + 32 * i;
@@ -71,7 +77,33 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) layernorm_warp_kernel(con
                 r.y = (v[i].y * rstd + shift) * g.y + bb.y;
                 r.z = (v[i].z * rstd + shift) * g.z + bb.z;
                 r.w = (v[i].w * rstd + shift) * g.w + bb.w;
-                orow[c] = r;
+                if (FORM == kF32) out[row * n4 + c] = r;
+                else if (FORM == kBf16)
+                    *reinterpret_cast<uint2*>(so.planes + (row * n4 + c) * 4) = make_uint2(sm100::pack_bf16x2(r.x, r.y), sm100::pack_bf16x2(r.z, r.w));
+                else {
+                    m = fmaxf(m, fmaxf(fmaxf(fabsf(r.x), fabsf(r.y)), fmaxf(fabsf(r.z), fabsf(r.w))));
+                    v[i] = r;
+                }
+            }
+        }
+        if (FORM == kSplitF16) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            float scale, inv;
+            sm100::split_scale(m, scale, inv);
+            if (lane == 0) {
+                so.inv[row] = inv;
+                so.amax[row] = m;
+            }
+#pragma unroll
+            for (int i = 0; i < NV; i++) {
+                int c = lane + 32 * i;
+                if (c < n4) {
+                    uint2 hi, lo;
+                    sm100::split_f16x4(v[i], scale, hi, lo);
+                    *reinterpret_cast<uint2*>(so.planes + (row * n4 + c) * 4) = hi;
+                    *reinterpret_cast<uint2*>(so.planes + so.plane + (row * n4 + c) * 4) = lo;
+                }
             }
         }
     }
@@ -121,6 +153,8 @@ template <bool ADD>
 int run_layernorm(const float* x, const float* z, const float* w, const float* b, float* out, int64_t M, int64_t N, float eps, ExecCtx& ctx) {
     if (M == 0 || N == 0) return 0;
     float inv_n = 1.0f / float(N);
+    const bool bf16 = ctx.gemm_mode == FXF_GEMM_BF16;
+    const SplitOut so = ctx.split_out;
     bool vec = N % 4 == 0 && N <= 1024 && aligned16(x) && aligned16(w) && aligned16(b) && aligned16(out) && (!ADD || aligned16(z));
     if (vec) {
         int n4 = int(N / 4), nv = (n4 + 31) / 32;
@@ -133,13 +167,18 @@ int run_layernorm(const float* x, const float* z, const float* w, const float* b
         auto Bv = reinterpret_cast<const float4*>(b);
         auto O = reinterpret_cast<float4*>(out);
         dim3 blk(kWarpsPerBlock * 32);
-#define FXF_LN_CASE(NV) case NV: layernorm_warp_kernel<NV, ADD><<<grid, blk, 0, ctx.stream>>>(X, Z, W, Bv, O, M, n4, inv_n, eps); break;
+        auto kernel = layernorm_warp_kernel<1, ADD, kF32>;
+#define FXF_LN_CASE(NV) \
+    case NV: kernel = so.planes == nullptr ? layernorm_warp_kernel<NV, ADD, kF32> : (bf16 ? layernorm_warp_kernel<NV, ADD, kBf16> : layernorm_warp_kernel<NV, ADD, kSplitF16>); break;
         switch (nv) {
             FXF_LN_CASE(1) FXF_LN_CASE(2) FXF_LN_CASE(3) FXF_LN_CASE(4)
             FXF_LN_CASE(5) FXF_LN_CASE(6) FXF_LN_CASE(7) FXF_LN_CASE(8)
         }
 #undef FXF_LN_CASE
+        FXF_CUDA(launch_dependent(kernel, dim3(grid), blk, 0, ctx.stream, 1, X, Z, W, Bv, O, so, M, n4, inv_n, eps));
+        if (so.parts_out) *so.parts_out = 1;
     } else {
+        FXF_CHECK(so.planes == nullptr, "layer_norm: rows this wide have no split form");
         int64_t cap = int64_t(ctx.sm_count) * 8;
         int grid = int(M < cap ? M : cap);
         layernorm_block_kernel<ADD><<<grid, 256, 0, ctx.stream>>>(x, z, w, b, out, M, N, inv_n, eps);
@@ -187,7 +226,7 @@ int k_add_layer_norm(Registry& reg, const TensorIds& in, const TensorIds& out, c
                                static_cast<const float*>(b.ptr), static_cast<float*>(o.ptr), M, N, p.floats[0], ctx);
 }
 
-std::unique_ptr<NodePlan> plan_layernorm(const Registry& reg, const TensorIds& in, const TensorIds& out, const Params&, const PlanEnv&) {
+std::unique_ptr<NodePlan> plan_layernorm(const Registry& reg, const TensorIds& in, const TensorIds& out, const Params& params, const PlanEnv&) {
     auto p = std::make_unique<LayerNormPlan>();
     double b = 0;
     for (auto id : in) b += double(reg[id].nbytes);
@@ -195,6 +234,15 @@ std::unique_ptr<NodePlan> plan_layernorm(const Registry& reg, const TensorIds& i
     p->bytes = b;
     p->flops = out.empty() ? 0 : 8.0 * double(numel(reg[out[0]]));
     p->variant = "warp-per-row vec128";
+    // the warp-per-row kernel can leave its rows in split form (8-element groups for the 16-byte rows of the f16 GEMM's loads)
+    int64_t n = 1;
+    if (!params.ints.empty() && int64_t(params.ints.size()) > params.ints[0])
+        for (int64_t i = 0; i < params.ints[0]; i++) n *= params.ints[1 + i];
+    if (!out.empty() && n > 0 && n % 8 == 0 && n <= 1024 && numel(reg[out[0]]) % n == 0) {
+        p->makes_split = true;
+        p->split_cols = n;
+        p->split_rows = numel(reg[out[0]]) / n;
+    }
     return p;
 }
 

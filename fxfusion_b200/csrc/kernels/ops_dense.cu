@@ -96,9 +96,11 @@ struct Slice {
     bool split = false;             // TF32 hi/lo copies wanted (tensor-core GEMM operand)
     bool bf16 = false;              // bf16 mode: one bf16 copy instead (hi points to it, lo stays NULL)
     bool mixed = false;             // mixed mode: hi = TF32 high part (fp32), lo -> bf16(w - hi)
+    bool f16 = false;               // operand of the f16 GEMM instead: split form (gemm_f16.cu), or its bf16 plane in bf16 mode
     bool drop = false;              // replaced by "no bias" (rank != 0 of a row-parallel product)
     size_t off_copy = 0, off_split = 0;  // byte offsets inside the plan's persistent memory
     const float *ptr = nullptr, *hi = nullptr, *lo = nullptr;  // resolved by prepare()
+    SplitMat mat;                   // likewise
     int64_t rows() const { return nrow[0] + nrow[1] + nrow[2]; }
     int64_t elems() const { return rows() * ncol; }
 };
@@ -120,6 +122,12 @@ struct DensePlan : NodePlan {
         x.row0[0] = 0; x.nrow[0] = rows;
         x.col0 = 0; x.ncol = cols; x.src_ld = cols;
         return x;
+    }
+    void reserve_f16(Slice& x) {   // the whole tensor in split form (f16 products are not sharded)
+        x.f16 = true;
+        x.bf16 = bf16_mode;
+        x.off_split = persist_bytes;
+        persist_bytes += round_up(size_t(x.elems()) * (bf16_mode ? 2 : 4), 256) + round_up(size_t(x.rows()) * 4, 256) + 256;
     }
     void reserve(Slice& x, bool want_split) {
         if (x.drop) return;
@@ -154,6 +162,19 @@ struct DensePlan : NodePlan {
                 }
                 x.ptr = dst;
             }
+            if (x.f16) {
+                FXF_CHECK(persist != nullptr && x.whole, "dense plan: persistent memory was not assigned");
+                char* base = static_cast<char*>(persist) + x.off_split;
+                SplitOut o;
+                o.planes = reinterpret_cast<uint16_t*>(base);
+                o.plane = x.elems();
+                o.inv = reinterpret_cast<float*>(base + round_up(size_t(x.elems()) * (x.bf16 ? 2 : 4), 256));
+                float* bound = reinterpret_cast<float*>(reinterpret_cast<char*>(o.inv) + round_up(size_t(x.rows()) * 4, 256));
+                FXF_CUDA(cudaMemsetAsync(bound, 0, 2 * sizeof(float), ctx.stream));
+                if (launch_split_rows(x.ptr, x.ncol, x.rows(), x.ncol, x.bf16, o, bound, ctx)) return 1;
+                x.mat = SplitMat{};
+                x.mat.planes = o.planes; x.mat.plane = o.plane; x.mat.inv = o.inv; x.mat.bound = bound;
+            }
             if (x.split) {
                 FXF_CHECK(persist != nullptr, "dense plan: persistent memory was not assigned");
                 float* h = reinterpret_cast<float*>(static_cast<char*>(persist) + x.off_split);
@@ -172,6 +193,8 @@ struct DensePlan : NodePlan {
                 }
             }
         }
+        for (int i = 0; i + 1 < n; i++)   // a weight's bias follows it
+            if (s[i].f16 && !s[i].bf16 && s[i + 1].ncol == 1 && !s[i + 1].drop && launch_bias_bound(s[i + 1].ptr, s[i + 1].rows(), const_cast<float*>(s[i].mat.bound), ctx)) return 1;
         prepared = true;
         return 0;
     }
@@ -181,6 +204,54 @@ inline const DensePlan* dense(const NodePlan* p) { return static_cast<const Dens
 // M < 64 (batch-sized layers, single-position decode steps) never takes the tensor-core path: those problems are weight
 // reads, served by the fp32 FFMA few-rows kernels from the fp32 weights (half the bytes of a hi/lo pair).
 bool want_tc(const PlanEnv& env, int64_t M, int64_t N, int64_t K) { return env.gemm_mode != FXF_GEMM_FP32_SIMT && gemm_tc_shape_ok(M, N, K); }
+
+// The f16 GEMM serves single-GPU engines in the default and the bf16 mode, from 64 rows on (fewer rows: see above).
+bool want_f16(const PlanEnv& env, int64_t M, int64_t N, int64_t K) {
+    if (env.tp_size > 1 || M < 64 || !gemm_f16_shape_ok(M, N, K)) return false;
+    return env.gemm_mode == FXF_GEMM_AUTO || (env.gemm_mode == FXF_GEMM_BF16 && gemm_tc_shape_ok(M, N, K));
+}
+void reserve_weight(DensePlan& p, Slice& w, const PlanEnv& env, int64_t M, int64_t N, int64_t K) {
+    if (want_f16(env, M, N, K)) p.reserve_f16(w);
+    else p.reserve(w, want_tc(env, M, N, K));
+}
+std::string variant_of(const PlanEnv& env, const Slice& w, int64_t M, int64_t N, int64_t K) {
+    GemmArgs g;
+    g.M = M; g.N = N; g.K = K;
+    std::string v = gemm_variant_name(g, env.gemm_mode, 148, env.tc_pairs);
+    return w.f16 ? v + " (split operands: tcgen05-" + gemm_f16_variant_name(M, N, K, w.bf16, 148) + ")" : v;
+}
+
+// Room for an activation matrix that has to be split before its product: planes, scales, row maxima.
+size_t split_area_bytes(int64_t M, int64_t K) { return round_up(size_t(M) * size_t(K) * 4, 256) + 2 * round_up(size_t(M) * 4, 256); }
+SplitOut split_area(void* area, int64_t M, int64_t K) {
+    SplitOut o;
+    char* b = static_cast<char*>(area);
+    o.planes = reinterpret_cast<uint16_t*>(b);
+    o.plane = M * K;
+    o.inv = reinterpret_cast<float*>(b + round_up(size_t(M) * size_t(K) * 4, 256));
+    o.amax = reinterpret_cast<float*>(reinterpret_cast<char*>(o.inv) + round_up(size_t(M) * 4, 256));
+    return o;
+}
+SplitMat as_operand(const SplitOut& o, int parts = 1) {
+    SplitMat m;
+    m.planes = o.planes; m.plane = o.plane; m.inv = o.inv; m.amax = o.amax; m.parts = parts;
+    return m;
+}
+// The split form of input `id` of a node: the tensor's own where its producer wrote it so, else split into `area` now.
+int split_input(const Registry& reg, uint32_t id, int64_t M, int64_t K, bool bf16, void* area, ExecCtx& ctx, SplitMat* out) {
+    if (const SplitMat* m = split_of(ctx, id)) {
+        *out = *m;
+        return 0;
+    }
+    const SplitOut o = split_area(area, M, K);
+    *out = as_operand(o);
+    return launch_split_rows(static_cast<const float*>(reg[id].ptr), K, M, K, bf16, o, nullptr, ctx);
+}
+void fill_f16(F16GemmArgs& g, const SplitMat& x, const Slice& w, const Slice* bias, float* out, int64_t M, int64_t ldo, bool relu) {
+    g.x = x; g.w = w.mat; g.bf16 = w.bf16;
+    g.bias = (bias && !bias->drop) ? bias->ptr : nullptr;
+    g.out = out; g.M = M; g.N = w.rows(); g.K = w.ncol; g.ldo = ldo; g.relu = relu;
+}
 
 void fill_gemm(GemmArgs& g, const float* x, const Slice& w, const Slice* bias, float* out, int64_t M, int64_t ldx, int64_t ldo, bool relu) {
     g.x = x; g.w = w.ptr; g.w_hi = w.hi; g.w_lo = w.lo; g.w_is_bf16 = w.bf16; g.w_mixed = w.mixed;
@@ -208,6 +279,17 @@ int run_linear(Registry& reg, const TensorIds& in, const TensorIds& out, bool re
     FXF_CHECK(numel(o) == M * N, "%s: output size mismatch", who);
     const DensePlan* pl = dense(plan);
     FXF_CHECK(pl != nullptr && pl->n == 2 && pl->prepared, "%s: the node was not prepared", who);
+    if (pl->s[0].f16) {
+        if (M == 0 || N == 0) return 0;
+        FXF_CHECK(split_of(ctx, in[0]) != nullptr || ctx.scratch_bytes >= split_area_bytes(M, K), "%s: scratch too small", who);
+        SplitMat xs;
+        if (split_input(reg, in[0], M, K, pl->s[0].bf16, ctx.scratch, ctx, &xs)) return 1;
+        F16GemmArgs f;
+        fill_f16(f, xs, pl->s[0], &pl->s[1], static_cast<float*>(o.ptr), M, N, relu);
+        f.split_out = ctx.split_out;
+        if (ctx.split_out.planes == nullptr) apply_fusion(ctx, f, false);
+        return launch_gemm_f16(f, ctx);
+    }
     GemmArgs g;
     fill_gemm(g, static_cast<const float*>(x.ptr), pl->s[0], &pl->s[1], static_cast<float*>(o.ptr) + pl->col_off, M, K, N, relu);
     if (pl->col_off == 0 && pl->s[0].rows() == N) apply_fusion(ctx, g, false);   // never with a column-sharded output
@@ -220,10 +302,25 @@ int k_linear(Registry& reg, const TensorIds& in, const TensorIds& out, const Par
     return run_linear(reg, in, out, false, plan, ctx, "linear");
 }
 
-int linear_on_rows(const NodePlan* plan, const float* x_rows, int64_t M, int64_t ldx, float* out, int64_t ldo, ExecCtx& ctx) {
+int linear_on_rows(const NodePlan* plan, const float* x_rows, const SplitMat* split_rows, int64_t M, int64_t ldx, float* out, int64_t ldo, ExecCtx& ctx) {
     const DensePlan* pl = dense(plan);
     FXF_CHECK(pl != nullptr && pl->n == 2 && pl->prepared, "linear (rows): the node was not prepared");
     if (M == 0 || pl->s[0].rows() == 0) return 0;
+    if (pl->s[0].f16) {
+        SplitMat xs;
+        if (split_rows != nullptr) xs = *split_rows;
+        else {
+            const int64_t K = pl->s[0].ncol;
+            FXF_CHECK(ctx.scratch_bytes >= split_area_bytes(M, K), "linear (rows): scratch too small");
+            const SplitOut o = split_area(ctx.scratch, M, K);
+            if (launch_split_rows(x_rows, ldx, M, K, pl->s[0].bf16, o, nullptr, ctx)) return 1;
+            xs = as_operand(o);
+        }
+        F16GemmArgs f;
+        fill_f16(f, xs, pl->s[0], &pl->s[1], out, M, ldo, false);
+        return launch_gemm_f16(f, ctx);
+    }
+    FXF_CHECK(split_rows == nullptr, "linear (rows): the rows are in split form but the weight is not");
     GemmArgs g;
     fill_gemm(g, x_rows, pl->s[0], &pl->s[1], out + pl->col_off, M, ldx, ldo, false);
     // few rows against a large weight: the tensor-core kernel streams the pre-split weight once; rows beyond M are zero fill
@@ -253,14 +350,18 @@ std::unique_ptr<NodePlan> plan_linear(const Registry& reg, const TensorIds& in, 
         p->col_off = r0;
         p->n_local = r1 - r0;
     }
-    p->reserve(ws, want_tc(env, M, p->n_local, K));
+    reserve_weight(*p, ws, env, M, p->n_local, K);
     p->reserve(bs, false);
     p->M = M;
+    if (ws.f16) {
+        p->takes_split = 1;
+        p->makes_split = N % 8 == 0;
+        p->split_rows = M; p->split_cols = N;
+        p->scratch_bytes = split_area_bytes(M, K);
+    }
     p->flops = 2.0 * double(M) * double(p->n_local) * double(K);
     p->bytes = 4.0 * (double(M) * K + double(p->n_local) * K + double(p->n_local) + double(M) * p->n_local);
-    GemmArgs g;
-    g.M = M; g.N = p->n_local; g.K = K;
-    p->variant = gemm_variant_name(g, env.gemm_mode, 148, env.tc_pairs);
+    p->variant = variant_of(env, ws, M, p->n_local, K);
     return p;
 }
 
@@ -291,6 +392,55 @@ static int finish_row_parallel(GemmArgs& g2, int64_t M, int64_t N, bool sharded,
 }
 
 // ---- FeedForward ------------------------------------------------------------------------------
+// On the f16 GEMM: the first product's epilogue leaves the hidden activation in split form, so it costs no more bytes than in
+// fp32 and the second product reads it as it is.  scratch: hidden planes | scales | row maxima | room to split x.
+static size_t ff_f16_bytes(int64_t M, int64_t K, int64_t F) {
+    return round_up(size_t(M) * size_t(F) * 4, 256) + round_up(size_t(M) * 4, 256) + round_up(size_t(M) * size_t(gemm_f16_split_parts(F)) * 4, 256) + split_area_bytes(M, K);
+}
+static int run_feedforward_f16(Registry& reg, const TensorIds& in, const float* x, float* out, int64_t M, int64_t K, int64_t F, int64_t P, const DensePlan* pl, ExecCtx& ctx) {
+    if (M == 0 || P == 0) return 0;
+    FXF_CHECK(ctx.scratch != nullptr && ctx.scratch_bytes >= ff_f16_bytes(M, K, F), "feedforward: scratch too small");
+    char* base = static_cast<char*>(ctx.scratch);
+    SplitOut h;
+    int parts = 1;
+    h.planes = reinterpret_cast<uint16_t*>(base);
+    h.plane = M * F;
+    h.inv = reinterpret_cast<float*>(base + round_up(size_t(M) * size_t(F) * 4, 256));
+    h.amax = reinterpret_cast<float*>(reinterpret_cast<char*>(h.inv) + round_up(size_t(M) * 4, 256));
+    h.parts_out = &parts;
+    char* area = reinterpret_cast<char*>(h.amax) + round_up(size_t(M) * size_t(gemm_f16_split_parts(F)) * 4, 256);
+    float* hidden = static_cast<float*>(ctx.scratch);
+    const bool both = pl->s[0].f16 && pl->s[2].f16;
+    if (pl->s[0].f16) {
+        SplitMat xs;
+        if (split_input(reg, in[0], M, K, pl->s[0].bf16, area, ctx, &xs)) return 1;
+        F16GemmArgs g1;
+        fill_f16(g1, xs, pl->s[0], &pl->s[1], both ? nullptr : hidden, M, F, true);
+        if (both) g1.split_out = h;
+        if (launch_gemm_f16(g1, ctx)) return 1;
+    } else {
+        GemmArgs g1;
+        fill_gemm(g1, x, pl->s[0], &pl->s[1], hidden, M, K, F, true);
+        if (launch_gemm(g1, ctx)) return 1;
+    }
+    if (!pl->s[2].f16) {
+        GemmArgs g2;
+        fill_gemm(g2, hidden, pl->s[2], &pl->s[3], out, M, F, P, false);
+        apply_fusion(ctx, g2, false);
+        return launch_gemm(g2, ctx);
+    }
+    SplitMat hs = as_operand(h, parts);
+    if (!both) {   // the hidden activation came from another kernel as fp32
+        FXF_CHECK(split_area_bytes(M, F) <= ctx.scratch_bytes - size_t(reinterpret_cast<char*>(area) - base), "feedforward: scratch too small to split the hidden activation");
+        const SplitOut o = split_area(area, M, F);
+        if (launch_split_rows(hidden, F, M, F, pl->s[2].bf16, o, nullptr, ctx)) return 1;
+        hs = as_operand(o);
+    }
+    F16GemmArgs g2;
+    fill_f16(g2, hs, pl->s[2], &pl->s[3], out, M, P, false);
+    apply_fusion(ctx, g2, false);
+    return launch_gemm_f16(g2, ctx);
+}
 // slices: s[0] = w1 rows of this rank [Fl, D], s[1] = b1 entries [Fl], s[2] = w2 columns of this rank [P, Fl], s[3] = b2
 int k_feedforward(Registry& reg, const TensorIds& in, const TensorIds& out, const Params&, const NodePlan* plan, ExecCtx& ctx) {
     FXF_CHECK(in.size() >= 5 && out.size() >= 1, "feedforward: expects [x, w1, b1, w2, b2]");
@@ -305,6 +455,7 @@ int k_feedforward(Registry& reg, const TensorIds& in, const TensorIds& out, cons
     const DensePlan* pl = dense(plan);
     FXF_CHECK(pl != nullptr && pl->n == 4 && pl->prepared, "feedforward: the node was not prepared");
     const int64_t Fl = pl->s[0].rows();
+    if (pl->s[0].f16 || pl->s[2].f16) return run_feedforward_f16(reg, in, static_cast<const float*>(x.ptr), static_cast<float*>(o.ptr), M, K, Fl, P, pl, ctx);
     size_t need = size_t(M) * size_t(Fl) * sizeof(float);
     FXF_CHECK(ctx.scratch_bytes >= need && (need == 0 || ctx.scratch != nullptr), "feedforward: scratch too small (%zu < %zu bytes)", ctx.scratch_bytes, need);
     float* hidden = static_cast<float*>(ctx.scratch);
@@ -338,18 +489,17 @@ std::unique_ptr<NodePlan> plan_feedforward(const Registry& reg, const TensorIds&
     } else if (env.tp_size > 1) {
         p->variant = "replicated ";
     }
-    p->reserve(s_w1, want_tc(env, M, Fl, K));
+    reserve_weight(*p, s_w1, env, M, Fl, K);
     p->reserve(s_b1, false);
-    p->reserve(s_w2, want_tc(env, M, P, Fl));
+    reserve_weight(*p, s_w2, env, M, P, Fl);
     p->reserve(s_b2, false);
     p->M = M;
     p->scratch_bytes = size_t(M) * size_t(Fl) * sizeof(float);
+    if (s_w1.f16 || s_w2.f16) p->scratch_bytes = ff_f16_bytes(M, std::max(K, Fl), Fl);
+    if (s_w1.f16) p->takes_split = 1;
     p->flops = 2.0 * double(M) * double(Fl) * double(K) + 2.0 * double(M) * double(P) * double(Fl);
     p->bytes = 4.0 * (double(M) * K + double(Fl) * K + Fl + double(P) * Fl + P + double(M) * P);
-    GemmArgs g1, g2;
-    g1.M = M; g1.N = Fl; g1.K = K;
-    g2.M = M; g2.N = P; g2.K = Fl;
-    p->variant += gemm_variant_name(g1, env.gemm_mode, 148, env.tc_pairs) + "+" + gemm_variant_name(g2, env.gemm_mode, 148, env.tc_pairs);
+    p->variant += variant_of(env, s_w1, M, Fl, K) + "+" + variant_of(env, s_w2, M, P, Fl);
     return p;
 }
 
@@ -385,13 +535,35 @@ int k_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const Params
     float* qkv = static_cast<float*>(ctx.scratch);
     float* cx = qkv + M * QKVl;
     float* vt = cx + M * Dl;  // only present when the plan reserved it
+    // f16 products: room for x and, later, the context in split form, ahead of V^T
+    const size_t area_bytes = (pl->s[0].f16 || pl->s[2].f16) ? split_area_bytes(M, D) : 0;
+    void* area = vt;
+    vt = reinterpret_cast<float*>(reinterpret_cast<char*>(vt) + area_bytes);
+    need += area_bytes;
+    FXF_CHECK(ctx.scratch_bytes >= need, "mha: scratch too small (%zu < %zu bytes)", ctx.scratch_bytes, need);
     const bool have_vt = ctx.scratch_bytes >= need + attention_tc_scratch_bytes(B, T, Hl);
+    if (M == 0) return 0;
 
+    bool v_transposed = false;
+    if (pl->s[0].f16) {
+        SplitMat xs;
+        if (split_input(reg, in[0], M, D, pl->s[0].bf16, area, ctx, &xs)) return 1;
+        F16GemmArgs f;
+        fill_f16(f, xs, pl->s[0], &pl->s[1], qkv, M, QKVl, false);
+        if (have_vt && hd == 64) {
+            f.vt_out = vt;
+            f.vt_flags = reinterpret_cast<unsigned char*>(vt + size_t(B) * size_t(Hl) * size_t(T) * 64);
+            f.vt_col0 = 2 * Dl;
+            f.vt_T = int(T); f.vt_heads = int(Hl); f.vt_n32 = int((T + 31) / 32);
+            v_transposed = gemm_f16_vt_ok(f, ctx);
+            if (!v_transposed) { f.vt_out = nullptr; f.vt_flags = nullptr; }
+        }
+        if (launch_gemm_f16(f, ctx)) return 1;
+    } else {
     GemmArgs g;
     fill_gemm(g, static_cast<const float*>(x.ptr), pl->s[0], &pl->s[1], qkv, M, D, QKVl, false);
     // Where the projection runs on a tensor-core variant whose column halves are multiples of half a head, its epilogue writes the V third
     // transposed (and the finite flags of V) straight into the attention kernel's V^T buffer: no transpose launch.
-    bool v_transposed = false;
     if (have_vt && hd == 64 && ctx.gemm_mode != FXF_GEMM_FP32_SIMT && use_tc(g, ctx.gemm_mode)) {
         g.vt_out = vt;
         g.vt_flags = reinterpret_cast<unsigned char*>(vt + size_t(B) * size_t(Hl) * size_t(T) * 64);
@@ -401,6 +573,7 @@ int k_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const Params
         if (!v_transposed) { g.vt_out = nullptr; g.vt_flags = nullptr; }
     }
     if (launch_gemm(g, ctx)) return 1;
+    }
 
     AttnArgs a;
     a.qkv = qkv; a.ctx = cx;
@@ -416,6 +589,14 @@ int k_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const Params
         if (launch_attention(a, ctx)) return 1;
     }
 
+    if (pl->s[2].f16) {
+        const SplitOut so = split_area(area, M, D);
+        if (launch_split_rows(cx, D, M, D, pl->s[2].bf16, so, nullptr, ctx)) return 1;
+        F16GemmArgs f2;
+        fill_f16(f2, as_operand(so), pl->s[2], &pl->s[3], static_cast<float*>(o.ptr), M, D, false);
+        apply_fusion(ctx, f2, false);
+        return launch_gemm_f16(f2, ctx);
+    }
     GemmArgs g2;
     fill_gemm(g2, cx, pl->s[2], &pl->s[3], static_cast<float*>(o.ptr), M, Dl, D, false);
     return finish_row_parallel(g2, M, D, pl->tp_sharded, ctx);
@@ -452,20 +633,19 @@ std::unique_ptr<NodePlan> plan_mha(const Registry& reg, const TensorIds& in, con
     } else if (env.tp_size > 1) {
         pl->variant = "replicated ";
     }
-    pl->reserve(s_wq, want_tc(env, M, 3 * Dl, D));
+    reserve_weight(*pl, s_wq, env, M, 3 * Dl, D);
     pl->reserve(s_bq, false);
-    pl->reserve(s_wo, want_tc(env, M, D, Dl));
+    reserve_weight(*pl, s_wo, env, M, D, Dl);
     pl->reserve(s_bo, false);
     pl->M = M;
     pl->scratch_bytes = size_t(M) * size_t(3 * Dl + Dl) * sizeof(float);
+    if (s_wq.f16 || s_wo.f16) pl->scratch_bytes += split_area_bytes(M, D);
+    if (s_wq.f16) pl->takes_split = 1;
     const bool tc_attn = env.gemm_mode != FXF_GEMM_FP32_SIMT && hd == 64 && T % 4 == 0 && T >= 16 && T <= 4096 && Dl % 4 == 0;   // the tcgen05 kernel covers at most 32 blocks of 128 keys
     if (tc_attn) pl->scratch_bytes += attention_tc_scratch_bytes(B, T, Hl);
     pl->flops = 2.0 * M * double(3 * Dl) * D + 4.0 * double(B) * Hl * double(T) * T * hd + 2.0 * double(M) * D * Dl;
     pl->bytes = 4.0 * (2.0 * double(M) * D + double(3 * Dl) * D + 3 * Dl + double(D) * Dl + D) + double(reg[in[1]].nbytes);
-    GemmArgs g1, g2;
-    g1.M = M; g1.N = 3 * Dl; g1.K = D;
-    g2.M = M; g2.N = D; g2.K = Dl;
-    pl->variant += gemm_variant_name(g1, env.gemm_mode, 148, env.tc_pairs) + (tc_attn ? "+attn-tcgen05-tf32+2bf16+" : "+flash-fp32+") + gemm_variant_name(g2, env.gemm_mode, 148, env.tc_pairs);
+    pl->variant += variant_of(env, s_wq, M, 3 * Dl, D) + (tc_attn ? "+attn-tcgen05-tf32+2bf16+" : "+flash-fp32+") + variant_of(env, s_wo, M, D, Dl);
     return pl;
 }
 
@@ -511,14 +691,31 @@ int k_cross_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const 
     float* kv = q + Mq * Dl;                        // [Mk, 2*Dl]
     float* cx = kv + Mk * 2 * Dl;                   // [Mq, Dl]
     float* vt = cx + Mq * Dl;                       // only present when the plan reserved it
+    const bool any_f16 = pl->s[0].f16 || pl->s[2].f16 || pl->s[4].f16;   // room to split x, memory and the context, one after the other
+    void* area = vt;
+    if (any_f16) {
+        vt = reinterpret_cast<float*>(reinterpret_cast<char*>(vt) + split_area_bytes(std::max(Mq, Mk), D));
+        need += split_area_bytes(std::max(Mq, Mk), D);
+        FXF_CHECK(ctx.scratch_bytes >= need, "cross_mha: scratch too small (%zu < %zu bytes)", ctx.scratch_bytes, need);
+    }
     const bool have_vt = ctx.scratch_bytes >= need + attention_tc_scratch_bytes(B, Tk, Hl);
+    if (Mq == 0) return 0;
 
-    GemmArgs g;
-    fill_gemm(g, static_cast<const float*>(x.ptr), pl->s[0], &pl->s[1], q, Mq, D, Dl, false);
-    if (launch_gemm(g, ctx)) return 1;
-    GemmArgs gk;
-    fill_gemm(gk, static_cast<const float*>(mem.ptr), pl->s[2], &pl->s[3], kv, Mk, D, 2 * Dl, false);
-    if (launch_gemm(gk, ctx)) return 1;
+    auto project = [&](int wi, uint32_t id, const FxfTensor& t, float* dst, int64_t rows, int64_t cols) {
+        if (pl->s[wi].f16) {
+            SplitMat xs;
+            if (rows == 0) return 0;
+            if (split_input(reg, id, rows, D, pl->s[wi].bf16, area, ctx, &xs)) return 1;
+            F16GemmArgs f;
+            fill_f16(f, xs, pl->s[wi], &pl->s[wi + 1], dst, rows, cols, false);
+            return launch_gemm_f16(f, ctx);
+        }
+        GemmArgs g;
+        fill_gemm(g, static_cast<const float*>(t.ptr), pl->s[wi], &pl->s[wi + 1], dst, rows, D, cols, false);
+        return launch_gemm(g, ctx);
+    };
+    if (project(0, in[0], x, q, Mq, Dl)) return 1;
+    if (project(2, in[1], mem, kv, Mk, 2 * Dl)) return 1;
 
     if (Tk == 0) {  // softmax over no keys: the context is an empty sum
         if (Mq * Dl > 0) FXF_CUDA(cudaMemsetAsync(cx, 0, size_t(Mq) * size_t(Dl) * sizeof(float), ctx.stream));
@@ -538,6 +735,14 @@ int k_cross_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const 
         }
     }
 
+    if (pl->s[4].f16) {
+        const SplitOut so = split_area(area, Mq, D);
+        if (launch_split_rows(cx, D, Mq, D, pl->s[4].bf16, so, nullptr, ctx)) return 1;
+        F16GemmArgs f2;
+        fill_f16(f2, as_operand(so), pl->s[4], &pl->s[5], static_cast<float*>(o.ptr), Mq, D, false);
+        apply_fusion(ctx, f2, false);
+        return launch_gemm_f16(f2, ctx);
+    }
     GemmArgs g2;
     fill_gemm(g2, cx, pl->s[4], &pl->s[5], static_cast<float*>(o.ptr), Mq, Dl, D, false);
     return finish_row_parallel(g2, Mq, D, pl->tp_sharded, ctx);
@@ -581,24 +786,22 @@ std::unique_ptr<NodePlan> plan_cross_mha(const Registry& reg, const TensorIds& i
     } else if (env.tp_size > 1) {
         pl->variant = "replicated ";
     }
-    pl->reserve(s_wq, want_tc(env, Mq, Dl, D));
+    reserve_weight(*pl, s_wq, env, Mq, Dl, D);
     pl->reserve(s_bq, false);
-    pl->reserve(s_wkv, want_tc(env, Mk, 2 * Dl, D));
+    reserve_weight(*pl, s_wkv, env, Mk, 2 * Dl, D);
     pl->reserve(s_bkv, false);
-    pl->reserve(s_wo, want_tc(env, Mq, D, Dl));
+    reserve_weight(*pl, s_wo, env, Mq, D, Dl);
     pl->reserve(s_bo, false);
     pl->M = Mq;
     pl->scratch_bytes = (size_t(Mq) * size_t(2 * Dl) + size_t(Mk) * size_t(2 * Dl)) * sizeof(float);
+    if (s_wq.f16 || s_wkv.f16 || s_wo.f16) pl->scratch_bytes += split_area_bytes(std::max(Mq, Mk), D);
+    pl->takes_split = (s_wq.f16 ? 1u : 0u) | (s_wkv.f16 ? 2u : 0u);
     const bool tc_attn = env.gemm_mode != FXF_GEMM_FP32_SIMT && hd == 64 && Tk % 4 == 0 && Tk >= 16 && Tk <= 4096 && Dl % 4 == 0;
     if (tc_attn) pl->scratch_bytes += attention_tc_scratch_bytes(B, Tk, Hl);
     pl->flops = 2.0 * double(Mq) * Dl * D + 2.0 * double(Mk) * 2 * Dl * D + 4.0 * double(B) * Hl * double(Tq) * Tk * hd + 2.0 * double(Mq) * D * Dl;
     pl->bytes = 4.0 * (2.0 * double(Mq) * D + double(Mk) * D + 2.0 * double(Dl) * D + 2.0 * double(Dl) * D + 3 * Dl + D) + double(reg[in[2]].nbytes);
-    GemmArgs g1, g2, g3;
-    g1.M = Mq; g1.N = Dl; g1.K = D;
-    g2.M = Mk; g2.N = 2 * Dl; g2.K = D;
-    g3.M = Mq; g3.N = D; g3.K = Dl;
-    pl->variant += gemm_variant_name(g1, env.gemm_mode, 148, env.tc_pairs) + "+" + gemm_variant_name(g2, env.gemm_mode, 148, env.tc_pairs) +
-                   (tc_attn ? "+attn-tcgen05-tf32+2bf16+" : "+flash-fp32+") + gemm_variant_name(g3, env.gemm_mode, 148, env.tc_pairs);
+    pl->variant += variant_of(env, s_wq, Mq, Dl, D) + "+" + variant_of(env, s_wkv, Mk, 2 * Dl, D) + (tc_attn ? "+attn-tcgen05-tf32+2bf16+" : "+flash-fp32+") +
+                   variant_of(env, s_wo, Mq, D, Dl);
     return pl;
 }
 

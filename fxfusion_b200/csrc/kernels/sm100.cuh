@@ -3,6 +3,7 @@
 // tcgen05.mma / commit / ld / st, and the TF32 hi/lo split.  Every CTA issues its own plain tile loads.
 #pragma once
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -79,6 +80,40 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar))
                  : "memory");
+}
+
+// true in one lane of a converged warp
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+// Programmatic dependent launch: everything the kernels before this one in the stream wrote is visible after the wait; the
+// launch signal lets the next kernel become resident (its own wait still holds it back until this one has finished).
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---- split form of an fp32 row: two fp16 planes of x * scale, scale a power of two ------------------------------------
+// scale = the power of two that brings `bound` into [2^14, 2^15]; inv = 1 / scale.  Bounds below 2^-99 count as 2^-99.
+__device__ __forceinline__ void split_scale(float bound, float& scale, float& inv) {
+    int e = int(__float_as_uint(bound) >> 23) & 255;   // bound < 2^(e - 126)
+    e = e < 27 ? 27 : e;
+    scale = __int_as_float((268 - e) << 23);
+    inv = __int_as_float((e - 14) << 23);
+}
+__device__ __forceinline__ void split_f16x2(float x, float y, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+__device__ __forceinline__ void split_f16x4(float4 v, float scale, uint2& hi, uint2& lo) {
+    split_f16x2(v.x * scale, v.y * scale, hi.x, lo.x);
+    split_f16x2(v.z * scale, v.w * scale, hi.y, lo.y);
 }
 
 // K-major operand tile whose rows are one swizzle span wide (BK floats = 128 or 64 bytes):
@@ -225,6 +260,38 @@ __device__ __forceinline__ void umma_bf16_ts_pair(uint32_t d_tmem, uint32_t a_tm
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// kind::f16 with fp16 operands, fp32 accumulate, A and B K-major, M x N tile (K = 16 per instruction).
+__host__ __device__ constexpr uint32_t umma_idesc_f16(int m, int n) { return (1u << 4) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24); }
+// kind::f16, both operands from shared memory; PAIR: 256-row tile over the two CTAs of a cluster
+template <bool PAIR>
+__device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    if (PAIR) {
+        umma_bf16_pair(d_tmem, a_desc, b_desc, idesc, accumulate);   // the instruction descriptor names the element type
+    } else {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    }
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar) & kPeerBitMask)
+                 : "memory");
+}
+// ---- tile stores (shared -> global, asynchronous bulk groups of the issuing thread) ----
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* src, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// at most N committed groups may still be reading their source
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // completion of the pair's MMAs arrives on `bar` in both CTAs (same offset in each)
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
     const uint16_t both = 3;

@@ -78,6 +78,26 @@ struct EpilogueFusion {
     bool consumed = false;
 };
 
+// ---- split form (kernels/gemm_f16.cu): an fp32 matrix [rows, K] as two fp16 planes and a power-of-two scale per row, or as
+// one bf16 plane in the bf16 mode -----------------------------------------------------------------------------------------
+struct SplitMat {
+    const uint16_t* planes = nullptr;   // hi plane [rows, K]; the lo plane lies `plane` elements behind it
+    int64_t plane = 0;
+    int64_t ld = 0;                     // elements between rows (0: dense)
+    const float* inv = nullptr;         // 1 / scale per row, `inv_stride` entries apart
+    int64_t inv_stride = 1;
+    const float* amax = nullptr;        // activations: max_k |x[r,k]| as `parts` partial maxima per row
+    int parts = 1;
+    const float* bound = nullptr;       // weights: {max_j ||w_j||_1, max_j |b_j|}
+};
+struct SplitOut {
+    uint16_t* planes = nullptr;
+    int64_t plane = 0;
+    float* inv = nullptr;
+    float* amax = nullptr;
+    int* parts_out = nullptr;           // host: how many partial maxima per row the producer writes
+};
+
 struct ExecCtx {
     cudaStream_t stream = nullptr;
     void* scratch = nullptr;       // shared by all nodes of an engine; nodes run one at a time
@@ -89,6 +109,10 @@ struct ExecCtx {
     int tp_rank = 0, tp_size = 1;  // tensor-parallel position; tp_size > 1 needs `comm`
     void* comm = nullptr;          // fxf_comm* (NCCL communicator wrapper), owned by the caller
     const PeerMap* peers = nullptr;  // set when the ranks' allocations are mapped into each other: all-reduce over peer memory
+    // Tensors in split form, by tensor id (planes == NULL: the plain fp32 tensor), and the form in which the current node has to
+    // leave its output (set by the engine around the node).
+    const std::vector<SplitMat>* splits = nullptr;
+    SplitOut split_out;
     EpilogueFusion fuse;             // set by the engine around a node whose following Add was folded into it
     TpExchange xchg;                 // set by the engine around a sharded node whose exchange absorbs the following Add / LayerNorm
     // workspace of the tensor-core GEMM's K-split last round: partial tiles and their ready flags (zero between
@@ -98,6 +122,8 @@ struct ExecCtx {
     int* gemm_flags = nullptr;
     int gemm_flag_count = 0;
     int tc_chunk_k = 0;            // K-elements per tensor-core accumulation chain (0 = the kernel's default)
+    int f16_variant = -1;          // >= 0: this entry of the f16 GEMM's variant table instead of the modelled choice (experiments)
+    bool weights_settled = false;  // inside an engine after its build: weights were written long before the current kernel chain
     int tc_pair = 0;               // 0: 256-wide tensor-core GEMM tiles are computed by CTA pairs (tcgen05 cta_group::2); 1: never
     // profiling: when `trace` is set every launch appends a record carrying the current tag
     std::vector<LaunchRecord>* trace = nullptr;
@@ -111,6 +137,9 @@ inline void tag_launch(ExecCtx& c, const char* name, double flops, double bytes)
     c.tag_bytes = bytes;
 }
 int trace_after_launch(ExecCtx& ctx);
+inline const SplitMat* split_of(const ExecCtx& ctx, uint32_t id) {
+    return ctx.splits != nullptr && id < ctx.splits->size() && (*ctx.splits)[id].planes != nullptr ? &(*ctx.splits)[id] : nullptr;
+}
 // Called by the op that owns the final GEMM of a node: redirects the output and attaches the residual of a folded Add.
 // `partial`: the node is sharded over the tensor-parallel ranks and its outputs are summed afterwards, so only rank 0 adds
 // the residual (like the bias); a node that is replicated on every rank adds it everywhere.
@@ -127,6 +156,11 @@ int launch_residual_epilogue(float* out, const float* residual, int64_t n, bool 
 
 struct NodePlan {
     virtual ~NodePlan() = default;
+    // split-form activations (struct SplitMat): bit i set = input i is only ever the f16 operand of this node's products; makes_split
+    // = output 0 can be written in split form, as split_rows x split_cols
+    uint32_t takes_split = 0;
+    bool makes_split = false;
+    int64_t split_rows = 0, split_cols = 0;
     size_t scratch_bytes = 0;   // shared scratch wanted at execute time
     size_t persist_bytes = 0;   // memory that must survive across runs (e.g. re-laid-out weights)
     void* persist = nullptr;    // assigned by the engine before prepare()
@@ -306,6 +340,49 @@ int launch_split_mixed(const float* w, float* hi, void* lo_bf16, int64_t n, Exec
 int simt_tile_choice(int64_t M, int64_t N, int sm_count);
 std::string gemm_variant_name(const GemmArgs& a, int gemm_mode, int sm_count, bool pairs = true);
 
+struct F16GemmArgs {
+    SplitMat x, w;
+    bool bf16 = false;
+    const float* bias = nullptr;
+    const float* residual = nullptr;
+    float* out = nullptr;               // fp32 result, or
+    SplitOut split_out;                 // the result in split form (pitch N)
+    int64_t M = 0, N = 0, K = 0, ldo = 0;
+    bool relu = false, conv_chain = false;
+    float* vt_out = nullptr;            // as GemmArgs::vt_*
+    unsigned char* vt_flags = nullptr;
+    int64_t vt_col0 = 0;
+    int vt_T = 0, vt_heads = 0, vt_n32 = 0;
+};
+bool gemm_f16_shape_ok(int64_t M, int64_t N, int64_t K);
+bool gemm_f16_vt_ok(const F16GemmArgs& a, const ExecCtx& ctx);
+int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx);
+std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, int sm_count);
+int gemm_f16_split_parts(int64_t N);    // partial maxima per row a split output of N columns needs room for
+int launch_split_rows(const float* x, int64_t ld, int64_t M, int64_t K, bool bf16, const SplitOut& out, float* bound, ExecCtx& ctx);
+int launch_bias_bound(const float* bias, int64_t n, float* bound, ExecCtx& ctx);
+
+// Launch as a programmatic dependent of the kernel before it in the stream (the kernel calls griddepcontrol.wait before it
+// touches anything another kernel of the stream writes or reads).
+template <class... KArgs, class... Args>
+inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = unsigned(cluster);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
 // Convolution (stride 1 or 2) as an implicit GEMM on the tensor cores: channels-last activation x [N,H,W,C], weights
 // repacked to [O, KH*KW*C] (tap-major, channel-minor) and split into TF32 hi/lo, channels-last output [N,HO,WO,O].
 struct ConvTcArgs {
@@ -322,7 +399,8 @@ struct ConvTcArgs {
 bool conv_tc_shape_ok(int64_t n_pix, int C, int O);
 // The Linear of a planned node applied to M rows that start at x_rows and lie ldx floats apart; row m of the result
 // goes to out + m * ldo (+ the column offset of this rank's block when the node's output columns are sharded).
-int linear_on_rows(const NodePlan* plan, const float* x_rows, int64_t M, int64_t ldx, float* out, int64_t ldo, ExecCtx& ctx);
+// split_rows: the same rows in split form where the tensor is kept so (x_rows is then not read).
+int linear_on_rows(const NodePlan* plan, const float* x_rows, const SplitMat* split_rows, int64_t M, int64_t ldx, float* out, int64_t ldo, ExecCtx& ctx);
 int launch_conv_tc(const ConvTcArgs& a, ExecCtx& ctx);
 // w_oihw [O,C,KH,KW] -> TF32 hi/lo halves laid out [O,KH,KW,C]
 int launch_convert_bf16(const float* w, void* out_bf16, int64_t n, ExecCtx& ctx);

@@ -1,0 +1,103 @@
+"""The f16 GEMM (kernels/gemm_f16.cu) and the split form of its operands: every tile variant at its edges, rows of any scale,
+and activations that stay in split form between the nodes of an engine."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import compare_outputs
+from fxfusion_b200 import lowering, wire
+from oracle.graph_oracle import GraphOracle
+
+pytestmark = pytest.mark.gpu
+ATOL, RTOL = 1e-4, 1e-3
+
+
+def _engine(builder, tmp_path, **kw):
+    from fxfusion_b200.engine import ExecutionEngine
+    graph = builder.finish()
+    path = tmp_path / f"{graph.name}.bin"
+    wire.dump(graph, path)
+    return graph, ExecutionEngine(str(path), "cuda:0", **kw)
+
+
+def _w(rng, n, k):
+    return (rng.standard_normal((n, k), dtype=np.float32) / math.sqrt(k)).astype(np.float32)
+
+
+# one shape per tile variant and then its edges: one row / column past a tile, K past a 64-deep slab, K-split last rounds,
+# outputs without 16-byte rows, a single column
+@pytest.mark.parametrize("M,N,K,variant", [
+    (8192, 2304, 768, "256x"), (8192, 768, 3072, "256x"), (985, 768, 768, "256x64-pair"), (16384, 512, 512, "256x128-pair"), (8192, 3072, 768, "256x192-pair"),
+    (64, 512, 512, "128x32"), (512, 1000, 256, "128x32"), (129, 33, 72, "128x"), (257, 129, 1096, ""), (300, 10, 512, "128x32"), (985, 1111, 264, ""), (64, 1, 16, ""), (513, 50257, 40, "")])
+def test_every_variant_at_its_edges(built_lib, tmp_path, M, N, K, variant):
+    rng = np.random.default_rng(M + N + K)
+    b = lowering.GraphBuilder(f"f16_{M}_{N}_{K}")
+    x = b.input((M, K), wire.DT_F32)
+    b.output(b.op("LinearRelu", [x, b.const(_w(rng, N, K)), b.const(rng.standard_normal(N, dtype=np.float32))], (M, N)))
+    graph, eng = _engine(b, tmp_path)
+    assert "split operands: tcgen05-f16x3-" + variant in eng.describe(), eng.describe()
+    xin = torch.randn(M, K, generator=torch.Generator().manual_seed(1))
+    ok, info = compare_outputs(eng.run([xin.cuda()])[0].cpu(), GraphOracle(graph).run([xin])[0], atol=ATOL, rtol=RTOL)
+    assert ok, info
+    assert eng.device_status() == 0
+    eng.close()
+
+
+def test_rows_keep_their_precision_at_any_scale(built_lib, tmp_path):
+    """Every row carries its own power-of-two scale: rows of 1e-30 and of 1e30 come out as accurately as rows of 1, weight
+    rows likewise, a row of zeros gives the bias, and elements 2^-16 of their row's maximum
+    keep their own precision."""
+    M, N, K = 130, 72, 200
+    rng = np.random.default_rng(7)
+    w = _w(rng, N, K) * (10.0 ** rng.integers(-6, 6, size=(N, 1))).astype(np.float32)
+    w[:, 0] = 0.0
+    b = lowering.GraphBuilder("f16_scales")
+    x = b.input((M, K), wire.DT_F32)
+    b.output(b.op("Linear", [x, b.const(w), b.const(np.zeros(N, np.float32))], (M, N)))
+    _, eng = _engine(b, tmp_path)
+    xin = torch.randn(M, K, generator=torch.Generator().manual_seed(2)) * 10.0 ** torch.linspace(-30, 30, M).unsqueeze(1)
+    xin[5] = 0.0
+    xin[6] *= 2.0 ** -16 / xin[6].abs().max()
+    xin[6, 0] = 1.0        # meets a zero weight: it sets the row's scale and nothing else
+    w64 = torch.from_numpy(w).double()
+    want = xin.double() @ w64.T
+    scale = xin.double().abs() @ w64.abs().T
+    got = eng.run([xin.cuda()])[0].cpu().double()
+    assert torch.equal(got[5], torch.zeros(N, dtype=torch.float64))
+    ok = scale > 0
+    assert ((got - want).abs()[ok] / scale[ok]).max().item() < 2e-6
+    eng.close()
+
+
+@pytest.mark.parametrize("M,D,F", [(64, 64, 256), (200, 768, 3072), (333, 136, 72)])
+@pytest.mark.parametrize("precision", ["auto", "bf16"])
+def test_activations_stay_in_split_form_between_nodes(built_lib, tmp_path, M, D, F, precision):
+    """LayerNorm -> FeedForward and LinearRelu -> LinearRelu -> Linear: the activation between two products is written in
+    split form by its producer; one that anything else reads (the second LayerNorm's residual) stays fp32."""
+    rng = np.random.default_rng(M)
+    b = lowering.GraphBuilder(f"f16_chain_{M}_{D}")
+    c = lambda n, k: (b.const(_w(rng, n, k)), b.const(rng.standard_normal(n, dtype=np.float32)))
+    x = b.input((M, D), wire.DT_F32)
+    ln = b.op("LayerNorm", [x, b.const(rng.standard_normal(D, dtype=np.float32)), b.const(rng.standard_normal(D, dtype=np.float32))], (M, D), ints=[1, D], floats=[1e-5])
+    ff = b.op("FeedForward", [ln, *c(F, D), *c(D, F)], (M, D))
+    add = b.op("Add", [x, ff], (M, D))
+    ln2 = b.op("LayerNorm", [add, b.const(np.ones(D, np.float32)), b.const(np.zeros(D, np.float32))], (M, D), ints=[1, D], floats=[1e-5])
+    h1 = b.op("LinearRelu", [ln2, *c(F, D)], (M, F))
+    h2 = b.op("LinearRelu", [h1, *c(D, F)], (M, D))
+    both = b.op("Add", [h2, ln2], (M, D))
+    b.output(b.op("Linear", [both, *c(40, D)], (M, 40)))
+    graph, eng = _engine(b, tmp_path, precision=precision)
+    text = eng.describe().splitlines()
+    split = [("output in split form" in t) for t in text if t.split()[1:2] and t.split()[1] in ("LayerNorm", "LinearRelu")]
+    assert split == [True, False, True, False], "\n".join(text)
+    xin = torch.randn(M, D, generator=torch.Generator().manual_seed(3))
+    got, want = eng.run([xin.cuda()])[0].cpu(), GraphOracle(graph).run([xin])[0]
+    if precision == "auto":
+        ok, info = compare_outputs(got, want, atol=ATOL * 5, rtol=RTOL)
+        assert ok, info
+    else:
+        assert ((got - want).abs().max() / want.abs().max()).item() < 2e-2
+    assert eng.device_status() == 0
+    eng.close()
