@@ -641,7 +641,7 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             if ((B.op != FXF_OP_ADD && B.op != FXF_OP_ADD_RELU) || B.in.size() != 2 || B.out.size() != 1 || B.folded || A.xchg) continue;
             // Convolutions are left alone: their layers are bandwidth-bound with short K loops, and the residual read in the
             // GEMM epilogue (16 KB in flight per SM) is slower than the separate AddRelu kernel (measured on ResNet-50).
-            if (A.op != FXF_OP_LINEAR && A.op != FXF_OP_FEEDFORWARD && A.op != FXF_OP_MHA && A.op != FXF_OP_CROSS_MHA) continue;
+            if (A.op != FXF_OP_LINEAR && A.op != FXF_OP_FEEDFORWARD && A.op != FXF_OP_MHA && A.op != FXF_OP_CROSS_MHA && A.op != FXF_OP_CACHED_MHA) continue;
             if (A.fuse_out >= 0 || A.out.size() != 1) continue;
             if (B.op == FXF_OP_ADD_RELU && A.plan->tp_sharded) continue;   // the ReLU would have to follow the all-reduce
             if (A.op == FXF_OP_LINEAR && e->opts.tp_size > 1 && e->opts.tp_shard_output) continue;

@@ -85,6 +85,10 @@ struct F16Params {
     int full_tiles, tail_tiles, tail_split;   // tiles of the last round are cut along K into tail_split parts
     int chunk_slabs;
     int early_w;                  // weight tiles may be requested before the previous kernel has finished
+    // Few rows against a large weight: the operands change places (map_x covers the weight, map_w the rows of x, BN = 32 or 64 of
+    // them) so that the weight streams through full 128-row tiles; out[column * ldo + row], bias per row, scales as named.
+    int swap;
+    int64_t w_inv_stride;
     float* ws;
     int* flags;
     int* status;
@@ -205,14 +209,13 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 if (PAIR) tma_load_3d_pair(s.a[st], &map_x, k * BK, tm * BM, 0, &s.full[st]);
                 else tma_load_3d(s.a[st], &map_x, k * BK, tm * BM, 0, &s.full[st]);
             };
-            auto load_w = [&](int st, int k, int tn) {   // also announces the bytes of the whole stage (of both CTAs: the leader's barrier)
-                if (PAIR) {
-                    if (rank == 0) mbar_expect_tx(&s.full[st], 2 * (kABytes + kBBytes));
-                    tma_load_3d_pair(s.b[st], &map_w, k * BK, tn * BN + rank * BNB, 0, &s.full[st]);
-                } else {
-                    mbar_expect_tx(&s.full[st], kABytes + kBBytes);
-                    tma_load_3d(s.b[st], &map_w, k * BK, tn * BN, 0, &s.full[st]);
-                }
+            auto load_w = [&](int st, int k, int tn) {
+                if (PAIR) tma_load_3d_pair(s.b[st], &map_w, k * BK, tn * BN + rank * BNB, 0, &s.full[st]);
+                else tma_load_3d(s.b[st], &map_w, k * BK, tn * BN, 0, &s.full[st]);
+            };
+            auto announce = [&](int st) {   // the bytes of the whole stage (of both CTAs: the leader's barrier)
+                if (!PAIR) mbar_expect_tx(&s.full[st], kABytes + kBBytes);
+                else if (rank == 0) mbar_expect_tx(&s.full[st], 2 * (kABytes + kBBytes));
             };
             uint32_t it = 0;
             bool first = true;
@@ -225,9 +228,16 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 if (first) {   // the ring is empty: fill it without waiting, the weights ahead of the previous kernel's end
                     const int pre = min(STAGES, un.k1 - un.k0);
                     if (!p.early_w) grid_dep_wait();
-                    for (int i = 0; i < pre; i++) load_w(i, un.k0 + i, tn);
+                    for (int i = 0; i < pre; i++) {
+                        announce(i);
+                        if (p.swap) load_x(i, un.k0 + i, tm);
+                        else load_w(i, un.k0 + i, tn);
+                    }
                     if (p.early_w) grid_dep_wait();
-                    for (int i = 0; i < pre; i++) load_x(i, un.k0 + i, tm);
+                    for (int i = 0; i < pre; i++) {
+                        if (p.swap) load_w(i, un.k0 + i, tn);
+                        else load_x(i, un.k0 + i, tm);
+                    }
                     k += pre;
                     it += pre;
                     first = false;
@@ -238,6 +248,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                         give_up(abort_flag, p.status, kErrWaitEmpty);
                         goto producer_done;
                     }
+                    announce(st);
                     load_w(st, k, tn);
                     load_x(st, k, tm);
                 }
@@ -327,6 +338,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             const int64_t col_base = int64_t(tn) * BN + chalf * HALF;
             // constants of the row and of the columns, fetched while the tensor core works
             const float ri = (row_ok && p.x_inv != nullptr) ? __ldg(p.x_inv + grow * p.x_inv_stride) : 1.f;
+            const float row_bias = (p.swap && row_ok && p.bias != nullptr) ? __ldg(p.bias + grow) : 0.f;
             float rscale = 1.f, rmax = 0.f;
             if (NPL == 2 && p.so != nullptr && !writes_partial && row_ok) {
                 float am = 0.f, inv;
@@ -337,8 +349,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             __syncwarp();
             for (int j = lane; j < HALF; j += 32) {
                 const int64_t c = col_base + j;
-                cinv[j] = (p.w_inv && c < p.N) ? __ldg(p.w_inv + c) : 1.f;
-                cbias[j] = (p.bias && c < p.N) ? __ldg(p.bias + c) : 0.f;
+                cinv[j] = (p.w_inv && c < p.N) ? __ldg(p.w_inv + c * p.w_inv_stride) : 1.f;
+                cbias[j] = (p.bias && !p.swap && c < p.N) ? __ldg(p.bias + c) : 0.f;
             }
             __syncwarp();
             float sum[HALF];
@@ -417,6 +429,17 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     // both factors are powers of two; the weight's goes first: the product of the two may leave the range of fp32
                     v[j] = fmaf(v[j] * ci.x, ri, cb.x); v[j + 1] = fmaf(v[j + 1] * ci.y, ri, cb.y);
                     v[j + 2] = fmaf(v[j + 2] * ci.z, ri, cb.z); v[j + 3] = fmaf(v[j + 3] * ci.w, ri, cb.w);
+                }
+                if (p.swap) {   // the 32 lanes write 32 consecutive columns of the result
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        if (row_ok && col + j < p.N) {
+                            const int64_t off = (col + j) * p.ldo + grow;
+                            float t = v[j] + row_bias;
+                            if (p.residual != nullptr) t += p.residual[off];
+                            p.out[off] = p.relu ? relu_keep_nan(t) : t;
+                        }
+                    continue;
                 }
                 if (transposes) {
                     // V third of a packed QKV projection, transposed per head: the 32 lanes write 32 consecutive keys of a V^T row
@@ -668,7 +691,7 @@ int make_out_map(CUtensorMap* map, const F16GemmArgs& a, int planes) {
     return 0;
 }
 
-constexpr int kChunkKDense = 1024, kChunkKConv = 64;
+constexpr int kChunkKDense = 1024, kChunkKConv = 64, kChunkKRows = 256;
 
 // Times in microseconds as measured on B200 inside a chain of launches: `slab` per 64-deep K-slab of a tile, `gap` what every
 // tile adds (its epilogue runs under the next tile's products), `drain` the exposed epilogue of the last one.
@@ -697,7 +720,7 @@ int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int w
     constexpr int BNB = PAIR ? BN / 2 : BN;
     CUtensorMap mx, mw, mo;
     if (make_map(&mx, a.x.planes, a.M, a.K, a.x.ld ? a.x.ld : a.K, a.x.plane, NPL, BM)) return 1;
-    if (make_map(&mw, a.w.planes, a.N, a.K, a.K, a.w.plane, NPL, BNB)) return 1;
+    if (make_map(&mw, a.w.planes, a.N, a.K, a.w.ld ? a.w.ld : a.K, a.w.plane, NPL, BNB)) return 1;
     mo = mx;
     if (p.tma_out && make_out_map(&mo, a, NPL)) return 1;
     const size_t smem = sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL)>) + 1024;
@@ -797,6 +820,7 @@ int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx) {
     p.bias = a.bias; p.residual = a.residual; p.out = a.out;
     p.x_inv = a.bf16 ? nullptr : a.x.inv; p.w_inv = a.bf16 ? nullptr : a.w.inv;
     p.x_inv_stride = a.x.inv_stride;
+    p.w_inv_stride = 1;
     p.M = a.M; p.N = a.N; p.K = a.K; p.ldo = split ? a.N : a.ldo;
     p.relu = a.relu ? 1 : 0;
     p.tma_out = (split || (a.ldo % 4 == 0 && aligned16(a.out) && (a.residual == nullptr || aligned16(a.residual)))) ? 1 : 0;
@@ -843,6 +867,32 @@ int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx) {
         case 5: return launch_variant<64, 4, false, 2>(a, p, ts, workers, ctx);
         default: return launch_variant<32, 4, false, 2>(a, p, ts, workers, ctx);
     }
+}
+
+// out[M,N] for M <= 64 rows in split form and a weight of at least a tile per SM (see F16Params::swap).  The persistent kernel
+// keeps its weight stream going across tiles: 32 x 50257 x 768 (154 MB) in 31 us = 4.9 TB/s.
+int launch_gemm_f16_swapped(const F16GemmArgs& a, ExecCtx& ctx) {
+    FXF_CHECK(a.M >= 1 && a.M <= 64 && gemm_f16_shape_ok(a.M, a.N, a.K) && !a.bf16 && a.x.planes && a.w.planes && a.out && a.split_out.planes == nullptr && a.vt_out == nullptr,
+              "f16 GEMM (swapped): unsupported operands");
+    F16GemmArgs t = a;
+    t.x = a.w; t.w = a.x;
+    t.M = a.N; t.N = a.M;
+    F16Params p{};
+    p.swap = 1;
+    p.bias = a.bias; p.residual = a.residual; p.out = a.out;
+    p.x_inv = a.w.inv; p.x_inv_stride = 1; p.w_inv = a.x.inv; p.w_inv_stride = a.x.inv_stride;
+    p.M = t.M; p.N = t.N; p.K = t.K; p.ldo = a.ldo;
+    p.relu = a.relu ? 1 : 0;
+    p.tiles_m = int((t.M + BM - 1) / BM);
+    p.tiles_n = 1;
+    p.full_tiles = p.tiles_m; p.tail_split = 1;
+    p.chunk_slabs = kChunkKRows / BK;
+    p.early_w = ctx.weights_settled ? 1 : 0;
+    p.status = ctx.status;
+    tag_launch(ctx, "gemm_f16x3_swapped_tcgen05", 2.0 * double(a.M) * double(a.N) * double(a.K),
+               4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.N) + double(a.M) * a.N));
+    const TailSplit ts{p.tiles_m, 0, 1, 0.0};
+    return a.M <= 32 ? launch_variant<32, 4, false, 2>(t, p, ts, ctx.sm_count, ctx) : launch_variant<64, 4, false, 2>(t, p, ts, ctx.sm_count, ctx);
 }
 
 }  // namespace fxf

@@ -1,0 +1,363 @@
+// Few-row GEMM for sm_100a:  out[M,N] = act(x[M,K] · w[N,K]^T + bias[N] (+ residual)),  M <= 64, on the tensor cores with the
+// f16x3 arithmetic of gemm_f16.cu (weights in the same split form; see there).
+//
+// These products are weight reads: single-position decode steps, batch-sized MLP layers, the last-row vocabulary projection.
+// The operands are swapped — a tile is 128 WEIGHT rows by all rows of x — so no tensor time goes into padding rows, and one
+// tile's K range is cut over a cluster of up to 8 CTAs, so that a 512-row weight already occupies 32 SMs.  Per CTA:
+//   * weight slabs (128 rows x 64, both planes, 32 KB) by TMA.  They do not depend on the kernel before this one, so the first
+//     STAGES slabs are requested before griddepcontrol.wait: the weight stream runs under the previous kernel;
+//   * x comes as fp32 (or in split form): all warps fetch this CTA's K range of the rows, take the maximum of each row over
+//     it, and write the two fp16 planes into swizzled shared memory.  The scale may differ between the CTAs of a cluster:
+//     their results are only added after it has been divided out;
+//   * MMAs of 128 x NB x 16; 64- to 128-deep chains in separate TMEM accumulators, added in fp32 registers;
+//   * every CTA owns a share of the tile: the others push their partial sums of it into its shared memory (one bulk copy each,
+//     counted on the owner's mbarrier), it adds them in rank order, applies scale, bias, residual and ReLU and stores rows of
+//     consecutive columns.  Pulling the partial tiles after a cluster barrier instead, with another barrier before the exit,
+//     cost 4000 to 7000 cycles of 9000 to 12000.
+// Bound: HBM (4 bytes per weight element) for the large weights, launch-to-launch latency for the small ones.
+#include <cuda.h>
+
+#include <algorithm>
+
+#include "../runtime.hpp"
+#include "sm100.cuh"
+
+namespace fxf {
+namespace {
+
+using namespace sm100;
+
+constexpr int BN = 128, BK = 64, kThreads = 256, kWarps = kThreads / 32;
+constexpr int kTmaWarp = 7, kMmaWarp = 6, kAccCols = 128, kMaxCluster = 16;   // TMEM columns per CTA
+enum : int { kErrRowsFull = 141, kErrRowsEmpty = 142, kErrRowsDone = 143, kErrRowsReduce = 144 };
+
+template <int NB, int STAGES, int XS>
+struct alignas(1024) RowsSmem {
+    uint16_t w[STAGES][2][BN * BK];   // [0] is reused for the partial tile [NB][128] once the products are done
+    uint16_t x[XS][2][NB * BK];
+    float recv[NB * BN + 64];         // [rank][share of the tile]: the cluster's partial sums of the elements this CTA owns
+    float x_inv[NB];
+    uint64_t full[STAGES], empty[STAGES], done, received;
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+struct RowsParams {
+    const float* x;               // [M] rows of K floats, ldx apart, or NULL:
+    const uint16_t* x_planes;     // the rows in split form, ld_planes elements apart, 1 / scale x_inv_stride entries apart
+    int64_t x_plane, ld_planes, x_inv_stride;
+    const float* x_inv;
+    int64_t ldx;
+    const float *w_inv, *bias, *residual;
+    float* out;
+    int M, N, K, slabs;
+    int64_t ldo;
+    int relu, early_w;
+    int* status;
+};
+
+__device__ __forceinline__ float relu_keep_nan(float v) { return v > 0.f ? v : (v != v ? v : 0.f); }
+__device__ __forceinline__ uint32_t cluster_nctarank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+// `bytes` (a multiple of 16) of this CTA's shared memory to the same-named location of CTA `rank`, counted on its barrier
+__device__ __forceinline__ void push_bulk(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar, uint32_t rank) {
+    uint32_t d, b;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(dst), "r"(rank));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(bar), "r"(rank));
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d), "r"(src), "r"(bytes), "r"(b) : "memory");
+}
+
+template <int NB, int STAGES, int XS>
+__global__ void __launch_bounds__(kThreads, STAGES <= 2 ? 2 : 1)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, RowsParams p) {
+    extern __shared__ unsigned char smem_raw[];
+    using Smem = RowsSmem<NB, STAGES, XS>;
+    Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    constexpr uint32_t kWBytes = 2 * BN * BK * 2;
+    constexpr uint32_t kIdesc = umma_idesc_f16(BN, NB);
+    constexpr int NACC = kAccCols / NB, COLS = NB >= 32 ? NB / 2 : NB, EPI_WARPS = NB >= 32 ? 8 : 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cs = int(cluster_nctarank()), rank = int(cluster_ctarank());
+    const int tile = blockIdx.x / cs, n0 = tile * BN;
+    const int m0 = blockIdx.y * NB, rows = min(NB, p.M - m0);   // this CTA's rows of x
+    const int s0 = int(int64_t(p.slabs) * rank / cs), s1 = int(int64_t(p.slabs) * (rank + 1) / cs), count = s1 - s0;
+    volatile int* abort_flag = &s.abort_flag;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < STAGES; i++) {
+            mbar_init(&s.full[i], 1);
+            mbar_init(&s.empty[i], 1);
+        }
+        mbar_init(&s.done, 1);
+        mbar_init(&s.received, 1);
+        s.abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem_base)), "r"(kAccCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // shares of the tile's M * 128 elements, a multiple of 16 bytes each
+    const int total = rows * BN, share = ((total + cs - 1) / cs + 3) & ~3, own0 = min(rank * share, total), own_n = min(share, total - own0);
+    if (threadIdx.x == 0 && cs > 1) mbar_expect_tx(&s.received, uint32_t(cs) * uint32_t(own_n) * 4u);
+    tc_fence_before();
+    __syncthreads();
+    if (cs > 1) cluster_sync_all();   // the peers' barriers exist (this runs under the previous kernel)
+    tc_fence_after();
+    const uint32_t tmem = s.tmem_base;
+    grid_dep_launch();
+
+    auto load_w = [&](int i) {   // slab i of this CTA
+        const int st = i % STAGES;
+        mbar_expect_tx(&s.full[st], kWBytes);
+        tma_load_3d(s.w[st], &map_w, (s0 + i) * BK, n0, 0, &s.full[st]);
+    };
+    const bool producer = warp == kTmaWarp && lane == 0;
+    int loaded = 0;   // producer: slabs requested so far
+    if (producer && p.early_w)
+        for (; loaded < min(STAGES, count); loaded++) load_w(loaded);
+    // constants of this thread's output column (shares start at multiples of 4 elements, not of 128)
+    const int nt = (own0 + threadIdx.x) & (BN - 1);
+    const bool n_ok = n0 + nt < p.N;
+    const float wi = n_ok ? __ldg(p.w_inv + n0 + nt) : 0.f, bi = (n_ok && p.bias) ? __ldg(p.bias + n0 + nt) : 0.f;
+    grid_dep_wait();
+    if (producer && !p.early_w)
+        for (; loaded < min(STAGES, count); loaded++) load_w(loaded);
+
+    float sum[COLS];
+#pragma unroll
+    for (int j = 0; j < COLS; j++) sum[j] = 0.f;
+    const int quarter = warp & 3, mbase = NB >= 32 ? (warp >> 2) * COLS : 0;
+    bool alive = true;
+    int round = 0;
+    for (int r0 = 0; r0 < count && alive; r0 += XS, round++) {
+        const int ns = min(XS, count - r0), kb = (s0 + r0) * BK;
+        // ---- this round's K range of the rows: fp32 -> two fp16 planes under one scale per row ----
+        constexpr int V = (XS + 1) / 2, ROWS = NB / kWarps;   // float4 per lane and row (128 floats = two slabs each), rows per warp
+        float4 v[ROWS][V];                                    // every row's loads are in flight before the first maximum
+#pragma unroll
+        for (int q = 0; q < ROWS; q++)
+#pragma unroll
+            for (int i = 0; i < V; i++) {
+                const int r = q * kWarps + warp, at = i * 128 + lane * 4, k = kb + at;
+                v[q][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r < rows && at < ns * BK && k < p.K) {
+                    if (p.x != nullptr) {
+                        v[q][i] = *reinterpret_cast<const float4*>(p.x + (m0 + r) * p.ldx + k);
+                    } else {
+                        const uint2 h = *reinterpret_cast<const uint2*>(p.x_planes + (m0 + r) * p.ld_planes + k), l = *reinterpret_cast<const uint2*>(p.x_planes + p.x_plane + (m0 + r) * p.ld_planes + k);
+                        const float inv = __ldg(p.x_inv + (m0 + r) * p.x_inv_stride);
+                        const float2 h0 = __half22float2(*reinterpret_cast<const __half2*>(&h.x)), h1 = __half22float2(*reinterpret_cast<const __half2*>(&h.y));
+                        const float2 l0 = __half22float2(*reinterpret_cast<const __half2*>(&l.x)), l1 = __half22float2(*reinterpret_cast<const __half2*>(&l.y));
+                        v[q][i] = make_float4((h0.x + l0.x) * inv, (h0.y + l0.y) * inv, (h1.x + l1.x) * inv, (h1.y + l1.y) * inv);
+                    }
+                }
+            }
+#pragma unroll
+        for (int q = 0; q < ROWS; q++) {
+            const int r = q * kWarps + warp;
+            float m = 0.f;
+#pragma unroll
+            for (int i = 0; i < V; i++) m = fmaxf(m, fmaxf(fmaxf(fabsf(v[q][i].x), fabsf(v[q][i].y)), fmaxf(fabsf(v[q][i].z), fabsf(v[q][i].w))));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            float scale, inv;
+            split_scale(m, scale, inv);
+            if (lane == 0) s.x_inv[r] = inv;
+#pragma unroll
+            for (int i = 0; i < V; i++) {
+                const int sl = i * 2 + (lane >> 4);
+                uint2 hi, lo;
+                split_f16x4(v[q][i], scale, hi, lo);
+                char* dst = reinterpret_cast<char*>(s.x[sl][0]) + r * 128 + ((((lane & 15) >> 1) ^ (r & 7)) << 4) + ((lane & 1) << 3);
+                *reinterpret_cast<uint2*>(dst) = hi;
+                *reinterpret_cast<uint2*>(dst + NB * BK * 2) = lo;
+            }
+        }
+        fence_async_smem();
+        __syncthreads();
+        if (warp == kMmaWarp) {
+            const uint32_t leader = elect_one();
+            for (int i = 0; i < ns; i++) {
+                const int g = r0 + i, st = g % STAGES;
+                if (!(__all_sync(0xffffffffu, mbar_wait(&s.full[st], (g / STAGES) & 1, abort_flag)))) {
+                    give_up(abort_flag, p.status, kErrRowsFull);
+                    break;
+                }
+                tc_fence_after();
+                if (leader) {
+                    const uint64_t a = umma_desc_k_major_bytes<128>(smem_u32(s.w[st][0])), b = umma_desc_k_major_bytes<128>(smem_u32(s.x[i][0]));
+                    constexpr uint64_t kALo = BN * BK * 2 / 16, kBLo = NB * BK * 2 / 16;
+                    const uint32_t acc = tmem + uint32_t(i % NACC) * NB;
+#pragma unroll
+                    for (int kk = 0; kk < BK / 16; kk++) {
+                        const uint64_t adv = uint64_t((kk * 32) >> 4);
+                        umma_f16_ss<false>(acc, a + kALo + adv, b + adv, kIdesc, (i >= NACC || kk > 0) ? 1u : 0u);
+                        umma_f16_ss<false>(acc, a + adv, b + kBLo + adv, kIdesc, 1u);
+                        umma_f16_ss<false>(acc, a + adv, b + adv, kIdesc, 1u);
+                    }
+                    umma_commit(&s.empty[st]);
+                    if (i + 1 == ns) umma_commit(&s.done);
+                }
+            }
+        }
+        if (producer) {   // the ring is refilled while the products run (the next round's slabs included)
+            for (; loaded < min(count, r0 + ns + STAGES); loaded++) {
+                if (!mbar_wait(&s.empty[loaded % STAGES], ((loaded / STAGES) - 1) & 1, abort_flag)) {
+                    give_up(abort_flag, p.status, kErrRowsEmpty);
+                    break;
+                }
+                load_w(loaded);
+            }
+        }
+        __syncwarp();
+        alive = __all_sync(0xffffffffu, mbar_wait(&s.done, round & 1, abort_flag));
+        if (!alive) give_up(abort_flag, p.status, kErrRowsDone);
+        tc_fence_after();
+        if (alive && warp < EPI_WARPS) {
+            const int nacc = min(ns, NACC);
+            for (int a = 0; a < nacc; a++) {
+                const uint32_t t = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(a * NB + mbase);
+                uint32_t d[COLS];
+                tmem_ld(t, d);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < COLS; j++) sum[j] = fmaf(__uint_as_float(d[j]), s.x_inv[mbase + j], sum[j]);
+            }
+        }
+        tc_fence_before();
+        alive = __syncthreads_and(alive ? 1 : 0) != 0;   // the x planes, scales and accumulators may be reused
+    }
+
+    // ---- partial tile to shared memory, then the sum over the cluster ----
+    float* part = reinterpret_cast<float*>(s.w[0]);
+    if (warp < EPI_WARPS) {
+#pragma unroll
+        for (int j = 0; j < COLS; j++) part[(mbase + j) * BN + quarter * 32 + lane] = sum[j];
+    }
+    if (cs > 1) fence_async_smem();
+    __syncthreads();
+    const float* mine = part + own0;
+    if (cs > 1) {
+        if (warp == 0) {
+            if (lane < cs) {
+                const int q0 = min(lane * share, total), qn = min(share, total - q0);
+                if (qn > 0) push_bulk(smem_u32(s.recv) + uint32_t(rank * qn) * 4u, smem_u32(part + q0), uint32_t(qn) * 4u, smem_u32(&s.received), uint32_t(lane));
+            }
+            __syncwarp();
+        }
+        if (!mbar_wait(&s.received, 0, abort_flag)) {
+            give_up(abort_flag, p.status, kErrRowsReduce);
+            alive = false;
+        }
+        mine = s.recv;
+        // All this CTA was sent has arrived.  Once that holds for the whole cluster everyone may leave: nothing that was pushed
+        // is still being read.  Arriving here (relaxed: no memory has to be ordered) takes the wait below off the path.
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    }
+    for (int i = threadIdx.x; alive && i < own_n; i += kThreads) {
+        float t[kMaxCluster], v = 0.f;
+#pragma unroll
+        for (int q = 0; q < kMaxCluster; q++) t[q] = q < cs ? mine[q * own_n + i] : 0.f;
+#pragma unroll
+        for (int q = 0; q < kMaxCluster; q++) v += t[q];
+        if (n_ok) {
+            const int64_t off = int64_t(m0 + ((own0 + i) >> 7)) * p.ldo + n0 + nt;
+            v = fmaf(v, wi, bi);
+            if (p.residual != nullptr) v += p.residual[off];
+            p.out[off] = p.relu ? relu_keep_nan(v) : v;
+        }
+    }
+    tc_fence_before();
+    if (cs > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kAccCols) : "memory");
+    }
+}
+
+int make_weight_map(CUtensorMap* map, const SplitMat& w, int64_t rows, int64_t cols) {
+    using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                       const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static EncodeTiledFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            return reinterpret_cast<EncodeTiledFn>(p);
+        return EncodeTiledFn(nullptr);
+    }();
+    FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
+    cuuint64_t dims[3] = {cuuint64_t(cols), cuuint64_t(rows), 2};
+    cuuint64_t strides[2] = {cuuint64_t(cols) * 2, cuuint64_t(w.plane) * 2};
+    cuuint32_t box[3] = {BK, BN, 2};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<uint16_t*>(w.planes), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    FXF_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (rows) failed with code %d", int(r));
+    return 0;
+}
+
+template <int NB, int STAGES, int XS>
+int launch_rows(const CUtensorMap& map, const RowsParams& p, int tiles, int cs, ExecCtx& ctx) {
+    const size_t smem = sizeof(RowsSmem<NB, STAGES, XS>) + 1024;
+    static_assert(sizeof(RowsSmem<NB, STAGES, XS>) + 1024 <= 227 * 1024, "shared memory of a CTA");
+    auto kernel = gemm_rows_kernel<NB, STAGES, XS>;
+    static bool configured[64] = {};
+    int dev = 0;
+    FXF_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        FXF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        FXF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    FXF_CUDA(launch_dependent(kernel, dim3(unsigned(tiles * cs), unsigned((p.M + NB - 1) / NB)), dim3(kThreads), smem, ctx.stream, cs, map, p));
+    FXF_LAUNCHED(ctx);
+    return 0;
+}
+
+}  // namespace
+
+bool gemm_rows_ok(int64_t M, int64_t N, int64_t K) { return M >= 1 && M <= 64 && gemm_f16_shape_ok(M, N, K); }
+// From a tile per SM on, a persistent kernel that streams its weights without a break between tiles is the better one
+// (launch_gemm_f16_swapped; 32 x 50257 x 768: 46 us here).
+bool gemm_rows_streams(int64_t M, int64_t N, int sm_count) { return M <= 64 && (N + BN - 1) / BN >= sm_count; }
+
+// x: fp32 rows `ldx` floats apart (16-byte aligned), or NULL with a.x in split form.
+int launch_gemm_rows(const F16GemmArgs& a, const float* x, int64_t ldx, ExecCtx& ctx) {
+    if (a.M == 0 || a.N == 0) return 0;
+    FXF_CHECK(gemm_rows_ok(a.M, a.N, a.K) && !a.bf16 && a.w.planes && a.out && (x != nullptr || a.x.planes != nullptr), "few-row GEMM: unsupported operands");
+    FXF_CHECK(x == nullptr || (aligned16(x) && ldx % 4 == 0), "few-row GEMM: unaligned rows");
+    CUtensorMap map;
+    if (make_weight_map(&map, a.w, a.N, a.K)) return 1;
+    RowsParams p{};
+    p.x = x; p.ldx = ldx;
+    if (x == nullptr) {
+        p.x_planes = a.x.planes; p.x_plane = a.x.plane; p.ld_planes = a.x.ld ? a.x.ld : a.K; p.x_inv = a.x.inv; p.x_inv_stride = a.x.inv_stride;
+    }
+    p.w_inv = a.w.inv; p.bias = a.bias; p.residual = a.residual; p.out = a.out;
+    p.M = int(a.M); p.N = int(a.N); p.K = int(a.K); p.ldo = a.ldo;
+    p.slabs = int((a.K + BK - 1) / BK);
+    p.relu = a.relu ? 1 : 0;
+    p.early_w = ctx.weights_settled ? 1 : 0;
+    p.status = ctx.status;
+    const int tiles = int((a.N + BN - 1) / BN);
+    // As many CTAs per tile as leave every SM at most two, up to 8 (a portable cluster); no more than give the fewest slabs.  A
+    // deep product with few tiles goes to clusters of 16 (32 x 768 x 3072: 7.4 -> 6.3 us); with more tiles they no longer find
+    // room beside the kernel before (32 x 3072 x 768: 6.9 -> 10.6 us).
+    int cs = std::max(1, std::min(std::min(8, p.slabs), 2 * ctx.sm_count / tiles));
+    if ((p.slabs + cs - 1) / cs > 2 && tiles * 16 * 3 <= ctx.sm_count * 2) cs = std::min(16, p.slabs);
+    const int per = (p.slabs + cs - 1) / cs;
+    cs = (p.slabs + per - 1) / per;
+    tag_launch(ctx, "gemm_f16x3_rows_tcgen05", 2.0 * double(a.M) * double(a.N) * double(a.K),
+               4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.N) + double(a.M) * a.N));
+    // two slabs per CTA: 70-100 KB of shared memory, so that this kernel's CTAs fit beside those of the kernel before it
+    if (a.M <= 16) return per <= 2 ? launch_rows<16, 2, 2>(map, p, tiles, cs, ctx) : launch_rows<16, 4, 8>(map, p, tiles, cs, ctx);
+    return per <= 2 ? launch_rows<32, 2, 2>(map, p, tiles, cs, ctx) : (per <= 4 ? launch_rows<32, 4, 4>(map, p, tiles, cs, ctx) : launch_rows<32, 4, 8>(map, p, tiles, cs, ctx));
+}
+
+}  // namespace fxf

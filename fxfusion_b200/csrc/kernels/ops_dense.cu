@@ -123,11 +123,11 @@ struct DensePlan : NodePlan {
         x.col0 = 0; x.ncol = cols; x.src_ld = cols;
         return x;
     }
-    void reserve_f16(Slice& x) {   // the whole tensor in split form (f16 products are not sharded)
+    void reserve_f16(Slice& x, bool as_bf16) {   // the whole tensor in split form (f16 products are not sharded)
         x.f16 = true;
-        x.bf16 = bf16_mode;
+        x.bf16 = as_bf16;
         x.off_split = persist_bytes;
-        persist_bytes += round_up(size_t(x.elems()) * (bf16_mode ? 2 : 4), 256) + round_up(size_t(x.rows()) * 4, 256) + 256;
+        persist_bytes += round_up(size_t(x.elems()) * (as_bf16 ? 2 : 4), 256) + round_up(size_t(x.rows()) * 4, 256) + 256;
     }
     void reserve(Slice& x, bool want_split) {
         if (x.drop) return;
@@ -201,24 +201,29 @@ struct DensePlan : NodePlan {
 };
 inline const DensePlan* dense(const NodePlan* p) { return static_cast<const DensePlan*>(p); }
 
-// M < 64 (batch-sized layers, single-position decode steps) never takes the tensor-core path: those problems are weight
-// reads, served by the fp32 FFMA few-rows kernels from the fp32 weights (half the bytes of a hi/lo pair).
+// The old tensor-core path (tensor parallelism, explicit arithmetic modes): M < 64 stays on the fp32 FFMA few-rows kernels there.
 bool want_tc(const PlanEnv& env, int64_t M, int64_t N, int64_t K) { return env.gemm_mode != FXF_GEMM_FP32_SIMT && gemm_tc_shape_ok(M, N, K); }
 
-// The f16 GEMM serves single-GPU engines in the default and the bf16 mode, from 64 rows on (fewer rows: see above).
+// Products in split form: single-GPU engines in the default and the bf16 mode.  Up to 64 rows (batch-sized layers, decode
+// steps) they run on the few-row kernels, in f16x3 whatever the mode; from 65 rows on the bf16 mode takes bf16 operands.
+constexpr int64_t kFewRows = 64;
 bool want_f16(const PlanEnv& env, int64_t M, int64_t N, int64_t K) {
-    if (env.tp_size > 1 || M < 64 || !gemm_f16_shape_ok(M, N, K)) return false;
-    return env.gemm_mode == FXF_GEMM_AUTO || (env.gemm_mode == FXF_GEMM_BF16 && gemm_tc_shape_ok(M, N, K));
+    if (env.tp_size > 1 || !gemm_f16_shape_ok(M, N, K)) return false;
+    return env.gemm_mode == FXF_GEMM_AUTO || (env.gemm_mode == FXF_GEMM_BF16 && (M <= kFewRows || gemm_tc_shape_ok(M, N, K)));
 }
 void reserve_weight(DensePlan& p, Slice& w, const PlanEnv& env, int64_t M, int64_t N, int64_t K) {
-    if (want_f16(env, M, N, K)) p.reserve_f16(w);
+    if (want_f16(env, M, N, K)) p.reserve_f16(w, p.bf16_mode && M > kFewRows);
     else p.reserve(w, want_tc(env, M, N, K));
 }
+// Whether a product wants its activation in split form from the producer: the tiled kernel and the streaming few-row kernel
+// load it so; the cluster kernel of gemm_rows.cu takes fp32 rows and splits its own K range.
+bool takes_split_rows(int64_t M, int64_t N) { return M > kFewRows || gemm_rows_streams(M, N, 148); }
 std::string variant_of(const PlanEnv& env, const Slice& w, int64_t M, int64_t N, int64_t K) {
     GemmArgs g;
     g.M = M; g.N = N; g.K = K;
     std::string v = gemm_variant_name(g, env.gemm_mode, 148, env.tc_pairs);
-    return w.f16 ? v + " (split operands: tcgen05-" + gemm_f16_variant_name(M, N, K, w.bf16, 148) + ")" : v;
+    if (!w.f16) return v;
+    return v + " (split operands: tcgen05-" + (M > kFewRows ? gemm_f16_variant_name(M, N, K, w.bf16, 148) : std::string(takes_split_rows(M, N) ? "f16x3-stream128" : "f16x3-rows128")) + ")";
 }
 
 // Room for an activation matrix that has to be split before its product: planes, scales, row maxima.
@@ -237,20 +242,28 @@ SplitMat as_operand(const SplitOut& o, int parts = 1) {
     m.planes = o.planes; m.plane = o.plane; m.inv = o.inv; m.amax = o.amax; m.parts = parts;
     return m;
 }
-// The split form of input `id` of a node: the tensor's own where its producer wrote it so, else split into `area` now.
-int split_input(const Registry& reg, uint32_t id, int64_t M, int64_t K, bool bf16, void* area, ExecCtx& ctx, SplitMat* out) {
-    if (const SplitMat* m = split_of(ctx, id)) {
-        *out = *m;
-        return 0;
+// One product on the split-form kernels: x as fp32 rows (`ldx` apart) or, where its producer wrote it so, in split form (`xs`).
+// `area` has room to split x (split_area_bytes).  fuse: the node's folded residual Add belongs to this product.
+int f16_product(const Slice& w, const Slice* bias, const float* x, int64_t ldx, const SplitMat* xs, float* out, int64_t M, int64_t ldo, bool relu, bool fuse, void* area,
+                ExecCtx& ctx, F16GemmArgs* extra = nullptr) {
+    F16GemmArgs f;
+    if (extra) f = *extra;   // split output, transposed columns
+    f.w = w.mat; f.bf16 = w.bf16;
+    f.bias = (bias && !bias->drop) ? bias->ptr : nullptr;
+    f.out = out; f.M = M; f.N = w.rows(); f.K = w.ncol; f.ldo = ldo; f.relu = relu;
+    if (M == 0 || f.N == 0) return 0;
+    if (fuse) apply_fusion(ctx, f, false);
+    const bool few = M <= kFewRows && !w.bf16 && f.split_out.planes == nullptr && f.vt_out == nullptr;
+    const bool clusters = few && !gemm_rows_streams(M, f.N, ctx.sm_count);
+    if (xs != nullptr) f.x = *xs;
+    else if (!(clusters && aligned16(x) && ldx % 4 == 0)) {
+        const SplitOut o = split_area(area, M, f.K);
+        if (launch_split_rows(x, ldx, M, f.K, w.bf16, o, nullptr, ctx)) return 1;
+        f.x = as_operand(o);
     }
-    const SplitOut o = split_area(area, M, K);
-    *out = as_operand(o);
-    return launch_split_rows(static_cast<const float*>(reg[id].ptr), K, M, K, bf16, o, nullptr, ctx);
-}
-void fill_f16(F16GemmArgs& g, const SplitMat& x, const Slice& w, const Slice* bias, float* out, int64_t M, int64_t ldo, bool relu) {
-    g.x = x; g.w = w.mat; g.bf16 = w.bf16;
-    g.bias = (bias && !bias->drop) ? bias->ptr : nullptr;
-    g.out = out; g.M = M; g.N = w.rows(); g.K = w.ncol; g.ldo = ldo; g.relu = relu;
+    if (clusters) return launch_gemm_rows(f, f.x.planes ? nullptr : x, ldx, ctx);
+    if (few) return launch_gemm_f16_swapped(f, ctx);
+    return launch_gemm_f16(f, ctx);
 }
 
 void fill_gemm(GemmArgs& g, const float* x, const Slice& w, const Slice* bias, float* out, int64_t M, int64_t ldx, int64_t ldo, bool relu) {
@@ -280,15 +293,11 @@ int run_linear(Registry& reg, const TensorIds& in, const TensorIds& out, bool re
     const DensePlan* pl = dense(plan);
     FXF_CHECK(pl != nullptr && pl->n == 2 && pl->prepared, "%s: the node was not prepared", who);
     if (pl->s[0].f16) {
-        if (M == 0 || N == 0) return 0;
         FXF_CHECK(split_of(ctx, in[0]) != nullptr || ctx.scratch_bytes >= split_area_bytes(M, K), "%s: scratch too small", who);
-        SplitMat xs;
-        if (split_input(reg, in[0], M, K, pl->s[0].bf16, ctx.scratch, ctx, &xs)) return 1;
-        F16GemmArgs f;
-        fill_f16(f, xs, pl->s[0], &pl->s[1], static_cast<float*>(o.ptr), M, N, relu);
-        f.split_out = ctx.split_out;
-        if (ctx.split_out.planes == nullptr) apply_fusion(ctx, f, false);
-        return launch_gemm_f16(f, ctx);
+        F16GemmArgs extra;
+        extra.split_out = ctx.split_out;
+        return f16_product(pl->s[0], &pl->s[1], static_cast<const float*>(x.ptr), K, split_of(ctx, in[0]), static_cast<float*>(o.ptr), M, N, relu,
+                           ctx.split_out.planes == nullptr, ctx.scratch, ctx, &extra);
     }
     GemmArgs g;
     fill_gemm(g, static_cast<const float*>(x.ptr), pl->s[0], &pl->s[1], static_cast<float*>(o.ptr) + pl->col_off, M, K, N, relu);
@@ -307,18 +316,8 @@ int linear_on_rows(const NodePlan* plan, const float* x_rows, const SplitMat* sp
     FXF_CHECK(pl != nullptr && pl->n == 2 && pl->prepared, "linear (rows): the node was not prepared");
     if (M == 0 || pl->s[0].rows() == 0) return 0;
     if (pl->s[0].f16) {
-        SplitMat xs;
-        if (split_rows != nullptr) xs = *split_rows;
-        else {
-            const int64_t K = pl->s[0].ncol;
-            FXF_CHECK(ctx.scratch_bytes >= split_area_bytes(M, K), "linear (rows): scratch too small");
-            const SplitOut o = split_area(ctx.scratch, M, K);
-            if (launch_split_rows(x_rows, ldx, M, K, pl->s[0].bf16, o, nullptr, ctx)) return 1;
-            xs = as_operand(o);
-        }
-        F16GemmArgs f;
-        fill_f16(f, xs, pl->s[0], &pl->s[1], out, M, ldo, false);
-        return launch_gemm_f16(f, ctx);
+        FXF_CHECK(split_rows != nullptr || ctx.scratch_bytes >= split_area_bytes(M, pl->s[0].ncol), "linear (rows): scratch too small");
+        return f16_product(pl->s[0], &pl->s[1], x_rows, ldx, split_rows, out, M, ldo, false, false, ctx.scratch, ctx);
     }
     FXF_CHECK(split_rows == nullptr, "linear (rows): the rows are in split form but the weight is not");
     GemmArgs g;
@@ -354,8 +353,8 @@ std::unique_ptr<NodePlan> plan_linear(const Registry& reg, const TensorIds& in, 
     p->reserve(bs, false);
     p->M = M;
     if (ws.f16) {
-        p->takes_split = 1;
-        p->makes_split = N % 8 == 0;
+        p->takes_split = takes_split_rows(M, N) ? 1 : 0;
+        p->makes_split = N % 8 == 0 && M > kFewRows;
         p->split_rows = M; p->split_cols = N;
         p->scratch_bytes = split_area_bytes(M, K);
     }
@@ -410,14 +409,11 @@ static int run_feedforward_f16(Registry& reg, const TensorIds& in, const float* 
     h.parts_out = &parts;
     char* area = reinterpret_cast<char*>(h.amax) + round_up(size_t(M) * size_t(gemm_f16_split_parts(F)) * 4, 256);
     float* hidden = static_cast<float*>(ctx.scratch);
-    const bool both = pl->s[0].f16 && pl->s[2].f16;
+    const bool keep_split = pl->s[0].f16 && pl->s[2].f16 && M > kFewRows && F % 8 == 0;
     if (pl->s[0].f16) {
-        SplitMat xs;
-        if (split_input(reg, in[0], M, K, pl->s[0].bf16, area, ctx, &xs)) return 1;
-        F16GemmArgs g1;
-        fill_f16(g1, xs, pl->s[0], &pl->s[1], both ? nullptr : hidden, M, F, true);
-        if (both) g1.split_out = h;
-        if (launch_gemm_f16(g1, ctx)) return 1;
+        F16GemmArgs extra;
+        if (keep_split) extra.split_out = h;
+        if (f16_product(pl->s[0], &pl->s[1], x, K, split_of(ctx, in[0]), keep_split ? nullptr : hidden, M, F, true, false, area, ctx, &extra)) return 1;
     } else {
         GemmArgs g1;
         fill_gemm(g1, x, pl->s[0], &pl->s[1], hidden, M, K, F, true);
@@ -429,17 +425,8 @@ static int run_feedforward_f16(Registry& reg, const TensorIds& in, const float* 
         apply_fusion(ctx, g2, false);
         return launch_gemm(g2, ctx);
     }
-    SplitMat hs = as_operand(h, parts);
-    if (!both) {   // the hidden activation came from another kernel as fp32
-        FXF_CHECK(split_area_bytes(M, F) <= ctx.scratch_bytes - size_t(reinterpret_cast<char*>(area) - base), "feedforward: scratch too small to split the hidden activation");
-        const SplitOut o = split_area(area, M, F);
-        if (launch_split_rows(hidden, F, M, F, pl->s[2].bf16, o, nullptr, ctx)) return 1;
-        hs = as_operand(o);
-    }
-    F16GemmArgs g2;
-    fill_f16(g2, hs, pl->s[2], &pl->s[3], out, M, P, false);
-    apply_fusion(ctx, g2, false);
-    return launch_gemm_f16(g2, ctx);
+    const SplitMat hs = as_operand(h, parts);
+    return f16_product(pl->s[2], &pl->s[3], hidden, F, keep_split ? &hs : nullptr, out, M, P, false, true, area, ctx);
 }
 // slices: s[0] = w1 rows of this rank [Fl, D], s[1] = b1 entries [Fl], s[2] = w2 columns of this rank [P, Fl], s[3] = b2
 int k_feedforward(Registry& reg, const TensorIds& in, const TensorIds& out, const Params&, const NodePlan* plan, ExecCtx& ctx) {
@@ -496,7 +483,7 @@ std::unique_ptr<NodePlan> plan_feedforward(const Registry& reg, const TensorIds&
     p->M = M;
     p->scratch_bytes = size_t(M) * size_t(Fl) * sizeof(float);
     if (s_w1.f16 || s_w2.f16) p->scratch_bytes = ff_f16_bytes(M, std::max(K, Fl), Fl);
-    if (s_w1.f16) p->takes_split = 1;
+    if (s_w1.f16) p->takes_split = takes_split_rows(M, Fl) ? 1 : 0;
     p->flops = 2.0 * double(M) * double(Fl) * double(K) + 2.0 * double(M) * double(P) * double(Fl);
     p->bytes = 4.0 * (double(M) * K + double(Fl) * K + Fl + double(P) * Fl + P + double(M) * P);
     p->variant += variant_of(env, s_w1, M, Fl, K) + "+" + variant_of(env, s_w2, M, P, Fl);
@@ -546,11 +533,9 @@ int k_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const Params
 
     bool v_transposed = false;
     if (pl->s[0].f16) {
-        SplitMat xs;
-        if (split_input(reg, in[0], M, D, pl->s[0].bf16, area, ctx, &xs)) return 1;
         F16GemmArgs f;
-        fill_f16(f, xs, pl->s[0], &pl->s[1], qkv, M, QKVl, false);
-        if (have_vt && hd == 64) {
+        if (have_vt && hd == 64 && M > kFewRows) {
+            f.M = M; f.N = QKVl; f.K = D;
             f.vt_out = vt;
             f.vt_flags = reinterpret_cast<unsigned char*>(vt + size_t(B) * size_t(Hl) * size_t(T) * 64);
             f.vt_col0 = 2 * Dl;
@@ -558,7 +543,7 @@ int k_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const Params
             v_transposed = gemm_f16_vt_ok(f, ctx);
             if (!v_transposed) { f.vt_out = nullptr; f.vt_flags = nullptr; }
         }
-        if (launch_gemm_f16(f, ctx)) return 1;
+        if (f16_product(pl->s[0], &pl->s[1], static_cast<const float*>(x.ptr), D, split_of(ctx, in[0]), qkv, M, QKVl, false, false, area, ctx, &f)) return 1;
     } else {
     GemmArgs g;
     fill_gemm(g, static_cast<const float*>(x.ptr), pl->s[0], &pl->s[1], qkv, M, D, QKVl, false);
@@ -590,12 +575,7 @@ int k_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const Params
     }
 
     if (pl->s[2].f16) {
-        const SplitOut so = split_area(area, M, D);
-        if (launch_split_rows(cx, D, M, D, pl->s[2].bf16, so, nullptr, ctx)) return 1;
-        F16GemmArgs f2;
-        fill_f16(f2, as_operand(so), pl->s[2], &pl->s[3], static_cast<float*>(o.ptr), M, D, false);
-        apply_fusion(ctx, f2, false);
-        return launch_gemm_f16(f2, ctx);
+        return f16_product(pl->s[2], &pl->s[3], cx, D, nullptr, static_cast<float*>(o.ptr), M, D, false, true, area, ctx);
     }
     GemmArgs g2;
     fill_gemm(g2, cx, pl->s[2], &pl->s[3], static_cast<float*>(o.ptr), M, Dl, D, false);
@@ -640,7 +620,7 @@ std::unique_ptr<NodePlan> plan_mha(const Registry& reg, const TensorIds& in, con
     pl->M = M;
     pl->scratch_bytes = size_t(M) * size_t(3 * Dl + Dl) * sizeof(float);
     if (s_wq.f16 || s_wo.f16) pl->scratch_bytes += split_area_bytes(M, D);
-    if (s_wq.f16) pl->takes_split = 1;
+    if (s_wq.f16) pl->takes_split = takes_split_rows(M, 3 * Dl) ? 1 : 0;
     const bool tc_attn = env.gemm_mode != FXF_GEMM_FP32_SIMT && hd == 64 && T % 4 == 0 && T >= 16 && T <= 4096 && Dl % 4 == 0;   // the tcgen05 kernel covers at most 32 blocks of 128 keys
     if (tc_attn) pl->scratch_bytes += attention_tc_scratch_bytes(B, T, Hl);
     pl->flops = 2.0 * M * double(3 * Dl) * D + 4.0 * double(B) * Hl * double(T) * T * hd + 2.0 * double(M) * D * Dl;
@@ -703,12 +683,7 @@ int k_cross_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const 
 
     auto project = [&](int wi, uint32_t id, const FxfTensor& t, float* dst, int64_t rows, int64_t cols) {
         if (pl->s[wi].f16) {
-            SplitMat xs;
-            if (rows == 0) return 0;
-            if (split_input(reg, id, rows, D, pl->s[wi].bf16, area, ctx, &xs)) return 1;
-            F16GemmArgs f;
-            fill_f16(f, xs, pl->s[wi], &pl->s[wi + 1], dst, rows, cols, false);
-            return launch_gemm_f16(f, ctx);
+            return f16_product(pl->s[wi], &pl->s[wi + 1], static_cast<const float*>(t.ptr), D, split_of(ctx, id), dst, rows, cols, false, false, area, ctx);
         }
         GemmArgs g;
         fill_gemm(g, static_cast<const float*>(t.ptr), pl->s[wi], &pl->s[wi + 1], dst, rows, D, cols, false);
@@ -736,12 +711,7 @@ int k_cross_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const 
     }
 
     if (pl->s[4].f16) {
-        const SplitOut so = split_area(area, Mq, D);
-        if (launch_split_rows(cx, D, Mq, D, pl->s[4].bf16, so, nullptr, ctx)) return 1;
-        F16GemmArgs f2;
-        fill_f16(f2, as_operand(so), pl->s[4], &pl->s[5], static_cast<float*>(o.ptr), Mq, D, false);
-        apply_fusion(ctx, f2, false);
-        return launch_gemm_f16(f2, ctx);
+        return f16_product(pl->s[4], &pl->s[5], cx, D, nullptr, static_cast<float*>(o.ptr), Mq, D, false, true, area, ctx);
     }
     GemmArgs g2;
     fill_gemm(g2, cx, pl->s[4], &pl->s[5], static_cast<float*>(o.ptr), Mq, Dl, D, false);
@@ -795,7 +765,7 @@ std::unique_ptr<NodePlan> plan_cross_mha(const Registry& reg, const TensorIds& i
     pl->M = Mq;
     pl->scratch_bytes = (size_t(Mq) * size_t(2 * Dl) + size_t(Mk) * size_t(2 * Dl)) * sizeof(float);
     if (s_wq.f16 || s_wkv.f16 || s_wo.f16) pl->scratch_bytes += split_area_bytes(std::max(Mq, Mk), D);
-    pl->takes_split = (s_wq.f16 ? 1u : 0u) | (s_wkv.f16 ? 2u : 0u);
+    pl->takes_split = (s_wq.f16 && takes_split_rows(Mq, Dl) ? 1u : 0u) | (s_wkv.f16 && takes_split_rows(Mk, 2 * Dl) ? 2u : 0u);
     const bool tc_attn = env.gemm_mode != FXF_GEMM_FP32_SIMT && hd == 64 && Tk % 4 == 0 && Tk >= 16 && Tk <= 4096 && Dl % 4 == 0;
     if (tc_attn) pl->scratch_bytes += attention_tc_scratch_bytes(B, Tk, Hl);
     pl->flops = 2.0 * double(Mq) * Dl * D + 2.0 * double(Mk) * 2 * Dl * D + 4.0 * double(B) * Hl * double(Tq) * Tk * hd + 2.0 * double(Mq) * D * Dl;
@@ -929,23 +899,31 @@ int k_cached_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const
     FXF_CHECK(numel(o) == B * D && x.dtype == FXF_F32 && o.dtype == FXF_F32, "cached_mha: output must be float32 [B,1,D]");
     const DensePlan* pl = dense(plan);
     FXF_CHECK(pl != nullptr && pl->n == 4 && pl->prepared && pl->persist != nullptr, "cached_mha: the node was not prepared");
-    size_t need = size_t(B) * size_t(4 * D) * sizeof(float);
+    const size_t core = round_up(size_t(B) * size_t(4 * D) * sizeof(float), 256);
+    size_t need = core + (pl->s[0].f16 || pl->s[2].f16 ? split_area_bytes(B, D) : 0);
     FXF_CHECK(ctx.scratch_bytes >= need && ctx.scratch != nullptr, "cached_mha: scratch too small (%zu < %zu bytes)", ctx.scratch_bytes, need);
     float* qkv = static_cast<float*>(ctx.scratch);
     float* cx = qkv + B * 3 * D;
     float* cache = reinterpret_cast<float*>(static_cast<char*>(pl->persist) + pl->cache_off);
+    void* area = static_cast<char*>(ctx.scratch) + core;
     if (B == 0) return 0;
-    GemmArgs g;
-    fill_gemm(g, static_cast<const float*>(x.ptr), pl->s[0], &pl->s[1], qkv, B, D, QKV, false);
-    if (launch_gemm(g, ctx)) return 1;
+    if (pl->s[0].f16) {
+        if (f16_product(pl->s[0], &pl->s[1], static_cast<const float*>(x.ptr), D, split_of(ctx, in[0]), qkv, B, QKV, false, false, area, ctx)) return 1;
+    } else {
+        GemmArgs g;
+        fill_gemm(g, static_cast<const float*>(x.ptr), pl->s[0], &pl->s[1], qkv, B, D, QKV, false);
+        if (launch_gemm(g, ctx)) return 1;
+    }
     tag_launch(ctx, "cached_attention_fp32", 4.0 * double(B) * H * double(T) * hd, 4.0 * 2.0 * double(B) * T * D);
     FXF_CHECK(T * sizeof(float) <= 160 * 1024, "cached_mha: static length %lld is too long for the score buffer", (long long)T);
     if (size_t(T) * sizeof(float) > 40 * 1024) FXF_CUDA(cudaFuncSetAttribute(cached_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(T * sizeof(float))));
     cached_attn_kernel<<<dim3(unsigned(H), unsigned(B)), kCachedAttnThreads, size_t(T) * sizeof(float), ctx.stream>>>(
         qkv, cache, static_cast<const int64_t*>(tok.ptr), static_cast<const int64_t*>(pos.ptr), cx, int(T), int(D), int(hd), p.floats[0], p.ints[4], ctx.status);
     FXF_LAUNCHED(ctx);
+    if (pl->s[2].f16) return f16_product(pl->s[2], &pl->s[3], cx, D, nullptr, static_cast<float*>(o.ptr), B, D, false, true, area, ctx);
     GemmArgs g2;
     fill_gemm(g2, cx, pl->s[2], &pl->s[3], static_cast<float*>(o.ptr), B, D, D, false);
+    apply_fusion(ctx, g2, false);
     return launch_gemm(g2, ctx);
 }
 
@@ -961,19 +939,18 @@ std::unique_ptr<NodePlan> plan_cached_mha(const Registry& reg, const TensorIds& 
     Slice& s_bq = pl->add(4, QKV, 1);
     Slice& s_wo = pl->add(5, D, D);
     Slice& s_bo = pl->add(6, D, 1);
-    pl->reserve(s_wq, want_tc(env, B, QKV, D));
+    reserve_weight(*pl, s_wq, env, B, QKV, D);
     pl->reserve(s_bq, false);
-    pl->reserve(s_wo, want_tc(env, B, D, D));
+    reserve_weight(*pl, s_wo, env, B, D, D);
     pl->reserve(s_bo, false);
+    if (s_wq.f16) pl->takes_split = takes_split_rows(B, QKV) ? 1 : 0;
     pl->cache_off = pl->persist_bytes;
     pl->persist_bytes += round_up(size_t(B) * size_t(T) * size_t(2 * D) * sizeof(float), 256);
     pl->M = B;
-    pl->scratch_bytes = size_t(B) * size_t(4 * D) * sizeof(float);
+    pl->scratch_bytes = round_up(size_t(B) * size_t(4 * D) * sizeof(float), 256) + (s_wq.f16 || s_wo.f16 ? split_area_bytes(B, D) : 0);
     pl->flops = 2.0 * double(B) * QKV * D + 4.0 * double(B) * H * double(T) * hd + 2.0 * double(B) * D * D;
     pl->bytes = 4.0 * (double(QKV) * D + double(D) * D + 2.0 * double(B) * T * D);
-    GemmArgs g1;
-    g1.M = B; g1.N = QKV; g1.K = D;
-    pl->variant = std::string(env.tp_size > 1 ? "replicated " : "") + gemm_variant_name(g1, env.gemm_mode, 148, env.tc_pairs) + "+cached-attn-fp32";
+    pl->variant = std::string(env.tp_size > 1 ? "replicated " : "") + variant_of(env, s_wq, B, QKV, D) + "+cached-attn-fp32";
     return pl;
 }
 

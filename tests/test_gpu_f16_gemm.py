@@ -30,7 +30,7 @@ def _w(rng, n, k):
 # outputs without 16-byte rows, a single column
 @pytest.mark.parametrize("M,N,K,variant", [
     (8192, 2304, 768, "256x"), (8192, 768, 3072, "256x"), (985, 768, 768, "256x64-pair"), (16384, 512, 512, "256x128-pair"), (8192, 3072, 768, "256x192-pair"),
-    (64, 512, 512, "128x32"), (512, 1000, 256, "128x32"), (129, 33, 72, "128x"), (257, 129, 1096, ""), (300, 10, 512, "128x32"), (985, 1111, 264, ""), (64, 1, 16, ""), (513, 50257, 40, "")])
+    (65, 512, 512, "128x32"), (512, 1000, 256, "128x32"), (129, 33, 72, "128x"), (257, 129, 1096, ""), (300, 10, 512, "128x32"), (985, 1111, 264, ""), (66, 1, 16, ""), (513, 50257, 40, "")])
 def test_every_variant_at_its_edges(built_lib, tmp_path, M, N, K, variant):
     rng = np.random.default_rng(M + N + K)
     b = lowering.GraphBuilder(f"f16_{M}_{N}_{K}")
@@ -71,7 +71,7 @@ def test_rows_keep_their_precision_at_any_scale(built_lib, tmp_path):
     eng.close()
 
 
-@pytest.mark.parametrize("M,D,F", [(64, 64, 256), (200, 768, 3072), (333, 136, 72)])
+@pytest.mark.parametrize("M,D,F", [(65, 64, 256), (200, 768, 3072), (333, 136, 72)])
 @pytest.mark.parametrize("precision", ["auto", "bf16"])
 def test_activations_stay_in_split_form_between_nodes(built_lib, tmp_path, M, D, F, precision):
     """LayerNorm -> FeedForward and LinearRelu -> LinearRelu -> Linear: the activation between two products is written in
@@ -99,5 +99,31 @@ def test_activations_stay_in_split_form_between_nodes(built_lib, tmp_path, M, D,
         assert ok, info
     else:
         assert ((got - want).abs().max() / want.abs().max()).item() < 2e-2
+    assert eng.device_status() == 0
+    eng.close()
+
+
+# the few-row kernels: row groups of 16 and 32, clusters of 1 to 16 CTAs over K, several rounds of slabs, a ragged K and N, and
+# the streaming kernel for weights of a tile per SM
+@pytest.mark.parametrize("M,N,K,variant", [
+    (1, 512, 512, "rows128"), (16, 129, 72, "rows128"), (17, 10, 512, "rows128"), (32, 768, 3072, "rows128"), (33, 127, 16, "rows128"), (64, 2304, 768, "rows128"),
+    (5, 1, 5000, "rows128"), (64, 512, 8200, "rows128"), (31, 12800, 264, "rows128"), (32, 18945, 768, "stream128"), (33, 19000, 520, "stream128"), (1, 50257, 768, "stream128")])
+def test_few_rows(built_lib, tmp_path, M, N, K, variant):
+    rng = np.random.default_rng(M + N + K)
+    b = lowering.GraphBuilder(f"rows_{M}_{N}_{K}")
+    x = b.input((M, K), wire.DT_F32)
+    r = b.input((M, N), wire.DT_F32)
+    lin = b.op("Linear", [x, b.const(_w(rng, N, K)), b.const(rng.standard_normal(N, dtype=np.float32))], (M, N))
+    b.output(b.op("AddRelu", [lin, r], (M, N)))
+    graph, eng = _engine(b, tmp_path)
+    assert "split operands: tcgen05-f16x3-" + variant in eng.describe() and "+AddRelu(residual" in eng.describe(), eng.describe()
+    gen = torch.Generator().manual_seed(1)
+    xin, rin = torch.randn(M, K, generator=gen), torch.randn(M, N, generator=gen)
+    xin *= 10.0 ** torch.linspace(-6, 6, K)   # K ranges of very different size: every CTA of a cluster scales its own
+    got, want = eng.run([xin.cuda(), rin.cuda()])[0].cpu(), GraphOracle(graph).run([xin, rin])[0]
+    assert ((got - want).abs().max() / want.abs().max()).item() < 2e-6
+    xin = torch.randn(M, K, generator=gen)
+    ok, info = compare_outputs(eng.run([xin.cuda(), rin.cuda()])[0].cpu(), GraphOracle(graph).run([xin, rin])[0], atol=2e-5, rtol=1e-4)
+    assert ok, info
     assert eng.device_status() == 0
     eng.close()
