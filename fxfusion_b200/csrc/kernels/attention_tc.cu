@@ -69,6 +69,7 @@ __device__ __forceinline__ void soft_sync(int quarter) { asm volatile("bar.sync 
 // vflags[(bh * 2 + half) * n32 + slab] (this kernel reports a slab under half 0 and clears half 1).
 __global__ void __launch_bounds__(256) attn_vt_kernel(const float* __restrict__ qkv, int64_t ld, int64_t v_off, int T, int H, float* __restrict__ vt,
                                                       unsigned char* __restrict__ vflags, int n32) {
+    grid_dep();
     // one block moves 64 keys x 64 head columns: rows of 256 bytes on both sides
     __shared__ float tile[HD][65];
     const int bh = blockIdx.y, b = bh / H, h = bh % H, t0 = blockIdx.x * 64, tid = threadIdx.x;
@@ -201,6 +202,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s.tmem_base;
+    grid_dep_wait();   // the set-up above ran under the previous kernel
 
     // ---- which key blocks matter to this CTA's 128 query rows ----
     const unsigned long long all_blocks = nblk >= 64 ? ~0ull : ((1ull << nblk) - 1ull);
@@ -491,6 +493,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
             }
             soft_sync(quarter);   // exch[] is reused by the next block (and by the final sum exchange)
         }
+        grid_dep_launch();
         s.exch[half][row] = l_run;
         soft_sync(quarter);
         const float l_tot = s.exch[0][row] + s.exch[1][row];
@@ -568,7 +571,7 @@ int launch_attention_tc(const AttnArgs& a, float* vt_scratch, ExecCtx& ctx, bool
     unsigned char* vflags = reinterpret_cast<unsigned char*>(vt_scratch + size_t(BH) * size_t(Tk) * HD);
     if (!v_transposed) {   // otherwise the projection's epilogue has written V^T and the flags already
         tag_launch(ctx, "attention_v_transpose", 0, 8.0 * double(BH) * Tk * HD);
-        attn_vt_kernel<<<pgrid, 256, 0, ctx.stream>>>(kvp, ldk, a.v_off, Tk, a.H, vt_scratch, vflags, n32);
+        dependent(attn_vt_kernel, pgrid, 256, 0, ctx)(kvp, ldk, a.v_off, Tk, a.H, vt_scratch, vflags, n32);
         FXF_LAUNCHED(ctx);
     }
 
@@ -603,7 +606,7 @@ int launch_attention_tc(const AttnArgs& a, float* vt_scratch, ExecCtx& ctx, bool
     dim3 grid(unsigned((a.T + BQ - 1) / BQ), unsigned(BH));
     tag_launch(ctx, "attention_tf32_bf16x2_tcgen05", 4.0 * double(a.B) * a.H * double(a.T) * Tk * a.hd,
                4.0 * 2.0 * double(a.B) * (double(a.T) + Tk) * double(a.H) * a.hd + double(a.B) * a.T * Tk);
-    attn_tc_kernel<<<grid, kAttnThreads, smem, ctx.stream>>>(mq, mk, mv, p);
+    dependent(attn_tc_kernel, grid, kAttnThreads, smem, ctx)(mq, mk, mv, p);
     FXF_LAUNCHED(ctx);
     return 0;
 }

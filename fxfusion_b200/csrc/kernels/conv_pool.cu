@@ -24,6 +24,7 @@
 #include <cmath>
 
 #include "../runtime.hpp"
+#include "sm100.cuh"
 
 namespace fxf {
 namespace {
@@ -48,6 +49,7 @@ constexpr int CBM = 64, CBN = 64, CBK = 16;
 
 __global__ void __launch_bounds__(256) conv2d_igemm_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                                                            float* __restrict__ out, ConvDesc d) {
+    sm100::grid_dep();
     __shared__ __align__(16) float As[CBK][CBM + 4];
     __shared__ __align__(16) float Bs[CBK][CBN + 4];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;  // tx -> pixels, ty -> channels
@@ -158,6 +160,7 @@ enum PoolOp { kMaxPool = 0, kAvgPool = 1, kAdaptiveAvg = 2 };
 
 template <int OP>
 __global__ void __launch_bounds__(256) pool2d_kernel(const float* __restrict__ x, float* __restrict__ out, PoolDesc d) {
+    sm100::grid_dep();
     int64_t total = d.N * d.C * d.HO * d.WO, stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
         int64_t n;
@@ -201,6 +204,7 @@ __global__ void __launch_bounds__(256) pool2d_kernel(const float* __restrict__ x
 
 // Global average of a row-major plane (output 1x1, NCHW input): one warp per (n,c) plane.
 __global__ void __launch_bounds__(256) global_avg_pool_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t NC, int HW) {
+    sm100::grid_dep();
     int lane = threadIdx.x & 31;
     int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5, nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
     for (int64_t p = warp; p < NC; p += nwarps) {
@@ -220,6 +224,7 @@ __global__ void __launch_bounds__(256) global_avg_pool_kernel(const float* __res
 // rearranged the same way (taps beyond k are zero): out[oy, ox] = sum_{qy,qx,ch} S[oy+qy, ox+qx, ch] * W'[o, qy, qx, ch].
 __global__ void __launch_bounds__(256) space_to_depth16_kernel(const float* __restrict__ x, float4* __restrict__ s, int64_t N, int C, int H, int W, int Hs, int Ws,
                                                                int ph, int pw, Strides4 xs) {
+    sm100::grid_dep();
     const int64_t total = N * Hs * Ws * 4, stride = int64_t(gridDim.x) * blockDim.x;   // one float4 = 4 of the 16 channels
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
         const int g = int(i & 3);
@@ -365,7 +370,7 @@ int run_conv(Registry& reg, const TensorIds& in, const TensorIds& out, const Par
         float* sbuf = static_cast<float*>(ctx.scratch);
         const int64_t total4 = int64_t(d.N) * cp->Hs * cp->Ws * 4;
         tag_launch(ctx, "space_to_depth16", 0, double(x.nbytes) + 16.0 * double(total4));
-        space_to_depth16_kernel<<<pool_grid(total4, ctx), 256, 0, ctx.stream>>>(static_cast<const float*>(x.ptr), reinterpret_cast<float4*>(sbuf), d.N, d.C, d.H, d.W,
+        dependent(space_to_depth16_kernel, pool_grid(total4, ctx), 256, 0, ctx)(static_cast<const float*>(x.ptr), reinterpret_cast<float4*>(sbuf), d.N, d.C, d.H, d.W,
                                                                                 cp->Hs, cp->Ws, d.ph, d.pw, d.xs);
         FXF_LAUNCHED(ctx);
         ConvTcArgs c;
@@ -402,7 +407,7 @@ int run_conv(Registry& reg, const TensorIds& in, const TensorIds& out, const Par
         dst = ctx.fuse.out;
         d.relu = 0;
     }
-    conv2d_igemm_kernel<<<grid, 256, 0, ctx.stream>>>(static_cast<const float*>(x.ptr), static_cast<const float*>(w.ptr), static_cast<const float*>(b.ptr), dst, d);
+    dependent(conv2d_igemm_kernel, grid, 256, 0, ctx)(static_cast<const float*>(x.ptr), static_cast<const float*>(w.ptr), static_cast<const float*>(b.ptr), dst, d);
     FXF_LAUNCHED(ctx);
     if (fused) {
         ctx.fuse.consumed = true;
@@ -445,7 +450,7 @@ int k_max_pool2d(Registry& reg, const TensorIds& in, const TensorIds& out, const
     FXF_CHECK(d.sh > 0 && d.sw > 0, "max_pool2d: stride must be positive");
     int64_t total = d.N * d.C * d.HO * d.WO;
     if (total == 0) return 0;
-    pool2d_kernel<kMaxPool><<<pool_grid(total, ctx), 256, 0, ctx.stream>>>(static_cast<const float*>(reg[in[0]].ptr), static_cast<float*>(reg[out[0]].ptr), d);
+    dependent(pool2d_kernel<kMaxPool>, pool_grid(total, ctx), 256, 0, ctx)(static_cast<const float*>(reg[in[0]].ptr), static_cast<float*>(reg[out[0]].ptr), d);
     FXF_LAUNCHED(ctx);
     return 0;
 }
@@ -459,7 +464,7 @@ int k_avg_pool2d(Registry& reg, const TensorIds& in, const TensorIds& out, const
     FXF_CHECK(d.sh > 0 && d.sw > 0, "avg_pool2d: stride must be positive");
     int64_t total = d.N * d.C * d.HO * d.WO;
     if (total == 0) return 0;
-    pool2d_kernel<kAvgPool><<<pool_grid(total, ctx), 256, 0, ctx.stream>>>(static_cast<const float*>(reg[in[0]].ptr), static_cast<float*>(reg[out[0]].ptr), d);
+    dependent(pool2d_kernel<kAvgPool>, pool_grid(total, ctx), 256, 0, ctx)(static_cast<const float*>(reg[in[0]].ptr), static_cast<float*>(reg[out[0]].ptr), d);
     FXF_LAUNCHED(ctx);
     return 0;
 }
@@ -474,11 +479,11 @@ int k_adaptive_avg_pool2d(Registry& reg, const TensorIds& in, const TensorIds& o
     if (total == 0) return 0;
     if (d.HO == 1 && d.WO == 1 && is_contiguous(reg[in[0]]) && is_contiguous(reg[out[0]])) {
         int64_t nc = d.N * d.C, blocks = (nc * 32 + 255) / 256, cap = int64_t(ctx.sm_count) * 8;
-        global_avg_pool_kernel<<<int(blocks < cap ? blocks : cap), 256, 0, ctx.stream>>>(static_cast<const float*>(reg[in[0]].ptr), static_cast<float*>(reg[out[0]].ptr), nc, d.H * d.W);
+        dependent(global_avg_pool_kernel, int(blocks < cap ? blocks : cap), 256, 0, ctx)(static_cast<const float*>(reg[in[0]].ptr), static_cast<float*>(reg[out[0]].ptr), nc, d.H * d.W);
     } else {
         // a channels-last input is walked channels-fastest, which keeps the strided window reads coalesced
         if (is_channels_last(reg[in[0]])) d.cl = 1;
-        pool2d_kernel<kAdaptiveAvg><<<pool_grid(total, ctx), 256, 0, ctx.stream>>>(static_cast<const float*>(reg[in[0]].ptr), static_cast<float*>(reg[out[0]].ptr), d);
+        dependent(pool2d_kernel<kAdaptiveAvg>, pool_grid(total, ctx), 256, 0, ctx)(static_cast<const float*>(reg[in[0]].ptr), static_cast<float*>(reg[out[0]].ptr), d);
     }
     FXF_LAUNCHED(ctx);
     return 0;

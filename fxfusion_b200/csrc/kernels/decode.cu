@@ -10,11 +10,13 @@
 #include <cmath>
 
 #include "../runtime.hpp"
+#include "sm100.cuh"
 
 namespace fxf {
 namespace {
 
 __global__ void __launch_bounds__(256) build_mask_kernel(const int64_t* __restrict__ tokens, uint8_t* __restrict__ mask, int B, int T, int cur, int64_t pad) {
+    sm100::grid_dep();
     int64_t total = int64_t(B) * T * T, stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
         int k = int(i % T);
@@ -27,6 +29,7 @@ __global__ void __launch_bounds__(256) build_mask_kernel(const int64_t* __restri
 
 // 4 keys per thread, one 32-bit store.
 __global__ void __launch_bounds__(256) build_mask_vec4_kernel(const int64_t* __restrict__ tokens, uint32_t* __restrict__ mask, int B, int T, int cur, int64_t pad) {
+    sm100::grid_dep();
     int T4 = T / 4;
     int64_t total = int64_t(B) * T * T4, stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -64,6 +67,7 @@ __device__ __forceinline__ bool better(const Best& a, const Best& b) {
 }
 
 __global__ void __launch_bounds__(1024) argmax_scatter_kernel(const float* __restrict__ logits, int64_t row_stride, int64_t row_off, int64_t* __restrict__ tokens, int T, int64_t V, int cur) {
+    sm100::grid_dep();
     __shared__ Best red[32];
     int b = blockIdx.x;
     const float* row = logits + int64_t(b) * row_stride + row_off;
@@ -106,6 +110,7 @@ struct alignas(16) Candidate {
 
 __global__ void __launch_bounds__(1024) argmax_partial_kernel(const float* __restrict__ logits, int64_t row_stride, int64_t row_off, Candidate* __restrict__ cand,
                                                               int64_t col0, int64_t ncols) {
+    sm100::grid_dep();
     __shared__ Best red[32];
     int b = blockIdx.x;
     const float* row = logits + int64_t(b) * row_stride + row_off;
@@ -138,6 +143,7 @@ __global__ void __launch_bounds__(1024) argmax_partial_kernel(const float* __res
 }
 
 __global__ void argmax_combine_scatter_kernel(const Candidate* __restrict__ all, int64_t* __restrict__ tokens, int B, int T, int cur, int n_ranks) {
+    sm100::grid_dep();
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= B) return;
     Best best{0.f, -1};
@@ -167,10 +173,10 @@ int decode_argmax_scatter_sharded_rows(const float* logits, int64_t row_stride, 
     FXF_CHECK(cur >= 1 && cur < T, "decode: current_len %d must be in [1, %d)", cur, T);
     if (B == 0) return 0;
     (void)V;
-    argmax_partial_kernel<<<B, 1024, 0, ctx.stream>>>(logits, row_stride, row_off, static_cast<Candidate*>(cand_local), col0, ncols);
+    dependent(argmax_partial_kernel, B, 1024, 0, ctx)(logits, row_stride, row_off, static_cast<Candidate*>(cand_local), col0, ncols);
     FXF_LAUNCHED(ctx);
     if (tp_all_gather(cand_local, cand_all, int64_t(B) * int64_t(sizeof(Candidate)), ctx)) return 1;
-    argmax_combine_scatter_kernel<<<(B + 127) / 128, 128, 0, ctx.stream>>>(static_cast<const Candidate*>(cand_all), tokens, B, T, cur, ctx.tp_size);
+    dependent(argmax_combine_scatter_kernel, (B + 127) / 128, 128, 0, ctx)(static_cast<const Candidate*>(cand_all), tokens, B, T, cur, ctx.tp_size);
     FXF_LAUNCHED(ctx);
     return 0;
 }
@@ -178,6 +184,7 @@ int decode_argmax_scatter_sharded_rows(const float* logits, int64_t row_stride, 
 namespace {
 // ids[b] = tokens[b, p]; *pos = p  — the inputs of one incremental decode step
 __global__ void step_prepare_kernel(const int64_t* __restrict__ tokens, int64_t* __restrict__ ids, int64_t* __restrict__ pos, int B, int T, int p) {
+    sm100::grid_dep();
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < B) ids[b] = tokens[int64_t(b) * T + p];
     if (b == 0) *pos = p;
@@ -186,7 +193,7 @@ __global__ void step_prepare_kernel(const int64_t* __restrict__ tokens, int64_t*
 
 int decode_step_prepare(const int64_t* tokens, int64_t* ids, int64_t* pos, int B, int T, int p, ExecCtx& ctx) {
     FXF_CHECK(p >= 0 && p < T, "decode: position %d is outside the static length %d", p, T);
-    step_prepare_kernel<<<(B + 127) / 128 > 0 ? (B + 127) / 128 : 1, 128, 0, ctx.stream>>>(tokens, ids, pos, B, T, p);
+    dependent(step_prepare_kernel, (B + 127) / 128 > 0 ? (B + 127) / 128 : 1, 128, 0, ctx)(tokens, ids, pos, B, T, p);
     FXF_LAUNCHED(ctx);
     return 0;
 }
@@ -197,10 +204,10 @@ int decode_build_mask(const int64_t* tokens, uint8_t* mask, int B, int T, int cu
     int64_t cap = int64_t(ctx.sm_count) * 8;
     if (T % 4 == 0 && (reinterpret_cast<uintptr_t>(mask) & 3) == 0) {
         int64_t total = int64_t(B) * T * (T / 4), blocks = (total + 255) / 256;
-        build_mask_vec4_kernel<<<int(blocks < cap ? blocks : cap), 256, 0, ctx.stream>>>(tokens, reinterpret_cast<uint32_t*>(mask), B, T, cur, pad);
+        dependent(build_mask_vec4_kernel, int(blocks < cap ? blocks : cap), 256, 0, ctx)(tokens, reinterpret_cast<uint32_t*>(mask), B, T, cur, pad);
     } else {
         int64_t total = int64_t(B) * T * T, blocks = (total + 255) / 256;
-        build_mask_kernel<<<int(blocks < cap ? blocks : cap), 256, 0, ctx.stream>>>(tokens, mask, B, T, cur, pad);
+        dependent(build_mask_kernel, int(blocks < cap ? blocks : cap), 256, 0, ctx)(tokens, mask, B, T, cur, pad);
     }
     FXF_LAUNCHED(ctx);
     return 0;
@@ -214,7 +221,7 @@ int decode_argmax_scatter_rows(const float* logits, int64_t row_stride, int64_t 
     FXF_CHECK(cur >= 1 && cur < T, "decode: current_len %d must be in [1, %d)", cur, T);
     FXF_CHECK(V >= 1, "decode: empty vocabulary");
     if (B == 0) return 0;
-    argmax_scatter_kernel<<<B, 1024, 0, ctx.stream>>>(logits, row_stride, row_off, tokens, T, V, cur);
+    dependent(argmax_scatter_kernel, B, 1024, 0, ctx)(logits, row_stride, row_off, tokens, T, V, cur);
     FXF_LAUNCHED(ctx);
     return 0;
 }

@@ -14,6 +14,7 @@
 //   embedding       csrc/kernels/cpu/embedding.cpp:5-11
 //   transpose       csrc/kernels/cpu/transpose.cpp:5-12 (materialised two-dim swap)
 #include "../runtime.hpp"
+#include "sm100.cuh"
 
 namespace fxf {
 namespace {
@@ -47,6 +48,7 @@ template <int OP> __device__ __forceinline__ float4 apply4(float4 a, float4 b) {
 template <int OP>
 __global__ void __launch_bounds__(kThreads) binary_vec4_kernel(const float4* __restrict__ a, const float4* __restrict__ b,
                                                                float4* __restrict__ out, int64_t n4, int64_t nb4) {
+    sm100::grid_dep();
     int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += stride) {
         float4 va = a[i];
@@ -65,6 +67,7 @@ struct BroadcastDesc {
 template <int OP>
 __global__ void __launch_bounds__(kThreads) binary_generic_kernel(const float* __restrict__ a, const float* __restrict__ b,
                                                                   float* __restrict__ out, int64_t n, BroadcastDesc d) {
+    sm100::grid_dep();
     int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
         int64_t rem = i, oa = 0, ob = 0;
@@ -117,7 +120,7 @@ int run_binary(const FxfTensor& a, const FxfTensor& b, const FxfTensor& out, Exe
     if (flat) { b_suffix = true; nb = n; na = n; }
     if (na == n && (flat || is_contiguous(a)) && b_suffix && n % 4 == 0 && nb % 4 == 0 && aligned16(a.ptr) && aligned16(b.ptr) && aligned16(out.ptr)) {
         int64_t n4 = n / 4;
-        binary_vec4_kernel<OP><<<grid_for(n4, ctx), kThreads, 0, ctx.stream>>>(
+        dependent(binary_vec4_kernel<OP>, grid_for(n4, ctx), kThreads, 0, ctx)(
             static_cast<const float4*>(a.ptr), static_cast<const float4*>(b.ptr), static_cast<float4*>(out.ptr), n4, nb / 4);
     } else {
         if (flat) {  // identical layouts but not 16-byte friendly: walk storage order with unit strides
@@ -125,7 +128,7 @@ int run_binary(const FxfTensor& a, const FxfTensor& b, const FxfTensor& out, Exe
             d.shape[0] = n;
             d.sa[0] = d.sb[0] = 1;
         }
-        binary_generic_kernel<OP><<<grid_for(n, ctx), kThreads, 0, ctx.stream>>>(
+        dependent(binary_generic_kernel<OP>, grid_for(n, ctx), kThreads, 0, ctx)(
             static_cast<const float*>(a.ptr), static_cast<const float*>(b.ptr), static_cast<float*>(out.ptr), n, d);
     }
     FXF_LAUNCHED(ctx);
@@ -140,6 +143,7 @@ template <int OP> __device__ __forceinline__ float unary(float x, float s) {
 }
 template <int OP>
 __global__ void __launch_bounds__(kThreads) unary_vec4_kernel(const float4* x, float4* out, int64_t n4, float s) {
+    sm100::grid_dep();
     int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += stride) {
         float4 v = x[i];
@@ -148,6 +152,7 @@ __global__ void __launch_bounds__(kThreads) unary_vec4_kernel(const float4* x, f
 }
 template <int OP>
 __global__ void __launch_bounds__(kThreads) unary_kernel(const float* x, float* out, int64_t n, float s) {
+    sm100::grid_dep();
     int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = unary<OP>(x[i], s);
 }
@@ -159,9 +164,9 @@ int run_unary(const FxfTensor& x, const FxfTensor& out, float s, ExecCtx& ctx) {
     FXF_CHECK(same_layout(x, out) || (is_contiguous(x) && is_contiguous(out)), "unary op: input and output layouts differ");
     if (n == 0) return 0;
     if (n % 4 == 0 && aligned16(x.ptr) && aligned16(out.ptr)) {
-        unary_vec4_kernel<OP><<<grid_for(n / 4, ctx), kThreads, 0, ctx.stream>>>(static_cast<const float4*>(x.ptr), static_cast<float4*>(out.ptr), n / 4, s);
+        dependent(unary_vec4_kernel<OP>, grid_for(n / 4, ctx), kThreads, 0, ctx)(static_cast<const float4*>(x.ptr), static_cast<float4*>(out.ptr), n / 4, s);
     } else {
-        unary_kernel<OP><<<grid_for(n, ctx), kThreads, 0, ctx.stream>>>(static_cast<const float*>(x.ptr), static_cast<float*>(out.ptr), n, s);
+        dependent(unary_kernel<OP>, grid_for(n, ctx), kThreads, 0, ctx)(static_cast<const float*>(x.ptr), static_cast<float*>(out.ptr), n, s);
     }
     FXF_LAUNCHED(ctx);
     return 0;
@@ -169,6 +174,7 @@ int run_unary(const FxfTensor& x, const FxfTensor& out, float s, ExecCtx& ctx) {
 
 // ---- size ---------------------------------------------------------------------------------
 __global__ void fill_i64_kernel(int64_t* out, int64_t v, int64_t n) {
+    sm100::grid_dep();
     int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) out[i] = v;
 }
@@ -176,6 +182,7 @@ __global__ void fill_i64_kernel(int64_t* out, int64_t v, int64_t n) {
 // ---- strided row copy (narrow) --------------------------------------------------------------
 // rows x row_bytes, source rows `src_pitch` bytes apart.  16-byte words when aligned.
 __global__ void __launch_bounds__(kThreads) rowcopy16_kernel(const uint4* src, uint4* dst, int64_t rows, int64_t row_w, int64_t src_pitch_w) {
+    sm100::grid_dep();
     int64_t total = rows * row_w, stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
         int64_t r = i / row_w, c = i - r * row_w;
@@ -184,6 +191,7 @@ __global__ void __launch_bounds__(kThreads) rowcopy16_kernel(const uint4* src, u
 }
 template <typename T>
 __global__ void __launch_bounds__(kThreads) rowcopy_kernel(const T* src, T* dst, int64_t rows, int64_t row_w, int64_t src_pitch_w) {
+    sm100::grid_dep();
     int64_t total = rows * row_w, stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
         int64_t r = i / row_w, c = i - r * row_w;
@@ -194,6 +202,7 @@ __global__ void __launch_bounds__(kThreads) rowcopy_kernel(const T* src, T* dst,
 // ---- embedding ----------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads) embedding_vec4_kernel(const int64_t* __restrict__ idx, const float4* __restrict__ w, float4* __restrict__ out,
                                                                   int64_t n_idx, int64_t d4, int64_t vocab, int* status) {
+    sm100::grid_dep();
     int64_t total = n_idx * d4, stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
         int64_t r = i / d4, c = i - r * d4;
@@ -208,6 +217,7 @@ __global__ void __launch_bounds__(kThreads) embedding_vec4_kernel(const int64_t*
 }
 __global__ void __launch_bounds__(kThreads) embedding_kernel(const int64_t* __restrict__ idx, const float* __restrict__ w, float* __restrict__ out,
                                                              int64_t n_idx, int64_t d, int64_t vocab, int* status) {
+    sm100::grid_dep();
     int64_t total = n_idx * d, stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
         int64_t r = i / d, c = i - r * d;
@@ -229,6 +239,7 @@ struct TransposeDesc {
 };
 template <typename T>
 __global__ void __launch_bounds__(kThreads) transpose_generic_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t n, TransposeDesc d) {
+    sm100::grid_dep();
     int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
         int64_t rem = i, off = 0;
@@ -243,6 +254,7 @@ __global__ void __launch_bounds__(kThreads) transpose_generic_kernel(const T* __
 // Batched [R, C] -> [C, R] through a 32x33 shared tile: both the read and the write are coalesced.
 template <typename T>
 __global__ void __launch_bounds__(256) transpose_tile_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t R, int64_t C, int64_t tiles_r, int64_t tiles_c, int64_t n_tiles) {
+    sm100::grid_dep();
     __shared__ T tile[32][33];
     int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
     for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
@@ -276,7 +288,7 @@ int run_transpose_typed(const FxfTensor& x, const FxfTensor& out, int d0, int d1
         int64_t R = x.shape[d0], C = x.shape[d1], batch = n / (R * C);
         int64_t tr = (R + 31) / 32, tc = (C + 31) / 32, tiles = batch * tr * tc;
         int grid = int(tiles < int64_t(ctx.sm_count) * 8 ? tiles : int64_t(ctx.sm_count) * 8);
-        transpose_tile_kernel<T><<<grid, 256, 0, ctx.stream>>>(static_cast<const T*>(x.ptr), static_cast<T*>(out.ptr), R, C, tr, tc, tiles);
+        dependent(transpose_tile_kernel<T>, grid, 256, 0, ctx)(static_cast<const T*>(x.ptr), static_cast<T*>(out.ptr), R, C, tr, tc, tiles);
     } else {
         TransposeDesc d;
         d.rank = rank;
@@ -285,7 +297,7 @@ int run_transpose_typed(const FxfTensor& x, const FxfTensor& out, int d0, int d1
             d.out_shape[k] = x.shape[src];
             d.in_stride_perm[k] = x.stride[src];
         }
-        transpose_generic_kernel<T><<<grid_for(n, ctx), kThreads, 0, ctx.stream>>>(static_cast<const T*>(x.ptr), static_cast<T*>(out.ptr), n, d);
+        dependent(transpose_generic_kernel<T>, grid_for(n, ctx), kThreads, 0, ctx)(static_cast<const T*>(x.ptr), static_cast<T*>(out.ptr), n, d);
     }
     FXF_LAUNCHED(ctx);
     return 0;
@@ -339,7 +351,7 @@ int k_size(Registry& reg, const TensorIds& in, const TensorIds& out, const Param
     FXF_CHECK(dim >= 0 && dim < x.rank, "size: dim out of range");
     FXF_CHECK(o.dtype == FXF_I64, "size: output must be int64");
     int64_t n = numel(o);
-    fill_i64_kernel<<<int((n + 255) / 256), 256, 0, ctx.stream>>>(static_cast<int64_t*>(o.ptr), x.shape[dim], n);
+    dependent(fill_i64_kernel, int((n + 255) / 256), 256, 0, ctx)(static_cast<int64_t*>(o.ptr), x.shape[dim], n);
     FXF_LAUNCHED(ctx);
     return 0;
 }
@@ -367,13 +379,13 @@ int k_narrow(Registry& reg, const TensorIds& in, const TensorIds& out, const Par
     const char* src = static_cast<const char*>(x.ptr) + start * inner * esz;
     char* dst = static_cast<char*>(o.ptr);
     if (row_bytes % 16 == 0 && pitch % 16 == 0 && aligned16(src) && aligned16(dst)) {
-        rowcopy16_kernel<<<grid_for(outer * row_bytes / 16, ctx), kThreads, 0, ctx.stream>>>(
+        dependent(rowcopy16_kernel, grid_for(outer * row_bytes / 16, ctx), kThreads, 0, ctx)(
             reinterpret_cast<const uint4*>(src), reinterpret_cast<uint4*>(dst), outer, row_bytes / 16, pitch / 16);
     } else if (esz == 4) {
-        rowcopy_kernel<uint32_t><<<grid_for(outer * row_bytes / 4, ctx), kThreads, 0, ctx.stream>>>(
+        dependent(rowcopy_kernel<uint32_t>, grid_for(outer * row_bytes / 4, ctx), kThreads, 0, ctx)(
             reinterpret_cast<const uint32_t*>(src), reinterpret_cast<uint32_t*>(dst), outer, row_bytes / 4, pitch / 4);
     } else {
-        rowcopy_kernel<uint8_t><<<grid_for(outer * row_bytes, ctx), kThreads, 0, ctx.stream>>>(
+        dependent(rowcopy_kernel<uint8_t>, grid_for(outer * row_bytes, ctx), kThreads, 0, ctx)(
             reinterpret_cast<const uint8_t*>(src), reinterpret_cast<uint8_t*>(dst), outer, row_bytes, pitch);
     }
     FXF_LAUNCHED(ctx);
@@ -390,10 +402,10 @@ int k_embedding(Registry& reg, const TensorIds& in, const TensorIds& out, const 
     FXF_CHECK(numel(o) == n_idx * D, "embedding: output size mismatch");
     if (n_idx * D == 0) return 0;
     if (D % 4 == 0 && aligned16(w.ptr) && aligned16(o.ptr)) {
-        embedding_vec4_kernel<<<grid_for(n_idx * D / 4, ctx), kThreads, 0, ctx.stream>>>(
+        dependent(embedding_vec4_kernel, grid_for(n_idx * D / 4, ctx), kThreads, 0, ctx)(
             static_cast<const int64_t*>(idx.ptr), static_cast<const float4*>(w.ptr), static_cast<float4*>(o.ptr), n_idx, D / 4, V, ctx.status);
     } else {
-        embedding_kernel<<<grid_for(n_idx * D, ctx), kThreads, 0, ctx.stream>>>(
+        dependent(embedding_kernel, grid_for(n_idx * D, ctx), kThreads, 0, ctx)(
             static_cast<const int64_t*>(idx.ptr), static_cast<const float*>(w.ptr), static_cast<float*>(o.ptr), n_idx, D, V, ctx.status);
     }
     FXF_LAUNCHED(ctx);

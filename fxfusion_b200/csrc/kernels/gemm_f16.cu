@@ -197,7 +197,6 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     if (PAIR) cluster_sync_all();   // the other CTA's barriers exist before anything of this CTA signals them
     tc_fence_after();
     const uint32_t tmem_base = s.tmem_base;
-    grid_dep_launch();
 
     // 384 x 168 registers at launch = 256 x 208 + 128 x 88
     if (warp >= kEpiWarps) {
@@ -374,6 +373,9 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 }
             }
             if (!alive) break;
+            // The next kernel may become resident once every CTA has come to its last store; earlier, its blocks would pile up on the
+            // SMs this launch leaves idle and run there one after the other.
+            if (unit + sched_n >= num_units) grid_dep_launch();
             if (adds_partials) {
                 int ok = 1;
                 if (lane == 0)

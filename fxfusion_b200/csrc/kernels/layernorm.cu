@@ -31,8 +31,7 @@ template <int NV, bool ADD, int FORM>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) layernorm_warp_kernel(const float4* __restrict__ x, const float4* __restrict__ z,
                                                                              const float4* __restrict__ w, const float4* __restrict__ b,
                                                                              float4* __restrict__ out, SplitOut so, int64_t M, int n4, float inv_n, float eps) {
-    sm100::grid_dep_launch();
-    sm100::grid_dep_wait();
+    sm100::grid_dep();
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int64_t row_stride = int64_t(gridDim.x) * kWarpsPerBlock;
     for (int64_t row = int64_t(blockIdx.x) * kWarpsPerBlock + warp; row < M; row += row_stride) {
@@ -123,6 +122,7 @@ __device__ float block_sum(float v, float* red) {
 template <bool ADD>
 __global__ void __launch_bounds__(256) layernorm_block_kernel(const float* __restrict__ x, const float* __restrict__ z, const float* __restrict__ w,
                                                               const float* __restrict__ b, float* __restrict__ out, int64_t M, int64_t N, float inv_n, float eps) {
+    sm100::grid_dep();
     __shared__ float red[32];
     for (int64_t row = blockIdx.x; row < M; row += gridDim.x) {
         const float* xr = x + row * N;
@@ -181,7 +181,7 @@ int run_layernorm(const float* x, const float* z, const float* w, const float* b
         FXF_CHECK(so.planes == nullptr, "layer_norm: rows this wide have no split form");
         int64_t cap = int64_t(ctx.sm_count) * 8;
         int grid = int(M < cap ? M : cap);
-        layernorm_block_kernel<ADD><<<grid, 256, 0, ctx.stream>>>(x, z, w, b, out, M, N, inv_n, eps);
+        dependent(layernorm_block_kernel<ADD>, grid, 256, 0, ctx)(x, z, w, b, out, M, N, inv_n, eps);
     }
     FXF_LAUNCHED(ctx);
     return 0;

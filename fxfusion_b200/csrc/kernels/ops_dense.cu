@@ -24,6 +24,7 @@
 #include <algorithm>
 
 #include "../runtime.hpp"
+#include "sm100.cuh"
 
 namespace fxf {
 
@@ -38,6 +39,7 @@ static bool use_tc(const GemmArgs& a, int gemm_mode) {
 
 namespace {
 __global__ void __launch_bounds__(256) residual_epilogue_kernel(float* __restrict__ out, const float* __restrict__ res, int64_t n, int relu) {
+    sm100::grid_dep();
     int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
         float v = out[i] + res[i];
@@ -51,7 +53,7 @@ int launch_residual_epilogue(float* out, const float* residual, int64_t n, bool 
     if (n == 0) return 0;
     int64_t blocks = (n + 255) / 256, cap = int64_t(ctx.sm_count) * 8;
     tag_launch(ctx, "residual_epilogue", double(n), 12.0 * double(n));
-    residual_epilogue_kernel<<<int(blocks < cap ? blocks : cap), 256, 0, ctx.stream>>>(out, residual, n, relu ? 1 : 0);
+    dependent(residual_epilogue_kernel, int(blocks < cap ? blocks : cap), 256, 0, ctx)(out, residual, n, relu ? 1 : 0);
     FXF_LAUNCHED(ctx);
     return 0;
 }
@@ -805,12 +807,97 @@ __device__ __forceinline__ float block_reduce(float v, float* red, bool is_max) 
     return r;
 }
 
-// One block per (head, sequence).  Phase 1: one key per thread (independent 16-byte loads of whole key rows keep many
+// Head sizes 32, 64 and 128.  One block per (head, sequence); HD / 4 lanes hold one key, so a key's row (and its value row) is
+// one coalesced access, and every lane group walks its own keys with an online softmax: four keys' K and V rows, eight 16-byte
+// loads per lane, are in flight before the first is used.  The groups' (max, sum, context) are merged through shared memory.
+// The row of the new position is taken from qkv (and stored): nothing in the kernel waits for that store.
+// Bound: HBM (the cache).  32 sequences, 12 heads, 256 positions (50 MB): 28 -> 10 us, 5 TB/s; the kernel it replaces had one key
+// per thread, that is 32 different rows in one load.
+template <int HD>
+__global__ void __launch_bounds__(kCachedAttnThreads) cached_attn_groups_kernel(const float* __restrict__ qkv, float* __restrict__ cache, const int64_t* __restrict__ tokens,
+                                                                                const int64_t* __restrict__ pos_ptr, float* __restrict__ ctxo, int T, int D, float scale_divisor,
+                                                                                int64_t pad, int* status) {
+    constexpr int L = HD / 4, GROUPS = kCachedAttnThreads / L, UNROLL = 4;
+    __shared__ float gm[GROUPS], gl[GROUPS];
+    __shared__ float go[GROUPS][HD + 4];
+    sm100::grid_dep();
+    const int h = blockIdx.x, b = blockIdx.y, l = threadIdx.x % L, g = threadIdx.x / L;
+    const int64_t pos64 = *pos_ptr;
+    if (pos64 < 0 || pos64 >= T) {   // uniform: a position outside the cache is reported, nothing is written
+        if (threadIdx.x == 0 && status) atomicCAS(status, 0, 3);
+        return;
+    }
+    const int pos = int(pos64), n_keys = pos + 1;
+    float* rows = cache + int64_t(b) * T * 2 * D + h * HD + l * 4;
+    const float* qrow = qkv + int64_t(b) * 3 * D + h * HD + l * 4;
+    const float4 q = *reinterpret_cast<const float4*>(qrow), knew = *reinterpret_cast<const float4*>(qrow + D), vnew = *reinterpret_cast<const float4*>(qrow + 2 * D);
+    if (g == 0) {
+        *reinterpret_cast<float4*>(rows + int64_t(pos) * 2 * D) = knew;
+        *reinterpret_cast<float4*>(rows + int64_t(pos) * 2 * D + D) = vnew;
+    }
+    float m = -INFINITY, sum = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int64_t* tok = tokens + int64_t(b) * T;
+    for (int jb = 0; jb < n_keys; jb += GROUPS * UNROLL) {   // the same trip count for every lane: the shuffles below span groups
+        const int j0 = jb + g;
+        float4 k[UNROLL], v[UNROLL];
+        bool in[UNROLL], keep[UNROLL];
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) {
+            const int j = j0 + u * GROUPS;
+            in[u] = j < n_keys;
+            k[u] = knew; v[u] = vnew;
+            if (in[u] && j != pos) {
+                k[u] = *reinterpret_cast<const float4*>(rows + int64_t(j) * 2 * D);
+                v[u] = *reinterpret_cast<const float4*>(rows + int64_t(j) * 2 * D + D);
+            }
+            keep[u] = in[u] && tok[j] != pad;
+        }
+        float s[UNROLL], mx = m;
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) {
+            float d = fmaf(q.x, k[u].x, fmaf(q.y, k[u].y, fmaf(q.z, k[u].z, q.w * k[u].w)));
+#pragma unroll
+            for (int w = L / 2; w > 0; w >>= 1) d += __shfl_xor_sync(0xffffffffu, d, w);
+            s[u] = keep[u] ? d / scale_divisor : -INFINITY;
+            mx = fmaxf(mx, s[u]);   // a NaN score does not move the maximum; it reaches the sum below
+        }
+        const float ms = mx == -INFINITY ? 0.f : mx, alpha = expf(m - ms);
+        m = mx;
+        sum *= alpha;
+        o.x *= alpha; o.y *= alpha; o.z *= alpha; o.w *= alpha;
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++)
+            if (in[u]) {   // masked keys keep their (zero-weighted) value row: a NaN there poisons the context
+                const float p = expf(s[u] - ms);
+                sum += p;
+                o.x = fmaf(p, v[u].x, o.x); o.y = fmaf(p, v[u].y, o.y); o.z = fmaf(p, v[u].z, o.z); o.w = fmaf(p, v[u].w, o.w);
+            }
+    }
+    *reinterpret_cast<float4*>(&go[g][l * 4]) = o;
+    if (l == 0) { gm[g] = m; gl[g] = sum; }
+    __syncthreads();
+    if (threadIdx.x < HD) {
+        float mall = -INFINITY;
+        for (int i = 0; i < GROUPS; i++) mall = fmaxf(mall, gm[i]);
+        const float ms = mall == -INFINITY ? 0.f : mall;
+        float acc = 0.f, lall = 0.f;
+        for (int i = 0; i < GROUPS; i++) {
+            const float a = expf(gm[i] - ms);
+            acc = fmaf(a, go[i][threadIdx.x], acc);
+            lall = fmaf(a, gl[i], lall);
+        }
+        ctxo[int64_t(b) * D + h * HD + threadIdx.x] = acc / lall;   // 0/0 = NaN when every key is masked
+    }
+}
+
+// Any other head size.  One block per (head, sequence).  Phase 1: one key per thread (independent 16-byte loads of whole key rows keep many
 // requests in flight), scores to shared memory; phase 2: probabilities; phase 3: threads = (output dim, key residue class),
 // value rows read coalesced.  Dynamic shared memory: T scores.
 __global__ void __launch_bounds__(kCachedAttnThreads) cached_attn_kernel(const float* __restrict__ qkv, float* __restrict__ cache, const int64_t* __restrict__ tokens,
                                                                          const int64_t* __restrict__ pos_ptr, float* __restrict__ ctxo, int T, int D, int hd,
                                                                          float scale_divisor, int64_t pad, int* status) {
+    sm100::grid_dep();
     extern __shared__ float scores[];
     __shared__ float red[kCachedAttnThreads / 32], qs[128], part_o[kCachedAttnThreads];
     const int h = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
@@ -915,10 +1002,16 @@ int k_cached_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const
         if (launch_gemm(g, ctx)) return 1;
     }
     tag_launch(ctx, "cached_attention_fp32", 4.0 * double(B) * H * double(T) * hd, 4.0 * 2.0 * double(B) * T * D);
-    FXF_CHECK(T * sizeof(float) <= 160 * 1024, "cached_mha: static length %lld is too long for the score buffer", (long long)T);
-    if (size_t(T) * sizeof(float) > 40 * 1024) FXF_CUDA(cudaFuncSetAttribute(cached_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(T * sizeof(float))));
-    cached_attn_kernel<<<dim3(unsigned(H), unsigned(B)), kCachedAttnThreads, size_t(T) * sizeof(float), ctx.stream>>>(
-        qkv, cache, static_cast<const int64_t*>(tok.ptr), static_cast<const int64_t*>(pos.ptr), cx, int(T), int(D), int(hd), p.floats[0], p.ints[4], ctx.status);
+    const dim3 attn_grid{unsigned(H), unsigned(B)};
+    const int64_t *tokp = static_cast<const int64_t*>(tok.ptr), *posp = static_cast<const int64_t*>(pos.ptr);
+    if ((hd == 32 || hd == 64 || hd == 128) && aligned16(qkv) && aligned16(cache)) {
+        auto kernel = hd == 32 ? cached_attn_groups_kernel<32> : (hd == 64 ? cached_attn_groups_kernel<64> : cached_attn_groups_kernel<128>);
+        dependent(kernel, attn_grid, kCachedAttnThreads, 0, ctx)(qkv, cache, tokp, posp, cx, int(T), int(D), p.floats[0], p.ints[4], ctx.status);
+    } else {
+        FXF_CHECK(T * sizeof(float) <= 160 * 1024, "cached_mha: static length %lld is too long for the score buffer", (long long)T);
+        if (size_t(T) * sizeof(float) > 40 * 1024) FXF_CUDA(cudaFuncSetAttribute(cached_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(T * sizeof(float))));
+        dependent(cached_attn_kernel, attn_grid, kCachedAttnThreads, size_t(T) * sizeof(float), ctx)(qkv, cache, tokp, posp, cx, int(T), int(D), int(hd), p.floats[0], p.ints[4], ctx.status);
+    }
     FXF_LAUNCHED(ctx);
     if (pl->s[2].f16) return f16_product(pl->s[2], &pl->s[3], cx, D, nullptr, static_cast<float*>(o.ptr), B, D, false, true, area, ctx);
     GemmArgs g2;

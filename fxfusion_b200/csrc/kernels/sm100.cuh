@@ -95,6 +95,10 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
 // launch signal lets the next kernel become resident (its own wait still holds it back until this one has finished).
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep() {   // first statement of a kernel with nothing to do ahead of its inputs
+    grid_dep_launch();
+    grid_dep_wait();
+}
 
 // ---- split form of an fp32 row: two fp16 planes of x * scale, scale a power of two ------------------------------------
 // scale = the power of two that brings `bound` into [2^14, 2^15]; inv = 1 / scale.  Bounds below 2^-99 count as 2^-99.

@@ -388,6 +388,21 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// dependent(kernel, grid, block, smem, ctx)(args...): the same with the look of a kernel launch; errors surface in FXF_LAUNCHED.
+template <class... KArgs>
+struct DependentLaunch {
+    void (*kernel)(KArgs...);
+    dim3 grid, block;
+    size_t smem;
+    cudaStream_t stream;
+    template <class... Args>
+    void operator()(Args... args) const { (void)launch_dependent(kernel, grid, block, smem, stream, 1, args...); }
+};
+template <class... KArgs>
+inline DependentLaunch<KArgs...> dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, const ExecCtx& ctx) {
+    return {kernel, grid, block, smem, ctx.stream};
+}
+
 // Convolution (stride 1 or 2) as an implicit GEMM on the tensor cores: channels-last activation x [N,H,W,C], weights
 // repacked to [O, KH*KW*C] (tap-major, channel-minor) and split into TF32 hi/lo, channels-last output [N,HO,WO,O].
 struct ConvTcArgs {
