@@ -74,6 +74,7 @@ struct Node {
     bool splits = false;
     size_t split_off = 0;
     int split_parts = 1;
+    bool clears_images = false;   // the first node on images in split form: the maxima of all of them are zeroed before it
 };
 
 }  // namespace
@@ -114,6 +115,7 @@ struct fxf_engine {
     bool peers_mapped = false;
     std::vector<SplitMat> splits;      // by tensor id: activations kept in split form in their arena slots
     std::vector<uint32_t> split_root;  // by tensor id: the tensor whose storage it shares
+    size_t image_off = 0, image_bytes = 0;   // scales and maxima of images in split form
     // decode that evaluates the final Linear only at the position whose logits are read
     int tail_node = -1;                // index of that Linear (the last node), -1 when the graph does not end in one
     size_t lastrow_off = 0, lastrow_bytes = 0;  // its [B,V] output
@@ -150,6 +152,7 @@ int run_node(fxf_engine* e, size_t i) {
         e->ctx.fuse.residual = static_cast<const float*>(e->reg[size_t(n.fuse_res)].ptr);
         e->ctx.fuse.out = static_cast<float*>(e->reg[size_t(n.fuse_out)].ptr);
         e->ctx.fuse.relu = n.fuse_relu;
+        e->ctx.fuse.residual_id = n.fuse_res;
     }
     e->ctx.xchg = TpExchange{};
     if (n.xchg) {
@@ -164,7 +167,15 @@ int run_node(fxf_engine* e, size_t i) {
         e->ctx.xchg.replicate_x = n.xchg_replicate_x;
     }
     e->ctx.split_out = SplitOut{};
-    if (n.splits) {
+    if (n.clears_images) FXF_CUDA(cudaMemsetAsync(e->base + e->image_off, 0, e->image_bytes, e->ctx.stream));
+    if (n.splits && n.plan->images) {
+        const SplitMat& m = e->splits[n.fuse_out >= 0 ? size_t(n.fuse_out) : n.out[0]];
+        SplitOut& so = e->ctx.split_out;
+        so.planes = const_cast<uint16_t*>(m.planes);
+        so.plane = m.plane;
+        so.inv = const_cast<float*>(m.inv);
+        so.amax = const_cast<float*>(m.amax);
+    } else if (n.splits) {
         const int64_t rows = n.plan->split_rows;
         SplitOut& so = e->ctx.split_out;
         so.planes = static_cast<uint16_t*>(e->reg[n.out[0]].ptr);
@@ -174,7 +185,7 @@ int run_node(fxf_engine* e, size_t i) {
         so.parts_out = &n.split_parts;
     }
     if (n.fn(e->reg, n.in, n.out, n.params, n.plan.get(), e->ctx)) return 1;
-    if (n.splits)
+    if (n.splits && !n.plan->images)
         for (size_t id = 0; id < e->splits.size(); id++)
             if (e->split_root[id] == e->split_root[n.out[0]]) e->splits[id].parts = n.split_parts;
     if (n.fuse_out >= 0) {
@@ -452,6 +463,14 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             n.split_off = cursor;
             cursor = round_up(cursor + size_t(n.plan->split_rows) * sizeof(float) * size_t(1 + parts), kAlign);
         }
+    e->image_off = cursor;
+    for (auto& n : e->nodes)
+        if (n.plan->image_role != NodePlan::kNoImages) {
+            n.split_off = cursor;
+            cursor = round_up(cursor + size_t(e->reg[n.out[0]].shape[0]) * sizeof(float) * 2, 16);
+        }
+    e->image_bytes = cursor - e->image_off;
+    cursor = round_up(cursor, kAlign);
     e->total_bytes = cursor;
 
     // ---- the one device allocation -----------------------------------------------------------
@@ -639,8 +658,8 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
         for (size_t bi = 1; !e->opts.no_epilogue_fusion && bi < e->nodes.size(); bi++) {
             Node &A = e->nodes[bi - 1], &B = e->nodes[bi];
             if ((B.op != FXF_OP_ADD && B.op != FXF_OP_ADD_RELU) || B.in.size() != 2 || B.out.size() != 1 || B.folded || A.xchg) continue;
-            // Convolutions are left alone: their layers are bandwidth-bound with short K loops, and the residual read in the
-            // GEMM epilogue (16 KB in flight per SM) is slower than the separate AddRelu kernel (measured on ResNet-50).
+            // Convolutions fold theirs below, where they work on images in split form (their epilogue requests the residual ahead
+            // of its use); on fp32 images the residual read in the epilogue is slower than the separate AddRelu kernel.
             if (A.op != FXF_OP_LINEAR && A.op != FXF_OP_FEEDFORWARD && A.op != FXF_OP_MHA && A.op != FXF_OP_CROSS_MHA && A.op != FXF_OP_CACHED_MHA) continue;
             if (A.fuse_out >= 0 || A.out.size() != 1) continue;
             if (B.op == FXF_OP_ADD_RELU && A.plan->tp_sharded) continue;   // the ReLU would have to follow the all-reduce
@@ -677,9 +696,108 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
 
         // -- an activation that only feeds products of the f16 GEMM is written in that GEMM's operand form by the node that
         // produces it (same bytes, same arena slot): no conversion pass, and the GEMM has nothing to convert.
+        // -- images in split form: a channels-last activation whose producer and readers all can keep it so (convolutions, max
+        // pooling, the residual Add of a convolution, global average pooling) is kept in the operand form of the f16 product, with
+        // one scale per image (kernels/gemm_f16.cu).  Optimistic set of tensors, demoted until every producer and reader agrees.
+        struct ImageFold { int add = -1; uint32_t res = 0, out = 0; bool relu = false; };
+        std::vector<ImageFold> folds(e->nodes.size());
+        std::vector<char> images(n_tensors, 0);
+        auto image_tensor = [&](uint32_t id) {
+            const FxfTensor& t = e->reg[id];
+            int64_t lo = 0, hi = 0;
+            return root(id) == id && meta[id].kind == kActivation && !escapes[id] && t.rank == 4 && t.dtype == FXF_F32 && t.shape[1] % 8 == 0 &&
+                   (is_channels_last(t) || (is_contiguous(t) && t.shape[2] * t.shape[3] == 1)) && numel(t) > 0 && arena_range(id, &lo, &hi);
+        };
+        auto overlap = [&](uint32_t a, uint32_t b) {
+            int64_t al = 0, ah = 0, bl = 0, bh = 0;
+            return arena_range(a, &al, &ah) && arena_range(b, &bl, &bh) && al < bh && bl < ah;
+        };
+        for (size_t i = 0; i < e->nodes.size(); i++) {
+            Node& n = e->nodes[i];
+            if (n.op == FXF_OP_MAX_POOL2D && e->reg[n.out[0]].rank == 4) n.plan->image_role = NodePlan::kImageMaxPool;
+            if (n.op == FXF_OP_ADAPTIVE_AVG_POOL2D && e->reg[n.out[0]].rank == 4 && e->reg[n.out[0]].shape[2] * e->reg[n.out[0]].shape[3] == 1 && is_contiguous(e->reg[n.out[0]]) &&
+                e->reg[n.out[0]].shape[0] <= 65535)
+                n.plan->image_role = NodePlan::kImageGlobalAvg;
+            const auto role = n.plan->image_role;
+            if (role == NodePlan::kNoImages || role == NodePlan::kImageGlobalAvg || n.out.size() != 1) continue;
+            uint32_t t = n.out[0];
+            if (role != NodePlan::kImageMaxPool && !e->opts.no_epilogue_fusion && i + 1 < e->nodes.size()) {
+                const Node& B = e->nodes[i + 1];   // the conditions of the fold above, and neither operand of the convolution may lie under the result
+                if ((B.op == FXF_OP_ADD || B.op == FXF_OP_ADD_RELU) && B.in.size() == 2 && B.out.size() == 1 && !B.folded && n_readers[t] == 1 && !escapes[t] &&
+                    (B.in[0] == t) != (B.in[1] == t)) {
+                    const uint32_t r = B.in[0] == t ? B.in[1] : B.in[0], o = B.out[0];
+                    if (image_tensor(r) && image_tensor(o) && same_shape(t, r) && same_shape(t, o) && producer[r] < int(i) && !overlap(r, o) && !overlap(n.in[0], o)) {
+                        folds[i] = ImageFold{int(i) + 1, r, o, B.op == FXF_OP_ADD_RELU};
+                        t = o;
+                    }
+                }
+            }
+            if (image_tensor(t)) images[t] = 1;
+        }
+        auto active = [&](size_t i) {
+            const Node& n = e->nodes[i];
+            const ImageFold& f = folds[i];
+            if (f.add >= 0 && !(images[f.res] && images[f.out])) return false;
+            const uint32_t o = f.add >= 0 ? f.out : n.out[0];
+            const FxfTensor& to = e->reg[o];   // what is not kept in split form leaves as fp32 pixels
+            if (!images[o] && !(is_channels_last(to) || (is_contiguous(to) && to.rank == 4 && (to.shape[2] * to.shape[3] == 1 || to.shape[1] == 1)))) return false;
+            switch (n.plan->image_role) {
+                case NodePlan::kImageConv: return images[n.in[0]] != 0;
+                case NodePlan::kImageStem: return true;
+                case NodePlan::kImageMaxPool: return images[n.in[0]] && images[n.out[0]];
+                case NodePlan::kImageGlobalAvg: return images[n.in[0]] != 0;
+                default: return false;
+            }
+        };
+        for (bool changed = true; changed;) {
+            changed = false;
+            for (uint32_t t = 0; t < n_tensors; t++) {
+                if (!images[t]) continue;
+                bool ok = false;
+                for (size_t i = 0; i < e->nodes.size(); i++) {
+                    const Node& n = e->nodes[i];
+                    if ((folds[i].add >= 0 ? folds[i].out : n.out[0]) == t && n.plan->image_role != NodePlan::kNoImages) ok = active(i);
+                }
+                for (size_t i = 0; i < e->nodes.size() && ok; i++)
+                    for (size_t k = 0; k < e->nodes[i].in.size(); k++) {
+                        const uint32_t id = e->nodes[i].in[k];
+                        if (root(id) != t) continue;
+                        const bool residual = i > 0 && folds[i - 1].add == int(i) && folds[i - 1].res == t && active(i - 1);
+                        ok = ok && id == t && (residual || (k == 0 && active(i)));
+                    }
+                if (!ok) { images[t] = 0; changed = true; }
+            }
+        }
         e->split_root.resize(n_tensors);
         for (uint32_t id = 0; id < n_tensors; id++) e->split_root[id] = root(id);
         e->splits.assign(n_tensors, SplitMat{});
+        bool first_image = true;
+        for (size_t i = 0; i < e->nodes.size(); i++) {
+            Node& n = e->nodes[i];
+            if (!active(i)) continue;
+            n.plan->images = true;
+            n.clears_images = first_image;
+            first_image = false;
+            const ImageFold& f = folds[i];
+            if (f.add >= 0) {
+                n.fuse_res = int(f.res); n.fuse_out = int(f.out); n.fuse_relu = f.relu;
+                e->nodes[size_t(f.add)].folded = true;
+            }
+            const uint32_t t = f.add >= 0 ? f.out : n.out[0];
+            if (!images[t]) continue;
+            n.splits = true;
+            SplitMat m;
+            m.planes = reinterpret_cast<const uint16_t*>(e->base + meta[t].offset);
+            m.plane = numel(e->reg[t]);
+            if (n.plan->image_role == NodePlan::kImageMaxPool) {   // scales and bounds of its input
+                m.inv = e->splits[n.in[0]].inv;
+                m.amax = e->splits[n.in[0]].amax;
+            } else {
+                m.inv = reinterpret_cast<const float*>(e->base + n.split_off);
+                m.amax = m.inv + e->reg[t].shape[0];
+            }
+            e->splits[t] = m;
+        }
         for (size_t pi = 0; pi < e->nodes.size() && e->opts.tp_size == 1; pi++) {
             Node& P = e->nodes[pi];
             if (!P.plan->makes_split || P.folded || P.xchg || P.fuse_out >= 0 || P.out.size() != 1) continue;

@@ -20,6 +20,9 @@
 //     and ReLU fused in its epilogue (weights split into TF32 hi/lo once, at engine build).
 //   * everything else: an implicit GEMM (rows = output pixels n*Ho*Wo, columns = output channels, depth =
 //     Cin/groups*Kh*Kw) on fp32 FFMA tiles of 64x64x16 with the im2col gather done while the A tile is staged.
+#include <cuda_fp16.h>
+
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 
@@ -271,8 +274,191 @@ __global__ void __launch_bounds__(256) conv_weight_s2d_split_kernel(const float*
     }
 }
 
+// ---- images in split form (one power-of-two scale per image; see gemm_f16.cu) -----------------------------------------
+// Filters of one output channel per block: [O, taps, Cp] with Cp = C padded to whole 64-deep K-slabs (S2D: [O, KH2, 4 pixels,
+// 16 channels] in the space-to-depth order above), as two fp16 planes, 1 / scale per row and the largest L1 norm of a row.
+template <bool S2D>
+__global__ void __launch_bounds__(128) conv_weight_f16_kernel(const float* __restrict__ w, uint16_t* __restrict__ planes, int64_t plane, float* __restrict__ inv_out,
+                                                              float* __restrict__ bound, int C, int KH, int KW, int Cp, int K) {
+    __shared__ float red[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, o = blockIdx.x;
+    const float* wo = w + int64_t(o) * C * KH * KW;
+    auto value = [&](int k) {
+        if (S2D) {
+            const int ch = k & 15, qx = (k >> 4) & 3, qy = k >> 6, r = ch / C, c = ch - r * C, ky = 2 * qy + (r >> 1), kx = 2 * qx + (r & 1);
+            return (r < 4 && ky < KH && kx < KW) ? wo[(c * KH + ky) * KW + kx] : 0.f;
+        }
+        const int tap = k / Cp, c = k - tap * Cp;
+        return c < C ? wo[c * KH * KW + tap] : 0.f;
+    };
+    float m = 0.f, l1 = 0.f;
+    for (int k = threadIdx.x; k < K; k += 128) {
+        const float a = fabsf(value(k));
+        m = fmaxf(m, a);
+        l1 += a;
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+        l1 += __shfl_xor_sync(0xffffffffu, l1, s);
+    }
+    if (lane == 0) { red[warp] = m; red[4 + warp] = l1; }
+    __syncthreads();
+    m = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+    float scale, inv;
+    sm100::split_scale(m, scale, inv);
+    if (threadIdx.x == 0) {
+        inv_out[o] = inv;
+        atomicMax(reinterpret_cast<int*>(bound), __float_as_int((red[4] + red[5] + red[6] + red[7]) * 1.0001f));
+    }
+    for (int k = threadIdx.x * 2; k < K; k += 256) {
+        uint32_t hi, lo;
+        sm100::split_f16x2(value(k) * scale, value(k + 1) * scale, hi, lo);
+        *reinterpret_cast<uint32_t*>(planes + int64_t(o) * K + k) = hi;
+        *reinterpret_cast<uint32_t*>(planes + plane + int64_t(o) * K + k) = lo;
+    }
+}
+
+// Largest finite magnitude of each image in kImageParts parts (grid: parts x images), so that nothing has to be zeroed before.
+constexpr int kImageParts = 16;
+__global__ void __launch_bounds__(256) image_amax_kernel(const float* __restrict__ x, int64_t per_image, float* __restrict__ amax) {
+    __shared__ float red[8];
+    sm100::grid_dep();
+    const float* src = x + int64_t(blockIdx.y) * per_image;
+    float m = 0.f;
+    auto take = [&](float v) {
+        v = fabsf(v);
+        m = fmaxf(m, v < INFINITY ? v : 0.f);
+    };
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && per_image % 4 == 0) {
+        for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < per_image / 4; i += kImageParts * 256) {
+            const float4 v = reinterpret_cast<const float4*>(src)[i];
+            take(v.x); take(v.y); take(v.z); take(v.w);
+        }
+    } else {
+        for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < per_image; i += kImageParts * 256) take(src[i]);
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int j = 1; j < 8; j++) m = fmaxf(m, red[j]);
+        amax[int64_t(blockIdx.y) * kImageParts + blockIdx.x] = m;
+    }
+}
+
+// space_to_depth16_kernel in split form: a thread writes half a pixel (8 channels) of both planes.  Grid: rows x images.
+__global__ void __launch_bounds__(128) space_to_depth16_f16_kernel(const float* __restrict__ x, uint16_t* __restrict__ s, int64_t plane, const float* __restrict__ amax,
+                                                                   float* __restrict__ inv_out, int C, int H, int W, int Hs, int Ws, int ph, int pw, Strides4 xs) {
+    sm100::grid_dep();
+    const int Y = blockIdx.x, n = blockIdx.y;
+    float m = 0.f, scale, inv;
+#pragma unroll
+    for (int j = 0; j < kImageParts; j++) m = fmaxf(m, amax[int64_t(n) * kImageParts + j]);
+    sm100::split_scale(m, scale, inv);
+    if (Y == 0 && threadIdx.x == 0) inv_out[n] = inv;
+    for (int i = threadIdx.x; i < Ws * 2; i += 128) {
+        const int X = i >> 1, half = i & 1;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int ch = half * 8 + j, r = ch / C, c = ch - r * C;   // r = ry*2 + rx
+            const int iy = 2 * Y + (r >> 1) - ph, ix = 2 * X + (r & 1) - pw;
+            v[j] = (r < 4 && iy >= 0 && iy < H && ix >= 0 && ix < W) ? x[int64_t(n) * xs.n + int64_t(c) * xs.c + int64_t(iy) * xs.h + int64_t(ix) * xs.w] : 0.f;
+        }
+        uint4 hi, lo;
+        sm100::split_f16x2(v[0] * scale, v[1] * scale, hi.x, lo.x);
+        sm100::split_f16x2(v[2] * scale, v[3] * scale, hi.y, lo.y);
+        sm100::split_f16x2(v[4] * scale, v[5] * scale, hi.z, lo.z);
+        sm100::split_f16x2(v[6] * scale, v[7] * scale, hi.w, lo.w);
+        uint16_t* dst = s + ((int64_t(n) * Hs + Y) * Ws + X) * 16 + half * 8;
+        *reinterpret_cast<uint4*>(dst) = hi;
+        *reinterpret_cast<uint4*>(dst + plane) = lo;
+    }
+}
+
+__device__ __forceinline__ float2 joined(uint32_t hi, uint32_t lo) {
+    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi)), l = __half22float2(*reinterpret_cast<const __half2*>(&lo));
+    return make_float2(h.x + l.x, h.y + l.y);
+}
+
+// Max pooling of images in split form: the scale of an image is common to its pixels, so the larger hi + lo is the larger value
+// and its two halves are the result; scales and bounds of the input hold for the output.  One thread: 8 channels of a pixel.
+__global__ void __launch_bounds__(256) max_pool_split_kernel(const uint16_t* __restrict__ x, int64_t xplane, uint16_t* __restrict__ out, int64_t oplane, PoolDesc d) {
+    sm100::grid_dep();
+    const int C8 = d.C / 8;
+    const int64_t total = d.N * d.HO * d.WO * C8, stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
+        const int c8 = int(i % C8);
+        const int64_t pix = i / C8;
+        const int ox = int(pix % d.WO), oy = int((pix / d.WO) % d.HO);
+        const int64_t n = pix / (int64_t(d.WO) * d.HO);
+        float best[8];
+        uint16_t hi[8], lo[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) { best[j] = -INFINITY; hi[j] = 0xfc00u; lo[j] = 0; }
+        for (int a = 0; a < d.kh; a++) {
+            const int iy = oy * d.sh - d.ph + a * d.dh;
+            if (iy < 0 || iy >= d.H) continue;
+            for (int b = 0; b < d.kw; b++) {
+                const int ix = ox * d.sw - d.pw + b * d.dw;
+                if (ix < 0 || ix >= d.W) continue;
+                const uint16_t* src = x + ((n * d.H + iy) * d.W + ix) * d.C + c8 * 8;
+                const uint4 h = *reinterpret_cast<const uint4*>(src), l = *reinterpret_cast<const uint4*>(src + xplane);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const uint32_t hw = (&h.x)[j], lw = (&l.x)[j];
+                    const float2 v = joined(hw, lw);
+                    if (v.x > best[2 * j] || v.x != v.x) { best[2 * j] = v.x; hi[2 * j] = uint16_t(hw); lo[2 * j] = uint16_t(lw); }
+                    if (v.y > best[2 * j + 1] || v.y != v.y) { best[2 * j + 1] = v.y; hi[2 * j + 1] = uint16_t(hw >> 16); lo[2 * j + 1] = uint16_t(lw >> 16); }
+                }
+            }
+        }
+        uint4 oh, ol;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            (&oh.x)[j] = uint32_t(hi[2 * j]) | (uint32_t(hi[2 * j + 1]) << 16);
+            (&ol.x)[j] = uint32_t(lo[2 * j]) | (uint32_t(lo[2 * j + 1]) << 16);
+        }
+        uint16_t* dst = out + pix * d.C + c8 * 8;
+        *reinterpret_cast<uint4*>(dst) = oh;
+        *reinterpret_cast<uint4*>(dst + oplane) = ol;
+    }
+}
+
+// Global average of images in split form: a warp takes 32 channels of an image, eight pixels at a time.
+__global__ void __launch_bounds__(128) global_avg_split_kernel(const uint16_t* __restrict__ x, int64_t plane, const float* __restrict__ inv, float* __restrict__ out, int C, int HW) {
+    sm100::grid_dep();
+    const int lane = threadIdx.x & 31, c = ((blockIdx.x * 4 + (threadIdx.x >> 5)) * 4 + (lane & 3)) * 8, n = blockIdx.y;
+    float s[8] = {};
+    if (c < C)
+        for (int i = lane >> 2; i < HW; i += 8) {
+            const uint16_t* src = x + (int64_t(n) * HW + i) * C + c;
+            const uint4 h = *reinterpret_cast<const uint4*>(src), l = *reinterpret_cast<const uint4*>(src + plane);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float2 v = joined((&h.x)[j], (&l.x)[j]);
+                s[2 * j] += v.x;
+                s[2 * j + 1] += v.y;
+            }
+        }
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1)
+#pragma unroll
+        for (int j = 0; j < 8; j++) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+    if (lane < 4 && c < C) {
+        const float f = inv[n];
+        float* dst = out + int64_t(n) * C + c;
+#pragma unroll
+        for (int j = 0; j < 8; j++) dst[j] = s[j] * f / float(HW);
+    }
+}
+
 // ---- host side ----------------------------------------------------------------------------------------
 struct ConvPlan : NodePlan {
+    SplitMat w_split;               // images: the filters for launch_conv_f16
+    int64_t k_split = 0;            // and the length of a filter's row
     bool gemm_1x1 = false;          // planned for the tensor-core GEMM (still needs channels-last tensors at run time)
     bool bf16 = false;              // bf16 mode: one bf16 copy of the weights instead of the TF32 hi/lo pair
     bool igemm_tc = false;          // k x k or strided 1x1, stride <= 2: planned for the tensor-core implicit GEMM (same run-time condition)
@@ -280,7 +466,27 @@ struct ConvPlan : NodePlan {
     int Hs = 0, Ws = 0, KH2 = 0, KW2 = 0;
     int64_t w_elems = 0;
     const float *w_hi = nullptr, *w_lo = nullptr;
+    size_t split_bytes(int64_t O) const { return size_t(O) * size_t(k_split) * 4 + round_up(size_t(O) * 4, 16) + 16; }
+    int prepare_split(const FxfTensor& w, const FxfTensor& b, ExecCtx& ctx) {
+        const int O = int(w.shape[0]), C = int(w.shape[1]), KH = int(w.shape[2]), KW = int(w.shape[3]), K = int(k_split);
+        variant = image_role == kImageStem ? "space-to-depth + tcgen05-f16x3 implicit GEMM on images in split form" : "tcgen05-f16x3 implicit GEMM on images in split form";
+        uint16_t* planes = static_cast<uint16_t*>(persist);
+        float* inv = reinterpret_cast<float*>(planes + int64_t(O) * K * 2);
+        float* bound = inv + round_up(size_t(O), 4);
+        FXF_CUDA(cudaMemsetAsync(bound, 0, 8, ctx.stream));
+        const bool stem = image_role == kImageStem;
+        tag_launch(ctx, "conv_weight_split_f16", 0, 8.0 * double(O) * K);
+        if (stem) conv_weight_f16_kernel<true><<<O, 128, 0, ctx.stream>>>(static_cast<const float*>(w.ptr), planes, int64_t(O) * K, inv, bound, C, KH, KW, 64, K);
+        else conv_weight_f16_kernel<false><<<O, 128, 0, ctx.stream>>>(static_cast<const float*>(w.ptr), planes, int64_t(O) * K, inv, bound, C, KH, KW, K / (KH * KW), K);
+        FXF_LAUNCHED(ctx);
+        w_split.planes = planes;
+        w_split.plane = int64_t(O) * K;
+        w_split.inv = inv;
+        w_split.bound = bound;
+        return launch_bias_bound(static_cast<const float*>(b.ptr), O, bound, ctx);
+    }
     int prepare(Registry& reg, const TensorIds& in, const TensorIds&, const Params&, ExecCtx& ctx) override {
+        if (images) return prepare_split(reg[in[1]], reg[in[2]], ctx);
         if (!gemm_1x1 && !igemm_tc && !s2d_tc) return 0;
         FXF_CHECK(persist != nullptr, "conv plan: persistent memory was not assigned");
         float* h = static_cast<float*>(persist);
@@ -350,6 +556,46 @@ int run_conv(Registry& reg, const TensorIds& in, const TensorIds& out, const Par
     int64_t n_pix = int64_t(d.N) * d.HO * d.WO;
     if (n_pix == 0 || d.O == 0) return 0;
     const ConvPlan* cp = static_cast<const ConvPlan*>(plan);
+    if (cp && cp->images) {
+        ConvF16Args c;
+        c.w = cp->w_split;
+        c.bias = static_cast<const float*>(b.ptr);
+        c.split_out = ctx.split_out;
+        c.out = static_cast<float*>(o.ptr);
+        c.N = d.N; c.C = d.C; c.H = d.H; c.W = d.W; c.O = d.O; c.KH = d.KH; c.KW = d.KW; c.HO = d.HO; c.WO = d.WO;
+        c.pad_h = d.ph; c.pad_w = d.pw; c.dil_h = d.dh; c.dil_w = d.dw; c.str_h = d.sh; c.str_w = d.sw;
+        c.relu = relu;
+        if (cp->image_role == NodePlan::kImageStem) {
+            FXF_CHECK(ctx.scratch != nullptr && ctx.scratch_bytes >= cp->scratch_bytes, "%s: scratch for the space-to-depth copy is missing", who);
+            const int Ws = d.WO + 3;
+            uint16_t* planes = static_cast<uint16_t*>(ctx.scratch);
+            const int64_t plane = int64_t(d.N) * cp->Hs * Ws * 16;
+            float *inv = reinterpret_cast<float*>(planes + 2 * plane), *amax = inv + d.N;
+            tag_launch(ctx, "image_amax", 0, double(x.nbytes));
+            dependent(image_amax_kernel, dim3(kImageParts, unsigned(d.N)), 256, 0, ctx)(static_cast<const float*>(x.ptr), int64_t(d.C) * d.H * d.W, amax);
+            FXF_LAUNCHED(ctx);
+            tag_launch(ctx, "space_to_depth16_f16", 0, double(x.nbytes) + 4.0 * double(plane));
+            dependent(space_to_depth16_f16_kernel, dim3(unsigned(cp->Hs), unsigned(d.N)), 128, 0, ctx)(static_cast<const float*>(x.ptr), planes, plane, amax, inv, d.C, d.H, d.W, cp->Hs, Ws,
+                                                                                                       d.ph, d.pw, d.xs);
+            FXF_LAUNCHED(ctx);
+            c.x.planes = planes; c.x.plane = plane; c.x.inv = inv; c.x.amax = amax; c.x.parts = kImageParts;
+            c.window = true;
+            c.KH = cp->KH2; c.KW = 1; c.H = cp->Hs;
+            c.pad_h = c.pad_w = 0; c.str_h = c.str_w = 1;
+        } else {
+            const SplitMat* sx = split_of(ctx, in[0]);
+            FXF_CHECK(sx != nullptr, "%s: the input is not in split form", who);
+            c.x = *sx;
+        }
+        if (ctx.fuse.out != nullptr) {
+            const SplitMat* sr = split_of(ctx, uint32_t(ctx.fuse.residual_id));
+            FXF_CHECK(sr != nullptr, "%s: the residual is not in split form", who);
+            c.res = *sr;
+            c.relu = relu || ctx.fuse.relu;
+            ctx.fuse.consumed = true;
+        }
+        return launch_conv_f16(c, ctx);
+    }
     const bool is_1x1 = d.KH == 1 && d.KW == 1 && d.sh == 1 && d.sw == 1 && d.ph == 0 && d.pw == 0 && d.groups == 1;
     if (is_1x1 && pixel_major(x) && pixel_major(o)) {
         GemmArgs g;
@@ -441,7 +687,7 @@ int k_conv2d_relu(Registry& reg, const TensorIds& in, const TensorIds& out, cons
     return run_conv(reg, in, out, p, true, plan, ctx, "conv2d_relu");
 }
 
-int k_max_pool2d(Registry& reg, const TensorIds& in, const TensorIds& out, const Params& p, const NodePlan*, ExecCtx& ctx) {
+int k_max_pool2d(Registry& reg, const TensorIds& in, const TensorIds& out, const Params& p, const NodePlan* plan, ExecCtx& ctx) {
     FXF_CHECK(in.size() >= 1 && out.size() >= 1 && p.ints.size() >= 9, "max_pool2d: expects 9 int params");
     PoolDesc d;
     if (pool_desc(reg[in[0]], reg[out[0]], &d, "max_pool2d")) return 1;
@@ -450,6 +696,13 @@ int k_max_pool2d(Registry& reg, const TensorIds& in, const TensorIds& out, const
     FXF_CHECK(d.sh > 0 && d.sw > 0, "max_pool2d: stride must be positive");
     int64_t total = d.N * d.C * d.HO * d.WO;
     if (total == 0) return 0;
+    if (plan != nullptr && plan->images) {
+        const SplitMat* sx = split_of(ctx, in[0]);
+        FXF_CHECK(sx != nullptr && ctx.split_out.planes != nullptr, "max_pool2d: input and output must be in split form");
+        dependent(max_pool_split_kernel, pool_grid(total / 8, ctx), 256, 0, ctx)(sx->planes, sx->plane, ctx.split_out.planes, ctx.split_out.plane, d);
+        FXF_LAUNCHED(ctx);
+        return 0;
+    }
     dependent(pool2d_kernel<kMaxPool>, pool_grid(total, ctx), 256, 0, ctx)(static_cast<const float*>(reg[in[0]].ptr), static_cast<float*>(reg[out[0]].ptr), d);
     FXF_LAUNCHED(ctx);
     return 0;
@@ -469,7 +722,7 @@ int k_avg_pool2d(Registry& reg, const TensorIds& in, const TensorIds& out, const
     return 0;
 }
 
-int k_adaptive_avg_pool2d(Registry& reg, const TensorIds& in, const TensorIds& out, const Params& p, const NodePlan*, ExecCtx& ctx) {
+int k_adaptive_avg_pool2d(Registry& reg, const TensorIds& in, const TensorIds& out, const Params& p, const NodePlan* plan, ExecCtx& ctx) {
     FXF_CHECK(in.size() >= 1 && out.size() >= 1 && p.ints.size() >= 2, "adaptive_avg_pool2d: expects [oh, ow]");
     PoolDesc d;
     if (pool_desc(reg[in[0]], reg[out[0]], &d, "adaptive_avg_pool2d")) return 1;
@@ -477,7 +730,11 @@ int k_adaptive_avg_pool2d(Registry& reg, const TensorIds& in, const TensorIds& o
     d.kh = d.kw = d.sh = d.sw = d.dh = d.dw = 1; d.ph = d.pw = 0;
     int64_t total = d.N * d.C * d.HO * d.WO;
     if (total == 0) return 0;
-    if (d.HO == 1 && d.WO == 1 && is_contiguous(reg[in[0]]) && is_contiguous(reg[out[0]])) {
+    if (plan != nullptr && plan->images) {
+        const SplitMat* sx = split_of(ctx, in[0]);
+        FXF_CHECK(sx != nullptr, "adaptive_avg_pool2d: the input is not in split form");
+        dependent(global_avg_split_kernel, dim3(unsigned((d.C + 127) / 128), unsigned(d.N)), 128, 0, ctx)(sx->planes, sx->plane, sx->inv, static_cast<float*>(reg[out[0]].ptr), d.C, d.H * d.W);
+    } else if (d.HO == 1 && d.WO == 1 && is_contiguous(reg[in[0]]) && is_contiguous(reg[out[0]])) {
         int64_t nc = d.N * d.C, blocks = (nc * 32 + 255) / 256, cap = int64_t(ctx.sm_count) * 8;
         dependent(global_avg_pool_kernel, int(blocks < cap ? blocks : cap), 256, 0, ctx)(static_cast<const float*>(reg[in[0]].ptr), static_cast<float*>(reg[out[0]].ptr), nc, d.H * d.W);
     } else {
@@ -526,6 +783,18 @@ std::unique_ptr<NodePlan> plan_conv(const Registry& reg, const TensorIds& in, co
             pl->variant = "space-to-depth + tcgen05-tf32x3 implicit GEMM when the output is channels-last, else igemm-simt64x64";
         } else {
             pl->variant = "igemm-simt64x64";
+        }
+        // on images in split form, if the engine finds that the neighbours can (it then sets `images`)
+        if (env.gemm_mode == FXF_GEMM_AUTO && env.tp_size == 1 && reg[in[0]].rank == 4 && M >= 1 && numel(reg[in[2]]) == O && O % 8 == 0 && o.shape[0] <= 65535) {
+            if (pl->s2d_tc && pl->KW2 <= 4 && pl->Hs <= 65535 && M < (int64_t(1) << 31) - 256 && is_contiguous(reg[in[0]])) {
+                pl->image_role = NodePlan::kImageStem;
+                pl->k_split = int64_t(pl->KH2) * 64;
+                pl->scratch_bytes = std::max(pl->scratch_bytes, size_t(o.shape[0]) * (size_t(pl->Hs) * size_t(o.shape[3] + 3) * 16 * 4 + 4 * (1 + kImageParts)));
+            } else if (!pl->s2d_tc && reg[in[0]].shape[1] == C && conv_f16_shape_ok(M, C, O, w.shape[2], w.shape[3], p.ints.data())) {
+                pl->image_role = NodePlan::kImageConv;
+                pl->k_split = is_1x1 ? C : w.shape[2] * w.shape[3] * ((C + 63) / 64) * 64;
+            }
+            if (pl->image_role != NodePlan::kNoImages) pl->persist_bytes = std::max(pl->persist_bytes, round_up(pl->split_bytes(O), 256));
         }
     }
     return pl;

@@ -72,7 +72,24 @@ struct alignas(1024) F16Smem {
     int abort_flag;
 };
 
+// Images (IMG kernels): rows are the pixels of channels-last images, with one scale and one maximum per image (`rpi` rows)
+// instead of per row; the maxima of the result are collected with atomics in so_amax[image], zeroed before the forward.
+// c_slabs > 0: a convolution as an implicit GEMM.  K-slab k is input-channel slab k % c_slabs of filter tap k / c_slabs; the
+// im2col mode of the TMA walks the 128 consecutive output pixels of a tile across row and image borders (stride and padding
+// are in the map, the tap is the load's offset, pixels outside the image read zero), so tiles are full for any image size.
+// c_slabs == 0: rows as they lie in memory (1x1 filters).
+struct ImageGeom {
+    unsigned rpi;
+    int c_slabs, KW, WO, HO;
+    int sw, sh, pw, ph, dw, dh;
+    int lo_image;                 // images between the two planes of x
+    const uint16_t* res;          // residual in split form, laid out like the result: res_inv / res_amax per image
+    int64_t res_plane;
+    const float *res_inv, *res_amax;
+};
+
 struct F16Params {
+    ImageGeom im;
     const float* bias;
     const float* residual;        // optional, addressed like `out`
     const float *x_inv, *w_inv;   // 1 / scale per row of x and per row of w (NULL in bf16 mode)
@@ -147,7 +164,7 @@ __device__ __forceinline__ void drain_chunk(uint32_t tacc, float (&sum)[HALF]) {
     }
 }
 
-template <int BN, int STAGES, bool PAIR, int NPL>
+template <int BN, int STAGES, bool PAIR, int NPL, bool IMG>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_o, F16Params p) {
     extern __shared__ unsigned char smem_raw[];
@@ -204,7 +221,27 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       if (warp == kTmaWarp) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
+            int px = 0, py = 0, pn = 0;   // input position of the tile's first pixel
+            auto locate = [&](int tm) {
+                if (!IMG || p.im.c_slabs == 0) return;
+                unsigned pix = unsigned(tm) * BM;
+                if (pix >= unsigned(p.M)) pix = 0;   // the second tile of a pair may lie behind the last row: nothing of it is stored
+                const unsigned n = pix / p.im.rpi, r = pix - n * p.im.rpi, oy = r / unsigned(p.im.WO), ox = r - oy * unsigned(p.im.WO);
+                px = int(ox) * p.im.sw - p.im.pw;
+                py = int(oy) * p.im.sh - p.im.ph;
+                pn = int(n);
+            };
             auto load_x = [&](int st, int k, int tm) {
+                if (IMG && p.im.c_slabs > 0) {
+                    const int tap = k / p.im.c_slabs, c = (k - tap * p.im.c_slabs) * BK, kh = tap / p.im.KW;
+                    const uint16_t ow = uint16_t((tap - kh * p.im.KW) * p.im.dw), oh = uint16_t(kh * p.im.dh);
+#pragma unroll
+                    for (int pl = 0; pl < NPL; pl++) {
+                        if (PAIR) tma_load_im2col_pair(s.a[st][pl], &map_x, c, px, py, pn + pl * p.im.lo_image, ow, oh, &s.full[st]);
+                        else tma_load_im2col(s.a[st][pl], &map_x, c, px, py, pn + pl * p.im.lo_image, ow, oh, &s.full[st]);
+                    }
+                    return;
+                }
                 if (PAIR) tma_load_3d_pair(s.a[st], &map_x, k * BK, tm * BM, 0, &s.full[st]);
                 else tma_load_3d(s.a[st], &map_x, k * BK, tm * BM, 0, &s.full[st]);
             };
@@ -223,6 +260,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 int tm, tn;
                 tile_coords(p, un.tile, tm, tn);
                 if (PAIR) tm = tm * 2 + rank;
+                locate(tm);
                 int k = un.k0;
                 if (first) {   // the ring is empty: fill it without waiting, the weights ahead of the previous kernel's end
                     const int pre = min(STAGES, un.k1 - un.k0);
@@ -336,14 +374,36 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             const bool row_ok = grow < p.M;
             const int64_t col_base = int64_t(tn) * BN + chalf * HALF;
             // constants of the row and of the columns, fetched while the tensor core works
-            const float ri = (row_ok && p.x_inv != nullptr) ? __ldg(p.x_inv + grow * p.x_inv_stride) : 1.f;
+            const int64_t image = IMG ? int64_t(unsigned(grow) / p.im.rpi) : 0;
+            const int64_t sx = IMG ? image : grow * p.x_inv_stride, so_at = IMG ? image : grow;   // where the row's scales stand
+            const float ri = (row_ok && p.x_inv != nullptr) ? __ldg(p.x_inv + sx) : 1.f;
+            const float res_inv = (IMG && p.im.res != nullptr && row_ok) ? __ldg(p.im.res_inv + image) : 0.f;
             const float row_bias = (p.swap && row_ok && p.bias != nullptr) ? __ldg(p.bias + grow) : 0.f;
             float rscale = 1.f, rmax = 0.f;
             if (NPL == 2 && p.so != nullptr && !writes_partial && row_ok) {
                 float am = 0.f, inv;
-                for (int j = 0; j < p.x_parts; j++) am = fmaxf(am, __ldg(p.x_amax + grow * p.x_inv_stride * p.x_parts + j));
-                split_scale(fmaf(am, __ldg(p.w_bound), __ldg(p.w_bound + 1)), rscale, inv);
-                if (chalf == 0 && tn == 0) p.so_inv[grow] = inv;
+                for (int j = 0; j < p.x_parts; j++) am = fmaxf(am, __ldg(p.x_amax + sx * p.x_parts + j));
+                float bound = fmaf(am, __ldg(p.w_bound), __ldg(p.w_bound + 1));
+                if (IMG && p.im.res != nullptr) bound += __ldg(p.im.res_amax + image);
+                split_scale(bound, rscale, inv);
+                if (chalf == 0 && tn == 0 && (!IMG || unsigned(grow) == unsigned(image) * p.im.rpi)) p.so_inv[so_at] = inv;
+            }
+            // both planes of the residual's next sixteen columns, requested a group ahead of their use
+            uint4 rn[IMG ? 4 : 1];
+            auto fetch_residual = [&](int64_t col) {
+                if (!IMG || p.im.res == nullptr || !row_ok || col >= p.N) return;
+                const uint16_t* src = p.im.res + grow * p.N + col;
+                rn[0] = __ldg(reinterpret_cast<const uint4*>(src));
+                rn[IMG ? 2 : 0] = __ldg(reinterpret_cast<const uint4*>(src + p.im.res_plane));
+                if (col + 8 < p.N) {
+                    rn[IMG ? 1 : 0] = __ldg(reinterpret_cast<const uint4*>(src + 8));
+                    rn[IMG ? 3 : 0] = __ldg(reinterpret_cast<const uint4*>(src + p.im.res_plane + 8));
+                }
+            };
+            if (IMG) {
+#pragma unroll
+                for (int j = 0; j < (IMG ? 4 : 1); j++) rn[j] = make_uint4(0u, 0u, 0u, 0u);
+                if (!writes_partial) fetch_residual(col_base);
             }
             __syncwarp();
             for (int j = lane; j < HALF; j += 32) {
@@ -386,7 +446,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     break;
                 }
             }
-            const bool transposes = p.vt_out != nullptr && col_base >= p.vt_col0;
+            const bool transposes = !IMG && p.vt_out != nullptr && col_base >= p.vt_col0;
             // rows that do not start on 16-byte boundaries (a pitch like the 50257-column vocabulary): row r starts `shift` floats
             // past one and is stored as aligned 16-byte pieces, 16 columns lagging by `shift`
             float* orow = p.out + grow * p.ldo + col_base;
@@ -420,10 +480,16 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     }
                 }
                 float4 r4[4];
-                if (p.residual != nullptr && p.tma_out) {
+                if (!IMG && p.residual != nullptr && p.tma_out) {
 #pragma unroll
                     for (int j = 0; j < 4; j++)
                         r4[j] = (row_ok && col + 4 * j < p.N) ? *reinterpret_cast<const float4*>(p.residual + grow * p.ldo + col + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                uint4 rc[IMG ? 4 : 1];
+                if (IMG) {
+#pragma unroll
+                    for (int j = 0; j < (IMG ? 4 : 1); j++) rc[j] = rn[j];
+                    if (g + 1 < HALF / 16) fetch_residual(col + 16);
                 }
 #pragma unroll
                 for (int j = 0; j < 16; j += 4) {
@@ -432,7 +498,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     v[j] = fmaf(v[j] * ci.x, ri, cb.x); v[j + 1] = fmaf(v[j + 1] * ci.y, ri, cb.y);
                     v[j + 2] = fmaf(v[j + 2] * ci.z, ri, cb.z); v[j + 3] = fmaf(v[j + 3] * ci.w, ri, cb.w);
                 }
-                if (p.swap) {   // the 32 lanes write 32 consecutive columns of the result
+                if (!IMG && p.swap) {   // the 32 lanes write 32 consecutive columns of the result
 #pragma unroll
                     for (int j = 0; j < 16; j++)
                         if (row_ok && col + j < p.N) {
@@ -461,7 +527,16 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     }
                     continue;
                 }
-                if (p.residual != nullptr) {
+                if (IMG && p.im.res != nullptr) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const uint32_t hw = (&rc[IMG ? j >> 2 : 0].x)[j & 3], lw = (&rc[IMG ? 2 + (j >> 2) : 0].x)[j & 3];
+                        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hw)), l = __half22float2(*reinterpret_cast<const __half2*>(&lw));
+                        v[2 * j] = fmaf(h.x + l.x, res_inv, v[2 * j]);
+                        v[2 * j + 1] = fmaf(h.y + l.y, res_inv, v[2 * j + 1]);
+                    }
+                }
+                if (!IMG && p.residual != nullptr) {
                     if (p.tma_out) {
 #pragma unroll
                         for (int j = 0; j < 4; j++) { v[4 * j] += r4[j].x; v[4 * j + 1] += r4[j].y; v[4 * j + 2] += r4[j].z; v[4 * j + 3] += r4[j].w; }
@@ -476,7 +551,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     for (int j = 0; j < 16; j++) v[j] = relu_keep_nan(v[j]);
                 }
                 char* stage = reinterpret_cast<char*>(s.stage_out[warp][NSTG > 1 ? sbuf : 0]);
-                if (p.tma_out) {
+                if (IMG || p.tma_out) {
                     if (lane == 0) bulk_wait_read<NSTG - 1>();   // the store that used this buffer has read it
                     __syncwarp();
                     if (p.so == nullptr) {
@@ -497,7 +572,12 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll
                             for (int e = 0; e < 4; e++) {
                                 const float x = v[8 * j + 2 * e], y = v[8 * j + 2 * e + 1];
-                                rmax = fmaxf(rmax, fmaxf(fabsf(x), fabsf(y)));
+                                if (IMG) {   // an infinite value must not take the scale of its whole image along
+                                    rmax = fmaxf(rmax, fabsf(x) < INFINITY ? fabsf(x) : 0.f);
+                                    rmax = fmaxf(rmax, fabsf(y) < INFINITY ? fabsf(y) : 0.f);
+                                } else {
+                                    rmax = fmaxf(rmax, fmaxf(fabsf(x), fabsf(y)));
+                                }
                                 split_f16x2(x * rscale, y * rscale, hp[e], lp[e]);
                             }
                             const int at = lane * 32 + ((j ^ ((lane >> 2) & 1)) << 4);
@@ -560,7 +640,21 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     }
                 }
             }
-            if (NPL == 2 && p.so != nullptr && !writes_partial && row_ok) p.so_amax[grow * p.so_parts + tn * 2 + chalf] = rmax;
+            if (NPL == 2 && p.so != nullptr && !writes_partial) {
+                if (!IMG) {
+                    if (row_ok) p.so_amax[grow * p.so_parts + tn * 2 + chalf] = rmax;
+                } else {   // non-negative floats order like integers
+                    unsigned* at = reinterpret_cast<unsigned*>(p.so_amax);
+                    const int first = __shfl_sync(0xffffffffu, int(image), 0);
+                    const unsigned m = row_ok ? __float_as_uint(rmax) : 0u;
+                    if (warp_all(!row_ok || int(image) == first)) {
+                        const unsigned all = __reduce_max_sync(0xffffffffu, m);
+                        if (lane == 0 && row_ok) atomicMax(at + first, all);
+                    } else if (row_ok) {
+                        atomicMax(at + image, m);
+                    }
+                }
+            }
             if (writes_partial) {
                 __threadfence();
                 __syncwarp();
@@ -717,17 +811,18 @@ TailSplit plan_tail(int64_t tiles, int num_k, const Variant& v, int workers, boo
     return best;
 }
 
-template <int BN, int STAGES, bool PAIR, int NPL>
-int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int workers, ExecCtx& ctx) {
+template <int BN, int STAGES, bool PAIR, int NPL, bool IMG = false>
+int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int workers, ExecCtx& ctx, const CUtensorMap* im2col = nullptr) {
     constexpr int BNB = PAIR ? BN / 2 : BN;
     CUtensorMap mx, mw, mo;
-    if (make_map(&mx, a.x.planes, a.M, a.K, a.x.ld ? a.x.ld : a.K, a.x.plane, NPL, BM)) return 1;
+    if (IMG && p.im.c_slabs > 0) mx = *im2col;
+    else if (make_map(&mx, a.x.planes, a.M, a.K, a.x.ld ? a.x.ld : a.K, a.x.plane, NPL, BM)) return 1;
     if (make_map(&mw, a.w.planes, a.N, a.K, a.w.ld ? a.w.ld : a.K, a.w.plane, NPL, BNB)) return 1;
     mo = mx;
     if (p.tma_out && make_out_map(&mo, a, NPL)) return 1;
     const size_t smem = sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL)>) + 1024;
     static_assert(sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL)>) + 1024 <= 227 * 1024, "shared memory of a CTA");
-    auto kernel = gemm_f16_kernel<BN, STAGES, PAIR, NPL>;
+    auto kernel = gemm_f16_kernel<BN, STAGES, PAIR, NPL, IMG>;
     static bool configured[64] = {};
     int dev = 0;
     FXF_CUDA(cudaGetDevice(&dev));
@@ -804,8 +899,7 @@ bool gemm_f16_vt_ok(const F16GemmArgs& a, const ExecCtx& ctx) {
     return pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, false, true, a.vt_col0, nullptr, nullptr, -1) >= 0;
 }
 
-int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx) {
-    if (a.M == 0 || a.N == 0) return 0;
+static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorMap* im2col, const char* tag, double flops, ExecCtx& ctx) {
     FXF_CHECK(gemm_f16_shape_ok(a.M, a.N, a.K) && a.x.planes && a.w.planes && aligned16(a.x.planes) && aligned16(a.w.planes) && (a.x.plane * 2) % 16 == 0,
               "f16 GEMM: unsupported operands (M=%lld N=%lld K=%lld)", (long long)a.M, (long long)a.N, (long long)a.K);
     const bool split = a.split_out.planes != nullptr;
@@ -830,6 +924,7 @@ int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx) {
     p.tiles_n = int((a.N + var.bn - 1) / var.bn);
     p.m_fastest = a.N > a.M ? 1 : 0;
     p.status = ctx.status;
+    if (im != nullptr) p.im = *im;
     if (ts.parts > 1 && (size_t(ts.tail) * ts.parts * per_unit * size_t(BM) * var.bn * sizeof(float) > ctx.gemm_ws_bytes ||
                          ts.tail * ts.parts * per_unit * kEpiWarps > ctx.gemm_flag_count))
         ts = TailSplit{int64_t(p.tiles_m) * p.tiles_n, 0, 1, 0.0};
@@ -847,8 +942,7 @@ int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx) {
     if (a.vt_out != nullptr) {
         p.vt_out = a.vt_out; p.vt_flags = a.vt_flags; p.vt_col0 = a.vt_col0; p.vt_T = a.vt_T; p.vt_heads = a.vt_heads; p.vt_n32 = a.vt_n32;
     }
-    tag_launch(ctx, a.bf16 ? "gemm_bf16_tcgen05" : "gemm_f16x3_tcgen05", 2.0 * double(a.M) * double(a.N) * double(a.K),
-               4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.N) + double(a.M) * a.N));
+    tag_launch(ctx, tag, flops, 4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.N) + double(a.M) * a.N));
     if (a.bf16) {
         switch (v) {
             case 0: return launch_variant<256, 6, true, 1>(a, p, ts, workers, ctx);
@@ -860,6 +954,17 @@ int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx) {
             default: return launch_variant<32, 8, false, 1>(a, p, ts, workers, ctx);
         }
     }
+    if (im != nullptr) {
+        switch (v) {
+            case 0: return launch_variant<256, 3, true, 2, true>(a, p, ts, workers, ctx, im2col);
+            case 1: return launch_variant<192, 3, true, 2, true>(a, p, ts, workers, ctx, im2col);
+            case 2: return launch_variant<128, 4, true, 2, true>(a, p, ts, workers, ctx, im2col);
+            case 3: return launch_variant<64, 4, true, 2, true>(a, p, ts, workers, ctx, im2col);
+            case 4: return launch_variant<128, 3, false, 2, true>(a, p, ts, workers, ctx, im2col);
+            case 5: return launch_variant<64, 4, false, 2, true>(a, p, ts, workers, ctx, im2col);
+            default: return launch_variant<32, 4, false, 2, true>(a, p, ts, workers, ctx, im2col);
+        }
+    }
     switch (v) {
         case 0: return launch_variant<256, 3, true, 2>(a, p, ts, workers, ctx);
         case 1: return launch_variant<192, 3, true, 2>(a, p, ts, workers, ctx);
@@ -869,6 +974,60 @@ int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx) {
         case 5: return launch_variant<64, 4, false, 2>(a, p, ts, workers, ctx);
         default: return launch_variant<32, 4, false, 2>(a, p, ts, workers, ctx);
     }
+}
+
+int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx) {
+    if (a.M == 0 || a.N == 0) return 0;
+    return launch_f16(a, nullptr, nullptr, a.bf16 ? "gemm_bf16_tcgen05" : "gemm_f16x3_tcgen05", 2.0 * double(a.M) * double(a.N) * double(a.K), ctx);
+}
+
+// The corners and offsets of a 4-D im2col map are 8-bit numbers, its strides at most 8; TMA needs 16-byte pixels and image rows.
+bool conv_f16_shape_ok(int64_t n_pix, int64_t C, int64_t O, int64_t KH, int64_t KW, const int64_t* geom) {
+    const int64_t sh = geom[0], sw = geom[1], ph = geom[2], pw = geom[3], dh = geom[4], dw = geom[5], groups = geom[6];
+    return groups == 1 && C >= 16 && C % 8 == 0 && O % 8 == 0 && n_pix >= 1 && n_pix < (int64_t(1) << 31) - 256 && sh >= 1 && sh <= 8 && sw >= 1 && sw <= 8 && ph >= 0 && ph <= 127 &&
+           pw >= 0 && pw <= 127 && dh >= 1 && dw >= 1 && (KH - 1) * dh <= 127 && (KW - 1) * dw <= 127 && KH * KW * ((C + 63) / 64) < (1 << 20);
+}
+
+int launch_conv_f16(const ConvF16Args& c, ExecCtx& ctx) {
+    const int64_t pixels = int64_t(c.N) * c.HO * c.WO;
+    if (pixels == 0 || c.O == 0) return 0;
+    const bool rows = !c.window && c.KH == 1 && c.KW == 1 && c.str_h == 1 && c.str_w == 1 && c.pad_h == 0 && c.pad_w == 0;
+    const int c_slabs = c.window ? 1 : (c.C + BK - 1) / BK, taps = c.window ? c.KH : c.KH * c.KW;
+    F16GemmArgs a;
+    a.x = c.x; a.w = c.w;
+    a.bias = c.bias; a.out = c.out; a.split_out = c.split_out;
+    a.M = pixels; a.N = c.O; a.K = rows ? c.C : int64_t(taps) * c_slabs * BK;
+    a.ldo = c.O;
+    a.relu = c.relu;
+    a.conv_chain = true;
+    FXF_CHECK(c.split_out.planes != nullptr || (c.O % 4 == 0 && aligned16(c.out)), "convolution (f16): the output needs 16-byte pixels");
+    FXF_CHECK(c.res.planes == nullptr || (c.O % 8 == 0 && aligned16(c.res.planes) && (c.res.plane * 2) % 16 == 0 && c.split_out.planes != nullptr), "convolution (f16): unsupported residual");
+    ImageGeom im{};
+    im.rpi = unsigned(c.HO * c.WO);
+    im.res = c.res.planes; im.res_plane = c.res.plane; im.res_inv = c.res.inv; im.res_amax = c.res.amax;
+    CUtensorMap map;
+    if (!rows) {
+        im.c_slabs = c_slabs; im.KW = c.window ? 1 : c.KW; im.WO = c.WO; im.HO = c.HO;
+        im.sw = c.str_w; im.sh = c.str_h; im.pw = c.pad_w; im.ph = c.pad_h; im.dw = c.dil_w; im.dh = c.dil_h;
+        im.lo_image = c.N;
+        const int64_t C = c.window ? BK : c.C, pitch = c.window ? 16 : c.C, W = c.window ? c.WO : c.W, row = c.window ? int64_t(c.WO + 3) * 16 : int64_t(c.W) * c.C;
+        FXF_CHECK(c.x.plane == int64_t(c.N) * c.H * row, "convolution (f16): the planes of x must follow each other");
+        static const auto fn = [] {
+            void* q = nullptr;
+            cudaDriverEntryPointQueryResult r;
+            return cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &q, cudaEnableDefault, &r) == cudaSuccess && r == cudaDriverEntryPointSuccess ? reinterpret_cast<decltype(&cuTensorMapEncodeIm2col)>(q) : nullptr;
+        }();
+        FXF_CHECK(fn != nullptr, "cuTensorMapEncodeIm2col is not available from the CUDA driver");
+        const int KW = im.KW;
+        cuuint64_t dims[4] = {cuuint64_t(C), cuuint64_t(W), cuuint64_t(c.H), cuuint64_t(2) * c.N};
+        cuuint64_t strides[3] = {cuuint64_t(pitch) * 2, cuuint64_t(row) * 2, cuuint64_t(row) * c.H * 2};
+        int lower[2] = {-c.pad_w, -c.pad_h}, upper[2] = {c.pad_w - (KW - 1) * c.dil_w, c.pad_h - (c.KH - 1) * c.dil_h};
+        cuuint32_t estr[4] = {1, cuuint32_t(c.str_w), cuuint32_t(c.str_h), 1};
+        CUresult r = fn(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<uint16_t*>(c.x.planes), dims, strides, lower, upper, BK, BM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        FXF_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeIm2col failed with code %d (%d x %d x %d x %d)", int(r), c.N, c.H, c.W, c.C);
+    }
+    return launch_f16(a, &im, rows ? nullptr : &map, "conv2d_f16x3_tcgen05", 2.0 * double(pixels) * c.O * c.C * c.KH * c.KW, ctx);
 }
 
 // out[M,N] for M <= 64 rows in split form and a weight of at least a tile per SM (see F16Params::swap).  The persistent kernel

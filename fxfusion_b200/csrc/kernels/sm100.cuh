@@ -285,6 +285,17 @@ __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m
                  ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar) & kPeerBitMask)
                  : "memory");
 }
+// im2col mode: pixels that follow (w, h, n) in the map's bounding box, each shifted by (ow, oh)
+__device__ __forceinline__ void tma_load_im2col(void* dst, const CUtensorMap* map, int c, int w, int h, int n, uint16_t ow, uint16_t oh, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6], {%7, %8};"
+                 ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c), "r"(w), "r"(h), "r"(n), "r"(smem_u32(bar)), "h"(ow), "h"(oh)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_im2col_pair(void* dst, const CUtensorMap* map, int c, int w, int h, int n, uint16_t ow, uint16_t oh, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6], {%7, %8};"
+                 ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c), "r"(w), "r"(h), "r"(n), "r"(smem_u32(bar) & kPeerBitMask), "h"(ow), "h"(oh)
+                 : "memory");
+}
 // ---- tile stores (shared -> global, asynchronous bulk groups of the issuing thread) ----
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* src, int c0, int c1, int c2) {
     asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"

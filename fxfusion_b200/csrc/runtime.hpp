@@ -76,6 +76,7 @@ struct EpilogueFusion {
     float* out = nullptr;
     bool relu = false;
     bool consumed = false;
+    int residual_id = -1;   // its tensor id (for a residual kept in split form)
 };
 
 // ---- split form (kernels/gemm_f16.cu): an fp32 matrix [rows, K] as two fp16 planes and a power-of-two scale per row, or as
@@ -161,6 +162,10 @@ struct NodePlan {
     uint32_t takes_split = 0;
     bool makes_split = false;
     int64_t split_rows = 0, split_cols = 0;
+    // channels-last images in split form, one scale per image (ConvF16Args): what the node can do with them
+    enum ImageRole { kNoImages, kImageConv, kImageStem, kImageMaxPool, kImageGlobalAvg };
+    ImageRole image_role = kNoImages;
+    bool images = false;        // decided by the engine before prepare(): the node runs on them
     size_t scratch_bytes = 0;   // shared scratch wanted at execute time
     size_t persist_bytes = 0;   // memory that must survive across runs (e.g. re-laid-out weights)
     void* persist = nullptr;    // assigned by the engine before prepare()
@@ -354,6 +359,20 @@ struct F16GemmArgs {
     int64_t vt_col0 = 0;
     int vt_T = 0, vt_heads = 0, vt_n32 = 0;
 };
+// Convolution over channels-last images in split form with one scale per image (x.inv, x.amax: one entry per image, x.parts
+// maxima each).  Filters in split form as [O, KH*KW, C padded to 64]; 1x1, stride 1, unpadded: [O, C].
+// window: x is [N, H, WO + 3, 16] and a filter row covers four consecutive pixels at once, filters [O, KH, 4*16] (KW = 1).
+struct ConvF16Args {
+    SplitMat x, w, res;                 // res: residual, laid out like the output (planes == NULL: none)
+    const float* bias = nullptr;
+    float* out = nullptr;
+    SplitOut split_out;                 // amax must be zero before the launch
+    int N = 0, C = 0, H = 0, W = 0, O = 0, KH = 0, KW = 0, HO = 0, WO = 0;
+    int pad_h = 0, pad_w = 0, dil_h = 1, dil_w = 1, str_h = 1, str_w = 1;
+    bool relu = false, window = false;
+};
+bool conv_f16_shape_ok(int64_t n_pix, int64_t C, int64_t O, int64_t KH, int64_t KW, const int64_t* geom);   // geom: sh, sw, ph, pw, dh, dw, groups
+int launch_conv_f16(const ConvF16Args& a, ExecCtx& ctx);
 bool gemm_f16_shape_ok(int64_t M, int64_t N, int64_t K);
 bool gemm_f16_vt_ok(const F16GemmArgs& a, const ExecCtx& ctx);
 int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx);

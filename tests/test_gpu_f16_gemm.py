@@ -127,3 +127,49 @@ def test_few_rows(built_lib, tmp_path, M, N, K, variant):
     assert ok, info
     assert eng.device_status() == 0
     eng.close()
+
+
+# channels-last images in split form: image borders inside a tile (14 x 14, 7 x 7), several images per tile, ragged channels,
+# asymmetric filters and padding, strides, dilation, a map of one pixel, and one image of many tiles
+@pytest.mark.parametrize("N,size,C,O,kh,kw,s,ph,pw,d", [
+    (2, 56, 64, 96, 3, 3, 1, 1, 1, 1), (5, 28, 40, 72, 3, 3, 2, 1, 1, 1), (3, 57, 128, 256, 1, 1, 2, 0, 0, 1), (7, 30, 24, 64, 5, 3, 1, 2, 0, 1), (2, 64, 64, 64, 3, 5, 1, 2, 4, 2),
+    (1, 26, 512, 128, 7, 7, 1, 0, 0, 1), (1, 224, 64, 256, 3, 3, 1, 1, 1, 1), (33, 12, 16, 200, 3, 3, 1, 1, 1, 1)])
+def test_images_in_split_form(built_lib, tmp_path, N, size, C, O, kh, kw, s, ph, pw, d):
+    """Stem, max pooling, convolutions, the residual AddRelu in the epilogue of one of them and global average pooling hand
+    the images on in split form; a convolution that feeds a plain average pooling leaves fp32 pixels."""
+    rng = np.random.default_rng(size + C)
+    gb = [1, 1, 1, 256, 1, 1]
+    b = lowering.GraphBuilder(f"images_{N}_{size}_{C}_{O}")
+
+    def conv(x, c, o, h, w, kh=1, kw=1, s=1, ph=0, pw=0, d=1, relu=True):
+        ho, wo = (h + 2 * ph - d * (kh - 1) - 1) // s + 1, (w + 2 * pw - d * (kw - 1) - 1) // s + 1
+        weight = (rng.standard_normal((o, c, kh, kw)) / math.sqrt(c * kh * kw)).astype(np.float32)
+        y = b.op("Conv2dRelu" if relu else "Conv2d", [x, b.const(weight), b.const(rng.standard_normal(o, dtype=np.float32))], (N, o, ho, wo), ints=[s, s, ph, pw, d, d, 1] + gb)
+        return y, ho, wo
+
+    x = b.input((N, 3, size, size), wire.DT_F32)
+    y, h, w = conv(x, 3, 64, size, size, 7, 7, 2, 3, 3)
+    h, w = (h - 1) // 2 + 1, (w - 1) // 2 + 1
+    y = b.op("MaxPool2d", [y], (N, 64, h, w), ints=[3, 3, 2, 2, 1, 1, 1, 1, 0] + gb)
+    y, h, w = conv(y, 64, C, h, w)
+    r, _, _ = conv(y, C, 2 * O, h, w, kh, kw, s, ph, pw, d, relu=False)
+    y, h, w = conv(y, C, O, h, w, kh, kw, s, ph, pw, d)
+    y, _, _ = conv(y, O, 2 * O, h, w, relu=False)
+    y = b.op("AddRelu", [y, r], (N, 2 * O, h, w))
+    z, _, _ = conv(y, 2 * O, 24, h, w)
+    z = b.op("AvgPool2d", [z], (N, 24, h, w), ints=[1, 1, 1, 1, 0, 0, 0] + gb)
+    b.output(conv(z, 24, 8, h, w)[0])
+    b.output(b.op("AdaptiveAvgPool2d", [y], (N, 2 * O, 1, 1), ints=[1, 1] + gb))
+    graph, eng = _engine(b, tmp_path)
+    text = eng.describe()
+    assert text.count("images in split form") == 6 and text.count("output in split form") == 6 and "+AddRelu(residual" in text, text
+    xin = torch.randn(N, 3, size, size, generator=torch.Generator().manual_seed(3)) * 10.0 ** torch.linspace(-8, 8, N).reshape(N, 1, 1, 1)
+    got, want = eng.run([xin.cuda()]), GraphOracle(graph).run([xin])
+    for g, t in zip(got, want):
+        scale = t.abs().amax(dim=(1, 2, 3), keepdim=True)
+        assert ((g.cpu() - t).abs() / scale).max().item() < 4e-6
+    eng.run([xin.cuda() * 1e-3])   # the maxima of one forward do not stay for the next
+    again = eng.run([xin.cuda()])
+    assert all(torch.equal(a.cpu(), g.cpu()) for a, g in zip(again, got))
+    assert eng.device_status() == 0
+    eng.close()
