@@ -38,6 +38,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "../runtime.hpp"
 #include "sm100.cuh"
@@ -50,11 +51,14 @@ using namespace sm100;
 constexpr int BM = 128, BK = 64;
 constexpr int kEpiWarps = 8, kTmaWarp = 8, kMmaWarp = 9, kThreads = 384;
 constexpr int ACC = 2;
-enum : int { kErrWaitFull = 131, kErrWaitEmpty = 133, kErrWaitAcc = 134, kErrWaitAccEmpty = 135, kErrWaitPartial = 136 };
+enum : int { kErrWaitFull = 131, kErrWaitEmpty = 133, kErrWaitAcc = 134, kErrWaitAccEmpty = 135, kErrWaitPartial = 136, kErrWaitResidual = 137 };
 
-// output staging buffers per epilogue warp: two where the operand ring leaves room, so that a store may still be reading one
-constexpr int staging_buffers(int bn, int bnb, int stages, int npl) {
-    return stages * npl * (BM + bnb) * BK * 2 + 2 * kEpiWarps * 2048 + kEpiWarps * bn * 4 <= 225 * 1024 ? 2 : 1;
+// output staging buffers per epilogue warp, as far as the operand ring leaves room: a store may still be reading one (images:
+// and the residual be on its way into two others)
+constexpr int staging_buffers(int bn, int bnb, int stages, int npl, bool images) {
+    const int room = 225 * 1024 - stages * npl * (BM + bnb) * BK * 2 - kEpiWarps * bn * 4;
+    const int fit = room / (kEpiWarps * 2048), want = images ? 4 : 2;
+    return fit < 1 ? 1 : (fit < want ? fit : want);
 }
 
 // BNB = weight rows held by this CTA; NPL = planes per operand (2: f16x3, 1: bf16)
@@ -68,6 +72,7 @@ struct alignas(1024) F16Smem {
     uint64_t empty[STAGES];
     uint64_t acc_full[ACC];
     uint64_t acc_empty[ACC];
+    uint64_t res_full[kEpiWarps][NSTG];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -98,6 +103,7 @@ struct F16Params {
     int64_t M, N, K, ldo;
     int relu;
     int tma_out;                  // the result leaves through map_o (16-byte aligned rows): fp32 [M, N] or both planes of the split form
+    int fast;                     // whole tiles take the short epilogue (rows in whole 32-byte sectors, of the residual too)
     int tiles_m, tiles_n, m_fastest;
     int full_tiles, tail_tiles, tail_split;   // tiles of the last round are cut along K into tail_split parts
     int chunk_slabs;
@@ -150,26 +156,59 @@ __device__ __forceinline__ void tile_coords(const F16Params& p, int tile, int& t
 }
 // a wait counts only if it succeeded for every lane, so that a warp gives up as a whole
 __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
-__device__ __forceinline__ float relu_keep_nan(float v) { return v > 0.f ? v : (v != v ? v : 0.f); }
+__device__ __forceinline__ float max_keep_nan(float v, float floor_at) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "f"(floor_at));
+    return r;
+}
+__device__ __forceinline__ float relu_keep_nan(float v) { return max_keep_nan(v, 0.f); }
 
+// v = sum[16 g ..], g known only at run time: a tree of branches (registers cannot be indexed)
+template <int LO, int HI, int HALF>
+__device__ __forceinline__ void pick_group(const float (&sum)[HALF], int g, float (&v)[16]) {
+    if constexpr (HI - LO == 1) {
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] = sum[LO * 16 + j];
+    } else {
+        constexpr int MID = (LO + HI) / 2;
+        if (g < MID) pick_group<LO, MID>(sum, g, v);
+        else pick_group<MID, HI>(sum, g, v);
+    }
+}
+
+template <int N>
+struct Words { uint32_t w[N]; };
+// 32 bytes of global memory at once: a whole sector per lane, so that lanes may own rows
+__device__ __forceinline__ void load32(const void* p, Words<8>& r) {
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7]) : "l"(p));
+}
+__device__ __forceinline__ void store32(void* p, const Words<8>& r) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r.w[0]), "r"(r.w[1]), "r"(r.w[2]), "r"(r.w[3]), "r"(r.w[4]), "r"(r.w[5]), "r"(r.w[6]),
+                 "r"(r.w[7]) : "memory");
+}
+
+// 32 columns at a time (16 where the thread's registers are full of sums): the loads of a batch are in flight together
 template <int HALF>
 __device__ __forceinline__ void drain_chunk(uint32_t tacc, float (&sum)[HALF]) {
+    constexpr int STEP = HALF <= 64 && HALF % 32 == 0 ? 32 : 16;
 #pragma unroll
-    for (int c = 0; c < HALF; c += 16) {
-        uint32_t r[16];
-        tmem_ld16(tacc + uint32_t(c), r);
+    for (int c = 0; c < HALF; c += STEP) {
+        uint32_t r[STEP];
+        tmem_ld(tacc + uint32_t(c), r);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 16; j++) sum[c + j] += __uint_as_float(r[j]);
+        for (int j = 0; j < STEP; j++) sum[c + j] += __uint_as_float(r[j]);
     }
 }
 
 template <int BN, int STAGES, bool PAIR, int NPL, bool IMG>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_o, F16Params p) {
+gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_r, F16Params p) {
     extern __shared__ unsigned char smem_raw[];
     constexpr int BNB = PAIR ? BN / 2 : BN;
-    using Smem = F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL)>;
+    constexpr int kStg = staging_buffers(BN, BNB, STAGES, NPL, IMG);
+    using Smem = F16Smem<BN, BNB, STAGES, NPL, kStg>;
     Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr uint32_t kABytes = NPL * BM * BK * 2, kBBytes = NPL * BNB * BK * 2;
     constexpr uint32_t kIdesc = NPL == 2 ? umma_idesc_f16(PAIR ? 2 * BM : BM, BN) : umma_idesc_bf16(PAIR ? 2 * BM : BM, BN);
@@ -192,6 +231,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             mbar_init(&s.acc_full[i], 1);
             mbar_init(&s.acc_empty[i], PAIR ? 2 * kEpiWarps : kEpiWarps);
         }
+        if (IMG)
+            for (int i = 0; i < kEpiWarps * kStg; i++) mbar_init(&s.res_full[0][0] + i, 1);
         s.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -199,6 +240,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         prefetch_tensormap(&map_x);
         prefetch_tensormap(&map_w);
         if (p.tma_out) prefetch_tensormap(&map_o);
+        if (IMG && p.im.res != nullptr) prefetch_tensormap(&map_r);
     }
     if (warp == kMmaWarp) {
         if (PAIR) {
@@ -354,11 +396,18 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         // running sums is spelled out): unrolled, its code missed the instruction cache at every group.  A group leaves as one
         // TMA store from a swizzled staging block; row-contiguous stores by the LSU, with the lanes re-arranged through shared
         // memory, took 250 instructions and 1900 cycles per group and bound every product of K <= 1024.
-        constexpr int HALF = BN / 2, NSTG = staging_buffers(BN, BNB, STAGES, NPL);
+        constexpr int HALF = BN / 2, NSTG = kStg;
+        // Narrow tiles belong to problems of a wave or two, where the store's latency counts (M = 512, N = 256, K = 256: 5.5 -> 4.4 us
+        // with stores from registers); wide ones are stored by TMA, which a row per lane would keep the load / store unit busy for.
+        constexpr bool DIRECT = !IMG && BN <= 64;
+        static_assert(!IMG || NSTG >= 2, "a residual needs a staging buffer besides the one being stored");
+        constexpr int AHEAD = NSTG >= 4 ? 2 : 1;   // images: groups between a residual's request and its use
         const int q = warp & 3, chalf = warp >> 2;
         const uint32_t lane_base = uint32_t(q * 32) << 16;
         float *cinv = s.col_inv[warp], *cbias = s.col_bias[warp];
-        uint32_t ccount = 0, sbuf = 0;
+        uint32_t ccount = 0, sbuf = 0, res_use = 0;   // chains, stored groups; parity of each residual buffer
+        int have_tn = -1;
+        const int M = int(p.M), N = int(p.N);
         grid_dep_wait();
         for (int unit = sched_id; unit < num_units; unit += sched_n) {
             const Unit un = get_unit(p, unit, num_k);
@@ -370,51 +419,75 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             const int slot = PAIR ? un.u * 2 + rank : un.u, pstep = PAIR ? 2 : 1;
             // partial tiles: [column half][row quarter][4-column group][lane] float4, so that every access is coalesced
             float4* ws_mine = reinterpret_cast<float4*>(p.ws + size_t(slot) * size_t(BM * BN)) + warp * (HALF / 4) * 32 + lane;
-            const int64_t trow = int64_t(tm) * BM + q * 32, grow = trow + lane;   // first row of this warp, row of this thread
-            const bool row_ok = grow < p.M;
-            const int64_t col_base = int64_t(tn) * BN + chalf * HALF;
+            const int trow = tm * BM + q * 32, grow = trow + lane;   // first row of this warp, row of this thread
+            const bool row_ok = grow < M;
+            const int col_base = tn * BN + chalf * HALF;
             // constants of the row and of the columns, fetched while the tensor core works
-            const int64_t image = IMG ? int64_t(unsigned(grow) / p.im.rpi) : 0;
-            const int64_t sx = IMG ? image : grow * p.x_inv_stride, so_at = IMG ? image : grow;   // where the row's scales stand
+            const int image = IMG ? int(unsigned(grow) / p.im.rpi) : 0;
+            const int64_t sx = IMG ? image : grow * p.x_inv_stride;
+            const int so_at = IMG ? image : grow;   // where the row's scales stand
             const float ri = (row_ok && p.x_inv != nullptr) ? __ldg(p.x_inv + sx) : 1.f;
             const float res_inv = (IMG && p.im.res != nullptr && row_ok) ? __ldg(p.im.res_inv + image) : 0.f;
             const float row_bias = (p.swap && row_ok && p.bias != nullptr) ? __ldg(p.bias + grow) : 0.f;
-            float rscale = 1.f, rmax = 0.f;
+            float rscale = 1.f, rinv = 0.f;
+            __half2 rmax = __half2half2(__ushort_as_half(0));   // largest |hi| of the row so far
             if (NPL == 2 && p.so != nullptr && !writes_partial && row_ok) {
-                float am = 0.f, inv;
+                float am = 0.f;
                 for (int j = 0; j < p.x_parts; j++) am = fmaxf(am, __ldg(p.x_amax + sx * p.x_parts + j));
                 float bound = fmaf(am, __ldg(p.w_bound), __ldg(p.w_bound + 1));
                 if (IMG && p.im.res != nullptr) bound += __ldg(p.im.res_amax + image);
-                split_scale(bound, rscale, inv);
-                if (chalf == 0 && tn == 0 && (!IMG || unsigned(grow) == unsigned(image) * p.im.rpi)) p.so_inv[so_at] = inv;
+                split_scale(bound, rscale, rinv);
+                if (chalf == 0 && tn == 0 && (!IMG || unsigned(grow) == unsigned(image) * p.im.rpi)) p.so_inv[so_at] = rinv;
             }
-            // both planes of the residual's next sixteen columns, requested a group ahead of their use
-            uint4 rn[IMG ? 4 : 1];
-            auto fetch_residual = [&](int64_t col) {
-                if (!IMG || p.im.res == nullptr || !row_ok || col >= p.N) return;
-                const uint16_t* src = p.im.res + grow * p.N + col;
-                rn[0] = __ldg(reinterpret_cast<const uint4*>(src));
-                rn[IMG ? 2 : 0] = __ldg(reinterpret_cast<const uint4*>(src + p.im.res_plane));
-                if (col + 8 < p.N) {
-                    rn[IMG ? 1 : 0] = __ldg(reinterpret_cast<const uint4*>(src + 8));
-                    rn[IMG ? 3 : 0] = __ldg(reinterpret_cast<const uint4*>(src + p.im.res_plane + 8));
+            const bool fast = p.fast && un.nparts == 1 && (IMG || p.vt_out == nullptr || col_base < p.vt_col0);
+            const int groups = writes_partial ? HALF / 16 : min(HALF, N - col_base + 15) / 16;   // warp-uniform; may be negative
+            // the residual's next sixteen columns, requested ahead of their use: fp32 into registers, images into staging buffers
+            Words<8> rn[2] = {};
+            auto fetch_residual = [&](int col) {
+                if (IMG || p.residual == nullptr || !row_ok || col >= N) return;
+                const float* src = p.residual + int64_t(grow) * p.ldo + col;
+                load32(src, rn[0]);
+                load32(src + 8, rn[1]);
+            };
+            auto request_image = [&](int ahead) {   // lane 0: group `ahead` from the one in hand, counted over the tiles of this warp
+                const uint32_t b = (sbuf + uint32_t(ahead)) % NSTG;
+                bulk_wait_read<NSTG - 1 - AHEAD>();   // the store that last used the buffer has read it
+                mbar_expect_tx(&s.res_full[warp][b], 2048);
+                return b;
+            };
+            const bool image_res = IMG && fast && p.im.res != nullptr;
+            if (fast) fetch_residual(col_base);
+            if (image_res && lane == 0)
+                for (int g = 0; g < min(AHEAD, groups); g++) {
+                    const uint32_t b = request_image(g);
+                    tma_load_3d(s.stage_out[warp][b], &map_r, col_base + g * 16, trow, 0, &s.res_full[warp][b]);
+                }
+            if (tn != have_tn) {
+                __syncwarp();
+                for (int j = lane; j < HALF; j += 32) {
+                    const int c = col_base + j;
+                    cinv[j] = (p.w_inv && c < N) ? __ldg(p.w_inv + c * p.w_inv_stride) : 1.f;
+                    cbias[j] = (p.bias && !p.swap && c < N) ? __ldg(p.bias + c) : 0.f;
+                }
+                __syncwarp();
+                have_tn = tn;
+            }
+            // A unit of one chain is read from its accumulator group by group; of several, the sums are in registers.
+            const bool single = un.k1 - un.k0 <= chunk;
+            const uint32_t tacc = tmem_base + (ccount % ACC) * uint32_t(BN) + lane_base + uint32_t(chalf * HALF);
+            auto release = [&](uint32_t buf) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (PAIR) mbar_arrive_leader(&s.acc_empty[buf]);
+                    else mbar_arrive(&s.acc_empty[buf]);
                 }
             };
-            if (IMG) {
-#pragma unroll
-                for (int j = 0; j < (IMG ? 4 : 1); j++) rn[j] = make_uint4(0u, 0u, 0u, 0u);
-                if (!writes_partial) fetch_residual(col_base);
-            }
-            __syncwarp();
-            for (int j = lane; j < HALF; j += 32) {
-                const int64_t c = col_base + j;
-                cinv[j] = (p.w_inv && c < p.N) ? __ldg(p.w_inv + c * p.w_inv_stride) : 1.f;
-                cbias[j] = (p.bias && !p.swap && c < p.N) ? __ldg(p.bias + c) : 0.f;
-            }
-            __syncwarp();
             float sum[HALF];
+            if (!single) {
 #pragma unroll
-            for (int j = 0; j < HALF; j++) sum[j] = 0.f;
+                for (int j = 0; j < HALF; j++) sum[j] = 0.f;
+            }
             bool alive = true;
             for (int kc0 = un.k0; kc0 < un.k1; kc0 += chunk, ccount++) {
                 const uint32_t buf = ccount % ACC;
@@ -424,12 +497,9 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     break;
                 }
                 tc_fence_after();
-                drain_chunk<HALF>(tmem_base + buf * uint32_t(BN) + lane_base + uint32_t(chalf * HALF), sum);
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    if (PAIR) mbar_arrive_leader(&s.acc_empty[buf]);
-                    else mbar_arrive(&s.acc_empty[buf]);
+                if (!single) {
+                    drain_chunk<HALF>(tmem_base + buf * uint32_t(BN) + lane_base + uint32_t(chalf * HALF), sum);
+                    release(buf);
                 }
             }
             if (!alive) break;
@@ -449,24 +519,129 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             const bool transposes = !IMG && p.vt_out != nullptr && col_base >= p.vt_col0;
             // rows that do not start on 16-byte boundaries (a pitch like the 50257-column vocabulary): row r starts `shift` floats
             // past one and is stored as aligned 16-byte pieces, 16 columns lagging by `shift`
-            float* orow = p.out + grow * p.ldo + col_base;
+            float* orow = p.out + int64_t(grow) * p.ldo + col_base;
             const int shift = int((reinterpret_cast<uintptr_t>(orow) >> 2) & 3);
             float c0 = 0.f, c1 = 0.f, c2 = 0.f;   // the last three columns of the previous group
-#pragma unroll 1
-            for (int g = 0; g < HALF / 16; g++) {
-                const int64_t col = col_base + g * 16;
-                if (col >= p.N && !writes_partial) break;   // warp-uniform
-                float v[16];
-#pragma unroll
-                for (int gg = 0; gg < HALF / 16; gg++)
-                    if (gg == g) {
-#pragma unroll
-                        for (int j = 0; j < 16; j++) v[j] = sum[gg * 16 + j];
+            // The common case, whole tiles that leave by TMA, without a branch but for the residual: with two warps per scheduler every
+            // branch costs its latency (a group took 1500 cycles with all cases in one body).
+            const float floor_at = p.relu ? 0.f : -INFINITY;
+            auto finish_fast = [&](int g, float (&v)[16], auto split_tag) {
+                constexpr bool SPLIT = decltype(split_tag)::value;
+                const int col = col_base + g * 16;
+                const Words<8> r0 = rn[0], r1 = rn[1];
+                fetch_residual(g + 1 < HALF / 16 ? col + 16 : N);
+                const uint32_t buf = sbuf % NSTG;
+                char* stage = reinterpret_cast<char*>(s.stage_out[warp][buf]);
+                if (image_res) {
+                    if (lane == 0 && g + AHEAD < groups) {
+                        const uint32_t b = request_image(AHEAD);
+                        tma_load_3d(s.stage_out[warp][b], &map_r, col + AHEAD * 16, trow, 0, &s.res_full[warp][b]);
                     }
+                    if (!warp_all(mbar_wait(&s.res_full[warp][buf], (res_use >> buf) & 1, abort_flag))) give_up(abort_flag, p.status, kErrWaitResidual);
+                    res_use ^= 1u << buf;
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) {
+                    const float4 ci = *reinterpret_cast<const float4*>(cinv + g * 16 + j), cb = *reinterpret_cast<const float4*>(cbias + g * 16 + j);
+                    // both factors are powers of two; the weight's goes first: the product of the two may leave the range of fp32
+                    v[j] = fmaf(v[j] * ci.x, ri, cb.x); v[j + 1] = fmaf(v[j + 1] * ci.y, ri, cb.y);
+                    v[j + 2] = fmaf(v[j + 2] * ci.z, ri, cb.z); v[j + 3] = fmaf(v[j + 3] * ci.w, ri, cb.w);
+                }
+                if (image_res) {
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        const int at = lane * 32 + ((j ^ ((lane >> 2) & 1)) << 4);
+                        const uint4 hq = *reinterpret_cast<const uint4*>(stage + at), lq = *reinterpret_cast<const uint4*>(stage + 1024 + at);
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const uint32_t hw = (&hq.x)[e], lw = (&lq.x)[e];
+                            const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hw)), l = __half22float2(*reinterpret_cast<const __half2*>(&lw));
+                            v[8 * j + 2 * e] = fmaf(h.x + l.x, res_inv, v[8 * j + 2 * e]);
+                            v[8 * j + 2 * e + 1] = fmaf(h.y + l.y, res_inv, v[8 * j + 2 * e + 1]);
+                        }
+                    }
+                } else if (!IMG && !SPLIT && p.residual != nullptr) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        v[j] += __uint_as_float(r0.w[j]);
+                        v[8 + j] += __uint_as_float(r1.w[j]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] = max_keep_nan(v[j], floor_at);
+                if constexpr (DIRECT) {
+                    Words<8> o0, o1;
+                    if constexpr (!SPLIT) {
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            o0.w[j] = __float_as_uint(v[j]);
+                            o1.w[j] = __float_as_uint(v[8 + j]);
+                        }
+                        if (row_ok) {
+                            float* dst = p.out + int64_t(grow) * p.ldo + col;
+                            store32(dst, o0);
+                            store32(dst + 8, o1);
+                        }
+                    } else if constexpr (NPL == 1) {
+#pragma unroll
+                        for (int j = 0; j < 8; j++) o0.w[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+                        if (row_ok) store32(p.so + int64_t(grow) * N + col, o0);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            split_f16x2(v[2 * j] * rscale, v[2 * j + 1] * rscale, o0.w[j], o1.w[j]);
+                            rmax = __hmax2(rmax, __habs2(*reinterpret_cast<const __half2*>(&o0.w[j])));
+                        }
+                        if (row_ok) {
+                            uint16_t* dst = p.so + int64_t(grow) * N + col;
+                            store32(dst, o0);
+                            store32(dst + p.so_plane, o1);
+                        }
+                    }
+                    return;
+                }
+                if (!image_res) {
+                    if (lane == 0) bulk_wait_read<NSTG - 1>();   // the store that used this buffer has read it
+                    __syncwarp();
+                }
+                if constexpr (!SPLIT) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        *reinterpret_cast<float4*>(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                } else if constexpr (NPL == 1) {
+#pragma unroll
+                    for (int j = 0; j < 2; j++)
+                        *reinterpret_cast<uint4*>(stage + lane * 32 + ((j ^ ((lane >> 2) & 1)) << 4)) =
+                            make_uint4(pack_bf16x2(v[8 * j], v[8 * j + 1]), pack_bf16x2(v[8 * j + 2], v[8 * j + 3]), pack_bf16x2(v[8 * j + 4], v[8 * j + 5]), pack_bf16x2(v[8 * j + 6], v[8 * j + 7]));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        uint4 hi, lo;
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            split_f16x2(v[8 * j + 2 * e] * rscale, v[8 * j + 2 * e + 1] * rscale, (&hi.x)[e], (&lo.x)[e]);
+                            rmax = __hmax2(rmax, __habs2(*reinterpret_cast<const __half2*>(&hi.x + e)));
+                        }
+                        const int at = lane * 32 + ((j ^ ((lane >> 2) & 1)) << 4);
+                        *reinterpret_cast<uint4*>(stage + at) = hi;
+                        *reinterpret_cast<uint4*>(stage + 1024 + at) = lo;
+                    }
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    if (trow < M) tma_store_3d(&map_o, stage, col, trow, 0);
+                    bulk_commit();
+                }
+                sbuf++;
+            };
+            // sixteen columns: scales, bias, residual, activation, store
+            auto finish = [&](int g, float (&v)[16]) {
+                const int col = col_base + g * 16;
                 if (writes_partial) {
 #pragma unroll
                     for (int j = 0; j < 4; j++) ws_mine[(g * 4 + j) * 32] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                    continue;
+                    return;
                 }
                 if (adds_partials) {
 #pragma unroll 1
@@ -483,13 +658,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 if (!IMG && p.residual != nullptr && p.tma_out) {
 #pragma unroll
                     for (int j = 0; j < 4; j++)
-                        r4[j] = (row_ok && col + 4 * j < p.N) ? *reinterpret_cast<const float4*>(p.residual + grow * p.ldo + col + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                uint4 rc[IMG ? 4 : 1];
-                if (IMG) {
-#pragma unroll
-                    for (int j = 0; j < (IMG ? 4 : 1); j++) rc[j] = rn[j];
-                    if (g + 1 < HALF / 16) fetch_residual(col + 16);
+                        r4[j] = (row_ok && col + 4 * j < N) ? *reinterpret_cast<const float4*>(p.residual + int64_t(grow) * p.ldo + col + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
                 for (int j = 0; j < 16; j += 4) {
@@ -501,19 +670,18 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 if (!IMG && p.swap) {   // the 32 lanes write 32 consecutive columns of the result
 #pragma unroll
                     for (int j = 0; j < 16; j++)
-                        if (row_ok && col + j < p.N) {
-                            const int64_t off = (col + j) * p.ldo + grow;
+                        if (row_ok && col + j < N) {
+                            const int64_t off = int64_t(col + j) * p.ldo + grow;
                             float t = v[j] + row_bias;
                             if (p.residual != nullptr) t += p.residual[off];
                             p.out[off] = p.relu ? relu_keep_nan(t) : t;
                         }
-                    continue;
+                    return;
                 }
                 if (transposes) {
                     // V third of a packed QKV projection, transposed per head: the 32 lanes write 32 consecutive keys of a V^T row
-                    const int64_t b = grow / p.vt_T, t = grow - b * p.vt_T, v0 = col - p.vt_col0, h = v0 >> 6;
-                    const int d0 = int(v0 & 63);
-                    float* dst = p.vt_out + ((b * p.vt_heads + h) * 64 + d0) * int64_t(p.vt_T) + t;
+                    const int b = grow / p.vt_T, t = grow - b * p.vt_T, v0 = col - int(p.vt_col0), h = v0 >> 6, d0 = v0 & 63;
+                    float* dst = p.vt_out + ((int64_t(b) * p.vt_heads + h) * 64 + d0) * int64_t(p.vt_T) + t;
                     bool bad = false;
 #pragma unroll
                     for (int d = 0; d < 16; d++) {
@@ -522,19 +690,25 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     }
                     const unsigned any_bad = __ballot_sync(0xffffffffu, row_ok && bad);
                     if (lane == 0 && row_ok) {
-                        unsigned char* fl = p.vt_flags + ((b * p.vt_heads + h) * 2 + (d0 >> 5)) * p.vt_n32 + (t >> 5);
+                        unsigned char* fl = p.vt_flags + ((int64_t(b) * p.vt_heads + h) * 2 + (d0 >> 5)) * p.vt_n32 + (t >> 5);
                         *fl = (any_bad != 0 || ((d0 & 16) && *fl != 0)) ? 1 : 0;   // two groups share a flag, in this order
                     }
-                    continue;
+                    return;
                 }
-                if (IMG && p.im.res != nullptr) {
+                if (IMG && p.im.res != nullptr && row_ok) {
 #pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const uint32_t hw = (&rc[IMG ? j >> 2 : 0].x)[j & 3], lw = (&rc[IMG ? 2 + (j >> 2) : 0].x)[j & 3];
-                        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hw)), l = __half22float2(*reinterpret_cast<const __half2*>(&lw));
-                        v[2 * j] = fmaf(h.x + l.x, res_inv, v[2 * j]);
-                        v[2 * j + 1] = fmaf(h.y + l.y, res_inv, v[2 * j + 1]);
-                    }
+                    for (int j = 0; j < 16; j += 8)
+                        if (col + j < N) {
+                            const uint16_t* src = p.im.res + int64_t(grow) * N + col + j;
+                            const uint4 hq = *reinterpret_cast<const uint4*>(src), lq = *reinterpret_cast<const uint4*>(src + p.im.res_plane);
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                const uint32_t hw = (&hq.x)[e], lw = (&lq.x)[e];
+                                const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hw)), l = __half22float2(*reinterpret_cast<const __half2*>(&lw));
+                                v[j + 2 * e] = fmaf(h.x + l.x, res_inv, v[j + 2 * e]);
+                                v[j + 2 * e + 1] = fmaf(h.y + l.y, res_inv, v[j + 2 * e + 1]);
+                            }
+                        }
                 }
                 if (!IMG && p.residual != nullptr) {
                     if (p.tma_out) {
@@ -543,14 +717,14 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     } else {
 #pragma unroll
                         for (int j = 0; j < 16; j++)
-                            if (row_ok && col + j < p.N) v[j] += p.residual[grow * p.ldo + col + j];
+                            if (row_ok && col + j < N) v[j] += p.residual[int64_t(grow) * p.ldo + col + j];
                     }
                 }
                 if (p.relu) {
 #pragma unroll
                     for (int j = 0; j < 16; j++) v[j] = relu_keep_nan(v[j]);
                 }
-                char* stage = reinterpret_cast<char*>(s.stage_out[warp][NSTG > 1 ? sbuf : 0]);
+                char* stage = reinterpret_cast<char*>(s.stage_out[warp][sbuf % NSTG]);
                 if (IMG || p.tma_out) {
                     if (lane == 0) bulk_wait_read<NSTG - 1>();   // the store that used this buffer has read it
                     __syncwarp();
@@ -572,13 +746,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll
                             for (int e = 0; e < 4; e++) {
                                 const float x = v[8 * j + 2 * e], y = v[8 * j + 2 * e + 1];
-                                if (IMG) {   // an infinite value must not take the scale of its whole image along
-                                    rmax = fmaxf(rmax, fabsf(x) < INFINITY ? fabsf(x) : 0.f);
-                                    rmax = fmaxf(rmax, fabsf(y) < INFINITY ? fabsf(y) : 0.f);
-                                } else {
-                                    rmax = fmaxf(rmax, fmaxf(fabsf(x), fabsf(y)));
-                                }
                                 split_f16x2(x * rscale, y * rscale, hp[e], lp[e]);
+                                rmax = __hmax2(rmax, __habs2(*reinterpret_cast<const __half2*>(hp + e)));
                             }
                             const int at = lane * 32 + ((j ^ ((lane >> 2) & 1)) << 4);
                             *reinterpret_cast<uint4*>(stage + at) = hi;
@@ -588,11 +757,11 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     fence_async_smem();
                     __syncwarp();
                     if (lane == 0) {
-                        if (trow < p.M) tma_store_3d(&map_o, stage, int(col), int(trow), 0);
+                        if (trow < M) tma_store_3d(&map_o, stage, col, trow, 0);
                         bulk_commit();
                     }
-                    sbuf ^= 1;
-                    continue;
+                    sbuf++;
+                    return;
                 }
                 // ---- unaligned rows: out[k] = column 16g - shift + k of the row, by two select steps over {previous three, v} ----
                 float u[18], w[16];
@@ -606,14 +775,14 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 }
                 if (row_ok && shift > 0) {   // the 4 - shift leading and the shift trailing columns of this block's row segment
                     if (g == 0) {
-                        if (col < p.N) orow[0] = v[0];
-                        if (shift < 3 && col + 1 < p.N) orow[1] = v[1];
-                        if (shift < 2 && col + 2 < p.N) orow[2] = v[2];
+                        if (col < N) orow[0] = v[0];
+                        if (shift < 3 && col + 1 < N) orow[1] = v[1];
+                        if (shift < 2 && col + 2 < N) orow[2] = v[2];
                     }
-                    if (g + 1 == HALF / 16 || col + 16 >= p.N) {
-                        if (col + 15 < p.N) orow[g * 16 + 15] = v[15];
-                        if (shift > 1 && col + 14 < p.N) orow[g * 16 + 14] = v[14];
-                        if (shift > 2 && col + 13 < p.N) orow[g * 16 + 13] = v[13];
+                    if (g + 1 == HALF / 16 || col + 16 >= N) {
+                        if (col + 15 < N) orow[g * 16 + 15] = v[15];
+                        if (shift > 1 && col + 14 < N) orow[g * 16 + 14] = v[14];
+                        if (shift > 2 && col + 13 < N) orow[g * 16 + 13] = v[13];
                     }
                 }
                 c0 = v[13]; c1 = v[14]; c2 = v[15];
@@ -626,27 +795,59 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll
                 for (int i = 0; i < 4; i++) {   // 4 lanes cover a row's 64 bytes, 8 rows per instruction
                     const int rr = i * 8 + (lane >> 2);
-                    const int64_t gr = trow + rr;
-                    float* rp = p.out + gr * p.ldo + col;
+                    const int gr = trow + rr;
+                    float* rp = p.out + int64_t(gr) * p.ldo + col;
                     const int a = int((reinterpret_cast<uintptr_t>(rp) >> 2) & 3), c = piece * 4 - a;
                     const float4 x = *reinterpret_cast<const float4*>(stage + rr * 64 + ((piece ^ ((rr >> 1) & 3)) << 4));
-                    if (gr >= p.M || (g == 0 && c < 0)) continue;   // the piece left of the block belongs to the neighbour
-                    if (col + c + 3 < p.N) {
+                    if (gr >= M || (g == 0 && c < 0)) continue;   // the piece left of the block belongs to the neighbour
+                    if (col + c + 3 < N) {
                         *reinterpret_cast<float4*>(rp + c) = x;
                     } else {
-                        if (col + c < p.N) rp[c] = x.x;
-                        if (col + c + 1 < p.N) rp[c + 1] = x.y;
-                        if (col + c + 2 < p.N) rp[c + 2] = x.z;
+                        if (col + c < N) rp[c] = x.x;
+                        if (col + c + 1 < N) rp[c + 1] = x.y;
+                        if (col + c + 2 < N) rp[c + 2] = x.z;
                     }
                 }
+            };
+            auto all_groups = [&](auto&& group) {
+                if (single) {
+                    uint32_t acc[16];
+                    tmem_ld16(tacc, acc);
+                    tmem_wait_ld();
+#pragma unroll 1
+                    for (int g = 0; g < groups; g++) {
+                        float v[16];
+#pragma unroll
+                        for (int j = 0; j < 16; j++) v[j] = __uint_as_float(acc[j]);
+                        tmem_ld16(tacc + uint32_t(min(g + 1, HALF / 16 - 1) * 16), acc);   // the next group's, behind this one's work
+                        group(g, v);
+                        tmem_wait_ld();
+                    }
+                    release((ccount - 1) % ACC);
+                } else {
+#pragma unroll 1
+                    for (int g = 0; g < groups; g++) {
+                        float v[16];
+                        pick_group<0, HALF / 16>(sum, g, v);
+                        group(g, v);
+                    }
+                }
+            };
+            if (fast) {
+                if (p.so == nullptr) all_groups([&](int g, float (&v)[16]) { finish_fast(g, v, std::false_type()); });
+                else all_groups([&](int g, float (&v)[16]) { finish_fast(g, v, std::true_type()); });
+            } else {
+                all_groups(finish);
             }
             if (NPL == 2 && p.so != nullptr && !writes_partial) {
+                // hi is within 2^-11 of the value; an infinite one must not take the scale of its whole image along
+                const float top = fminf(fmaxf(__low2float(rmax), __high2float(rmax)) * 1.0005f, 32768.f) * rinv;
                 if (!IMG) {
-                    if (row_ok) p.so_amax[grow * p.so_parts + tn * 2 + chalf] = rmax;
+                    if (row_ok) p.so_amax[int64_t(grow) * p.so_parts + tn * 2 + chalf] = top;
                 } else {   // non-negative floats order like integers
                     unsigned* at = reinterpret_cast<unsigned*>(p.so_amax);
                     const int first = __shfl_sync(0xffffffffu, int(image), 0);
-                    const unsigned m = row_ok ? __float_as_uint(rmax) : 0u;
+                    const unsigned m = row_ok ? __float_as_uint(top) : 0u;
                     if (warp_all(!row_ok || int(image) == first)) {
                         const unsigned all = __reduce_max_sync(0xffffffffu, m);
                         if (lane == 0 && row_ok) atomicMax(at + first, all);
@@ -782,12 +983,12 @@ int make_out_map(CUtensorMap* map, const F16GemmArgs& a, int planes) {
     cuuint32_t estr[3] = {1, 1, 1};
     void* base = split ? static_cast<void*>(a.split_out.planes) : static_cast<void*>(a.out);
     CUresult r = fn(map, split ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    split ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                    split ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     FXF_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (f16 output) failed with code %d", int(r));
     return 0;
 }
 
-constexpr int kChunkKDense = 1024, kChunkKConv = 64, kChunkKRows = 256;
+constexpr int kChunkKDense = 1024, kChunkKConv = 128, kChunkKRows = 256;
 
 // Times in microseconds as measured on B200 inside a chain of launches: `slab` per 64-deep K-slab of a tile, `gap` what every
 // tile adds (its epilogue runs under the next tile's products), `drain` the exposed epilogue of the last one.
@@ -814,14 +1015,21 @@ TailSplit plan_tail(int64_t tiles, int num_k, const Variant& v, int workers, boo
 template <int BN, int STAGES, bool PAIR, int NPL, bool IMG = false>
 int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int workers, ExecCtx& ctx, const CUtensorMap* im2col = nullptr) {
     constexpr int BNB = PAIR ? BN / 2 : BN;
-    CUtensorMap mx, mw, mo;
+    CUtensorMap mx, mw, mo, mr;
     if (IMG && p.im.c_slabs > 0) mx = *im2col;
     else if (make_map(&mx, a.x.planes, a.M, a.K, a.x.ld ? a.x.ld : a.K, a.x.plane, NPL, BM)) return 1;
     if (make_map(&mw, a.w.planes, a.N, a.K, a.w.ld ? a.w.ld : a.K, a.w.plane, NPL, BNB)) return 1;
     mo = mx;
     if (p.tma_out && make_out_map(&mo, a, NPL)) return 1;
-    const size_t smem = sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL)>) + 1024;
-    static_assert(sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL)>) + 1024 <= 227 * 1024, "shared memory of a CTA");
+    mr = mo;
+    if (IMG && p.im.res != nullptr) {   // laid out like the result
+        F16GemmArgs r = a;
+        r.split_out.planes = const_cast<uint16_t*>(p.im.res);
+        r.split_out.plane = p.im.res_plane;
+        if (make_out_map(&mr, r, NPL)) return 1;
+    }
+    const size_t smem = sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL, IMG)>) + 1024;
+    static_assert(sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL, IMG)>) + 1024 <= 227 * 1024, "shared memory of a CTA");
     auto kernel = gemm_f16_kernel<BN, STAGES, PAIR, NPL, IMG>;
     static bool configured[64] = {};
     int dev = 0;
@@ -832,7 +1040,7 @@ int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int w
     }
     const int64_t units = ts.full + ts.tail * ts.parts;
     const int grid = int(std::min<int64_t>(units, workers)) * (PAIR ? 2 : 1);
-    FXF_CUDA(launch_dependent(kernel, dim3(unsigned(grid)), dim3(kThreads), smem, ctx.stream, PAIR ? 2 : 1, mx, mw, mo, p));
+    FXF_CUDA(launch_dependent(kernel, dim3(unsigned(grid)), dim3(kThreads), smem, ctx.stream, PAIR ? 2 : 1, mx, mw, mo, mr, p));
     FXF_LAUNCHED(ctx);
     return 0;
 }
@@ -840,7 +1048,7 @@ int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int w
 }  // namespace
 
 bool gemm_f16_shape_ok(int64_t M, int64_t N, int64_t K) {
-    return M >= 1 && N >= 1 && K >= 16 && K % 8 == 0 && M < (int64_t(1) << 31) && N < (int64_t(1) << 31) && K < (int64_t(1) << 31);
+    return M >= 1 && N >= 1 && K >= 16 && K % 8 == 0 && M < (int64_t(1) << 31) - 512 && N < (int64_t(1) << 31) - 512 && K < (int64_t(1) << 31);
 }
 
 int gemm_f16_split_parts(int64_t N) { return int((N + 31) / 32) * 2; }
@@ -920,6 +1128,8 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     p.M = a.M; p.N = a.N; p.K = a.K; p.ldo = split ? a.N : a.ldo;
     p.relu = a.relu ? 1 : 0;
     p.tma_out = (split || (a.ldo % 4 == 0 && aligned16(a.out) && (a.residual == nullptr || aligned16(a.residual)))) ? 1 : 0;
+    auto sector = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 31) == 0; };
+    p.fast = a.N % 16 == 0 && (split ? sector(a.split_out.planes) && a.split_out.plane % 16 == 0 : a.ldo % 8 == 0 && sector(a.out)) && sector(a.residual) ? 1 : 0;
     p.tiles_m = int((a.M + rows - 1) / rows);
     p.tiles_n = int((a.N + var.bn - 1) / var.bn);
     p.m_fastest = a.N > a.M ? 1 : 0;
@@ -956,12 +1166,12 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     }
     if (im != nullptr) {
         switch (v) {
-            case 0: return launch_variant<256, 3, true, 2, true>(a, p, ts, workers, ctx, im2col);
+            case 0: return launch_variant<256, 2, true, 2, true>(a, p, ts, workers, ctx, im2col);
             case 1: return launch_variant<192, 3, true, 2, true>(a, p, ts, workers, ctx, im2col);
-            case 2: return launch_variant<128, 4, true, 2, true>(a, p, ts, workers, ctx, im2col);
+            case 2: return launch_variant<128, 3, true, 2, true>(a, p, ts, workers, ctx, im2col);
             case 3: return launch_variant<64, 4, true, 2, true>(a, p, ts, workers, ctx, im2col);
-            case 4: return launch_variant<128, 3, false, 2, true>(a, p, ts, workers, ctx, im2col);
-            case 5: return launch_variant<64, 4, false, 2, true>(a, p, ts, workers, ctx, im2col);
+            case 4: return launch_variant<128, 2, false, 2, true>(a, p, ts, workers, ctx, im2col);
+            case 5: return launch_variant<64, 3, false, 2, true>(a, p, ts, workers, ctx, im2col);
             default: return launch_variant<32, 4, false, 2, true>(a, p, ts, workers, ctx, im2col);
         }
     }
