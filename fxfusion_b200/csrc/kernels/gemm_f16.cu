@@ -49,30 +49,29 @@ namespace {
 using namespace sm100;
 
 constexpr int BM = 128, BK = 64;
-constexpr int kEpiWarps = 8, kTmaWarp = 8, kMmaWarp = 9, kThreads = 384;
 constexpr int ACC = 2;
 enum : int { kErrWaitFull = 131, kErrWaitEmpty = 133, kErrWaitAcc = 134, kErrWaitAccEmpty = 135, kErrWaitPartial = 136, kErrWaitResidual = 137 };
 
 // output staging buffers per epilogue warp, as far as the operand ring leaves room: a store may still be reading one (images:
 // and the residual be on its way into two others)
-constexpr int staging_buffers(int bn, int bnb, int stages, int npl, bool images) {
-    const int room = 225 * 1024 - stages * npl * (BM + bnb) * BK * 2 - kEpiWarps * bn * 4;
-    const int fit = room / (kEpiWarps * 2048), want = images ? 4 : 2;
+constexpr int staging_buffers(int bn, int bnb, int stages, int npl, bool images, int warps) {
+    const int room = 225 * 1024 - stages * npl * (BM + bnb) * BK * 2 - 32 * bn;
+    const int fit = room / (warps * 2048), want = images ? 4 : 2;
     return fit < 1 ? 1 : (fit < want ? fit : want);
 }
 
 // BNB = weight rows held by this CTA; NPL = planes per operand (2: f16x3, 1: bf16)
-template <int BN, int BNB, int STAGES, int NPL, int NSTG>
+template <int BN, int BNB, int STAGES, int NPL, int NSTG, int EW>
 struct alignas(1024) F16Smem {
     uint16_t a[STAGES][NPL][BM * BK];
     uint16_t b[STAGES][NPL][BNB * BK];
-    float stage_out[kEpiWarps][NSTG][32 * 16];       // 32 rows x 16 columns per epilogue warp (64-byte rows, 64-byte swizzle)
-    float col_inv[kEpiWarps][BN / 2], col_bias[kEpiWarps][BN / 2];   // 1 / scale and bias of a warp's columns
+    float stage_out[EW][NSTG][32 * 16];       // 32 rows x 16 columns per epilogue warp (64-byte rows, 64-byte swizzle)
+    float col_inv[EW][BN * 4 / EW], col_bias[EW][BN * 4 / EW];   // 1 / scale and bias of a warp's columns
     uint64_t full[STAGES];
     uint64_t empty[STAGES];
     uint64_t acc_full[ACC];
     uint64_t acc_empty[ACC];
-    uint64_t res_full[kEpiWarps][NSTG];
+    uint64_t res_full[EW][NSTG];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -202,13 +201,17 @@ __device__ __forceinline__ void drain_chunk(uint32_t tacc, float (&sum)[HALF]) {
     }
 }
 
-template <int BN, int STAGES, bool PAIR, int NPL, bool IMG>
-__global__ void __launch_bounds__(kThreads, 1)
+// EW epilogue warps: eight, or sixteen for units of a single chain, which need no registers for sums.  Those are short products
+// (K <= 128) bound by the epilogue, where a scheduler with two of its warps issues an instruction every other cycle:
+// 128 images of 56 x 56, 64 -> 256 channels with residual 215 -> 178 us (7.7 TB/s would take 120).
+template <int BN, int STAGES, bool PAIR, int NPL, bool IMG, int EW>
+__global__ void __launch_bounds__(EW * 32 + 128, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_r, F16Params p) {
     extern __shared__ unsigned char smem_raw[];
     constexpr int BNB = PAIR ? BN / 2 : BN;
-    constexpr int kStg = staging_buffers(BN, BNB, STAGES, NPL, IMG);
-    using Smem = F16Smem<BN, BNB, STAGES, NPL, kStg>;
+    constexpr int kStg = staging_buffers(BN, BNB, STAGES, NPL, IMG, EW);
+    constexpr int kTmaWarp = EW, kMmaWarp = EW + 1, PARTS = EW / 4;
+    using Smem = F16Smem<BN, BNB, STAGES, NPL, kStg, EW>;
     Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr uint32_t kABytes = NPL * BM * BK * 2, kBBytes = NPL * BNB * BK * 2;
     constexpr uint32_t kIdesc = NPL == 2 ? umma_idesc_f16(PAIR ? 2 * BM : BM, BN) : umma_idesc_bf16(PAIR ? 2 * BM : BM, BN);
@@ -229,10 +232,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         }
         for (int i = 0; i < ACC; i++) {
             mbar_init(&s.acc_full[i], 1);
-            mbar_init(&s.acc_empty[i], PAIR ? 2 * kEpiWarps : kEpiWarps);
+            mbar_init(&s.acc_empty[i], PAIR ? 2 * EW : EW);
         }
         if (IMG)
-            for (int i = 0; i < kEpiWarps * kStg; i++) mbar_init(&s.res_full[0][0] + i, 1);
+            for (int i = 0; i < EW * kStg; i++) mbar_init(&s.res_full[0][0] + i, 1);
         s.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -257,9 +260,12 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     tc_fence_after();
     const uint32_t tmem_base = s.tmem_base;
 
-    // 384 x 168 registers at launch = 256 x 208 + 128 x 88
-    if (warp >= kEpiWarps) {
-      if (BN >= 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    // registers at launch: 384 x 168 = 256 x 208 + 128 x 88, 640 x 96 = 512 x 104 + 128 x 64
+    if (warp >= EW) {
+      if (BN >= 128) {
+          if (EW == 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+          else asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+      }
       if (warp == kTmaWarp) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
@@ -390,19 +396,22 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         }
       }
     } else {
-        if (BN >= 128) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
-        // ---------------- epilogue (warp w owns TMEM lanes 32*(w%4).. and column half w/4) ----------------
-        // One thread owns one row of its warp's 32 x HALF block.  The group loop stays rolled (only picking a group's sixteen
+        if (BN >= 128) {
+            if (EW == 16) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+            else asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+        }
+        // ---------------- epilogue (warp w owns TMEM lanes 32*(w%4).. and column part w/4) ----------------
+        // One thread owns one row of its warp's 32 x COLS block.  The group loop stays rolled (only picking a group's sixteen
         // running sums is spelled out): unrolled, its code missed the instruction cache at every group.  A group leaves as one
         // TMA store from a swizzled staging block; row-contiguous stores by the LSU, with the lanes re-arranged through shared
         // memory, took 250 instructions and 1900 cycles per group and bound every product of K <= 1024.
-        constexpr int HALF = BN / 2, NSTG = kStg;
+        constexpr int COLS = BN / PARTS, NSTG = kStg;
         // Narrow tiles belong to problems of a wave or two, where the store's latency counts (M = 512, N = 256, K = 256: 5.5 -> 4.4 us
         // with stores from registers); wide ones are stored by TMA, which a row per lane would keep the load / store unit busy for.
         constexpr bool DIRECT = !IMG && BN <= 64;
         static_assert(!IMG || NSTG >= 2, "a residual needs a staging buffer besides the one being stored");
         constexpr int AHEAD = NSTG >= 4 ? 2 : 1;   // images: groups between a residual's request and its use
-        const int q = warp & 3, chalf = warp >> 2;
+        const int q = warp & 3, part = warp >> 2;
         const uint32_t lane_base = uint32_t(q * 32) << 16;
         float *cinv = s.col_inv[warp], *cbias = s.col_bias[warp];
         uint32_t ccount = 0, sbuf = 0, res_use = 0;   // chains, stored groups; parity of each residual buffer
@@ -418,10 +427,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             const bool adds_partials = un.nparts > 1 && un.part == 0;
             const int slot = PAIR ? un.u * 2 + rank : un.u, pstep = PAIR ? 2 : 1;
             // partial tiles: [column half][row quarter][4-column group][lane] float4, so that every access is coalesced
-            float4* ws_mine = reinterpret_cast<float4*>(p.ws + size_t(slot) * size_t(BM * BN)) + warp * (HALF / 4) * 32 + lane;
+            float4* ws_mine = reinterpret_cast<float4*>(p.ws + size_t(slot) * size_t(BM * BN)) + warp * (COLS / 4) * 32 + lane;
             const int trow = tm * BM + q * 32, grow = trow + lane;   // first row of this warp, row of this thread
             const bool row_ok = grow < M;
-            const int col_base = tn * BN + chalf * HALF;
+            const int col_base = tn * BN + part * COLS;
             // constants of the row and of the columns, fetched while the tensor core works
             const int image = IMG ? int(unsigned(grow) / p.im.rpi) : 0;
             const int64_t sx = IMG ? image : grow * p.x_inv_stride;
@@ -437,10 +446,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 float bound = fmaf(am, __ldg(p.w_bound), __ldg(p.w_bound + 1));
                 if (IMG && p.im.res != nullptr) bound += __ldg(p.im.res_amax + image);
                 split_scale(bound, rscale, rinv);
-                if (chalf == 0 && tn == 0 && (!IMG || unsigned(grow) == unsigned(image) * p.im.rpi)) p.so_inv[so_at] = rinv;
+                if (part == 0 && tn == 0 && (!IMG || unsigned(grow) == unsigned(image) * p.im.rpi)) p.so_inv[so_at] = rinv;
             }
             const bool fast = p.fast && un.nparts == 1 && (IMG || p.vt_out == nullptr || col_base < p.vt_col0);
-            const int groups = writes_partial ? HALF / 16 : min(HALF, N - col_base + 15) / 16;   // warp-uniform; may be negative
+            const int groups = writes_partial ? COLS / 16 : min(COLS, N - col_base + 15) / 16;   // warp-uniform; may be negative
             // the residual's next sixteen columns, requested ahead of their use: fp32 into registers, images into staging buffers
             Words<8> rn[2] = {};
             auto fetch_residual = [&](int col) {
@@ -464,7 +473,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 }
             if (tn != have_tn) {
                 __syncwarp();
-                for (int j = lane; j < HALF; j += 32) {
+                for (int j = lane; j < COLS; j += 32) {
                     const int c = col_base + j;
                     cinv[j] = (p.w_inv && c < N) ? __ldg(p.w_inv + c * p.w_inv_stride) : 1.f;
                     cbias[j] = (p.bias && !p.swap && c < N) ? __ldg(p.bias + c) : 0.f;
@@ -473,8 +482,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 have_tn = tn;
             }
             // A unit of one chain is read from its accumulator group by group; of several, the sums are in registers.
-            const bool single = un.k1 - un.k0 <= chunk;
-            const uint32_t tacc = tmem_base + (ccount % ACC) * uint32_t(BN) + lane_base + uint32_t(chalf * HALF);
+            const bool single = EW == 16 || un.k1 - un.k0 <= chunk;
+            const uint32_t tacc = tmem_base + (ccount % ACC) * uint32_t(BN) + lane_base + uint32_t(part * COLS);
             auto release = [&](uint32_t buf) {
                 tc_fence_before();
                 __syncwarp();
@@ -483,10 +492,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     else mbar_arrive(&s.acc_empty[buf]);
                 }
             };
-            float sum[HALF];
-            if (!single) {
+            float sum[EW == 16 ? 16 : COLS];   // (a single chain keeps none)
+            if (EW == 8 && !single) {
 #pragma unroll
-                for (int j = 0; j < HALF; j++) sum[j] = 0.f;
+                for (int j = 0; j < COLS; j++) sum[j] = 0.f;
             }
             bool alive = true;
             for (int kc0 = un.k0; kc0 < un.k1; kc0 += chunk, ccount++) {
@@ -497,9 +506,11 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     break;
                 }
                 tc_fence_after();
-                if (!single) {
-                    drain_chunk<HALF>(tmem_base + buf * uint32_t(BN) + lane_base + uint32_t(chalf * HALF), sum);
-                    release(buf);
+                if constexpr (EW == 8) {
+                    if (!single) {
+                        drain_chunk<COLS>(tmem_base + buf * uint32_t(BN) + lane_base + uint32_t(part * COLS), sum);
+                        release(buf);
+                    }
                 }
             }
             if (!alive) break;
@@ -509,7 +520,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             if (adds_partials) {
                 int ok = 1;
                 if (lane == 0)
-                    for (int pp = 1; pp < un.nparts && ok; pp++) ok = flag_wait(p.flags + (slot + pp * pstep) * kEpiWarps + warp, abort_flag) ? 1 : 0;
+                    for (int pp = 1; pp < un.nparts && ok; pp++) ok = flag_wait(p.flags + (slot + pp * pstep) * EW + warp, abort_flag) ? 1 : 0;
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) {
                     give_up(abort_flag, p.status, kErrWaitPartial);
@@ -529,7 +540,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 constexpr bool SPLIT = decltype(split_tag)::value;
                 const int col = col_base + g * 16;
                 const Words<8> r0 = rn[0], r1 = rn[1];
-                fetch_residual(g + 1 < HALF / 16 ? col + 16 : N);
+                fetch_residual(g + 1 < COLS / 16 ? col + 16 : N);
                 const uint32_t buf = sbuf % NSTG;
                 char* stage = reinterpret_cast<char*>(s.stage_out[warp][buf]);
                 if (image_res) {
@@ -779,7 +790,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                         if (shift < 3 && col + 1 < N) orow[1] = v[1];
                         if (shift < 2 && col + 2 < N) orow[2] = v[2];
                     }
-                    if (g + 1 == HALF / 16 || col + 16 >= N) {
+                    if (g + 1 == COLS / 16 || col + 16 >= N) {
                         if (col + 15 < N) orow[g * 16 + 15] = v[15];
                         if (shift > 1 && col + 14 < N) orow[g * 16 + 14] = v[14];
                         if (shift > 2 && col + 13 < N) orow[g * 16 + 13] = v[13];
@@ -819,16 +830,16 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                         float v[16];
 #pragma unroll
                         for (int j = 0; j < 16; j++) v[j] = __uint_as_float(acc[j]);
-                        tmem_ld16(tacc + uint32_t(min(g + 1, HALF / 16 - 1) * 16), acc);   // the next group's, behind this one's work
+                        tmem_ld16(tacc + uint32_t(min(g + 1, COLS / 16 - 1) * 16), acc);   // the next group's, behind this one's work
                         group(g, v);
                         tmem_wait_ld();
                     }
                     release((ccount - 1) % ACC);
-                } else {
+                } else if constexpr (EW == 8) {
 #pragma unroll 1
                     for (int g = 0; g < groups; g++) {
                         float v[16];
-                        pick_group<0, HALF / 16>(sum, g, v);
+                        pick_group<0, COLS / 16>(sum, g, v);
                         group(g, v);
                     }
                 }
@@ -843,27 +854,21 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 // hi is within 2^-11 of the value; an infinite one must not take the scale of its whole image along
                 const float top = fminf(fmaxf(__low2float(rmax), __high2float(rmax)) * 1.0005f, 32768.f) * rinv;
                 if (!IMG) {
-                    if (row_ok) p.so_amax[int64_t(grow) * p.so_parts + tn * 2 + chalf] = top;
-                } else {   // non-negative floats order like integers
-                    unsigned* at = reinterpret_cast<unsigned*>(p.so_amax);
-                    const int first = __shfl_sync(0xffffffffu, int(image), 0);
-                    const unsigned m = row_ok ? __float_as_uint(top) : 0u;
-                    if (warp_all(!row_ok || int(image) == first)) {
-                        const unsigned all = __reduce_max_sync(0xffffffffu, m);
-                        if (lane == 0 && row_ok) atomicMax(at + first, all);
-                    } else if (row_ok) {
-                        atomicMax(at + image, m);
-                    }
+                    if (row_ok) p.so_amax[int64_t(grow) * p.so_parts + tn * PARTS + part] = top;
+                } else {   // one atomic per image among the warp's rows (an atomic per row: 85 us instead of 60 for 7 x 7 images)
+                    const unsigned same = __match_any_sync(0xffffffffu, row_ok ? image : -1);
+                    const unsigned all = __reduce_max_sync(same, __float_as_uint(top));   // non-negative floats order like integers
+                    if (row_ok && lane == __ffs(same) - 1) atomicMax(reinterpret_cast<unsigned*>(p.so_amax) + image, all);
                 }
             }
             if (writes_partial) {
                 __threadfence();
                 __syncwarp();
-                if (lane == 0) flag_set(p.flags + slot * kEpiWarps + warp, 1);
+                if (lane == 0) flag_set(p.flags + slot * EW + warp, 1);
             } else if (adds_partials) {
                 __syncwarp();
                 if (lane == 0)
-                    for (int pp = 1; pp < un.nparts; pp++) flag_set(p.flags + (slot + pp * pstep) * kEpiWarps + warp, 0);
+                    for (int pp = 1; pp < un.nparts; pp++) flag_set(p.flags + (slot + pp * pstep) * EW + warp, 0);
             }
         }
         if (p.tma_out && lane == 0) bulk_wait_all();
@@ -994,8 +999,13 @@ constexpr int kChunkKDense = 1024, kChunkKConv = 128, kChunkKRows = 256;
 // tile adds (its epilogue runs under the next tile's products), `drain` the exposed epilogue of the last one.
 struct Variant { bool pair; int bn; double slab, gap, drain; };
 const Variant kVariants[] = {
-    {true, 256, 0.88, 1.5, 6.8}, {true, 192, 0.78, 0.6, 4.9}, {true, 128, 0.54, 0.4, 2.8}, {true, 64, 0.37, 0.2, 1.5},
-    {false, 128, 0.64, 0.3, 2.0}, {false, 64, 0.47, 0.3, 1.0}, {false, 32, 0.39, 0.2, 0.3},
+    {true, 256, 0.88, 1.5, 6.0}, {true, 192, 0.78, 0.6, 4.0}, {true, 128, 0.54, 0.4, 2.9}, {true, 64, 0.37, 0.2, 1.9},
+    {false, 128, 0.64, 0.3, 2.1}, {false, 64, 0.47, 0.3, 1.3}, {false, 32, 0.39, 0.2, 0.6},
+};
+// Images: chains of 128, and an epilogue that often outlasts the products (it is part of `gap`).
+const Variant kImageVariants[] = {
+    {true, 256, 1.15, 5.0, 4.0}, {true, 192, 0.80, 4.4, 3.5}, {true, 128, 0.62, 3.2, 2.5}, {true, 64, 0.43, 2.2, 1.5},
+    {false, 128, 0.74, 2.9, 2.0}, {false, 64, 0.55, 1.6, 1.0}, {false, 32, 0.46, 1.3, 0.5},
 };
 struct TailSplit { int64_t full, tail; int parts; double us; };
 // Whole tiles first, then the remainder R = tiles % workers cut along K into s parts each (see F16Params).
@@ -1012,7 +1022,7 @@ TailSplit plan_tail(int64_t tiles, int num_k, const Variant& v, int workers, boo
     return best;
 }
 
-template <int BN, int STAGES, bool PAIR, int NPL, bool IMG = false>
+template <int BN, int STAGES, bool PAIR, int NPL, bool IMG = false, int EW = 8>
 int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int workers, ExecCtx& ctx, const CUtensorMap* im2col = nullptr) {
     constexpr int BNB = PAIR ? BN / 2 : BN;
     CUtensorMap mx, mw, mo, mr;
@@ -1028,9 +1038,9 @@ int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int w
         r.split_out.plane = p.im.res_plane;
         if (make_out_map(&mr, r, NPL)) return 1;
     }
-    const size_t smem = sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL, IMG)>) + 1024;
-    static_assert(sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL, IMG)>) + 1024 <= 227 * 1024, "shared memory of a CTA");
-    auto kernel = gemm_f16_kernel<BN, STAGES, PAIR, NPL, IMG>;
+    const size_t smem = sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL, IMG, EW), EW>) + 1024;
+    static_assert(sizeof(F16Smem<BN, BNB, STAGES, NPL, staging_buffers(BN, BNB, STAGES, NPL, IMG, EW), EW>) + 1024 <= 227 * 1024, "shared memory of a CTA");
+    auto kernel = gemm_f16_kernel<BN, STAGES, PAIR, NPL, IMG, EW>;
     static bool configured[64] = {};
     int dev = 0;
     FXF_CUDA(cudaGetDevice(&dev));
@@ -1040,7 +1050,7 @@ int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int w
     }
     const int64_t units = ts.full + ts.tail * ts.parts;
     const int grid = int(std::min<int64_t>(units, workers)) * (PAIR ? 2 : 1);
-    FXF_CUDA(launch_dependent(kernel, dim3(unsigned(grid)), dim3(kThreads), smem, ctx.stream, PAIR ? 2 : 1, mx, mw, mo, mr, p));
+    FXF_CUDA(launch_dependent(kernel, dim3(unsigned(grid)), dim3(EW * 32 + 128), smem, ctx.stream, PAIR ? 2 : 1, mx, mw, mo, mr, p));
     FXF_LAUNCHED(ctx);
     return 0;
 }
@@ -1073,12 +1083,12 @@ int launch_bias_bound(const float* bias, int64_t n, float* bound, ExecCtx& ctx) 
 
 // The variant with the least modelled time.  Wide pair tiles win once they fill the machine; smaller problems take narrower
 // tiles until every SM has one.  `force` >= 0 picks an entry of kVariants.
-static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pairs, bool k_split, bool vt, int64_t vt_col0, TailSplit* out_ts, int* out_workers, int force) {
+static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pairs, bool k_split, bool vt, int64_t vt_col0, bool images, TailSplit* out_ts, int* out_workers, int force) {
     const int num_k = int((K + BK - 1) / BK);
     int best = -1;
     double best_us = 0;
     for (int i = 0; i < int(sizeof(kVariants) / sizeof(kVariants[0])); i++) {
-        const Variant& v = kVariants[i];
+        const Variant& v = images ? kImageVariants[i] : kVariants[i];
         if (force >= 0 && i != force) continue;
         if (v.pair && (!pairs || M <= BM || sm_count < 2)) continue;
         if (vt && ((v.bn / 2) % 32 != 0 || vt_col0 % (v.bn / 2) != 0)) continue;   // a warp's columns: whole halves of a head
@@ -1096,7 +1106,7 @@ static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pair
 }
 
 std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, int sm_count) {
-    const int v = pick_variant(M, N, K, sm_count, true, true, false, 0, nullptr, nullptr, -1);
+    const int v = pick_variant(M, N, K, sm_count, true, true, false, 0, false, nullptr, nullptr, -1);
     if (v < 0) return "none";
     return strfmt("%s-%dx%d%s", bf16 ? "bf16" : "f16x3", kVariants[v].pair ? 256 : 128, kVariants[v].bn, kVariants[v].pair ? "-pair" : "");
 }
@@ -1104,7 +1114,7 @@ std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, in
 bool gemm_f16_vt_ok(const F16GemmArgs& a, const ExecCtx& ctx) {
     if (a.vt_out == nullptr || a.vt_flags == nullptr || a.residual != nullptr || a.relu || a.split_out.planes != nullptr) return false;
     if (a.vt_T <= 0 || a.vt_T % 32 != 0 || a.M % a.vt_T != 0 || (a.N - a.vt_col0) != int64_t(a.vt_heads) * 64) return false;
-    return pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, false, true, a.vt_col0, nullptr, nullptr, -1) >= 0;
+    return pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, false, true, a.vt_col0, false, nullptr, nullptr, -1) >= 0;
 }
 
 static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorMap* im2col, const char* tag, double flops, ExecCtx& ctx) {
@@ -1116,7 +1126,7 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     TailSplit ts{};
     int workers = 0;
     const bool ks = ctx.gemm_ws != nullptr && ctx.gemm_flags != nullptr;
-    const int v = pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, ks, a.vt_out != nullptr, a.vt_col0, &ts, &workers, ctx.f16_variant);
+    const int v = pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, ks, a.vt_out != nullptr, a.vt_col0, im != nullptr, &ts, &workers, ctx.f16_variant);
     FXF_CHECK(v >= 0, "f16 GEMM: no kernel variant for M=%lld N=%lld K=%lld", (long long)a.M, (long long)a.N, (long long)a.K);
     const Variant& var = kVariants[v];
     const int rows = var.pair ? 2 * BM : BM, per_unit = var.pair ? 2 : 1;
@@ -1136,7 +1146,7 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     p.status = ctx.status;
     if (im != nullptr) p.im = *im;
     if (ts.parts > 1 && (size_t(ts.tail) * ts.parts * per_unit * size_t(BM) * var.bn * sizeof(float) > ctx.gemm_ws_bytes ||
-                         ts.tail * ts.parts * per_unit * kEpiWarps > ctx.gemm_flag_count))
+                         ts.tail * ts.parts * per_unit * 8 > ctx.gemm_flag_count))
         ts = TailSplit{int64_t(p.tiles_m) * p.tiles_n, 0, 1, 0.0};
     p.full_tiles = int(ts.full); p.tail_tiles = int(ts.tail); p.tail_split = ts.parts;
     p.chunk_slabs = std::max(1, (ctx.tc_chunk_k > 0 ? ctx.tc_chunk_k : (a.conv_chain ? kChunkKConv : kChunkKDense)) / BK);
@@ -1166,7 +1176,9 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     }
     if (im != nullptr) {
         switch (v) {
-            case 0: return launch_variant<256, 2, true, 2, true>(a, p, ts, workers, ctx, im2col);
+            case 0:
+                if (a.K <= int64_t(p.chunk_slabs) * BK) return launch_variant<256, 2, true, 2, true, 16>(a, p, ts, workers, ctx, im2col);
+                return launch_variant<256, 2, true, 2, true>(a, p, ts, workers, ctx, im2col);
             case 1: return launch_variant<192, 3, true, 2, true>(a, p, ts, workers, ctx, im2col);
             case 2: return launch_variant<128, 3, true, 2, true>(a, p, ts, workers, ctx, im2col);
             case 3: return launch_variant<64, 4, true, 2, true>(a, p, ts, workers, ctx, im2col);
