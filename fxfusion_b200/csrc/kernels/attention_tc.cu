@@ -67,7 +67,7 @@ __device__ __forceinline__ void soft_sync(int quarter) { asm volatile("bar.sync 
 // ---- V transpose -------------------------------------------------------------------------------------
 // Also records, per (batch*head, half of the head's 64 columns, 32-key slab), whether any V element is NaN or infinite:
 // vflags[(bh * 2 + half) * n32 + slab] (this kernel reports a slab under half 0 and clears half 1).
-__global__ void __launch_bounds__(256) attn_vt_kernel(const float* __restrict__ qkv, int64_t ld, int64_t v_off, int T, int H, float* __restrict__ vt,
+__global__ void __launch_bounds__(256) attn_vt_kernel(const float* __restrict__ qkv, int64_t ld, int64_t v_off, int T, int Tp, int H, float* __restrict__ vt,
                                                       unsigned char* __restrict__ vflags, int n32) {
     grid_dep();
     // one block moves 64 keys x 64 head columns: rows of 256 bytes on both sides
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256) attn_vt_kernel(const float* __restrict__ 
     }
     for (int idx = tid; idx < HD * 64; idx += 256) {
         int d = idx >> 6, tt = idx & 63, t = t0 + tt;
-        if (t < T) vt[(int64_t(bh) * HD + d) * T + t] = tile[d][tt];
+        if (t < T) vt[(int64_t(bh) * HD + d) * Tp + t] = tile[d][tt];
     }
 }
 
@@ -128,6 +128,7 @@ struct AttnTcParams {
     float inv_scale;      // 1 / scale_divisor, used only when that is exact
     int scale_is_pow2;
     int mask_vec16;       // mask rows may be fetched as aligned 16-byte words
+    int mask_words;       // mask bytes of a row are consecutive: fetched as the aligned 4-byte words around them
     int* status;
 };
 
@@ -216,6 +217,35 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
             if (m16.x | m16.y | m16.z | m16.w) mine |= 1ull << (vv / (BKEY / 16));
         }
         // a block whose V rows hold NaN or infinity is kept: 0 * inf has to reach the output
+        for (int sl = threadIdx.x; sl < p.n32; sl += kAttnThreads)
+            if (p.vflags[int64_t(bh) * 2 * p.n32 + sl] | p.vflags[(int64_t(bh) * 2 + 1) * p.n32 + sl]) mine |= 1ull << (sl / (BKEY / 32));
+        const unsigned int lo32 = __reduce_or_sync(0xffffffffu, (unsigned int)(mine & 0xffffffffull));
+        const unsigned int hi32 = __reduce_or_sync(0xffffffffu, (unsigned int)(mine >> 32));
+        mine = (unsigned long long)lo32 | ((unsigned long long)hi32 << 32);
+        if (lane == 0 && mine) atomicOr(&s.need_blocks, mine);
+        __syncthreads();
+    } else if (p.mask_words && nblk <= 64) {
+        unsigned long long mine = 0;
+        const uint8_t* mh = p.mask + int64_t(b) * p.mask_sb + int64_t(h) * p.mask_sh;
+        const int per_row = Tk / 4 + 2, rows = min(BQ, T - q0);
+        for (int idx = threadIdx.x; idx < rows * per_row; idx += kAttnThreads) {
+            const int rr = idx / per_row;
+            const uint8_t* row = mh + int64_t(q0 + rr) * p.mask_sq;
+            const int k = (idx - rr * per_row) * 4 - int(reinterpret_cast<uintptr_t>(row) & 3);   // key of the word's first byte
+            if (k >= Tk || k <= -4) continue;
+            uint32_t w = *reinterpret_cast<const uint32_t*>(row + k);
+            if (k < 0) w &= 0xffffffffu << (-8 * k);
+            if (k + 4 > Tk) w &= 0xffffffffu >> (8 * (k + 4 - Tk));
+            if (w == 0) continue;
+            const int first = max(k, 0) / BKEY, last = min(k + 3, Tk - 1) / BKEY;
+            if (first == last) {
+                mine |= 1ull << first;
+            } else {   // a word across the border of two blocks
+                const int cut = last * BKEY - k;
+                if (w & (0xffffffffu >> (32 - 8 * cut))) mine |= 1ull << first;
+                if (w >> (8 * cut)) mine |= 1ull << last;
+            }
+        }
         for (int sl = threadIdx.x; sl < p.n32; sl += kAttnThreads)
             if (p.vflags[int64_t(bh) * 2 * p.n32 + sl] | p.vflags[(int64_t(bh) * 2 + 1) * p.n32 + sl]) mine |= 1ull << (sl / (BKEY / 32));
         const unsigned int lo32 = __reduce_or_sync(0xffffffffu, (unsigned int)(mine & 0xffffffffull));
@@ -377,39 +407,50 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
             const uint32_t par = i & 1;
             // ---- stage this warp's share of the mask: rows of its quarter, the 32 keys of its half ----
             const int key0 = blk * BKEY + half * 32;
-            if (p.mask_vec16) {
-#pragma unroll
-                for (int it = 0; it < 2; it++) {
-                    const int rr = quarter * 32 + it * 16 + (lane >> 1), kq = key0 + (lane & 1) * 16, qq = q0 + rr;
-                    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                    if (qq < T && kq < Tk) v = *reinterpret_cast<const uint4*>(mhead + int64_t(qq) * p.mask_sq + kq);
-                    *reinterpret_cast<uint4*>(s.mask_rows + rr * kMaskPitch + half * 32 + (lane & 1) * 16) = v;
-                }
-            } else {
-                for (int idx = lane; idx < 32 * 32; idx += 32) {
-                    const int rr = quarter * 32 + (idx >> 5), kc = key0 + (idx & 31), qq = q0 + rr;
-                    unsigned char v = 0;
-                    if (qq < T && kc < Tk) v = mhead[int64_t(qq) * p.mask_sq + int64_t(kc) * p.mask_sk];
-                    s.mask_rows[rr * kMaskPitch + half * 32 + (idx & 31)] = v;
-                }
-            }
-            __syncwarp();
             uint32_t keep = 0;
-            {
+            // 0x01 per non-zero byte, gathered into 4 bits by one multiply
+            auto nonzero4 = [](uint32_t w) { return (((__vcmpne4(w, 0u) & 0x01010101u) * 0x01020408u) >> 24) & 0xFu; };
+            if (p.mask_words && !p.mask_vec16) {
+                // rows at any address: this thread's 32 bytes from the nine aligned words around them (none lies wholly outside the row)
+                const uint8_t* src = mhead + int64_t(qi) * p.mask_sq + key0;
+                const int n = row_ok ? min(32, Tk - key0) : 0, off = int(reinterpret_cast<uintptr_t>(src) & 3);
+                const uint32_t* wp = reinterpret_cast<const uint32_t*>(src - off);
+                uint32_t w = n > 0 ? wp[0] : 0u;
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const uint32_t nw = (k * 4 + 4 < n + off) ? wp[k + 1] : 0u;
+                    keep |= nonzero4(__funnelshift_r(w, nw, 8 * off)) << (4 * k);
+                    w = nw;
+                }
+                if (n < 32) keep &= n > 0 ? (1u << n) - 1u : 0u;
+            } else {
+                if (p.mask_vec16) {
+#pragma unroll
+                    for (int it = 0; it < 2; it++) {
+                        const int rr = quarter * 32 + it * 16 + (lane >> 1), kq = key0 + (lane & 1) * 16, qq = q0 + rr;
+                        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                        if (qq < T && kq < Tk) v = *reinterpret_cast<const uint4*>(mhead + int64_t(qq) * p.mask_sq + kq);
+                        *reinterpret_cast<uint4*>(s.mask_rows + rr * kMaskPitch + half * 32 + (lane & 1) * 16) = v;
+                    }
+                } else {
+                    for (int idx = lane; idx < 32 * 32; idx += 32) {
+                        const int rr = quarter * 32 + (idx >> 5), kc = key0 + (idx & 31), qq = q0 + rr;
+                        unsigned char v = 0;
+                        if (qq < T && kc < Tk) v = mhead[int64_t(qq) * p.mask_sq + int64_t(kc) * p.mask_sk];
+                        s.mask_rows[rr * kMaskPitch + half * 32 + (idx & 31)] = v;
+                    }
+                }
+                __syncwarp();
                 const uint4* mp = reinterpret_cast<const uint4*>(s.mask_rows + row * kMaskPitch + half * 32);
 #pragma unroll
                 for (int w = 0; w < 2; w++) {
                     const uint4 m16 = mp[w];
                     const uint32_t words[4] = {m16.x, m16.y, m16.z, m16.w};
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        // 0x01 per non-zero byte, gathered into 4 bits by one multiply
-                        const uint32_t nz = __vcmpne4(words[k], 0u) & 0x01010101u;
-                        keep |= ((nz * 0x01020408u) >> 24 & 0xFu) << (16 * w + 4 * k);
-                    }
+                    for (int k = 0; k < 4; k++) keep |= nonzero4(words[k]) << (16 * w + 4 * k);
                 }
+                __syncwarp();
             }
-            __syncwarp();
             // ---- pass 1: scale, mask, log2 domain, partial row maximum; processed scores go back to TMEM ----
             if (alive && !mbar_wait(&s.bar_s, par, abort_flag)) { give_up(abort_flag, p.status, kErrAttnS); alive = false; }
             float tmax = -INFINITY;
@@ -547,7 +588,7 @@ int make_map3(CUtensorMap* map, const float* base, int64_t n0, int64_t n1, int64
 bool attention_tc_supported(const AttnArgs& a, int gemm_mode) {
     if (gemm_mode == FXF_GEMM_FP32_SIMT) return false;
     const int Tk = a.kv ? a.Tk : a.T;
-    if (a.hd != HD || Tk % 4 != 0 || Tk < 16 || a.T < 1) return false;   // V^T rows (Tk floats) must be 16-byte multiples
+    if (a.hd != HD || Tk < 16 || a.T < 1) return false;
     if ((Tk + BKEY - 1) / BKEY > 64) return false;   // the kernel tracks its key blocks in one 64-bit word: at most 4096 keys
     if (a.ld_qkv % 4 != 0 || a.ld_ctx % 4 != 0 || (a.q_off | a.k_off | a.v_off) % 4 != 0) return false;
     if (a.kv && (a.ld_kv % 4 != 0 || !aligned16(a.kv))) return false;
@@ -555,9 +596,9 @@ bool attention_tc_supported(const AttnArgs& a, int gemm_mode) {
     return true;
 }
 
-// V^T [B*H, 64, T] followed by one "non-finite" byte per (batch*head, column half of the head, 32-key slab)
+// V^T [B*H, 64, T] (rows padded to 16 bytes) followed by one "non-finite" byte per (batch*head, column half of the head, 32-key slab)
 size_t attention_tc_scratch_bytes(int64_t B, int64_t T, int64_t H) {
-    return size_t(B) * size_t(T) * size_t(H) * HD * sizeof(float) + round_up(size_t(2) * size_t(B) * size_t(H) * size_t((T + 31) / 32), 256);
+    return size_t(B) * round_up(size_t(T), 4) * size_t(H) * HD * sizeof(float) + round_up(size_t(2) * size_t(B) * size_t(H) * size_t((T + 31) / 32), 256);
 }
 
 int launch_attention_tc(const AttnArgs& a, float* vt_scratch, ExecCtx& ctx, bool v_transposed) {
@@ -566,12 +607,12 @@ int launch_attention_tc(const AttnArgs& a, float* vt_scratch, ExecCtx& ctx, bool
     const int Tk = a.kv ? a.Tk : a.T;                     // keys per batch
     const float* kvp = a.kv ? a.kv : a.qkv;               // where K and V live
     const int64_t ldk = a.kv ? a.ld_kv : a.ld_qkv;
-    const int n32 = (Tk + 31) / 32;
+    const int n32 = (Tk + 31) / 32, Tp = (Tk + 3) / 4 * 4;   // V^T rows are 16-byte multiples
     dim3 pgrid(unsigned((Tk + 63) / 64), unsigned(BH));
-    unsigned char* vflags = reinterpret_cast<unsigned char*>(vt_scratch + size_t(BH) * size_t(Tk) * HD);
+    unsigned char* vflags = reinterpret_cast<unsigned char*>(vt_scratch + size_t(BH) * size_t(Tp) * HD);
     if (!v_transposed) {   // otherwise the projection's epilogue has written V^T and the flags already
         tag_launch(ctx, "attention_v_transpose", 0, 8.0 * double(BH) * Tk * HD);
-        dependent(attn_vt_kernel, pgrid, 256, 0, ctx)(kvp, ldk, a.v_off, Tk, a.H, vt_scratch, vflags, n32);
+        dependent(attn_vt_kernel, pgrid, 256, 0, ctx)(kvp, ldk, a.v_off, Tk, Tp, a.H, vt_scratch, vflags, n32);
         FXF_LAUNCHED(ctx);
     }
 
@@ -579,7 +620,7 @@ int launch_attention_tc(const AttnArgs& a, float* vt_scratch, ExecCtx& ctx, bool
     // Q and K tiles come straight out of the packed projection: [B, T, ld] with the row pitch of qkv
     if (make_map3(&mq, a.qkv, a.ld_qkv, a.T, a.B, a.ld_qkv * 4, int64_t(a.T) * a.ld_qkv * 4, BQ)) return 1;
     if (make_map3(&mk, kvp, ldk, Tk, a.B, ldk * 4, int64_t(Tk) * ldk * 4, BKEY)) return 1;
-    if (make_map3(&mv, vt_scratch, Tk, HD, BH, int64_t(Tk) * 4, int64_t(Tk) * HD * 4, HD)) return 1;
+    if (make_map3(&mv, vt_scratch, Tk, HD, BH, int64_t(Tp) * 4, int64_t(Tp) * HD * 4, HD)) return 1;
     AttnTcParams p;
     p.vflags = vflags; p.n32 = int((Tk + 31) / 32);
     p.mask = a.mask; p.ctx = a.ctx; p.B = a.B; p.T = a.T; p.Tk = Tk; p.H = a.H; p.ld_ctx = a.ld_ctx;
@@ -593,6 +634,7 @@ int launch_attention_tc(const AttnArgs& a, float* vt_scratch, ExecCtx& ctx, bool
         p.inv_scale = p.scale_is_pow2 ? 1.0f / a.scale_divisor : 0.f;
     }
     p.mask_vec16 = (a.mask_sk == 1 && Tk % 16 == 0 && a.mask_sb % 16 == 0 && a.mask_sh % 16 == 0 && a.mask_sq % 16 == 0 && aligned16(a.mask)) ? 1 : 0;
+    p.mask_words = a.mask_sk == 1 ? 1 : 0;
     p.status = ctx.status;
     size_t smem = sizeof(AttnTcSmem) + 1024;
     static bool configured[64] = {};

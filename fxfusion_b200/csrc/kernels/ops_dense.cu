@@ -623,7 +623,7 @@ std::unique_ptr<NodePlan> plan_mha(const Registry& reg, const TensorIds& in, con
     pl->scratch_bytes = size_t(M) * size_t(3 * Dl + Dl) * sizeof(float);
     if (s_wq.f16 || s_wo.f16) pl->scratch_bytes += split_area_bytes(M, D);
     if (s_wq.f16) pl->takes_split = takes_split_rows(M, 3 * Dl) ? 1 : 0;
-    const bool tc_attn = env.gemm_mode != FXF_GEMM_FP32_SIMT && hd == 64 && T % 4 == 0 && T >= 16 && T <= 4096 && Dl % 4 == 0;   // the tcgen05 kernel covers at most 32 blocks of 128 keys
+    const bool tc_attn = env.gemm_mode != FXF_GEMM_FP32_SIMT && hd == 64 && T >= 16 && T <= 4096 && Dl % 4 == 0;   // the tcgen05 kernel covers at most 32 blocks of 128 keys
     if (tc_attn) pl->scratch_bytes += attention_tc_scratch_bytes(B, T, Hl);
     pl->flops = 2.0 * M * double(3 * Dl) * D + 4.0 * double(B) * Hl * double(T) * T * hd + 2.0 * double(M) * D * Dl;
     pl->bytes = 4.0 * (2.0 * double(M) * D + double(3 * Dl) * D + 3 * Dl + double(D) * Dl + D) + double(reg[in[1]].nbytes);
@@ -768,7 +768,7 @@ std::unique_ptr<NodePlan> plan_cross_mha(const Registry& reg, const TensorIds& i
     pl->scratch_bytes = (size_t(Mq) * size_t(2 * Dl) + size_t(Mk) * size_t(2 * Dl)) * sizeof(float);
     if (s_wq.f16 || s_wkv.f16 || s_wo.f16) pl->scratch_bytes += split_area_bytes(std::max(Mq, Mk), D);
     pl->takes_split = (s_wq.f16 && takes_split_rows(Mq, Dl) ? 1u : 0u) | (s_wkv.f16 && takes_split_rows(Mk, 2 * Dl) ? 2u : 0u);
-    const bool tc_attn = env.gemm_mode != FXF_GEMM_FP32_SIMT && hd == 64 && Tk % 4 == 0 && Tk >= 16 && Tk <= 4096 && Dl % 4 == 0;
+    const bool tc_attn = env.gemm_mode != FXF_GEMM_FP32_SIMT && hd == 64 && Tk >= 16 && Tk <= 4096 && Dl % 4 == 0;
     if (tc_attn) pl->scratch_bytes += attention_tc_scratch_bytes(B, Tk, Hl);
     pl->flops = 2.0 * double(Mq) * Dl * D + 2.0 * double(Mk) * 2 * Dl * D + 4.0 * double(B) * Hl * double(Tq) * Tk * hd + 2.0 * double(Mq) * D * Dl;
     pl->bytes = 4.0 * (2.0 * double(Mq) * D + double(Mk) * D + 2.0 * double(Dl) * D + 2.0 * double(Dl) * D + 3 * Dl + D) + double(reg[in[2]].nbytes);
