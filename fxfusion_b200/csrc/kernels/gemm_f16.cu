@@ -103,6 +103,7 @@ struct F16Params {
     int relu;
     int tma_out;                  // the result leaves through map_o (16-byte aligned rows): fp32 [M, N] or both planes of the split form
     int fast;                     // whole tiles take the short epilogue (rows in whole 32-byte sectors, of the residual too)
+    int lean;                     // plain fp32 rows at any 4-byte address: whole tiles take the short epilogue for them
     int tiles_m, tiles_n, m_fastest;
     int full_tiles, tail_tiles, tail_split;   // tiles of the last round are cut along K into tail_split parts
     int chunk_slabs;
@@ -646,6 +647,65 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 }
                 sbuf++;
             };
+            // The same for rows that do not start on 16-byte boundaries: row r starts `shift` floats past one and leaves as aligned 16-byte
+            // pieces, sixteen columns lagging by `shift`; the 4 - shift first and the shift last columns of the block on their own.
+            // (8192 x 50257 x 768, the logits of a 50257-word vocabulary: 1500 -> 1350 us.)
+            constexpr bool LEAN = !IMG && BN >= 128;   // (its code costs the one-wave problems of the narrow tiles 0.3 us)
+            const bool lean = LEAN && p.lean && un.nparts == 1 && col_base + COLS <= N && (p.vt_out == nullptr || col_base < p.vt_col0);
+            float* piece_at[4];   // this lane's pieces of the group in hand: rows i * 8 + lane / 4, sixteen bytes each
+            uint32_t piece_ok = 0, piece_left = 0;   // bit i: the row exists; its first piece belongs to the block on the left
+            if (lean) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int gr = trow + i * 8 + (lane >> 2);
+                    float* rp = p.out + int64_t(gr) * p.ldo + col_base;
+                    const int c = (lane & 3) * 4 - int((reinterpret_cast<uintptr_t>(rp) >> 2) & 3);
+                    piece_at[i] = rp + c;
+                    piece_ok |= (gr < M ? 1u : 0u) << i;
+                    piece_left |= (c < 0 ? 1u : 0u) << i;
+                }
+            }
+            auto finish_lean = [&](int g, float (&v)[16]) {
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) {
+                    const float4 ci = *reinterpret_cast<const float4*>(cinv + g * 16 + j), cb = *reinterpret_cast<const float4*>(cbias + g * 16 + j);
+                    v[j] = max_keep_nan(fmaf(v[j] * ci.x, ri, cb.x), floor_at); v[j + 1] = max_keep_nan(fmaf(v[j + 1] * ci.y, ri, cb.y), floor_at);
+                    v[j + 2] = max_keep_nan(fmaf(v[j + 2] * ci.z, ri, cb.z), floor_at); v[j + 3] = max_keep_nan(fmaf(v[j + 3] * ci.w, ri, cb.w), floor_at);
+                }
+                const bool s1 = shift & 1, s2 = shift & 2;
+                float u[18], w[16];   // w[k] = column 16 g - shift + k, by two select steps over {previous three, v}
+                u[0] = s1 ? c0 : c1; u[1] = s1 ? c1 : c2; u[2] = s1 ? c2 : v[0];
+#pragma unroll
+                for (int k = 3; k < 18; k++) u[k] = s1 ? v[k - 3] : v[k - 2];
+#pragma unroll
+                for (int k = 0; k < 16; k++) w[k] = s2 ? u[k] : u[k + 2];
+                c0 = v[13]; c1 = v[14]; c2 = v[15];
+                if (row_ok && shift > 0) {
+                    if (g == 0) {
+                        orow[0] = v[0];
+                        if (shift < 3) orow[1] = v[1];
+                        if (shift < 2) orow[2] = v[2];
+                    }
+                    if (g + 1 == COLS / 16) {
+                        orow[COLS - 1] = v[15];
+                        if (shift > 1) orow[COLS - 2] = v[14];
+                        if (shift > 2) orow[COLS - 3] = v[13];
+                    }
+                }
+                char* stage = reinterpret_cast<char*>(s.stage_out[warp][0]);
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    *reinterpret_cast<float4*>(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = make_float4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+                __syncwarp();
+                const uint32_t skip = g == 0 ? piece_left : 0u;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {   // 4 lanes cover a row's 64 bytes, 8 rows per instruction
+                    const int rr = i * 8 + (lane >> 2);
+                    const float4 x = *reinterpret_cast<const float4*>(stage + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
+                    if ((piece_ok & ~skip) >> i & 1u) *reinterpret_cast<float4*>(piece_at[i] + g * 16) = x;
+                }
+            };
             // sixteen columns: scales, bias, residual, activation, store
             auto finish = [&](int g, float (&v)[16]) {
                 const int col = col_base + g * 16;
@@ -847,6 +907,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             if (fast) {
                 if (p.so == nullptr) all_groups([&](int g, float (&v)[16]) { finish_fast(g, v, std::false_type()); });
                 else all_groups([&](int g, float (&v)[16]) { finish_fast(g, v, std::true_type()); });
+            } else if (lean) {
+                if constexpr (LEAN) all_groups(finish_lean);
             } else {
                 all_groups(finish);
             }
@@ -1007,6 +1069,11 @@ const Variant kImageVariants[] = {
     {true, 256, 1.15, 5.0, 4.0}, {true, 192, 0.80, 4.4, 3.5}, {true, 128, 0.62, 3.2, 2.5}, {true, 64, 0.43, 2.2, 1.5},
     {false, 128, 0.74, 2.9, 2.0}, {false, 64, 0.55, 1.6, 1.0}, {false, 32, 0.46, 1.3, 0.5},
 };
+// bf16: a third of the products, so that the epilogue shows (in `gap`).
+const Variant kBf16Variants[] = {
+    {true, 256, 0.36, 1.0, 4.0}, {true, 192, 0.26, 3.0, 4.0}, {true, 128, 0.24, 1.7, 2.9}, {true, 64, 0.22, 0.4, 1.9},
+    {false, 128, 0.28, 1.6, 2.1}, {false, 64, 0.24, 0.3, 1.3}, {false, 32, 0.22, 0.3, 0.6},
+};
 struct TailSplit { int64_t full, tail; int parts; double us; };
 // Whole tiles first, then the remainder R = tiles % workers cut along K into s parts each (see F16Params).
 TailSplit plan_tail(int64_t tiles, int num_k, const Variant& v, int workers, bool allowed) {
@@ -1083,12 +1150,12 @@ int launch_bias_bound(const float* bias, int64_t n, float* bound, ExecCtx& ctx) 
 
 // The variant with the least modelled time.  Wide pair tiles win once they fill the machine; smaller problems take narrower
 // tiles until every SM has one.  `force` >= 0 picks an entry of kVariants.
-static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pairs, bool k_split, bool vt, int64_t vt_col0, bool images, TailSplit* out_ts, int* out_workers, int force) {
+static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pairs, bool k_split, bool vt, int64_t vt_col0, const Variant* table, TailSplit* out_ts, int* out_workers, int force) {
     const int num_k = int((K + BK - 1) / BK);
     int best = -1;
     double best_us = 0;
     for (int i = 0; i < int(sizeof(kVariants) / sizeof(kVariants[0])); i++) {
-        const Variant& v = images ? kImageVariants[i] : kVariants[i];
+        const Variant& v = table[i];
         if (force >= 0 && i != force) continue;
         if (v.pair && (!pairs || M <= BM || sm_count < 2)) continue;
         if (vt && ((v.bn / 2) % 32 != 0 || vt_col0 % (v.bn / 2) != 0)) continue;   // a warp's columns: whole halves of a head
@@ -1106,7 +1173,7 @@ static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pair
 }
 
 std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, int sm_count) {
-    const int v = pick_variant(M, N, K, sm_count, true, true, false, 0, false, nullptr, nullptr, -1);
+    const int v = pick_variant(M, N, K, sm_count, true, true, false, 0, bf16 ? kBf16Variants : kVariants, nullptr, nullptr, -1);
     if (v < 0) return "none";
     return strfmt("%s-%dx%d%s", bf16 ? "bf16" : "f16x3", kVariants[v].pair ? 256 : 128, kVariants[v].bn, kVariants[v].pair ? "-pair" : "");
 }
@@ -1114,7 +1181,7 @@ std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, in
 bool gemm_f16_vt_ok(const F16GemmArgs& a, const ExecCtx& ctx) {
     if (a.vt_out == nullptr || a.vt_flags == nullptr || a.residual != nullptr || a.relu || a.split_out.planes != nullptr) return false;
     if (a.vt_T <= 0 || a.vt_T % 32 != 0 || a.M % a.vt_T != 0 || (a.N - a.vt_col0) != int64_t(a.vt_heads) * 64) return false;
-    return pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, false, true, a.vt_col0, false, nullptr, nullptr, -1) >= 0;
+    return pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, false, true, a.vt_col0, a.bf16 ? kBf16Variants : kVariants, nullptr, nullptr, -1) >= 0;
 }
 
 static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorMap* im2col, const char* tag, double flops, ExecCtx& ctx) {
@@ -1126,7 +1193,7 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     TailSplit ts{};
     int workers = 0;
     const bool ks = ctx.gemm_ws != nullptr && ctx.gemm_flags != nullptr;
-    const int v = pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, ks, a.vt_out != nullptr, a.vt_col0, im != nullptr, &ts, &workers, ctx.f16_variant);
+    const int v = pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, ks, a.vt_out != nullptr, a.vt_col0, im != nullptr ? kImageVariants : (a.bf16 ? kBf16Variants : kVariants), &ts, &workers, ctx.f16_variant);
     FXF_CHECK(v >= 0, "f16 GEMM: no kernel variant for M=%lld N=%lld K=%lld", (long long)a.M, (long long)a.N, (long long)a.K);
     const Variant& var = kVariants[v];
     const int rows = var.pair ? 2 * BM : BM, per_unit = var.pair ? 2 : 1;
@@ -1140,6 +1207,7 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     p.tma_out = (split || (a.ldo % 4 == 0 && aligned16(a.out) && (a.residual == nullptr || aligned16(a.residual)))) ? 1 : 0;
     auto sector = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 31) == 0; };
     p.fast = a.N % 16 == 0 && (split ? sector(a.split_out.planes) && a.split_out.plane % 16 == 0 : a.ldo % 8 == 0 && sector(a.out)) && sector(a.residual) ? 1 : 0;
+    p.lean = !split && !p.tma_out && a.residual == nullptr ? 1 : 0;
     p.tiles_m = int((a.M + rows - 1) / rows);
     p.tiles_n = int((a.N + var.bn - 1) / var.bn);
     p.m_fastest = a.N > a.M ? 1 : 0;
@@ -1165,7 +1233,9 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     tag_launch(ctx, tag, flops, 4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.N) + double(a.M) * a.N));
     if (a.bf16) {
         switch (v) {
-            case 0: return launch_variant<256, 6, true, 1>(a, p, ts, workers, ctx);
+            case 0:
+                if (a.K <= int64_t(p.chunk_slabs) * BK && ts.parts == 1 && !p.lean) return launch_variant<256, 4, true, 1, false, 16>(a, p, ts, workers, ctx);
+                return launch_variant<256, 6, true, 1>(a, p, ts, workers, ctx);
             case 1: return launch_variant<192, 6, true, 1>(a, p, ts, workers, ctx);
             case 2: return launch_variant<128, 6, true, 1>(a, p, ts, workers, ctx);
             case 3: return launch_variant<64, 6, true, 1>(a, p, ts, workers, ctx);
