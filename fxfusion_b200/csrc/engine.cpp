@@ -820,6 +820,22 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             m.plane = P.plan->split_rows * P.plan->split_cols;
             m.inv = reinterpret_cast<const float*>(e->base + P.split_off);
             m.amax = m.inv + P.plan->split_rows;
+            if (P.op == FXF_OP_LAYER_NORM || P.op == FXF_OP_ADD_LAYER_NORM) {   // |(x - mean) / std| < sqrt(D), whatever x
+                auto largest = [&](uint32_t id, int64_t n) {   // of a constant; infinity: unknown
+                    if (meta[id].kind != kConstant || meta[id].data == nullptr || numel(e->reg[id]) != n || e->reg[id].dtype != FXF_F32) return INFINITY;
+                    float top = 0.f;
+                    for (int64_t k = 0; k < n; k++) {
+                        float v;
+                        std::memcpy(&v, reinterpret_cast<const char*>(meta[id].data) + k * 4, 4);
+                        top = std::fabs(v) <= top ? top : std::fabs(v);   // (NaN ends up in top and stays)
+                    }
+                    return top;
+                };
+                const int64_t D = P.plan->split_cols;
+                const size_t at = P.op == FXF_OP_LAYER_NORM ? 1 : 2;
+                if (P.in.size() > at + 1) m.cap = 1.001f * (std::sqrt(float(D)) * largest(P.in[at], D) + largest(P.in[at + 1], D));
+                if (!std::isfinite(m.cap)) m.cap = 0.f;
+            }
             for (uint32_t id = 0; id < n_tensors; id++)
                 if (root(id) == t) e->splits[id] = m;
         }

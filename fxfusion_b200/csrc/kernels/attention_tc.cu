@@ -130,6 +130,13 @@ struct AttnTcParams {
     int mask_vec16;       // mask rows may be fetched as aligned 16-byte words
     int mask_words;       // mask bytes of a row are consecutive: fetched as the aligned 4-byte words around them
     int* status;
+    // context in split form (AttnArgs::split_ctx), NULL: fp32 in ctx
+    uint16_t* so;
+    int64_t so_plane;
+    float* so_inv;
+    int so_bf16;
+    const float* v_bound;
+    float v_cap;
 };
 
 // x - (x with its 13 low mantissa bits cleared): the part of x a TF32 MMA does not see.  The difference is exact in fp32 and
@@ -542,10 +549,32 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
             // one reciprocal per row instead of 32 divisions; a fully masked row has o = 0 and l = 0: 0 * inf = NaN, as the
             // reference softmax gives
             const float inv_l = 1.0f / l_tot;
-            float* dst = p.ctx + (int64_t(b) * T + qi) * p.ld_ctx + int64_t(h) * HD + half * 32;
+            const int64_t at = (int64_t(b) * T + qi) * p.ld_ctx + int64_t(h) * HD + half * 32;
+            if (p.so == nullptr) {
+                float* dst = p.ctx + at;
 #pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<float4*>(dst + j) = make_float4(o[j] * inv_l, o[j + 1] * inv_l, o[j + 2] * inv_l, o[j + 3] * inv_l);
+                for (int j = 0; j < 32; j += 4)
+                    *reinterpret_cast<float4*>(dst + j) = make_float4(o[j] * inv_l, o[j + 1] * inv_l, o[j + 2] * inv_l, o[j + 3] * inv_l);
+            } else if (p.so_bf16) {
+                uint16_t* dst = p.so + at;
+#pragma unroll
+                for (int j = 0; j < 32; j += 8)
+                    *reinterpret_cast<uint4*>(dst + j) = make_uint4(pack_bf16x2(o[j] * inv_l, o[j + 1] * inv_l), pack_bf16x2(o[j + 2] * inv_l, o[j + 3] * inv_l),
+                                                                    pack_bf16x2(o[j + 4] * inv_l, o[j + 5] * inv_l), pack_bf16x2(o[j + 6] * inv_l, o[j + 7] * inv_l));
+            } else {   // a scale that no masked row can move: what a query does not see must not change a bit of its result
+                float scale, inv;
+                split_scale(fmaf(p.v_cap, __ldg(p.v_bound), __ldg(p.v_bound + 1)) * 1.001f, scale, inv);
+                if (h == 0 && half == 0) p.so_inv[int64_t(b) * T + qi] = inv;
+                uint16_t* dst = p.so + at;
+#pragma unroll
+                for (int j = 0; j < 32; j += 8) {
+                    uint4 hi, lo;
+#pragma unroll
+                    for (int e = 0; e < 4; e++) split_f16x2(o[j + 2 * e] * inv_l * scale, o[j + 2 * e + 1] * inv_l * scale, (&hi.x)[e], (&lo.x)[e]);
+                    *reinterpret_cast<uint4*>(dst + j) = hi;
+                    *reinterpret_cast<uint4*>(dst + p.so_plane + j) = lo;
+                }
+            }
         }
     }
     tc_fence_before();
@@ -636,6 +665,10 @@ int launch_attention_tc(const AttnArgs& a, float* vt_scratch, ExecCtx& ctx, bool
     p.mask_vec16 = (a.mask_sk == 1 && Tk % 16 == 0 && a.mask_sb % 16 == 0 && a.mask_sh % 16 == 0 && a.mask_sq % 16 == 0 && aligned16(a.mask)) ? 1 : 0;
     p.mask_words = a.mask_sk == 1 ? 1 : 0;
     p.status = ctx.status;
+    p.so = a.split_ctx.planes; p.so_plane = a.split_ctx.plane; p.so_inv = a.split_ctx.inv; p.so_bf16 = a.split_bf16 ? 1 : 0;
+    p.v_cap = a.v_cap; p.v_bound = a.v_bound;
+    FXF_CHECK(p.so == nullptr || (a.ld_ctx % 8 == 0 && (p.so_plane * 2) % 16 == 0 && (a.split_bf16 || (p.so_inv && p.v_cap > 0.f && p.v_bound))),
+              "attention: a context in split form needs 16-byte rows and the bound of V");
     size_t smem = sizeof(AttnTcSmem) + 1024;
     static bool configured[64] = {};
     int dev = 0;

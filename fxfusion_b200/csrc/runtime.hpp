@@ -89,6 +89,7 @@ struct SplitMat {
     int64_t inv_stride = 1;
     const float* amax = nullptr;        // activations: max_k |x[r,k]| as `parts` partial maxima per row
     int parts = 1;
+    float cap = 0.f;                    // activations: no |x| exceeds it whatever the input (normalised rows); 0: unknown
     const float* bound = nullptr;       // weights: {max_j ||w_j||_1, max_j |b_j|}
 };
 struct SplitOut {
@@ -462,6 +463,12 @@ struct AttnArgs {
     int64_t ld_ctx = 0;
     int64_t mask_sb = 0, mask_sh = 0, mask_sq = 0, mask_sk = 0;  // mask strides (bytes): batch, head, query, key
     float scale_divisor = 1.f;
+    // Tensor-core kernel only: the context in split form [B*T, H*hd] (or its bf16 plane) instead of `ctx`.  A context row is a convex
+    // combination of V rows, so all of them share one scale, from |v| <= v_cap * v_bound[0] + v_bound[1].
+    SplitOut split_ctx;
+    bool split_bf16 = false;
+    float v_cap = 0.f;                  // SplitMat::cap of the rows that V is projected from
+    const float* v_bound = nullptr;     // SplitMat::bound of the projection
 };
 int launch_attention(const AttnArgs& a, ExecCtx& ctx);
 // Sum `n` floats in place over the tensor-parallel ranks (NCCL all-reduce on ctx.stream); no-op for tp_size 1.
