@@ -215,6 +215,34 @@ __global__ void __launch_bounds__(kThreads) embedding_vec4_kernel(const int64_t*
         }
     }
 }
+// out[r] = w[idx[r]] * scale + rows[r % period], product and sum rounded one after the other as the separate nodes do
+template <int VEC>
+__global__ void __launch_bounds__(kThreads) embedding_scale_add_kernel(const int64_t* __restrict__ idx, const float* __restrict__ w, float scale, const float* __restrict__ rows,
+                                                                       int64_t period, float* __restrict__ out, int64_t n_idx, int64_t d, int64_t vocab, int* status) {
+    sm100::grid_dep();
+    const int64_t per_row = d / VEC, total = n_idx * per_row, stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
+        const int64_t r = i / per_row, c = (i - r * per_row) * VEC, row = idx[r];
+        const bool ok = row >= 0 && row < vocab;
+        if (!ok && status) atomicCAS(status, 0, 2);
+        const float* src = w + row * d + c;
+        const float* add = rows + (r % period) * d + c;
+        float v[VEC], a[VEC];
+        if constexpr (VEC == 4) {
+            const float4 x = ok ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f), y = *reinterpret_cast<const float4*>(add);
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+            a[0] = y.x; a[1] = y.y; a[2] = y.z; a[3] = y.w;
+        } else {
+            v[0] = ok ? *src : 0.f;
+            a[0] = *add;
+        }
+#pragma unroll
+        for (int j = 0; j < VEC; j++) v[j] = __fadd_rn(__fmul_rn(v[j], scale), a[j]);
+        if constexpr (VEC == 4) *reinterpret_cast<float4*>(out + r * d + c) = make_float4(v[0], v[1], v[2], v[3]);
+        else out[r * d + c] = v[0];
+    }
+}
+
 __global__ void __launch_bounds__(kThreads) embedding_kernel(const int64_t* __restrict__ idx, const float* __restrict__ w, float* __restrict__ out,
                                                              int64_t n_idx, int64_t d, int64_t vocab, int* status) {
     sm100::grid_dep();
@@ -411,6 +439,20 @@ int k_embedding(Registry& reg, const TensorIds& in, const TensorIds& out, const 
     FXF_LAUNCHED(ctx);
     return 0;
 }
+int launch_embedding_scale_add(const FxfTensor& idx, const FxfTensor& w, float scale, const FxfTensor& rows, const FxfTensor& out, ExecCtx& ctx) {
+    const int64_t n_idx = numel(idx), D = w.shape[1], V = w.shape[0], period = numel(rows) / (D > 0 ? D : 1);
+    FXF_CHECK(numel(out) == n_idx * D && period * D == numel(rows), "embedding: output size mismatch");
+    if (n_idx * D == 0) return 0;
+    tag_launch(ctx, "embedding_scale_add", 2.0 * double(n_idx) * D, 8.0 * double(n_idx) * D);
+    auto f = [&](const FxfTensor& t) { return static_cast<float*>(t.ptr); };
+    if (D % 4 == 0 && aligned16(w.ptr) && aligned16(rows.ptr) && aligned16(out.ptr))
+        dependent(embedding_scale_add_kernel<4>, grid_for(n_idx * D / 4, ctx), kThreads, 0, ctx)(static_cast<const int64_t*>(idx.ptr), f(w), scale, f(rows), period, f(out), n_idx, D, V, ctx.status);
+    else
+        dependent(embedding_scale_add_kernel<1>, grid_for(n_idx * D, ctx), kThreads, 0, ctx)(static_cast<const int64_t*>(idx.ptr), f(w), scale, f(rows), period, f(out), n_idx, D, V, ctx.status);
+    FXF_LAUNCHED(ctx);
+    return 0;
+}
+
 int k_transpose(Registry& reg, const TensorIds& in, const TensorIds& out, const Params& p, const NodePlan*, ExecCtx& ctx) {
     FXF_CHECK(in.size() >= 1 && out.size() >= 1 && p.ints.size() >= 2, "transpose: expects [dim0, dim1]");
     const FxfTensor& x = reg[in[0]];

@@ -173,3 +173,26 @@ def test_images_in_split_form(built_lib, tmp_path, N, size, C, O, kh, kw, s, ph,
     assert all(torch.equal(a.cpu(), g.cpu()) for a, g in zip(again, got))
     assert eng.device_status() == 0
     eng.close()
+
+
+@pytest.mark.parametrize("B,T,D,P,lead", [(2, 5, 64, 9, 0), (3, 7, 30, 7, 2), (1, 1, 4, 1, 0)])
+def test_embedding_scale_add_is_one_pass(built_lib, tmp_path, B, T, D, P, lead):
+    """Embedding -> Mul -> Add of a slice of a positional table: one launch with the roundings of the separate nodes; an index
+    outside the table still sets the status."""
+    rng = np.random.default_rng(T)
+    b = lowering.GraphBuilder(f"emb_{B}_{T}_{D}")
+    ids = b.input((B, T), wire.DT_I64)
+    mul = b.op("Mul", [b.op("Embedding", [ids, b.const(rng.standard_normal((11, D), dtype=np.float32))], (B, T, D))], (B, T, D), ints=[1], floats=[math.sqrt(D)])
+    size = b.op("Size", [mul], (), wire.DT_I64, ints=[1])
+    nar = b.op("Narrow", [b.const(rng.standard_normal((1, P + lead, D), dtype=np.float32)), size], (1, T, D), ints=[1, lead, -1])
+    b.output(b.op("Add", [mul, nar], (B, T, D)))
+    graph, eng = _engine(b, tmp_path)
+    x = torch.randint(0, 11, (B, T), generator=torch.Generator().manual_seed(0))
+    assert torch.equal(eng.run([x.cuda()])[0].cpu(), GraphOracle(graph).run([x])[0])
+    eng.profile_launches()
+    assert len(eng.profile_launches()) == 1
+    assert eng.device_status() == 0
+    x[0, 0] = 11
+    eng.run([x.cuda()])
+    assert eng.device_status() != 0
+    eng.close()
