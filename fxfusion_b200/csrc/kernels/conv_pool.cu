@@ -15,6 +15,9 @@
 //       ints = [oh, ow, ...]; window i = [floor(i*H/oh), ceil((i+1)*H/oh))
 //
 // Convolution paths:
+//   * channels-last images in split form (default mode, single GPU; the engine decides which tensors are kept so): every
+//     convolution is an f16x3 product (gemm_f16.cu), 1x1 filters over the pixels as rows, others through the im2col mode of the
+//     TMA, the stem over a space-to-depth copy.  What follows serves other modes, NCHW tensors and single calls.
 //   * 1x1, stride 1, no padding, channels-last in and out: the convolution IS the GEMM
 //     out[pixel, o] = x[pixel, :] · w[o, :] + b[o]  — it runs on the tcgen05 3xTF32 GEMM kernel with the bias
 //     and ReLU fused in its epilogue (weights split into TF32 hi/lo once, at engine build).

@@ -1055,6 +1055,9 @@ int make_out_map(CUtensorMap* map, const F16GemmArgs& a, int planes) {
     return 0;
 }
 
+// K-elements per accumulation chain.  Convolutions run 50 deep without normalisation: ResNet-50's logits lie 1.1e-5 from fp64 with
+// chains of 128 (5.7e-6 with 64; three TF32 products in chains of 64: 1.4e-5), and a chain of 64 drains at every slab
+// (128 images of 56 x 56, 64 channels, 3x3: 136 against 114 us).
 constexpr int kChunkKDense = 1024, kChunkKConv = 128, kChunkKRows = 256;
 
 // Times in microseconds as measured on B200 inside a chain of launches: `slab` per 64-deep K-slab of a tile, `gap` what every
@@ -1149,14 +1152,13 @@ int launch_bias_bound(const float* bias, int64_t n, float* bound, ExecCtx& ctx) 
 }
 
 // The variant with the least modelled time.  Wide pair tiles win once they fill the machine; smaller problems take narrower
-// tiles until every SM has one.  `force` >= 0 picks an entry of kVariants.
-static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pairs, bool k_split, bool vt, int64_t vt_col0, const Variant* table, TailSplit* out_ts, int* out_workers, int force) {
+// tiles until every SM has one.
+static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pairs, bool k_split, bool vt, int64_t vt_col0, const Variant* table, TailSplit* out_ts, int* out_workers) {
     const int num_k = int((K + BK - 1) / BK);
     int best = -1;
     double best_us = 0;
     for (int i = 0; i < int(sizeof(kVariants) / sizeof(kVariants[0])); i++) {
         const Variant& v = table[i];
-        if (force >= 0 && i != force) continue;
         if (v.pair && (!pairs || M <= BM || sm_count < 2)) continue;
         if (vt && ((v.bn / 2) % 32 != 0 || vt_col0 % (v.bn / 2) != 0)) continue;   // a warp's columns: whole halves of a head
         const int rows = v.pair ? 2 * BM : BM, workers = v.pair ? sm_count / 2 : sm_count;
@@ -1173,7 +1175,7 @@ static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pair
 }
 
 std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, int sm_count) {
-    const int v = pick_variant(M, N, K, sm_count, true, true, false, 0, bf16 ? kBf16Variants : kVariants, nullptr, nullptr, -1);
+    const int v = pick_variant(M, N, K, sm_count, true, true, false, 0, bf16 ? kBf16Variants : kVariants, nullptr, nullptr);
     if (v < 0) return "none";
     return strfmt("%s-%dx%d%s", bf16 ? "bf16" : "f16x3", kVariants[v].pair ? 256 : 128, kVariants[v].bn, kVariants[v].pair ? "-pair" : "");
 }
@@ -1181,7 +1183,7 @@ std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, in
 bool gemm_f16_vt_ok(const F16GemmArgs& a, const ExecCtx& ctx) {
     if (a.vt_out == nullptr || a.vt_flags == nullptr || a.residual != nullptr || a.relu || a.split_out.planes != nullptr) return false;
     if (a.vt_T <= 0 || a.vt_T % 32 != 0 || a.M % a.vt_T != 0 || (a.N - a.vt_col0) != int64_t(a.vt_heads) * 64) return false;
-    return pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, false, true, a.vt_col0, a.bf16 ? kBf16Variants : kVariants, nullptr, nullptr, -1) >= 0;
+    return pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, false, true, a.vt_col0, a.bf16 ? kBf16Variants : kVariants, nullptr, nullptr) >= 0;
 }
 
 static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorMap* im2col, const char* tag, double flops, ExecCtx& ctx) {
@@ -1193,7 +1195,7 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     TailSplit ts{};
     int workers = 0;
     const bool ks = ctx.gemm_ws != nullptr && ctx.gemm_flags != nullptr;
-    const int v = pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, ks, a.vt_out != nullptr, a.vt_col0, im != nullptr ? kImageVariants : (a.bf16 ? kBf16Variants : kVariants), &ts, &workers, ctx.f16_variant);
+    const int v = pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, ks, a.vt_out != nullptr, a.vt_col0, im != nullptr ? kImageVariants : (a.bf16 ? kBf16Variants : kVariants), &ts, &workers);
     FXF_CHECK(v >= 0, "f16 GEMM: no kernel variant for M=%lld N=%lld K=%lld", (long long)a.M, (long long)a.N, (long long)a.K);
     const Variant& var = kVariants[v];
     const int rows = var.pair ? 2 * BM : BM, per_unit = var.pair ? 2 : 1;

@@ -831,7 +831,7 @@ __device__ __forceinline__ float block_reduce(float v, float* red, bool is_max) 
 // one coalesced access, and every lane group walks its own keys with an online softmax: four keys' K and V rows, eight 16-byte
 // loads per lane, are in flight before the first is used.  The groups' (max, sum, context) are merged through shared memory.
 // The row of the new position is taken from qkv (and stored): nothing in the kernel waits for that store.
-// Bound: HBM (the cache).  32 sequences, 12 heads, 256 positions (50 MB): 28 -> 10 us, 5 TB/s; the kernel it replaces had one key
+// Bound: HBM (the cache).  32 sequences, 12 heads, 256 positions (50 MB): 28 -> 17 us, launch included, 3 TB/s; the kernel it replaces had one key
 // per thread, that is 32 different rows in one load.
 template <int HD>
 __global__ void __launch_bounds__(kCachedAttnThreads) cached_attn_groups_kernel(const float* __restrict__ qkv, float* __restrict__ cache, const int64_t* __restrict__ tokens,

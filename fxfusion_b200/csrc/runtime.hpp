@@ -124,7 +124,6 @@ struct ExecCtx {
     int* gemm_flags = nullptr;
     int gemm_flag_count = 0;
     int tc_chunk_k = 0;            // K-elements per tensor-core accumulation chain (0 = the kernel's default)
-    int f16_variant = -1;          // >= 0: this entry of the f16 GEMM's variant table instead of the modelled choice (experiments)
     bool weights_settled = false;  // inside an engine after its build: weights were written long before the current kernel chain
     int tc_pair = 0;               // 0: 256-wide tensor-core GEMM tiles are computed by CTA pairs (tcgen05 cta_group::2); 1: never
     // profiling: when `trace` is set every launch appends a record carrying the current tag
