@@ -552,7 +552,7 @@ int k_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const Params
     bool v_transposed = false;
     if (pl->s[0].f16) {
         F16GemmArgs f;
-        if (have_vt && hd == 64 && M > kFewRows) {
+        if (have_vt && hd == 64 && M > kFewRows && T >= 16 && T <= 4096) {   // (where the attention kernel will run)
             f.M = M; f.N = QKVl; f.K = D;
             f.vt_out = vt;
             f.vt_flags = reinterpret_cast<unsigned char*>(vt + size_t(B) * size_t(Hl) * size_t(T) * 64);
@@ -701,9 +701,22 @@ int k_cross_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const 
     const bool have_vt = ctx.scratch_bytes >= need + attention_tc_scratch_bytes(B, Tk, Hl);
     if (Mq == 0) return 0;
 
+    // the V half of the packed projection transposed by its epilogue, as in MHA (64 x 256 keys: 17 us per layer for the launch it saves)
+    F16GemmArgs vt_args;
+    bool v_transposed = false;
+    if (pl->s[2].f16 && have_vt && hd == 64 && Mk > kFewRows && Tk >= 16 && Tk <= 4096) {
+        F16GemmArgs& f = vt_args;
+        f.M = Mk; f.N = 2 * Dl; f.K = D;
+        f.vt_out = vt;
+        f.vt_flags = reinterpret_cast<unsigned char*>(vt + size_t(B) * size_t(Hl) * size_t(Tk) * 64);
+        f.vt_col0 = Dl;
+        f.vt_T = int(Tk); f.vt_heads = int(Hl); f.vt_n32 = int((Tk + 31) / 32);
+        v_transposed = gemm_f16_vt_ok(f, ctx);
+    }
     auto project = [&](int wi, uint32_t id, const FxfTensor& t, float* dst, int64_t rows, int64_t cols) {
         if (pl->s[wi].f16) {
-            return f16_product(pl->s[wi], &pl->s[wi + 1], static_cast<const float*>(t.ptr), D, split_of(ctx, id), dst, rows, cols, false, false, area, ctx);
+            return f16_product(pl->s[wi], &pl->s[wi + 1], static_cast<const float*>(t.ptr), D, split_of(ctx, id), dst, rows, cols, false, false, area, ctx,
+                               wi == 2 && v_transposed ? &vt_args : nullptr);
         }
         GemmArgs g;
         fill_gemm(g, static_cast<const float*>(t.ptr), pl->s[wi], &pl->s[wi + 1], dst, rows, D, cols, false);
@@ -726,8 +739,9 @@ int k_cross_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const 
         a.scale_divisor = p.floats[0];
         if (have_vt && attention_tc_supported(a, ctx.gemm_mode)) {
             cs = context_in_split_form(a, pl->s[2], pl->s[4], split_of(ctx, in[1]), cx, area, Mq, D);
-            if (launch_attention_tc(a, vt, ctx)) return 1;
+            if (launch_attention_tc(a, vt, ctx, v_transposed)) return 1;
         } else {
+            FXF_CHECK(!v_transposed, "cross_mha: the projection wrote V transposed but the tensor-core attention kernel cannot run");
             if (launch_attention(a, ctx)) return 1;
         }
     }

@@ -54,7 +54,7 @@ def test_any_sequence_length(built_lib, tmp_path, T, kind):
 
 
 @pytest.mark.parametrize("precision", ["auto", "bf16"])
-@pytest.mark.parametrize("B,T,Tk", [(2, 65, 65), (3, 40, 17), (1, 200, 130), (5, 256, 64)])
+@pytest.mark.parametrize("B,T,Tk", [(2, 65, 65), (3, 40, 17), (1, 200, 130), (5, 256, 64), (3, 33, 96)])
 def test_context_leaves_in_split_form(built_lib, tmp_path, B, T, Tk, precision):
     """LayerNorm -> MHA -> LayerNorm -> CrossMHA over a normalised memory: neither context passes through a conversion kernel."""
     from fxfusion_b200.engine import ExecutionEngine
