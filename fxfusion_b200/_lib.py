@@ -46,6 +46,7 @@ SIGNATURES = {
     "fxf_comm_rank": (C.c_int, [C.c_void_p]),
     "fxf_comm_size": (C.c_int, [C.c_void_p]),
     "fxf_engine_create_tp": (C.c_int, [C.c_char_p, C.c_int, C.POINTER(FxfEngineOptions), C.c_void_p, C.POINTER(C.c_void_p)]),
+    "fxf_gemm_workspace": (C.c_int, [C.c_int64, C.c_int64, C.c_int64, C.c_int, C.c_int, C.c_int, C.c_int] + [C.POINTER(C.c_int64)] * 4),
     "fxf_gemm_variant": (C.c_int, [C.c_int64, C.c_int64, C.c_int64, C.c_int, C.c_int, C.c_char_p, C.c_size_t]),
     "fxf_tp_exchange_emulated": (C.c_int, [C.c_int] + [C.POINTER(C.c_void_p)] * 4 + [C.c_void_p, C.c_void_p, C.c_float, C.c_int64, C.c_int64, C.c_int,
                                             C.c_void_p, C.c_int64, C.c_int, C.c_int, C.c_void_p]),

@@ -432,14 +432,14 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
     e->status_off = cursor;
     cursor += kAlign;
     if (e->opts.gemm_mode != FXF_GEMM_FP32_SIMT) {
-        // K-split workspace of the tensor-core GEMM: one 128 x 256 partial tile and eight flags (one per epilogue warp) per SM
+        // K-split workspace of the tensor-core GEMM
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
         e->gemm_ws_off = cursor;
-        e->gemm_ws_bytes = round_up(size_t(sms) * 128 * 256 * sizeof(float), kAlign);
+        e->gemm_ws_bytes = round_up(size_t(sms) * kSplitTileBytes, kAlign);
         cursor += e->gemm_ws_bytes;
         e->gemm_flags_off = cursor;
-        e->gemm_flags_bytes = round_up(size_t(sms) * 8 * sizeof(int), kAlign);
+        e->gemm_flags_bytes = round_up(size_t(sms) * kSplitFlagsPerSm * sizeof(int), kAlign);
         cursor += e->gemm_flags_bytes;
     }
     if (e->head_sharded && !e->input_ids.empty() && e->reg[e->input_ids[0]].rank >= 1) {
@@ -1281,7 +1281,7 @@ static int make_call(int op_code, const FxfTensor* reg, int n_reg, const uint32_
 
 // A single kernel call that may reach the tensor-core GEMM (its plan keeps split weights) also carries that kernel's
 // K-split workspace behind its scratch: partial tiles for up to kCallWsSms SMs, then the flags.
-constexpr size_t kCallWsSms = 160, kCallWsTile = size_t(128) * 256 * sizeof(float), kCallFlagBytes = 8192;
+constexpr size_t kCallWsSms = 160, kCallWsTile = kSplitTileBytes, kCallFlagBytes = kCallWsSms * kSplitFlagsPerSm * sizeof(int);
 static size_t call_ws_bytes(const NodePlan& plan, int gemm_mode) {
     return (gemm_mode != FXF_GEMM_FP32_SIMT && plan.persist_bytes > 0) ? kCallWsSms * kCallWsTile + kCallFlagBytes : 0;
 }
@@ -1344,6 +1344,23 @@ int fxf_gemm_variant(int64_t M, int64_t N, int64_t K, int gemm_mode, int sm_coun
     size_t k = std::min(out_bytes - 1, v.size());
     std::memcpy(out, v.data(), k);
     out[k] = 0;
+    return 0;
+}
+
+int fxf_gemm_workspace(int64_t M, int64_t N, int64_t K, int gemm_mode, int images, int tc_chunk_k, int sm_count, int64_t* bytes, int64_t* bytes_kept, int64_t* flags, int64_t* flags_kept) {
+    FXF_CHECK(bytes && bytes_kept && flags && flags_kept, "fxf_gemm_workspace: NULL argument");
+    FXF_CHECK(gemm_f16_shape_ok(M, N, K) && (gemm_mode == FXF_GEMM_AUTO || gemm_mode == FXF_GEMM_BF16) && sm_count >= 0, "fxf_gemm_workspace: no product on operands in split form");
+    F16Limits lim;
+    if (sm_count > 0) lim.sm_count = sm_count;
+    lim.chunk_k = tc_chunk_k;
+    lim.ws_bytes = size_t(lim.sm_count) * kSplitTileBytes;
+    lim.flag_count = int64_t(lim.sm_count) * kSplitFlagsPerSm;
+    const F16Plan p = gemm_f16_plan(M, N, K, images ? F16Form::kImages : (gemm_mode == FXF_GEMM_BF16 ? F16Form::kBf16 : F16Form::kRows), lim);
+    FXF_CHECK(p.variant >= 0, "fxf_gemm_workspace: no kernel variant");
+    *bytes = int64_t(p.ws_bytes);
+    *bytes_kept = int64_t(lim.ws_bytes);
+    *flags = p.flags;
+    *flags_kept = lim.flag_count;
     return 0;
 }
 

@@ -1093,7 +1093,7 @@ TailSplit plan_tail(int64_t tiles, int num_k, const Variant& v, int workers, boo
 }
 
 template <int BN, int STAGES, bool PAIR, int NPL, bool IMG = false, int EW = 8>
-int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int workers, ExecCtx& ctx, const CUtensorMap* im2col = nullptr) {
+int launch_variant(const F16GemmArgs& a, F16Params p, const F16Plan& plan, ExecCtx& ctx, const CUtensorMap* im2col = nullptr) {
     constexpr int BNB = PAIR ? BN / 2 : BN;
     CUtensorMap mx, mw, mo, mr;
     if (IMG && p.im.c_slabs > 0) mx = *im2col;
@@ -1118,8 +1118,8 @@ int launch_variant(const F16GemmArgs& a, F16Params p, const TailSplit& ts, int w
         FXF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    const int64_t units = ts.full + ts.tail * ts.parts;
-    const int grid = int(std::min<int64_t>(units, workers)) * (PAIR ? 2 : 1);
+    const int64_t units = plan.full + plan.tail * plan.parts;
+    const int grid = int(std::min<int64_t>(units, plan.workers)) * (PAIR ? 2 : 1);
     FXF_CUDA(launch_dependent(kernel, dim3(unsigned(grid)), dim3(EW * 32 + 128), smem, ctx.stream, PAIR ? 2 : 1, mx, mw, mo, mr, p));
     FXF_LAUNCHED(ctx);
     return 0;
@@ -1174,6 +1174,31 @@ static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pair
     return best;
 }
 
+// Which instance a product runs on, how its tiles are cut, and what it then uses of the K-split workspace: a partial tile per CTA
+// of a cut tile, and one flag for each of its epilogue warps.  Where that does not fit, every tile is computed whole.
+static F16Plan plan_launch(int64_t M, int64_t N, int64_t K, F16Form form, bool lean, bool vt, int64_t vt_col0, const F16Limits& lim) {
+    F16Plan r;
+    TailSplit ts{};
+    r.variant = pick_variant(M, N, K, lim.sm_count, lim.pairs, lim.ws_bytes > 0 && lim.flag_count > 0, vt, vt_col0,
+                             form == F16Form::kImages ? kImageVariants : (form == F16Form::kBf16 ? kBf16Variants : kVariants), &ts, &r.workers);
+    if (r.variant < 0) return r;
+    const Variant& var = kVariants[r.variant];
+    const int64_t chunk_k = lim.chunk_k > 0 ? lim.chunk_k : (form == F16Form::kImages ? kChunkKConv : kChunkKDense);
+    r.chunk_slabs = int(std::max<int64_t>(1, chunk_k / BK));
+    r.epilogue_warps = r.variant == 0 && K <= int64_t(r.chunk_slabs) * BK && (form == F16Form::kImages || (form == F16Form::kBf16 && ts.parts == 1 && !lean)) ? 16 : 8;
+    const int64_t ctas = ts.tail * ts.parts * (var.pair ? 2 : 1);
+    r.ws_bytes = ts.parts > 1 ? size_t(ctas) * BM * size_t(var.bn) * sizeof(float) : 0;
+    r.flags = ts.parts > 1 ? ctas * r.epilogue_warps : 0;
+    if (r.ws_bytes > lim.ws_bytes || r.flags > lim.flag_count) {
+        ts = TailSplit{ts.full + ts.tail, 0, 1, 0.0};
+        r.ws_bytes = 0;
+        r.flags = 0;
+    }
+    r.full = ts.full; r.tail = ts.tail; r.parts = ts.parts;
+    return r;
+}
+F16Plan gemm_f16_plan(int64_t M, int64_t N, int64_t K, F16Form form, const F16Limits& lim) { return plan_launch(M, N, K, form, false, false, 0, lim); }
+
 std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, int sm_count) {
     const int v = pick_variant(M, N, K, sm_count, true, true, false, 0, bf16 ? kBf16Variants : kVariants, nullptr, nullptr);
     if (v < 0) return "none";
@@ -1192,13 +1217,17 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     const bool split = a.split_out.planes != nullptr;
     FXF_CHECK(split || a.out != nullptr, "f16 GEMM: no output");
     FXF_CHECK(!split || (a.N % 8 == 0 && a.residual == nullptr && a.vt_out == nullptr), "f16 GEMM: a split output needs N %% 8 == 0 and no residual");
-    TailSplit ts{};
-    int workers = 0;
-    const bool ks = ctx.gemm_ws != nullptr && ctx.gemm_flags != nullptr;
-    const int v = pick_variant(a.M, a.N, a.K, ctx.sm_count, ctx.tc_pair != 1, ks, a.vt_out != nullptr, a.vt_col0, im != nullptr ? kImageVariants : (a.bf16 ? kBf16Variants : kVariants), &ts, &workers);
+    const bool tma_out = split || (a.ldo % 4 == 0 && aligned16(a.out) && (a.residual == nullptr || aligned16(a.residual)));
+    const bool lean = !split && !tma_out && a.residual == nullptr;
+    const F16Form form = im != nullptr ? F16Form::kImages : (a.bf16 ? F16Form::kBf16 : F16Form::kRows);
+    F16Limits lim;
+    lim.sm_count = ctx.sm_count; lim.pairs = ctx.tc_pair != 1; lim.chunk_k = ctx.tc_chunk_k;
+    if (ctx.gemm_ws != nullptr && ctx.gemm_flags != nullptr) { lim.ws_bytes = ctx.gemm_ws_bytes; lim.flag_count = ctx.gemm_flag_count; }
+    const F16Plan plan = plan_launch(a.M, a.N, a.K, form, lean, a.vt_out != nullptr, a.vt_col0, lim);
+    const int v = plan.variant;
     FXF_CHECK(v >= 0, "f16 GEMM: no kernel variant for M=%lld N=%lld K=%lld", (long long)a.M, (long long)a.N, (long long)a.K);
     const Variant& var = kVariants[v];
-    const int rows = var.pair ? 2 * BM : BM, per_unit = var.pair ? 2 : 1;
+    const int rows = var.pair ? 2 * BM : BM;
     F16Params p{};
     p.bias = a.bias; p.residual = a.residual; p.out = a.out;
     p.x_inv = a.bf16 ? nullptr : a.x.inv; p.w_inv = a.bf16 ? nullptr : a.w.inv;
@@ -1206,20 +1235,17 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     p.w_inv_stride = 1;
     p.M = a.M; p.N = a.N; p.K = a.K; p.ldo = split ? a.N : a.ldo;
     p.relu = a.relu ? 1 : 0;
-    p.tma_out = (split || (a.ldo % 4 == 0 && aligned16(a.out) && (a.residual == nullptr || aligned16(a.residual)))) ? 1 : 0;
+    p.tma_out = tma_out ? 1 : 0;
     auto sector = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 31) == 0; };
     p.fast = a.N % 16 == 0 && (split ? sector(a.split_out.planes) && a.split_out.plane % 16 == 0 : a.ldo % 8 == 0 && sector(a.out)) && sector(a.residual) ? 1 : 0;
-    p.lean = !split && !p.tma_out && a.residual == nullptr ? 1 : 0;
+    p.lean = lean ? 1 : 0;
     p.tiles_m = int((a.M + rows - 1) / rows);
     p.tiles_n = int((a.N + var.bn - 1) / var.bn);
     p.m_fastest = a.N > a.M ? 1 : 0;
     p.status = ctx.status;
     if (im != nullptr) p.im = *im;
-    if (ts.parts > 1 && (size_t(ts.tail) * ts.parts * per_unit * size_t(BM) * var.bn * sizeof(float) > ctx.gemm_ws_bytes ||
-                         ts.tail * ts.parts * per_unit * 8 > ctx.gemm_flag_count))
-        ts = TailSplit{int64_t(p.tiles_m) * p.tiles_n, 0, 1, 0.0};
-    p.full_tiles = int(ts.full); p.tail_tiles = int(ts.tail); p.tail_split = ts.parts;
-    p.chunk_slabs = std::max(1, (ctx.tc_chunk_k > 0 ? ctx.tc_chunk_k : (a.conv_chain ? kChunkKConv : kChunkKDense)) / BK);
+    p.full_tiles = int(plan.full); p.tail_tiles = int(plan.tail); p.tail_split = plan.parts;
+    p.chunk_slabs = plan.chunk_slabs;
     p.ws = ctx.gemm_ws; p.flags = ctx.gemm_flags;
     p.early_w = ctx.weights_settled ? 1 : 0;
     if (split) {
@@ -1236,37 +1262,37 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     if (a.bf16) {
         switch (v) {
             case 0:
-                if (a.K <= int64_t(p.chunk_slabs) * BK && ts.parts == 1 && !p.lean) return launch_variant<256, 4, true, 1, false, 16>(a, p, ts, workers, ctx);
-                return launch_variant<256, 6, true, 1>(a, p, ts, workers, ctx);
-            case 1: return launch_variant<192, 6, true, 1>(a, p, ts, workers, ctx);
-            case 2: return launch_variant<128, 6, true, 1>(a, p, ts, workers, ctx);
-            case 3: return launch_variant<64, 6, true, 1>(a, p, ts, workers, ctx);
-            case 4: return launch_variant<128, 6, false, 1>(a, p, ts, workers, ctx);
-            case 5: return launch_variant<64, 8, false, 1>(a, p, ts, workers, ctx);
-            default: return launch_variant<32, 8, false, 1>(a, p, ts, workers, ctx);
+                if (plan.epilogue_warps == 16) return launch_variant<256, 4, true, 1, false, 16>(a, p, plan, ctx);
+                return launch_variant<256, 6, true, 1>(a, p, plan, ctx);
+            case 1: return launch_variant<192, 6, true, 1>(a, p, plan, ctx);
+            case 2: return launch_variant<128, 6, true, 1>(a, p, plan, ctx);
+            case 3: return launch_variant<64, 6, true, 1>(a, p, plan, ctx);
+            case 4: return launch_variant<128, 6, false, 1>(a, p, plan, ctx);
+            case 5: return launch_variant<64, 8, false, 1>(a, p, plan, ctx);
+            default: return launch_variant<32, 8, false, 1>(a, p, plan, ctx);
         }
     }
     if (im != nullptr) {
         switch (v) {
             case 0:
-                if (a.K <= int64_t(p.chunk_slabs) * BK) return launch_variant<256, 2, true, 2, true, 16>(a, p, ts, workers, ctx, im2col);
-                return launch_variant<256, 2, true, 2, true>(a, p, ts, workers, ctx, im2col);
-            case 1: return launch_variant<192, 3, true, 2, true>(a, p, ts, workers, ctx, im2col);
-            case 2: return launch_variant<128, 3, true, 2, true>(a, p, ts, workers, ctx, im2col);
-            case 3: return launch_variant<64, 4, true, 2, true>(a, p, ts, workers, ctx, im2col);
-            case 4: return launch_variant<128, 2, false, 2, true>(a, p, ts, workers, ctx, im2col);
-            case 5: return launch_variant<64, 3, false, 2, true>(a, p, ts, workers, ctx, im2col);
-            default: return launch_variant<32, 4, false, 2, true>(a, p, ts, workers, ctx, im2col);
+                if (plan.epilogue_warps == 16) return launch_variant<256, 2, true, 2, true, 16>(a, p, plan, ctx, im2col);
+                return launch_variant<256, 2, true, 2, true>(a, p, plan, ctx, im2col);
+            case 1: return launch_variant<192, 3, true, 2, true>(a, p, plan, ctx, im2col);
+            case 2: return launch_variant<128, 3, true, 2, true>(a, p, plan, ctx, im2col);
+            case 3: return launch_variant<64, 4, true, 2, true>(a, p, plan, ctx, im2col);
+            case 4: return launch_variant<128, 2, false, 2, true>(a, p, plan, ctx, im2col);
+            case 5: return launch_variant<64, 3, false, 2, true>(a, p, plan, ctx, im2col);
+            default: return launch_variant<32, 4, false, 2, true>(a, p, plan, ctx, im2col);
         }
     }
     switch (v) {
-        case 0: return launch_variant<256, 3, true, 2>(a, p, ts, workers, ctx);
-        case 1: return launch_variant<192, 3, true, 2>(a, p, ts, workers, ctx);
-        case 2: return launch_variant<128, 4, true, 2>(a, p, ts, workers, ctx);
-        case 3: return launch_variant<64, 4, true, 2>(a, p, ts, workers, ctx);
-        case 4: return launch_variant<128, 3, false, 2>(a, p, ts, workers, ctx);
-        case 5: return launch_variant<64, 4, false, 2>(a, p, ts, workers, ctx);
-        default: return launch_variant<32, 4, false, 2>(a, p, ts, workers, ctx);
+        case 0: return launch_variant<256, 3, true, 2>(a, p, plan, ctx);
+        case 1: return launch_variant<192, 3, true, 2>(a, p, plan, ctx);
+        case 2: return launch_variant<128, 4, true, 2>(a, p, plan, ctx);
+        case 3: return launch_variant<64, 4, true, 2>(a, p, plan, ctx);
+        case 4: return launch_variant<128, 3, false, 2>(a, p, plan, ctx);
+        case 5: return launch_variant<64, 4, false, 2>(a, p, plan, ctx);
+        default: return launch_variant<32, 4, false, 2>(a, p, plan, ctx);
     }
 }
 
@@ -1293,7 +1319,6 @@ int launch_conv_f16(const ConvF16Args& c, ExecCtx& ctx) {
     a.M = pixels; a.N = c.O; a.K = rows ? c.C : int64_t(taps) * c_slabs * BK;
     a.ldo = c.O;
     a.relu = c.relu;
-    a.conv_chain = true;
     FXF_CHECK(c.split_out.planes != nullptr || (c.O % 4 == 0 && aligned16(c.out)), "convolution (f16): the output needs 16-byte pixels");
     FXF_CHECK(c.res.planes == nullptr || (c.O % 8 == 0 && aligned16(c.res.planes) && (c.res.plane * 2) % 16 == 0 && c.split_out.planes != nullptr), "convolution (f16): unsupported residual");
     ImageGeom im{};
@@ -1346,8 +1371,10 @@ int launch_gemm_f16_swapped(const F16GemmArgs& a, ExecCtx& ctx) {
     p.status = ctx.status;
     tag_launch(ctx, "gemm_f16x3_swapped_tcgen05", 2.0 * double(a.M) * double(a.N) * double(a.K),
                4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.N) + double(a.M) * a.N));
-    const TailSplit ts{p.tiles_m, 0, 1, 0.0};
-    return a.M <= 32 ? launch_variant<32, 4, false, 2>(t, p, ts, ctx.sm_count, ctx) : launch_variant<64, 4, false, 2>(t, p, ts, ctx.sm_count, ctx);
+    F16Plan plan;
+    plan.workers = ctx.sm_count;
+    plan.full = p.tiles_m;
+    return a.M <= 32 ? launch_variant<32, 4, false, 2>(t, p, plan, ctx) : launch_variant<64, 4, false, 2>(t, p, plan, ctx);
 }
 
 }  // namespace fxf

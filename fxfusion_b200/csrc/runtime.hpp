@@ -354,7 +354,7 @@ struct F16GemmArgs {
     float* out = nullptr;               // fp32 result, or
     SplitOut split_out;                 // the result in split form (pitch N)
     int64_t M = 0, N = 0, K = 0, ldo = 0;
-    bool relu = false, conv_chain = false;
+    bool relu = false;
     float* vt_out = nullptr;            // as GemmArgs::vt_*
     unsigned char* vt_flags = nullptr;
     int64_t vt_col0 = 0;
@@ -378,6 +378,25 @@ bool gemm_f16_shape_ok(int64_t M, int64_t N, int64_t K);
 bool gemm_f16_vt_ok(const F16GemmArgs& a, const ExecCtx& ctx);
 int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx);
 std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, int sm_count);
+// How a product in split form is launched, and what it uses of the K-split workspace (host side, no device needed).
+enum class F16Form { kRows, kBf16, kImages };
+struct F16Limits {
+    int sm_count = 148;
+    bool pairs = true;
+    int chunk_k = 0;                    // ExecCtx::tc_chunk_k
+    size_t ws_bytes = 0;                // K-split workspace and its flags; 0: every tile is computed whole
+    int64_t flag_count = 0;
+};
+struct F16Plan {
+    int variant = -1, epilogue_warps = 8, workers = 0, parts = 1, chunk_slabs = 1;
+    int64_t full = 0, tail = 0;         // whole tiles, and tiles cut along K into `parts`
+    size_t ws_bytes = 0;
+    int64_t flags = 0;
+};
+F16Plan gemm_f16_plan(int64_t M, int64_t N, int64_t K, F16Form form, const F16Limits& lim);
+// The workspace an engine keeps: per SM one 128 x 256 partial tile and a flag for each epilogue warp of the instance that has most.
+constexpr size_t kSplitTileBytes = size_t(128) * 256 * sizeof(float);
+constexpr int kSplitFlagsPerSm = 16;
 int gemm_f16_split_parts(int64_t N);    // partial maxima per row a split output of N columns needs room for
 int launch_split_rows(const float* x, int64_t ld, int64_t M, int64_t K, bool bf16, const SplitOut& out, float* bound, ExecCtx& ctx);
 // M <= 64 rows (kernels/gemm_rows.cu): x as fp32 rows, or NULL with a.x in split form; no split output, no transposed columns

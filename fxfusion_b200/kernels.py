@@ -119,3 +119,10 @@ def gemm_variant(M: int, N: int, K: int, precision: str = "auto", sm_count: int 
     buf = C.create_string_buffer(96)
     _lib.check(_lib.lib().fxf_gemm_variant(M, N, K, _lib.GEMM_MODES[precision], sm_count, buf, len(buf)))
     return buf.value.decode()
+
+
+def gemm_workspace(M: int, N: int, K: int, precision: str = "auto", images: bool = False, tc_chunk_k: int = 0, sm_count: int = 148) -> dict:
+    """What a product on operands in split form uses of the K-split workspace, and how much of it an engine keeps (host-side query)."""
+    v = [C.c_int64() for _ in range(4)]
+    _lib.check(_lib.lib().fxf_gemm_workspace(M, N, K, _lib.GEMM_MODES[precision], int(images), tc_chunk_k, sm_count, *[C.byref(x) for x in v]))
+    return dict(zip(("bytes", "bytes_kept", "flags", "flags_kept"), (x.value for x in v)))

@@ -71,3 +71,21 @@ def test_gemm_dispatch_rule_is_a_host_side_query(built_lib):
     assert gemm_variant(8192, 3072, 768, precision="bf16") == "tcgen05-bf16-128x192"
     assert gemm_variant(8192, 3072, 768, precision="fp32_simt") == "simt128x128"
     assert gemm_variant(32, 512, 512) == "skinny32x8"                                # the MLP of the first benchmark configuration
+
+
+def test_tiles_cut_along_k_fit_their_workspace(built_lib):
+    """A product whose last round of tiles is cut along K writes one partial tile per CTA and one flag per epilogue warp: never
+    more of them than the engine keeps, for any chain length (long chains give short convolutions sixteen epilogue warps)."""
+    from fxfusion_b200.kernels import gemm_workspace
+    widest = 0
+    for images, precision in ((True, "auto"), (False, "auto"), (False, "bf16")):
+        for chunk in (0, 64, 512, 1024, 4608):
+            for M in (49, 196, 985, 3136, 196 * 81, 56 * 56 * 7, 200704):
+                for N in (24, 64, 256, 512, 1024, 2048, 3072):
+                    for K in (64, 128, 256, 512, 576, 2304, 4608):
+                        for sms in (148, 132):
+                            w = gemm_workspace(M, N, K, precision, images, chunk, sms)
+                            assert w["bytes"] <= w["bytes_kept"] and w["flags"] <= w["flags_kept"], (M, N, K, precision, images, chunk, sms, w)
+                            widest = max(widest, w["flags"])
+    assert gemm_workspace(81 * 196, 1024, 512, images=True, tc_chunk_k=512)["flags"] == 1920
+    assert widest > 148 * 8

@@ -196,3 +196,35 @@ def test_embedding_scale_add_is_one_pass(built_lib, tmp_path, B, T, D, P, lead):
     eng.run([x.cuda()])
     assert eng.device_status() != 0
     eng.close()
+
+
+@pytest.mark.parametrize("N,O,chunk", [(81, 1024, 512), (81, 1024, 0), (20, 1024, 1024)])
+def test_short_convolutions_with_long_chains(built_lib, tmp_path, N, O, chunk):
+    """1x1 convolutions of 14 x 14 images, 512 channels: with chains as long as their depth they run with sixteen epilogue warps
+    and cut tiles along K (fxf_gemm_workspace: 1920 flags at 81 images), residual and maxima included."""
+    from fxfusion_b200.kernels import gemm_workspace
+    cut = gemm_workspace(N * 196, O, 512, images=True, tc_chunk_k=chunk)
+    assert cut["flags"] <= cut["flags_kept"] and (chunk != 512 or cut["flags"] == 1920)
+    rng = np.random.default_rng(N)
+    gb = [1, 1, 1, 256, 1, 1]
+    b = lowering.GraphBuilder(f"cut_{N}_{O}_{chunk}")
+
+    def conv(x, c, o, k, s, p, h, relu=True):
+        w = (rng.standard_normal((o, c, k, k)) / math.sqrt(c * k * k)).astype(np.float32)
+        return b.op("Conv2dRelu" if relu else "Conv2d", [x, b.const(w), b.const(rng.standard_normal(o, dtype=np.float32))], (N, o, h, h), ints=[s, s, p, p, 1, 1, 1] + gb)
+
+    x = b.input((N, 3, 28, 28), wire.DT_F32)
+    y = conv(x, 3, 512, 7, 2, 3, 14)
+    r = conv(y, 512, O, 1, 1, 0, 14, relu=False)
+    y = b.op("AddRelu", [conv(y, 512, O, 1, 1, 0, 14, relu=False), r], (N, O, 14, 14))
+    y = conv(y, O, 512, 1, 1, 0, 14)
+    b.output(b.op("AdaptiveAvgPool2d", [y], (N, 512, 1, 1), ints=[1, 1] + gb))
+    graph, eng = _engine(b, tmp_path, tc_chunk_k=chunk)
+    assert eng.describe().count("output in split form") == 4, eng.describe()
+    xin = torch.randn(N, 3, 28, 28, generator=torch.Generator().manual_seed(5))
+    want = GraphOracle(graph).run([xin])[0]
+    for _ in range(3):   # the flags are zero again after every launch
+        got = eng.run([xin.cuda()])[0].cpu()
+        assert ((got - want).abs().max() / want.abs().max()).item() < (4e-6 if chunk == 0 else 4e-5)
+    assert eng.device_status() == 0
+    eng.close()
