@@ -561,6 +561,14 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             *hi = meta[r].offset + int64_t(e->reg[r].nbytes);
             return true;
         };
+        // whether a tensor will be bound to a 16-byte address: split form is read and written in such pieces, and a file may place
+        // activations (and slices of constants) at any offset
+        std::vector<int64_t> view_off(n_tensors, -1);   // slices of constants that are views: bytes behind the constant's begin
+        auto on_16_bytes = [&](uint32_t id) {
+            int64_t lo = 0, hi = 0;
+            const int64_t view = view_off[root(id)];
+            return view >= 0 ? view % 16 == 0 : (!arena_range(id, &lo, &hi) || lo % 16 == 0);
+        };
 
         // -- tensor parallelism: [sharded contraction -> Add -> LayerNorm] or [sharded contraction -> AddLayerNorm] becomes the
         // contraction plus ONE exchange kernel over peer memory that sums the ranks' partial outputs, adds the residual and
@@ -729,6 +737,7 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
                 if (outer != 1 || o.shape[dim] != length || start < 0 || start + length > x.shape[dim] || numel(o) != length * inner || numel(o) == 0) continue;
                 n.view_of = int(n.in[0]);
                 n.view_off = size_t(start * inner) * size_t(dtype_size(x.dtype));
+                view_off[n.out[0]] = int64_t(n.view_off);
                 n.folded = true;
             }
             for (auto& n : e->nodes) {
@@ -779,7 +788,7 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             const FxfTensor& t = e->reg[id];
             int64_t lo = 0, hi = 0;
             return root(id) == id && meta[id].kind == kActivation && !escapes[id] && t.rank == 4 && t.dtype == FXF_F32 && t.shape[1] % 8 == 0 &&
-                   (is_channels_last(t) || (is_contiguous(t) && t.shape[2] * t.shape[3] == 1)) && numel(t) > 0 && arena_range(id, &lo, &hi);
+                   (is_channels_last(t) || (is_contiguous(t) && t.shape[2] * t.shape[3] == 1)) && numel(t) > 0 && arena_range(id, &lo, &hi) && on_16_bytes(id);
         };
         auto overlap = [&](uint32_t a, uint32_t b) {
             int64_t al = 0, ah = 0, bl = 0, bh = 0;
@@ -813,6 +822,7 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             if (f.add >= 0 && !(images[f.res] && images[f.out])) return false;
             const uint32_t o = f.add >= 0 ? f.out : n.out[0];
             const FxfTensor& to = e->reg[o];   // what is not kept in split form leaves as fp32 pixels
+            if (!images[o] && n.plan->image_role != NodePlan::kImageGlobalAvg && !on_16_bytes(o)) return false;
             if (!images[o] && !(is_channels_last(to) || (is_contiguous(to) && to.rank == 4 && (to.shape[2] * to.shape[3] == 1 || to.shape[1] == 1)))) return false;
             switch (n.plan->image_role) {
                 case NodePlan::kImageConv: return images[n.in[0]] != 0;
@@ -876,7 +886,9 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             if (!P.plan->makes_split || P.folded || P.xchg || P.fuse_out >= 0 || P.out.size() != 1) continue;
             const uint32_t t = root(P.out[0]);
             int64_t lo = 0, hi = 0;
-            if (escapes[t] || meta[t].kind != kActivation || producer[t] != int(pi) || n_readers[t] == 0 || !arena_range(t, &lo, &hi)) continue;
+            if (escapes[t] || meta[t].kind != kActivation || producer[t] != int(pi) || n_readers[t] == 0 || !arena_range(t, &lo, &hi) || !on_16_bytes(t)) continue;
+            const bool norm = P.op == FXF_OP_LAYER_NORM || P.op == FXF_OP_ADD_LAYER_NORM;   // (only its vector kernel writes split form)
+            if (norm && !std::all_of(P.in.begin(), P.in.end(), on_16_bytes)) continue;
             if (numel(e->reg[P.out[0]]) != P.plan->split_rows * P.plan->split_cols || e->reg[P.out[0]].dtype != FXF_F32 || !is_contiguous(e->reg[P.out[0]])) continue;
             bool ok = true;
             for (size_t ri = 0; ri < e->nodes.size() && ok; ri++)
@@ -893,7 +905,7 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             m.plane = P.plan->split_rows * P.plan->split_cols;
             m.inv = reinterpret_cast<const float*>(e->base + P.split_off);
             m.amax = m.inv + P.plan->split_rows;
-            if (P.op == FXF_OP_LAYER_NORM || P.op == FXF_OP_ADD_LAYER_NORM) {   // |(x - mean) / std| < sqrt(D), whatever x
+            if (norm) {   // |(x - mean) / std| < sqrt(D), whatever x
                 auto largest = [&](uint32_t id, int64_t n) {   // of a constant; infinity: unknown
                     if (meta[id].kind != kConstant || meta[id].data == nullptr || numel(e->reg[id]) != n || e->reg[id].dtype != FXF_F32) return INFINITY;
                     float top = 0.f;

@@ -228,3 +228,81 @@ def test_short_convolutions_with_long_chains(built_lib, tmp_path, N, O, chunk):
         assert ((got - want).abs().max() / want.abs().max()).item() < (4e-6 if chunk == 0 else 4e-5)
     assert eng.device_status() == 0
     eng.close()
+
+
+@pytest.mark.parametrize("pad_x,pad_y", [(0, 0), (12, 0), (0, 4), (12, 4)])
+def test_rows_at_any_offset(built_lib, tmp_path, pad_x, pad_y):
+    """A graph file may place activations at any multiple of four bytes: where a LayerNorm, its input, its weights (a slice of a
+    constant) or a product's result does not lie on a 16-byte address, the rows stay fp32 and the results are the same."""
+    M, D, F = 70, 64, 96
+    rng = np.random.default_rng(1)
+    b = lowering.GraphBuilder(f"offsets_{pad_x}_{pad_y}", alignment=4)
+    c = lambda n, k: (b.const(_w(rng, n, k)), b.const(rng.standard_normal(n, dtype=np.float32)))
+    pads = []
+
+    def pad(nbytes):   # an activation that lives to the end, so that what follows lies `nbytes` further on
+        if nbytes:
+            pads.append(b.op("Relu", [b.input((nbytes // 4,), wire.DT_F32)], (nbytes // 4,)))
+
+    def slice_from(lead):   # a slice of a constant, `lead` floats behind its begin
+        return b.op("Narrow", [b.const(rng.standard_normal(D + 4, dtype=np.float32))], (D,), ints=[0, lead, D])
+
+    x0 = b.input((M, D), wire.DT_F32)
+    pad(pad_x)
+    x = b.op("Relu", [x0], (M, D))
+    pad(pad_y)
+    ln = b.op("LayerNorm", [x, slice_from(4), slice_from(0)], (M, D), ints=[1, D], floats=[1e-5])
+    ln2 = b.op("LayerNorm", [x, slice_from(1), slice_from(0)], (M, D), ints=[1, D], floats=[1e-5])   # never: its weights lie on 4 bytes
+    h = b.op("LinearRelu", [ln, *c(F, D)], (M, F))
+    g = b.op("FeedForward", [ln2, *c(F, D), *c(D, F)], (M, D))
+    h2 = b.op("Linear", [h, *c(D, F)], (M, D))
+    b.output(b.op("Add", [h2, g], (M, D)))
+    for p in pads:
+        b.output(p)
+    graph, eng = _engine(b, tmp_path)
+    text = eng.describe().splitlines()
+    split = [("output in split form" in t) for t in text if t.split()[1:2] and t.split()[1] in ("LayerNorm", "LinearRelu")]
+    assert split == [pad_x == 0 and pad_y == 0, False, (pad_x + pad_y) % 16 == 0], "\n".join(text)
+    gen = torch.Generator().manual_seed(3)
+    xin = [torch.randn(M, D, generator=gen)] + [torch.randn(n // 4, generator=gen) for n in (pad_x, pad_y) if n]
+    got, want = eng.run([t.cuda() for t in xin]), GraphOracle(graph).run(xin)
+    for o, w in zip(got, want):
+        ok, info = compare_outputs(o.cpu(), w, atol=ATOL, rtol=RTOL)
+        assert ok, info
+    assert eng.device_status() == 0
+    eng.close()
+
+
+@pytest.mark.parametrize("pad,later", [(0, False), (4, False), (12, False), (8, True)])
+def test_images_at_any_offset(built_lib, tmp_path, pad, later):
+    """The same for images: what does not lie on a 16-byte address is kept as fp32 pixels (`later`: from the second convolution's
+    result on), whatever its neighbours could do."""
+    N, rng, gb = 3, np.random.default_rng(2), [1, 1, 1, 256, 1, 1]
+    b = lowering.GraphBuilder(f"image_offsets_{pad}_{later}", alignment=4)
+
+    def conv(x, c, o, h, k, s, p, relu=True):
+        ho = (h + 2 * p - k) // s + 1
+        w = (rng.standard_normal((o, c, k, k)) / math.sqrt(c * k * k)).astype(np.float32)
+        return b.op("Conv2dRelu" if relu else "Conv2d", [x, b.const(w), b.const(rng.standard_normal(o, dtype=np.float32))], (N, o, ho, ho), ints=[s, s, p, p, 1, 1, 1] + gb)
+
+    x = b.input((N, 3, 48, 48), wire.DT_F32)
+    odd = b.input((pad // 4,), wire.DT_F32) if pad else None
+    keep = b.op("Relu", [odd], (pad // 4,)) if pad and not later else None
+    y = b.op("MaxPool2d", [conv(x, 3, 64, 48, 7, 2, 3)], (N, 64, 12, 12), ints=[3, 3, 2, 2, 1, 1, 1, 1, 0] + gb)
+    r = conv(y, 64, 128, 12, 1, 1, 0, relu=False)
+    if pad and later:
+        keep = b.op("Relu", [odd], (pad // 4,))
+    t = conv(y, 64, 64, 12, 3, 1, 1)
+    y = b.op("AddRelu", [conv(t, 64, 128, 12, 1, 1, 0, relu=False), r], (N, 128, 12, 12))
+    b.output(b.op("AdaptiveAvgPool2d", [conv(y, 128, 72, 12, 3, 2, 1)], (N, 72, 1, 1), ints=[1, 1] + gb))
+    if keep is not None:
+        b.output(keep)
+    graph, eng = _engine(b, tmp_path)
+    count = eng.describe().count("output in split form")
+    assert count == 6 if pad == 0 else (count == 0 if not later else count < 6), eng.describe()
+    gen = torch.Generator().manual_seed(4)
+    xin = [torch.randn(N, 3, 48, 48, generator=gen)] + ([torch.randn(pad // 4, generator=gen)] if pad else [])
+    got, want = eng.run([t.cuda() for t in xin]), GraphOracle(graph).run(xin)
+    assert ((got[0].cpu() - want[0]).abs().max() / want[0].abs().max()).item() < 4e-6
+    assert eng.device_status() == 0
+    eng.close()
