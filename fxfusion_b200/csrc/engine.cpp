@@ -395,6 +395,13 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
     }
 
     // ---- plans (they see the final layouts) ---------------------------------------------------------
+    std::vector<char> constants(n_tensors, 0);
+    for (uint32_t id = 0; id < n_tensors; id++) {
+        uint32_t r = id;
+        for (int guard = 0; guard < 64 && meta[r].alias_of >= 0 && uint32_t(meta[r].alias_of) < n_tensors; guard++) r = uint32_t(meta[r].alias_of);
+        constants[id] = meta[r].kind == kConstant;
+    }
+    env.constants = &constants;
     for (auto& n : e->nodes) {
         const int op = n.op;
         const OpEntry& entry = op_entry(op);

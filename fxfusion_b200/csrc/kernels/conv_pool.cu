@@ -774,14 +774,15 @@ std::unique_ptr<NodePlan> plan_conv(const Registry& reg, const TensorIds& in, co
         pl->flops = 2.0 * double(numel(o)) * double(w.shape[1]) * double(w.shape[2]) * double(w.shape[3]);
         pl->bytes = double(reg[in[0]].nbytes) + double(w.nbytes) + double(reg[in[2]].nbytes) + double(o.nbytes);
         const int64_t M = o.shape[0] * o.shape[2] * o.shape[3], O = w.shape[0], C = w.shape[1];
+        const bool tc = env.gemm_mode != FXF_GEMM_FP32_SIMT && env.is_constant(in[1]);   // filters are re-laid out at build time
         const bool is_1x1 = w.shape[2] == 1 && w.shape[3] == 1 && p.ints[0] == 1 && p.ints[1] == 1 && p.ints[2] == 0 && p.ints[3] == 0 && p.ints[6] == 1;
-        if (is_1x1 && env.gemm_mode != FXF_GEMM_FP32_SIMT && gemm_tc_shape_ok(M, O, C)) {
+        if (is_1x1 && tc && gemm_tc_shape_ok(M, O, C)) {
             pl->gemm_1x1 = true;
             pl->w_elems = O * C;
             pl->bf16 = env.gemm_mode == FXF_GEMM_BF16 && C % 8 == 0;
             pl->persist_bytes = round_up(size_t(2) * size_t(pl->w_elems) * sizeof(float), 256);
             pl->variant = pl->bf16 ? "1x1 -> tcgen05-bf16 GEMM when channels-last, else igemm-simt64x64" : "1x1 -> tcgen05-tf32x3 GEMM when channels-last, else igemm-simt64x64";
-        } else if (!is_1x1 && p.ints[0] >= 1 && p.ints[0] <= 2 && p.ints[1] >= 1 && p.ints[1] <= 2 && p.ints[6] == 1 && env.gemm_mode != FXF_GEMM_FP32_SIMT && conv_tc_shape_ok(M, int(C), int(O)) &&
+        } else if (!is_1x1 && p.ints[0] >= 1 && p.ints[0] <= 2 && p.ints[1] >= 1 && p.ints[1] <= 2 && p.ints[6] == 1 && tc && conv_tc_shape_ok(M, int(C), int(O)) &&
                    reg[in[0]].rank == 4 && reg[in[0]].shape[1] == C) {
             pl->igemm_tc = true;
             pl->w_elems = O * C * w.shape[2] * w.shape[3];
@@ -789,7 +790,7 @@ std::unique_ptr<NodePlan> plan_conv(const Registry& reg, const TensorIds& in, co
             pl->persist_bytes = round_up(size_t(2) * size_t(pl->w_elems) * sizeof(float), 256);
             pl->variant = pl->bf16 ? "tcgen05-bf16 implicit GEMM when channels-last, else igemm-simt64x64" : "tcgen05-tf32x3 implicit GEMM when channels-last, else igemm-simt64x64";
         } else if (!is_1x1 && p.ints[0] == 2 && p.ints[1] == 2 && p.ints[4] == 1 && p.ints[5] == 1 && p.ints[6] == 1 && C >= 1 && C <= 4 && O >= 64 &&
-                   env.gemm_mode != FXF_GEMM_FP32_SIMT && reg[in[0]].rank == 4 && reg[in[0]].shape[1] == C && M >= 64) {
+                   tc && reg[in[0]].rank == 4 && reg[in[0]].shape[1] == C && M >= 64) {
             // stem: space-to-depth copy (16 channels) in the shared scratch, then a stride-1 tensor-core convolution
             const FxfTensor& x = reg[in[0]];
             pl->s2d_tc = true;
@@ -806,7 +807,7 @@ std::unique_ptr<NodePlan> plan_conv(const Registry& reg, const TensorIds& in, co
             pl->variant = "igemm-simt64x64";
         }
         // on images in split form, if the engine finds that the neighbours can (it then sets `images`)
-        if (env.gemm_mode == FXF_GEMM_AUTO && env.tp_size == 1 && reg[in[0]].rank == 4 && M >= 1 && numel(reg[in[2]]) == O && O % 8 == 0 && o.shape[0] <= 65535) {
+        if (env.gemm_mode == FXF_GEMM_AUTO && tc && env.is_constant(in[2]) && env.tp_size == 1 && reg[in[0]].rank == 4 && M >= 1 && numel(reg[in[2]]) == O && O % 8 == 0 && o.shape[0] <= 65535) {
             if (pl->s2d_tc && pl->KW2 <= 4 && pl->Hs <= 65535 && M < (int64_t(1) << 31) - 256 && is_contiguous(reg[in[0]])) {
                 pl->image_role = NodePlan::kImageStem;
                 pl->k_split = int64_t(pl->KH2) * 64;

@@ -213,9 +213,12 @@ bool want_f16(const PlanEnv& env, int64_t M, int64_t N, int64_t K) {
     if (env.tp_size > 1 || !gemm_f16_shape_ok(M, N, K)) return false;
     return env.gemm_mode == FXF_GEMM_AUTO || (env.gemm_mode == FXF_GEMM_BF16 && (M <= kFewRows || gemm_tc_shape_ok(M, N, K)));
 }
-void reserve_weight(DensePlan& p, Slice& w, const PlanEnv& env, int64_t M, int64_t N, int64_t K) {
-    if (want_f16(env, M, N, K)) p.reserve_f16(w, p.bf16_mode && M > kFewRows);
-    else p.reserve(w, want_tc(env, M, N, K));
+// A weight's bias is the input after it.  Both have to be constants for split form: its conversion happens at build time and
+// includes a bound of the bias, and the few-row kernel reads both ahead of the end of the kernel before it.
+void reserve_weight(DensePlan& p, Slice& w, const TensorIds& in, const PlanEnv& env, int64_t M, int64_t N, int64_t K) {
+    const bool constant = env.is_constant(in[size_t(w.input)]);
+    if (constant && env.is_constant(in[size_t(w.input) + 1]) && want_f16(env, M, N, K)) p.reserve_f16(w, p.bf16_mode && M > kFewRows);
+    else p.reserve(w, constant && want_tc(env, M, N, K));
 }
 // Whether a product wants its activation in split form from the producer: the tiled kernel and the streaming few-row kernel
 // load it so; the cluster kernel of gemm_rows.cu takes fp32 rows and splits its own K range.
@@ -223,7 +226,7 @@ bool takes_split_rows(int64_t M, int64_t N) { return M > kFewRows || gemm_rows_s
 std::string variant_of(const PlanEnv& env, const Slice& w, int64_t M, int64_t N, int64_t K) {
     GemmArgs g;
     g.M = M; g.N = N; g.K = K;
-    std::string v = gemm_variant_name(g, env.gemm_mode, 148, env.tc_pairs);
+    std::string v = gemm_variant_name(g, w.f16 || w.split ? env.gemm_mode : FXF_GEMM_FP32_SIMT, 148, env.tc_pairs);
     if (!w.f16) return v;
     return v + " (split operands: tcgen05-" + (M > kFewRows ? gemm_f16_variant_name(M, N, K, w.bf16, 148) : std::string(takes_split_rows(M, N) ? "f16x3-stream128" : "f16x3-rows128")) + ")";
 }
@@ -351,7 +354,7 @@ std::unique_ptr<NodePlan> plan_linear(const Registry& reg, const TensorIds& in, 
         p->col_off = r0;
         p->n_local = r1 - r0;
     }
-    reserve_weight(*p, ws, env, M, p->n_local, K);
+    reserve_weight(*p, ws, in, env, M, p->n_local, K);
     p->reserve(bs, false);
     p->M = M;
     if (ws.f16) {
@@ -478,9 +481,9 @@ std::unique_ptr<NodePlan> plan_feedforward(const Registry& reg, const TensorIds&
     } else if (env.tp_size > 1) {
         p->variant = "replicated ";
     }
-    reserve_weight(*p, s_w1, env, M, Fl, K);
+    reserve_weight(*p, s_w1, in, env, M, Fl, K);
     p->reserve(s_b1, false);
-    reserve_weight(*p, s_w2, env, M, P, Fl);
+    reserve_weight(*p, s_w2, in, env, M, P, Fl);
     p->reserve(s_b2, false);
     p->M = M;
     p->scratch_bytes = size_t(M) * size_t(Fl) * sizeof(float);
@@ -633,9 +636,9 @@ std::unique_ptr<NodePlan> plan_mha(const Registry& reg, const TensorIds& in, con
     } else if (env.tp_size > 1) {
         pl->variant = "replicated ";
     }
-    reserve_weight(*pl, s_wq, env, M, 3 * Dl, D);
+    reserve_weight(*pl, s_wq, in, env, M, 3 * Dl, D);
     pl->reserve(s_bq, false);
-    reserve_weight(*pl, s_wo, env, M, D, Dl);
+    reserve_weight(*pl, s_wo, in, env, M, D, Dl);
     pl->reserve(s_bo, false);
     pl->M = M;
     pl->scratch_bytes = size_t(M) * size_t(3 * Dl + Dl) * sizeof(float);
@@ -792,11 +795,11 @@ std::unique_ptr<NodePlan> plan_cross_mha(const Registry& reg, const TensorIds& i
     } else if (env.tp_size > 1) {
         pl->variant = "replicated ";
     }
-    reserve_weight(*pl, s_wq, env, Mq, Dl, D);
+    reserve_weight(*pl, s_wq, in, env, Mq, Dl, D);
     pl->reserve(s_bq, false);
-    reserve_weight(*pl, s_wkv, env, Mk, 2 * Dl, D);
+    reserve_weight(*pl, s_wkv, in, env, Mk, 2 * Dl, D);
     pl->reserve(s_bkv, false);
-    reserve_weight(*pl, s_wo, env, Mq, D, Dl);
+    reserve_weight(*pl, s_wo, in, env, Mq, D, Dl);
     pl->reserve(s_bo, false);
     pl->M = Mq;
     pl->scratch_bytes = (size_t(Mq) * size_t(2 * Dl) + size_t(Mk) * size_t(2 * Dl)) * sizeof(float);
@@ -1066,9 +1069,9 @@ std::unique_ptr<NodePlan> plan_cached_mha(const Registry& reg, const TensorIds& 
     Slice& s_bq = pl->add(4, QKV, 1);
     Slice& s_wo = pl->add(5, D, D);
     Slice& s_bo = pl->add(6, D, 1);
-    reserve_weight(*pl, s_wq, env, B, QKV, D);
+    reserve_weight(*pl, s_wq, in, env, B, QKV, D);
     pl->reserve(s_bq, false);
-    reserve_weight(*pl, s_wo, env, B, D, D);
+    reserve_weight(*pl, s_wo, in, env, B, D, D);
     pl->reserve(s_bo, false);
     if (s_wq.f16) pl->takes_split = takes_split_rows(B, QKV) ? 1 : 0;
     pl->cache_off = pl->persist_bytes;

@@ -183,6 +183,10 @@ struct PlanEnv {
     int tp_rank = 0, tp_size = 1;     // tensor-parallel position of this engine
     bool shard_output_cols = false;   // this node is the graph's final Linear and its columns are sharded over the ranks
     bool tc_pairs = true;             // the engine lets CTA pairs compute the widest GEMM tiles (reported in variant names)
+    // By tensor id: the tensor is a constant of the graph (NULL: a single call, whose tensors are what they are while it runs).
+    // Only those may be converted at build time; a weight that the graph computes or takes as an input is read as it is.
+    const std::vector<char>* constants = nullptr;
+    bool is_constant(uint32_t id) const { return constants == nullptr || (id < constants->size() && (*constants)[id]); }
 };
 
 using KernelFn = int (*)(Registry&, const TensorIds&, const TensorIds&, const Params&, const NodePlan*, ExecCtx&);

@@ -306,3 +306,66 @@ def test_images_at_any_offset(built_lib, tmp_path, pad, later):
     assert ((got[0].cpu() - want[0]).abs().max() / want[0].abs().max()).item() < 4e-6
     assert eng.device_status() == 0
     eng.close()
+
+
+@pytest.mark.parametrize("M", [1, 32, 70, 300])
+@pytest.mark.parametrize("what", ["weight", "bias", "both"])
+def test_weights_that_are_not_constants(built_lib, tmp_path, M, what):
+    """Only constants are converted at build time: a weight or bias that is an input of the graph, or computed by the node
+    before, is read when the product runs."""
+    K, N = 72, 136
+    rng = np.random.default_rng(M)
+    b = lowering.GraphBuilder(f"live_{M}_{what}")
+    x = b.input((M, K), wire.DT_F32)
+    w1, w2, b1, b2 = _w(rng, N, K), _w(rng, K, N), rng.standard_normal(N, dtype=np.float32), rng.standard_normal(K, dtype=np.float32)
+    given = []
+
+    def weight(a):
+        if what == "bias":
+            return b.const(a)
+        given.append(a)
+        return b.input(a.shape, wire.DT_F32)
+
+    def bias(a):
+        if what == "weight":
+            return b.const(a)
+        given.append(a)
+        return b.op("Mul", [b.input(a.shape, wire.DT_F32)], a.shape, ints=[1], floats=[2.0])
+
+    ff = [weight(w1), bias(b1), weight(w2), bias(b2)]
+    y = b.op("FeedForward", [x, *ff], (M, K))
+    y = b.op("LinearRelu", [y, ff[0], ff[1]], (M, N))
+    b.output(b.op("Linear", [y, b.const(w2), bias(b2) if what != "weight" else b.const(b2)], (M, K)))
+    graph, eng = _engine(b, tmp_path)
+    gen = torch.Generator().manual_seed(1)
+    for scale in (1.0, 3.0):   # the second run brings other weights
+        xin = [torch.randn(M, K, generator=gen)] + [torch.from_numpy(a * np.float32(scale)) for a in given]
+        ok, info = compare_outputs(eng.run([t.cuda() for t in xin])[0].cpu(), GraphOracle(graph).run(xin)[0], atol=1e-3, rtol=1e-3)
+        assert ok, info
+    assert eng.device_status() == 0
+    eng.close()
+
+
+def test_filters_that_are_not_constants(built_lib, tmp_path):
+    """A convolution between images in split form whose filters are an input of the graph: it reads them when it runs, and its
+    neighbours keep the images it touches as fp32 pixels."""
+    N, rng, gb = 2, np.random.default_rng(3), [1, 1, 1, 256, 1, 1]
+    b = lowering.GraphBuilder("live_filters")
+    w = lambda o, c, k: (rng.standard_normal((o, c, k, k)) / math.sqrt(c * k * k)).astype(np.float32)
+    bias = lambda o: b.const(rng.standard_normal(o, dtype=np.float32))
+    x = b.input((N, 3, 32, 32), wire.DT_F32)
+    y = b.op("Conv2dRelu", [x, b.const(w(64, 3, 7)), bias(64)], (N, 64, 16, 16), ints=[2, 2, 3, 3, 1, 1, 1] + gb)
+    y = b.op("Conv2dRelu", [y, b.const(w(64, 64, 3)), bias(64)], (N, 64, 16, 16), ints=[1, 1, 1, 1, 1, 1, 1] + gb)
+    live = w(128, 64, 3)
+    y = b.op("Conv2dRelu", [y, b.input(live.shape, wire.DT_F32), bias(128)], (N, 128, 16, 16), ints=[1, 1, 1, 1, 1, 1, 1] + gb)
+    y = b.op("Conv2dRelu", [y, b.input((64, 128, 1, 1), wire.DT_F32), bias(64)], (N, 64, 16, 16), ints=[1, 1, 0, 0, 1, 1, 1] + gb)
+    b.output(b.op("AdaptiveAvgPool2d", [y], (N, 64, 1, 1), ints=[1, 1] + gb))
+    graph, eng = _engine(b, tmp_path)
+    assert eng.describe().count("output in split form") == 1, eng.describe()
+    gen = torch.Generator().manual_seed(1)
+    for scale in (1.0, 2.0):
+        xin = [torch.randn(N, 3, 32, 32, generator=gen), torch.from_numpy(live * np.float32(scale)), torch.from_numpy(w(64, 128, 1))]
+        ok, info = compare_outputs(eng.run([t.cuda() for t in xin])[0].cpu(), GraphOracle(graph).run(xin)[0], atol=ATOL, rtol=RTOL)
+        assert ok, info
+    assert eng.device_status() == 0
+    eng.close()
