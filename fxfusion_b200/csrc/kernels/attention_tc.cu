@@ -585,22 +585,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
     }
 }
 
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            return reinterpret_cast<EncodeTiledFn>(p);
-        return EncodeTiledFn(nullptr);
-    }();
-    return fn;
-}
 // fp32 tensor seen as [n2, n1, n0] with n0 contiguous and byte strides s1 (dim 1), s2 (dim 2);
 // box [1, box1, 32 floats], 128-byte swizzle, zero fill outside.
 int make_map3(CUtensorMap* map, const float* base, int64_t n0, int64_t n1, int64_t n2, int64_t s1, int64_t s2, int box1) {
-    EncodeTiledFn fn = encode_fn();
+    const auto fn = encode_tiled_fn();
     FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
     cuuint64_t dims[3] = {cuuint64_t(n0), cuuint64_t(n1), cuuint64_t(n2)};
     cuuint64_t strides[2] = {cuuint64_t(s1), cuuint64_t(s2)};

@@ -279,24 +279,20 @@ __global__ void __launch_bounds__(256) conv_weight_s2d_split_kernel(const float*
 
 // ---- images in split form (one power-of-two scale per image; see gemm_f16.cu) -----------------------------------------
 // Filters of one output channel per block: [O, taps, Cp] with Cp = C padded to whole 64-deep K-slabs (S2D: [O, KH2, 4 pixels,
-// 16 channels] in the space-to-depth order above), as two fp16 planes, 1 / scale per row and the largest L1 norm of a row.
+// 16 channels] in the space-to-depth order above), as two fp16 planes, 1 / scale per row and the row's L1 norm.  The filters are
+// read once, in memory order, and re-ordered in shared memory (`staged`: they fit there).
 template <bool S2D>
 __global__ void __launch_bounds__(128) conv_weight_f16_kernel(const float* __restrict__ w, uint16_t* __restrict__ planes, int64_t plane, float* __restrict__ inv_out,
-                                                              float* __restrict__ bound, int C, int KH, int KW, int Cp, int K) {
+                                                              float* __restrict__ l1_out, int C, int KH, int KW, int Cp, int K, int staged) {
+    extern __shared__ float filters[];
     __shared__ float red[8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, o = blockIdx.x;
-    const float* wo = w + int64_t(o) * C * KH * KW;
-    auto value = [&](int k) {
-        if (S2D) {
-            const int ch = k & 15, qx = (k >> 4) & 3, qy = k >> 6, r = ch / C, c = ch - r * C, ky = 2 * qy + (r >> 1), kx = 2 * qx + (r & 1);
-            return (r < 4 && ky < KH && kx < KW) ? wo[(c * KH + ky) * KW + kx] : 0.f;
-        }
-        const int tap = k / Cp, c = k - tap * Cp;
-        return c < C ? wo[c * KH * KW + tap] : 0.f;
-    };
+    sm100::grid_dep();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, o = blockIdx.x, n = C * KH * KW;
+    const float* wo = w + int64_t(o) * n;
     float m = 0.f, l1 = 0.f;
-    for (int k = threadIdx.x; k < K; k += 128) {
-        const float a = fabsf(value(k));
+    for (int i = threadIdx.x; i < n; i += 128) {
+        const float v = wo[i], a = fabsf(v);
+        if (staged) filters[i] = v;
         m = fmaxf(m, a);
         l1 += a;
     }
@@ -312,8 +308,17 @@ __global__ void __launch_bounds__(128) conv_weight_f16_kernel(const float* __res
     sm100::split_scale(m, scale, inv);
     if (threadIdx.x == 0) {
         inv_out[o] = inv;
-        atomicMax(reinterpret_cast<int*>(bound), __float_as_int((red[4] + red[5] + red[6] + red[7]) * 1.0001f));
+        l1_out[o] = (red[4] + red[5]) + (red[6] + red[7]);
     }
+    const float* src = staged ? filters : wo;
+    auto value = [&](int k) {
+        if (S2D) {
+            const int ch = k & 15, qx = (k >> 4) & 3, qy = k >> 6, r = ch / C, c = ch - r * C, ky = 2 * qy + (r >> 1), kx = 2 * qx + (r & 1);
+            return (r < 4 && ky < KH && kx < KW) ? src[(c * KH + ky) * KW + kx] : 0.f;
+        }
+        const int tap = k / Cp, c = k - tap * Cp;
+        return c < C ? src[c * KH * KW + tap] : 0.f;
+    };
     for (int k = threadIdx.x * 2; k < K; k += 256) {
         uint32_t hi, lo;
         sm100::split_f16x2(value(k) * scale, value(k + 1) * scale, hi, lo);
@@ -486,24 +491,26 @@ struct ConvPlan : NodePlan {
     int Hs = 0, Ws = 0, KH2 = 0, KW2 = 0;
     int64_t w_elems = 0;
     const float *w_hi = nullptr, *w_lo = nullptr;
-    size_t split_bytes(int64_t O) const { return size_t(O) * size_t(k_split) * 4 + round_up(size_t(O) * 4, 16) + 16; }
+    size_t split_bytes(int64_t O) const { return size_t(O) * size_t(k_split) * 4 + 2 * round_up(size_t(O) * 4, 16) + 16; }   // planes, scales, bound, L1 norms
     int prepare_split(const FxfTensor& w, const FxfTensor& b, ExecCtx& ctx) {
         const int O = int(w.shape[0]), C = int(w.shape[1]), KH = int(w.shape[2]), KW = int(w.shape[3]), K = int(k_split);
         variant = image_role == kImageStem ? "space-to-depth + tcgen05-f16x3 implicit GEMM on images in split form" : "tcgen05-f16x3 implicit GEMM on images in split form";
         uint16_t* planes = static_cast<uint16_t*>(persist);
         float* inv = reinterpret_cast<float*>(planes + int64_t(O) * K * 2);
         float* bound = inv + round_up(size_t(O), 4);
-        FXF_CUDA(cudaMemsetAsync(bound, 0, 8, ctx.stream));
+        float* l1 = bound + 4;
         const bool stem = image_role == kImageStem;
+        const size_t filter_bytes = size_t(C) * KH * KW * sizeof(float);
+        const int staged = filter_bytes <= 48 * 1024 - 64 ? 1 : 0;
         tag_launch(ctx, "conv_weight_split_f16", 0, 8.0 * double(O) * K);
-        if (stem) conv_weight_f16_kernel<true><<<O, 128, 0, ctx.stream>>>(static_cast<const float*>(w.ptr), planes, int64_t(O) * K, inv, bound, C, KH, KW, 64, K);
-        else conv_weight_f16_kernel<false><<<O, 128, 0, ctx.stream>>>(static_cast<const float*>(w.ptr), planes, int64_t(O) * K, inv, bound, C, KH, KW, K / (KH * KW), K);
+        dependent(stem ? conv_weight_f16_kernel<true> : conv_weight_f16_kernel<false>, O, 128, staged ? filter_bytes : 0, ctx)(
+            static_cast<const float*>(w.ptr), planes, int64_t(O) * K, inv, l1, C, KH, KW, stem ? 64 : K / (KH * KW), K, staged);
         FXF_LAUNCHED(ctx);
         w_split.planes = planes;
         w_split.plane = int64_t(O) * K;
         w_split.inv = inv;
         w_split.bound = bound;
-        return launch_bias_bound(static_cast<const float*>(b.ptr), O, bound, ctx);
+        return launch_weight_bound(l1, O, static_cast<const float*>(b.ptr), O, bound, ctx);
     }
     int prepare(Registry& reg, const TensorIds& in, const TensorIds&, const Params&, ExecCtx& ctx) override {
         if (images) return prepare_split(reg[in[1]], reg[in[2]], ctx);

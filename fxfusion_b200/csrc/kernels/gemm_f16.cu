@@ -13,7 +13,7 @@
 // of two, so multiplying by 1 / (s_x s_w) in the epilogue is exact.
 // Both planes of [rows, K] take the bytes of the fp32 matrix: a tensor of the engine keeps its arena slot in either form.
 //
-// Who splits.  Weights: once per engine (split_rows_kernel).  Activations: the kernel that produces them, where it knows a
+// Who splits.  Weights: once per engine (split_rows_kernel, split_form.cu).  Activations: the kernel that produces them, where it knows a
 // bound of each row: LayerNorm holds the row, and this kernel's own epilogue bounds its output rows by
 //     |y[r,j]| <= amax_r * max_j ||w_j||_1 + max_j |b_j|
 // (amax_r = max_k |x[r,k]|, kept beside the planes).  Anything else goes through split_rows_kernel first.
@@ -37,7 +37,6 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <mutex>
 #include <type_traits>
 
 #include "../runtime.hpp"
@@ -156,12 +155,6 @@ __device__ __forceinline__ void tile_coords(const F16Params& p, int tile, int& t
 }
 // a wait counts only if it succeeded for every lane, so that a warp gives up as a whole
 __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
-__device__ __forceinline__ float max_keep_nan(float v, float floor_at) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "f"(floor_at));
-    return r;
-}
-__device__ __forceinline__ float relu_keep_nan(float v) { return max_keep_nan(v, 0.f); }
 
 // v = sum[16 g ..], g known only at run time: a tree of branches (registers cannot be indexed)
 template <int LO, int HI, int HALF>
@@ -946,87 +939,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     }
 }
 
-// ---- fp32 rows -> split form ---------------------------------------------------------------------------
-// One block per row (rows are hundreds to thousands of floats): maximum, then the two planes from the row's second read,
-// which hits L1 / L2.  bound != NULL also raises bound[0] to the largest L1 norm of a row (weights; one atomic per row).
-// MODE 0: f16 planes; 1: bf16 plane only.
-template <int MODE>
-__global__ void __launch_bounds__(128) split_rows_kernel(const float* __restrict__ x, int64_t ld, uint16_t* __restrict__ planes, int64_t plane, float* __restrict__ inv_out,
-                                                         float* __restrict__ amax_out, float* __restrict__ bound, int64_t M, int K) {
-    __shared__ float red[8];
-    grid_dep_launch();
-    grid_dep_wait();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int64_t r = blockIdx.x; r < M; r += gridDim.x) {
-        const float* xr = x + r * ld;
-        uint16_t* hr = planes + r * K;
-        const bool vec = (reinterpret_cast<uintptr_t>(xr) & 15) == 0;
-        auto load = [&](int k) {
-            return vec ? *reinterpret_cast<const float4*>(xr + k) : make_float4(xr[k], xr[k + 1], xr[k + 2], xr[k + 3]);
-        };
-        if (MODE == 1) {
-            for (int k = threadIdx.x * 4; k < K; k += 512) {
-                const float4 v = load(k);
-                *reinterpret_cast<uint2*>(hr + k) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
-            }
-            continue;
-        }
-        float m = 0.f, l1 = 0.f;
-        for (int k = threadIdx.x * 4; k < K; k += 512) {
-            const float4 v = load(k);
-            m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-            l1 += (fabsf(v.x) + fabsf(v.y)) + (fabsf(v.z) + fabsf(v.w));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            l1 += __shfl_xor_sync(0xffffffffu, l1, o);
-        }
-        __syncthreads();
-        if (lane == 0) { red[warp] = m; red[4 + warp] = l1; }
-        __syncthreads();
-        m = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
-        float scale, inv;
-        split_scale(m, scale, inv);
-        if (threadIdx.x == 0) {
-            inv_out[r] = inv;
-            if (amax_out) amax_out[r] = m;
-            if (bound) atomicMax(reinterpret_cast<int*>(bound), __float_as_int((red[4] + red[5] + red[6] + red[7]) * 1.0001f));   // non-negative floats order like ints
-        }
-        for (int k = threadIdx.x * 4; k < K; k += 512) {
-            uint2 hi, lo;
-            split_f16x4(load(k), scale, hi, lo);
-            *reinterpret_cast<uint2*>(hr + k) = hi;
-            *reinterpret_cast<uint2*>(hr + plane + k) = lo;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256) bias_bound_kernel(const float* __restrict__ b, int64_t n, float* __restrict__ bound) {
-    float m = 0.f;
-    if (b != nullptr)
-        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) m = fmaxf(m, fabsf(b[i]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(bound + 1), __float_as_int(m));
-}
-
 // ---- host side -------------------------------------------------------------------------------------
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            return reinterpret_cast<EncodeTiledFn>(p);
-        return EncodeTiledFn(nullptr);
-    }();
-    return fn;
-}
 // [planes][rows][cols] 16-bit elements, `ld` elements between rows and `plane` between planes; box = 64 columns x box_rows x all planes
 int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int64_t plane, int planes, int box_rows) {
-    EncodeTiledFn fn = encode_fn();
+    const auto fn = encode_tiled_fn();
     FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
     cuuint64_t dims[3] = {cuuint64_t(cols), cuuint64_t(rows), cuuint64_t(planes)};
     cuuint64_t strides[2] = {cuuint64_t(ld) * 2, cuuint64_t(planes > 1 ? plane : rows * ld) * 2};
@@ -1040,7 +956,7 @@ int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int
 
 // the result as the epilogue stores it: boxes of 32 rows x 16 columns, fp32 (64-byte rows) or split form (32-byte rows, all planes)
 int make_out_map(CUtensorMap* map, const F16GemmArgs& a, int planes) {
-    EncodeTiledFn fn = encode_fn();
+    const auto fn = encode_tiled_fn();
     FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
     const bool split = a.split_out.planes != nullptr;
     const cuuint64_t esz = split ? 2 : 4, pitch = cuuint64_t(split ? a.N : a.ldo) * esz;
@@ -1132,24 +1048,6 @@ bool gemm_f16_shape_ok(int64_t M, int64_t N, int64_t K) {
 }
 
 int gemm_f16_split_parts(int64_t N) { return int((N + 31) / 32) * 2; }
-
-int launch_split_rows(const float* x, int64_t ld, int64_t M, int64_t K, bool bf16, const SplitOut& out, float* bound, ExecCtx& ctx) {
-    if (M == 0) return 0;
-    FXF_CHECK(K % 8 == 0 && out.planes != nullptr, "split rows: K must be a multiple of 8");
-    const int grid = int(std::min<int64_t>(M, int64_t(ctx.sm_count) * 16));
-    tag_launch(ctx, bf16 ? "split_rows_bf16" : "split_rows_f16", 0, (bf16 ? 6.0 : 8.0) * double(M) * double(K));
-    if (bf16) FXF_CUDA(launch_dependent(split_rows_kernel<1>, dim3(grid), dim3(128), 0, ctx.stream, 1, x, ld, out.planes, out.plane, out.inv, out.amax, bound, M, int(K)));
-    else FXF_CUDA(launch_dependent(split_rows_kernel<0>, dim3(grid), dim3(128), 0, ctx.stream, 1, x, ld, out.planes, out.plane, out.inv, out.amax, bound, M, int(K)));
-    FXF_LAUNCHED(ctx);
-    return 0;
-}
-
-int launch_bias_bound(const float* bias, int64_t n, float* bound, ExecCtx& ctx) {
-    tag_launch(ctx, "bias_bound", 0, 4.0 * double(n));
-    bias_bound_kernel<<<1, 256, 0, ctx.stream>>>(bias, n, bound);
-    FXF_LAUNCHED(ctx);
-    return 0;
-}
 
 // The variant with the least modelled time.  Wide pair tiles win once they fill the machine; smaller problems take narrower
 // tiles until every SM has one.

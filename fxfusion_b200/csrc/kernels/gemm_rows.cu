@@ -56,7 +56,6 @@ struct RowsParams {
     int* status;
 };
 
-__device__ __forceinline__ float relu_keep_nan(float v) { return v > 0.f ? v : (v != v ? v : 0.f); }
 __device__ __forceinline__ uint32_t cluster_nctarank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
@@ -122,10 +121,18 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, RowsParams p) {
     // constants of this thread's output column (shares start at multiples of 4 elements, not of 128)
     const int nt = (own0 + threadIdx.x) & (BN - 1);
     const bool n_ok = n0 + nt < p.N;
-    const float wi = n_ok ? __ldg(p.w_inv + n0 + nt) : 0.f, bi = (n_ok && p.bias) ? __ldg(p.bias + n0 + nt) : 0.f;
+    float wi = 0.f, bi = 0.f;
+    auto column_constants = [&]() {
+        if (n_ok) wi = p.w_inv[n0 + nt];
+        if (n_ok && p.bias) bi = p.bias[n0 + nt];
+    };
+    if (p.early_w) column_constants();
     grid_dep_wait();
-    if (producer && !p.early_w)
-        for (; loaded < min(STAGES, count); loaded++) load_w(loaded);
+    if (!p.early_w) {   // the weight's conversion may be the kernel before this one
+        column_constants();
+        if (producer)
+            for (; loaded < min(STAGES, count); loaded++) load_w(loaded);
+    }
 
     float sum[COLS];
 #pragma unroll
@@ -282,15 +289,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, RowsParams p) {
 }
 
 int make_weight_map(CUtensorMap* map, const SplitMat& w, int64_t rows, int64_t cols) {
-    using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                       const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            return reinterpret_cast<EncodeTiledFn>(p);
-        return EncodeTiledFn(nullptr);
-    }();
+    const auto fn = encode_tiled_fn();
     FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
     cuuint64_t dims[3] = {cuuint64_t(cols), cuuint64_t(rows), 2};
     cuuint64_t strides[2] = {cuuint64_t(cols) * 2, cuuint64_t(w.plane) * 2};

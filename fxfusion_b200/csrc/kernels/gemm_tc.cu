@@ -973,24 +973,9 @@ TailSplit plan_tail(int64_t tiles, int64_t K, int bn, int sms, bool allowed) {
 }
 
 // ---- host side -------------------------------------------------------------------------------------
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    });
-    return fn;
-}
-
 // 2-D fp32 row-major [rows, cols] with row pitch `ld` floats; box = [box_rows, bk floats], rows one swizzle span wide.
 int make_map(CUtensorMap* map, const float* base, int64_t rows, int64_t cols, int64_t ld, int box_rows, int bk) {
-    EncodeTiledFn fn = encode_tiled_fn();
+    const auto fn = encode_tiled_fn();
     FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
     cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
     cuuint64_t strides[1] = {cuuint64_t(ld) * sizeof(float)};
@@ -1005,7 +990,7 @@ int make_map(CUtensorMap* map, const float* base, int64_t rows, int64_t cols, in
 
 // bf16 weight matrix [rows, cols] (row pitch `ld` elements): box [box_rows, bk], rows of bk * 2 bytes = one swizzle span
 int make_map_bf16(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows, int bk) {
-    EncodeTiledFn fn = encode_tiled_fn();
+    const auto fn = encode_tiled_fn();
     FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
     cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
     cuuint64_t strides[1] = {cuuint64_t(ld) * 2};
@@ -1021,7 +1006,7 @@ int make_map_bf16(CUtensorMap* map, const void* base, int64_t rows, int64_t cols
 // channels-last activation [N,H,W,C] as a 4-D map; box = [BNI, BH, BW, bk channels], 64-byte swizzle (bk = 16).
 // With a traversal stride s the box extent is given in input pixels (BW * s) and ceil(extent / s) = BW are loaded.
 int make_map_nhwc(CUtensorMap* map, const float* base, int N, int H, int W, int C, int bni, int bh, int bw, int bk, int sh, int sw) {
-    EncodeTiledFn fn = encode_tiled_fn();
+    const auto fn = encode_tiled_fn();
     FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
     cuuint64_t dims[4] = {cuuint64_t(C), cuuint64_t(W), cuuint64_t(H), cuuint64_t(N)};
     cuuint64_t strides[3] = {cuuint64_t(C) * 4, cuuint64_t(W) * C * 4, cuuint64_t(H) * W * C * 4};

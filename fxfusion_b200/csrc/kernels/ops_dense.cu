@@ -105,6 +105,7 @@ struct Slice {
     SplitMat mat;                   // likewise
     int64_t rows() const { return nrow[0] + nrow[1] + nrow[2]; }
     int64_t elems() const { return rows() * ncol; }
+    static float* l1(float* bound) { return bound + 64; }   // the L1 norms of the rows lie behind the bound
 };
 
 struct DensePlan : NodePlan {
@@ -129,7 +130,7 @@ struct DensePlan : NodePlan {
         x.f16 = true;
         x.bf16 = as_bf16;
         x.off_split = persist_bytes;
-        persist_bytes += round_up(size_t(x.elems()) * (as_bf16 ? 2 : 4), 256) + round_up(size_t(x.rows()) * 4, 256) + 256;
+        persist_bytes += round_up(size_t(x.elems()) * (as_bf16 ? 2 : 4), 256) + (as_bf16 ? 1 : 2) * round_up(size_t(x.rows()) * 4, 256) + 256;   // planes, scales, L1 norms, bound
     }
     void reserve(Slice& x, bool want_split) {
         if (x.drop) return;
@@ -172,8 +173,7 @@ struct DensePlan : NodePlan {
                 o.plane = x.elems();
                 o.inv = reinterpret_cast<float*>(base + round_up(size_t(x.elems()) * (x.bf16 ? 2 : 4), 256));
                 float* bound = reinterpret_cast<float*>(reinterpret_cast<char*>(o.inv) + round_up(size_t(x.rows()) * 4, 256));
-                FXF_CUDA(cudaMemsetAsync(bound, 0, 2 * sizeof(float), ctx.stream));
-                if (launch_split_rows(x.ptr, x.ncol, x.rows(), x.ncol, x.bf16, o, bound, ctx)) return 1;
+                if (launch_split_rows(x.ptr, x.ncol, x.rows(), x.ncol, x.bf16, o, x.bf16 ? nullptr : x.l1(bound), ctx)) return 1;
                 x.mat = SplitMat{};
                 x.mat.planes = o.planes; x.mat.plane = o.plane; x.mat.inv = o.inv; x.mat.bound = bound;
             }
@@ -196,7 +196,10 @@ struct DensePlan : NodePlan {
             }
         }
         for (int i = 0; i + 1 < n; i++)   // a weight's bias follows it
-            if (s[i].f16 && !s[i].bf16 && s[i + 1].ncol == 1 && !s[i + 1].drop && launch_bias_bound(s[i + 1].ptr, s[i + 1].rows(), const_cast<float*>(s[i].mat.bound), ctx)) return 1;
+            if (s[i].f16 && !s[i].bf16) {
+                float* bound = const_cast<float*>(s[i].mat.bound);
+                if (launch_weight_bound(s[i].l1(bound), s[i].rows(), s[i + 1].drop ? nullptr : s[i + 1].ptr, s[i + 1].rows(), bound, ctx)) return 1;
+            }
         prepared = true;
         return 0;
     }

@@ -100,6 +100,13 @@ __device__ __forceinline__ void grid_dep() {   // first statement of a kernel wi
     grid_dep_wait();
 }
 
+__device__ __forceinline__ float max_keep_nan(float v, float floor_at) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "f"(floor_at));
+    return r;
+}
+__device__ __forceinline__ float relu_keep_nan(float v) { return max_keep_nan(v, 0.f); }
+
 // ---- split form of an fp32 row: two fp16 planes of x * scale, scale a power of two ------------------------------------
 // scale = the power of two that brings `bound` into [2^14, 2^15]; inv = 1 / scale.  Bounds below 2^-99 count as 2^-99.
 __device__ __forceinline__ void split_scale(float bound, float& scale, float& inv) {
@@ -400,6 +407,17 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// ---- host side: the driver's tensor-map encoder (NULL: not available) ---------------------------------------------------
+inline auto encode_tiled_fn() {
+    static const auto fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+        return ok ? reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(p) : nullptr;
+    }();
+    return fn;
+}
 
 }  // namespace sm100
 }  // namespace fxf

@@ -402,13 +402,14 @@ F16Plan gemm_f16_plan(int64_t M, int64_t N, int64_t K, F16Form form, const F16Li
 constexpr size_t kSplitTileBytes = size_t(128) * 256 * sizeof(float);
 constexpr int kSplitFlagsPerSm = 16;
 int gemm_f16_split_parts(int64_t N);    // partial maxima per row a split output of N columns needs room for
-int launch_split_rows(const float* x, int64_t ld, int64_t M, int64_t K, bool bf16, const SplitOut& out, float* bound, ExecCtx& ctx);
+// kernels/split_form.cu.  l1_out (weights): the L1 norm of each row; bound = {largest of them, largest |bias|} (SplitMat::bound).
+int launch_split_rows(const float* x, int64_t ld, int64_t M, int64_t K, bool bf16, const SplitOut& out, float* l1_out, ExecCtx& ctx);
+int launch_weight_bound(const float* l1, int64_t rows, const float* bias, int64_t n, float* bound, ExecCtx& ctx);
 // M <= 64 rows (kernels/gemm_rows.cu): x as fp32 rows, or NULL with a.x in split form; no split output, no transposed columns
 bool gemm_rows_ok(int64_t M, int64_t N, int64_t K);
 int launch_gemm_rows(const F16GemmArgs& a, const float* x, int64_t ldx, ExecCtx& ctx);
 bool gemm_rows_streams(int64_t M, int64_t N, int sm_count);   // launch_gemm_f16_swapped (x in split form) is the better one
 int launch_gemm_f16_swapped(const F16GemmArgs& a, ExecCtx& ctx);
-int launch_bias_bound(const float* bias, int64_t n, float* bound, ExecCtx& ctx);
 
 // Launch as a programmatic dependent of the kernel before it in the stream (the kernel calls griddepcontrol.wait before it
 // touches anything another kernel of the stream writes or reads).
