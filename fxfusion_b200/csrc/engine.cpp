@@ -310,6 +310,7 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
     env.tp_rank = e->opts.tp_rank;
     env.tp_size = e->opts.tp_size;
     env.tc_pairs = e->opts.tc_pair != 1;
+    cudaDeviceGetAttribute(&env.sm_count, cudaDevAttrMultiProcessorCount, e->device);
     for (uint32_t i = 0; i < n_nodes; i++) {
         fbs::Table nt = g.table_at(fbs::GraphF::nodes, i);
         int op = nt.scalar<int8_t>(fbs::NodeF::op_code, 0);
@@ -440,8 +441,7 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
     cursor += kAlign;
     if (e->opts.gemm_mode != FXF_GEMM_FP32_SIMT) {
         // K-split workspace of the tensor-core GEMM
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
+        const int sms = env.sm_count;
         e->gemm_ws_off = cursor;
         e->gemm_ws_bytes = round_up(size_t(sms) * kSplitTileBytes, kAlign);
         cursor += e->gemm_ws_bytes;

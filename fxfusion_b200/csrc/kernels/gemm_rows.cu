@@ -3,7 +3,7 @@
 //
 // These products are weight reads: single-position decode steps, batch-sized MLP layers, the last-row vocabulary projection.
 // The operands are swapped — a tile is 128 WEIGHT rows by all rows of x — so no tensor time goes into padding rows, and one
-// tile's K range is cut over a cluster of up to 8 CTAs, so that a 512-row weight already occupies 32 SMs.  Per CTA:
+// tile's K range is cut over a cluster of up to 16 CTAs (pick_cluster), so that a 512-row weight already occupies 32 SMs.  Per CTA:
 //   * weight slabs (128 rows x 64, both planes, 32 KB) by TMA.  They do not depend on the kernel before this one, so the first
 //     STAGES slabs are requested before griddepcontrol.wait: the weight stream runs under the previous kernel;
 //   * x comes as fp32 (or in split form): all warps fetch this CTA's K range of the rows, take the maximum of each row over
@@ -18,6 +18,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "../runtime.hpp"
 #include "sm100.cuh"
@@ -301,21 +302,85 @@ int make_weight_map(CUtensorMap* map, const SplitMat& w, int64_t rows, int64_t c
     return 0;
 }
 
+// The instances: rows of x per CTA, K-slabs per CTA that fit without refilling the rings, CTAs per SM (two slabs take 70-100 KB of
+// shared memory: two CTAs share an SM, or one stands beside one of the kernel before it).
+using RowsKernel = void (*)(const CUtensorMap, RowsParams);
+struct RowsInstance { int index, rows, slabs, per_sm; RowsKernel kernel; size_t smem; };
 template <int NB, int STAGES, int XS>
-int launch_rows(const CUtensorMap& map, const RowsParams& p, int tiles, int cs, ExecCtx& ctx) {
-    const size_t smem = sizeof(RowsSmem<NB, STAGES, XS>) + 1024;
+RowsInstance instance(int index) {
     static_assert(sizeof(RowsSmem<NB, STAGES, XS>) + 1024 <= 227 * 1024, "shared memory of a CTA");
-    auto kernel = gemm_rows_kernel<NB, STAGES, XS>;
-    static bool configured[64] = {};
+    return {index, NB, XS, STAGES <= 2 ? 2 : 1, gemm_rows_kernel<NB, STAGES, XS>, sizeof(RowsSmem<NB, STAGES, XS>) + 1024};
+}
+const RowsInstance& instance_for(int64_t M, int per) {
+    static const RowsInstance all[] = {instance<16, 2, 2>(0), instance<16, 4, 8>(1), instance<32, 2, 2>(2), instance<32, 4, 4>(3), instance<32, 4, 8>(4)};
+    return all[M <= 16 ? (per <= 2 ? 0 : 1) : (per <= 2 ? 2 : (per <= 4 ? 3 : 4))];
+}
+int configure(const RowsInstance& r) {
+    static std::atomic<unsigned> done[64];   // a bit per instance
     int dev = 0;
     FXF_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        FXF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        FXF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        if (dev >= 0 && dev < 64) configured[dev] = true;
+    if (dev >= 0 && dev < 64 && (done[dev].load(std::memory_order_relaxed) >> r.index & 1u)) return 0;
+    FXF_CUDA(cudaFuncSetAttribute(r.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(r.smem)));
+    FXF_CUDA(cudaFuncSetAttribute(r.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (dev >= 0 && dev < 64) done[dev].fetch_or(1u << r.index, std::memory_order_relaxed);
+    return 0;
+}
+
+// Clusters of `cs` CTAs, one CTA per SM, that the device holds at once.  A cluster lives inside one GPC, so this is not the number of
+// SMs over cs, and differs between devices of the same kind.  Asked once per device: the answer does not change.  (148 SMs here:
+// 33 clusters of 4, 22 of 6, 15 of 8, 7 of 11 to 16.)
+int clusters_resident(int cs, int* out) {
+    static std::atomic<int> known[64][kMaxCluster + 1];   // answer + 1
+    int dev = 0;
+    FXF_CUDA(cudaGetDevice(&dev));
+    std::atomic<int>* slot = dev >= 0 && dev < 64 ? &known[dev][cs] : nullptr;
+    *out = slot != nullptr ? slot->load(std::memory_order_relaxed) - 1 : -1;
+    if (*out >= 0) return 0;
+    const RowsInstance& r = instance_for(1, kMaxCluster);   // one CTA per SM
+    if (configure(r)) return 1;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(cs);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(unsigned(cs));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = r.smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FXF_CUDA(cudaOccupancyMaxActiveClusters(out, r.kernel, &cfg));
+    if (slot != nullptr) slot->store(*out + 1, std::memory_order_relaxed);
+    return 0;
+}
+
+// CTAs per tile: the least modelled time over all cluster sizes.  In a chain of launches with weights from HBM a K-slab of a CTA takes
+// 0.27 us for one row and 0.9 us for 32; clusters that do not fit the device at once form another wave of 4 us and its slabs; and
+// the fuller the device, the less of the next kernel can start beside this one, up to 1.6 us.  Fitted to 511 shapes on 148 SMs (1 to
+// 64 rows, 1 to 140 tiles, K = 200 to 6144, chains of 16): 0.5 % above the best measured size on average, and 16 % below the rule
+// before it (up to 8 CTAs; 16 for at most 6 tiles), whose choice was the better one by at most 12 %.  Some of them, us per launch
+// of 32 rows:
+//   N =  768, K = 1536:  8 CTAs 6.2, 12 5.8      N = 2048, K = 1536:  8 12.7 (16 clusters; the device holds 15), 6 7.8, 12 7.4
+//   N = 1024, K = 2048:  8 CTAs 7.1, 16 6.4      N = 2304, K =  768:  6  6.7, 4 7.4, 12 10.9
+int pick_cluster(int64_t M, int tiles, int slabs, int* cs_out) {
+    double best = 0;
+    *cs_out = 0;
+    for (int cs = 1; cs <= std::min(kMaxCluster, slabs); cs++) {
+        const int per = (slabs + cs - 1) / cs;
+        if ((slabs + per - 1) / per != cs) continue;   // no more CTAs than give the fewest slabs
+        const RowsInstance& inst = instance_for(M, per);
+        int resident = 0;
+        if (clusters_resident(cs, &resident)) return 1;
+        resident *= inst.per_sm;
+        if (resident < 1) continue;
+        const int64_t clusters = int64_t(tiles) * ((M + inst.rows - 1) / inst.rows);
+        const double fill = std::min(1.0, double(clusters) / resident), slab = 0.25 + 0.02 * double(std::min<int64_t>(M, 32));
+        const double us = double((clusters + resident - 1) / resident) * (slab * per + 4.0) + 1.6 * fill;
+        if (*cs_out == 0 || us < best) {
+            *cs_out = cs;
+            best = us;
+        }
     }
-    FXF_CUDA(launch_dependent(kernel, dim3(unsigned(tiles * cs), unsigned((p.M + NB - 1) / NB)), dim3(kThreads), smem, ctx.stream, cs, map, p));
-    FXF_LAUNCHED(ctx);
+    FXF_CHECK(*cs_out > 0, "few-row GEMM: no cluster size fits the device");
     return 0;
 }
 
@@ -345,18 +410,15 @@ int launch_gemm_rows(const F16GemmArgs& a, const float* x, int64_t ldx, ExecCtx&
     p.early_w = ctx.weights_settled ? 1 : 0;
     p.status = ctx.status;
     const int tiles = int((a.N + BN - 1) / BN);
-    // As many CTAs per tile as leave every SM at most two, up to 8 (a portable cluster); no more than give the fewest slabs.  A
-    // deep product with few tiles goes to clusters of 16 (32 x 768 x 3072: 7.4 -> 6.3 us); with more tiles they no longer find
-    // room beside the kernel before (32 x 3072 x 768: 6.9 -> 10.6 us).
-    int cs = std::max(1, std::min(std::min(8, p.slabs), 2 * ctx.sm_count / tiles));
-    if ((p.slabs + cs - 1) / cs > 2 && tiles * 16 * 3 <= ctx.sm_count * 2) cs = std::min(16, p.slabs);
-    const int per = (p.slabs + cs - 1) / cs;
-    cs = (p.slabs + per - 1) / per;
+    int cs = 0;
+    if (pick_cluster(a.M, tiles, p.slabs, &cs)) return 1;
+    const RowsInstance& inst = instance_for(a.M, (p.slabs + cs - 1) / cs);
+    if (configure(inst)) return 1;
     tag_launch(ctx, "gemm_f16x3_rows_tcgen05", 2.0 * double(a.M) * double(a.N) * double(a.K),
                4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.N) + double(a.M) * a.N));
-    // two slabs per CTA: 70-100 KB of shared memory, so that this kernel's CTAs fit beside those of the kernel before it
-    if (a.M <= 16) return per <= 2 ? launch_rows<16, 2, 2>(map, p, tiles, cs, ctx) : launch_rows<16, 4, 8>(map, p, tiles, cs, ctx);
-    return per <= 2 ? launch_rows<32, 2, 2>(map, p, tiles, cs, ctx) : (per <= 4 ? launch_rows<32, 4, 4>(map, p, tiles, cs, ctx) : launch_rows<32, 4, 8>(map, p, tiles, cs, ctx));
+    FXF_CUDA(launch_dependent(inst.kernel, dim3(unsigned(tiles * cs), unsigned((a.M + inst.rows - 1) / inst.rows)), dim3(kThreads), inst.smem, ctx.stream, cs, map, p));
+    FXF_LAUNCHED(ctx);
+    return 0;
 }
 
 }  // namespace fxf

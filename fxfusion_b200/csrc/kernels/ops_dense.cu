@@ -225,13 +225,13 @@ void reserve_weight(DensePlan& p, Slice& w, const TensorIds& in, const PlanEnv& 
 }
 // Whether a product wants its activation in split form from the producer: the tiled kernel and the streaming few-row kernel
 // load it so; the cluster kernel of gemm_rows.cu takes fp32 rows and splits its own K range.
-bool takes_split_rows(int64_t M, int64_t N) { return M > kFewRows || gemm_rows_streams(M, N, 148); }
+bool takes_split_rows(const PlanEnv& env, int64_t M, int64_t N) { return M > kFewRows || gemm_rows_streams(M, N, env.sm_count); }
 std::string variant_of(const PlanEnv& env, const Slice& w, int64_t M, int64_t N, int64_t K) {
     GemmArgs g;
     g.M = M; g.N = N; g.K = K;
-    std::string v = gemm_variant_name(g, w.f16 || w.split ? env.gemm_mode : FXF_GEMM_FP32_SIMT, 148, env.tc_pairs);
+    std::string v = gemm_variant_name(g, w.f16 || w.split ? env.gemm_mode : FXF_GEMM_FP32_SIMT, env.sm_count, env.tc_pairs);
     if (!w.f16) return v;
-    return v + " (split operands: tcgen05-" + (M > kFewRows ? gemm_f16_variant_name(M, N, K, w.bf16, 148) : std::string(takes_split_rows(M, N) ? "f16x3-stream128" : "f16x3-rows128")) + ")";
+    return v + " (split operands: tcgen05-" + (M > kFewRows ? gemm_f16_variant_name(M, N, K, w.bf16, env.sm_count) : std::string(takes_split_rows(env, M, N) ? "f16x3-stream128" : "f16x3-rows128")) + ")";
 }
 
 // Room for an activation matrix that has to be split before its product: planes, scales, row maxima.
@@ -361,7 +361,7 @@ std::unique_ptr<NodePlan> plan_linear(const Registry& reg, const TensorIds& in, 
     p->reserve(bs, false);
     p->M = M;
     if (ws.f16) {
-        p->takes_split = takes_split_rows(M, N) ? 1 : 0;
+        p->takes_split = takes_split_rows(env, M, N) ? 1 : 0;
         p->makes_split = N % 8 == 0 && M > kFewRows;
         p->split_rows = M; p->split_cols = N;
         p->scratch_bytes = split_area_bytes(M, K);
@@ -491,7 +491,7 @@ std::unique_ptr<NodePlan> plan_feedforward(const Registry& reg, const TensorIds&
     p->M = M;
     p->scratch_bytes = size_t(M) * size_t(Fl) * sizeof(float);
     if (s_w1.f16 || s_w2.f16) p->scratch_bytes = ff_f16_bytes(M, std::max(K, Fl), Fl);
-    if (s_w1.f16) p->takes_split = takes_split_rows(M, Fl) ? 1 : 0;
+    if (s_w1.f16) p->takes_split = takes_split_rows(env, M, Fl) ? 1 : 0;
     p->flops = 2.0 * double(M) * double(Fl) * double(K) + 2.0 * double(M) * double(P) * double(Fl);
     p->bytes = 4.0 * (double(M) * K + double(Fl) * K + Fl + double(P) * Fl + P + double(M) * P);
     p->variant += variant_of(env, s_w1, M, Fl, K) + "+" + variant_of(env, s_w2, M, P, Fl);
@@ -646,7 +646,7 @@ std::unique_ptr<NodePlan> plan_mha(const Registry& reg, const TensorIds& in, con
     pl->M = M;
     pl->scratch_bytes = size_t(M) * size_t(3 * Dl + Dl) * sizeof(float);
     if (s_wq.f16 || s_wo.f16) pl->scratch_bytes += split_area_bytes(M, D);
-    if (s_wq.f16) pl->takes_split = takes_split_rows(M, 3 * Dl) ? 1 : 0;
+    if (s_wq.f16) pl->takes_split = takes_split_rows(env, M, 3 * Dl) ? 1 : 0;
     const bool tc_attn = env.gemm_mode != FXF_GEMM_FP32_SIMT && hd == 64 && T >= 16 && T <= 4096 && Dl % 4 == 0;   // the tcgen05 kernel covers at most 32 blocks of 128 keys
     if (tc_attn) pl->scratch_bytes += attention_tc_scratch_bytes(B, T, Hl);
     pl->flops = 2.0 * M * double(3 * Dl) * D + 4.0 * double(B) * Hl * double(T) * T * hd + 2.0 * double(M) * D * Dl;
@@ -807,7 +807,7 @@ std::unique_ptr<NodePlan> plan_cross_mha(const Registry& reg, const TensorIds& i
     pl->M = Mq;
     pl->scratch_bytes = (size_t(Mq) * size_t(2 * Dl) + size_t(Mk) * size_t(2 * Dl)) * sizeof(float);
     if (s_wq.f16 || s_wkv.f16 || s_wo.f16) pl->scratch_bytes += split_area_bytes(std::max(Mq, Mk), D);
-    pl->takes_split = (s_wq.f16 && takes_split_rows(Mq, Dl) ? 1u : 0u) | (s_wkv.f16 && takes_split_rows(Mk, 2 * Dl) ? 2u : 0u);
+    pl->takes_split = (s_wq.f16 && takes_split_rows(env, Mq, Dl) ? 1u : 0u) | (s_wkv.f16 && takes_split_rows(env, Mk, 2 * Dl) ? 2u : 0u);
     const bool tc_attn = env.gemm_mode != FXF_GEMM_FP32_SIMT && hd == 64 && Tk >= 16 && Tk <= 4096 && Dl % 4 == 0;
     if (tc_attn) pl->scratch_bytes += attention_tc_scratch_bytes(B, Tk, Hl);
     pl->flops = 2.0 * double(Mq) * Dl * D + 2.0 * double(Mk) * 2 * Dl * D + 4.0 * double(B) * Hl * double(Tq) * Tk * hd + 2.0 * double(Mq) * D * Dl;
@@ -1076,7 +1076,7 @@ std::unique_ptr<NodePlan> plan_cached_mha(const Registry& reg, const TensorIds& 
     pl->reserve(s_bq, false);
     reserve_weight(*pl, s_wo, in, env, B, D, D);
     pl->reserve(s_bo, false);
-    if (s_wq.f16) pl->takes_split = takes_split_rows(B, QKV) ? 1 : 0;
+    if (s_wq.f16) pl->takes_split = takes_split_rows(env, B, QKV) ? 1 : 0;
     pl->cache_off = pl->persist_bytes;
     pl->persist_bytes += round_up(size_t(B) * size_t(T) * size_t(2 * D) * sizeof(float), 256);
     pl->M = B;

@@ -180,6 +180,7 @@ struct NodePlan {
 // What a plan builder needs to know about the engine it plans for.
 struct PlanEnv {
     int gemm_mode = FXF_GEMM_AUTO;
+    int sm_count = 148;               // of the device that will run the plan
     int tp_rank = 0, tp_size = 1;     // tensor-parallel position of this engine
     bool shard_output_cols = false;   // this node is the graph's final Linear and its columns are sharded over the ranks
     bool tc_pairs = true;             // the engine lets CTA pairs compute the widest GEMM tiles (reported in variant names)

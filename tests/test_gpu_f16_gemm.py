@@ -129,6 +129,12 @@ def test_few_rows(built_lib, tmp_path, M, N, K, variant):
     eng.close()
 
 
+# cluster sizes between the powers of two (K-slabs divided unevenly, several rounds of them), and grids of more than one wave
+@pytest.mark.parametrize("M,N,K", [(32, 2048, 3072), (20, 2944, 3080), (64, 2944, 1536), (3, 1500, 1536), (64, 896, 1000), (2, 8192, 704), (48, 4096, 4096)])
+def test_few_rows_of_any_cluster(built_lib, tmp_path, M, N, K):
+    test_few_rows(built_lib, tmp_path, M, N, K, "rows128")
+
+
 # channels-last images in split form: image borders inside a tile (14 x 14, 7 x 7), several images per tile, ragged channels,
 # asymmetric filters and padding, strides, dilation, a map of one pixel, and one image of many tiles
 @pytest.mark.parametrize("N,size,C,O,kh,kw,s,ph,pw,d", [
