@@ -9,7 +9,7 @@
 //   * x comes as fp32 (or in split form): all warps fetch this CTA's K range of the rows, take the maximum of each row over
 //     it, and write the two fp16 planes into swizzled shared memory.  The scale may differ between the CTAs of a cluster:
 //     their results are only added after it has been divided out;
-//   * MMAs of 128 x NB x 16; 64- to 128-deep chains in separate TMEM accumulators, added in fp32 registers;
+//   * MMAs of 128 x NB x 16; chains of one to three slabs in separate TMEM accumulators, added in fp32 registers;
 //   * every CTA owns a share of the tile: the others push their partial sums of it into its shared memory (one bulk copy each,
 //     counted on the owner's mbarrier), it adds them in rank order, applies scale, bias, residual and ReLU and stores rows of
 //     consecutive columns.  Pulling the partial tiles after a cluster barrier instead, with another barrier before the exit,
@@ -78,7 +78,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, RowsParams p) {
     Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr uint32_t kWBytes = 2 * BN * BK * 2;
     constexpr uint32_t kIdesc = umma_idesc_f16(BN, NB);
-    constexpr int NACC = kAccCols / NB, COLS = NB >= 32 ? NB / 2 : NB, EPI_WARPS = NB >= 32 ? 8 : 4;
+    // One accumulator for all corrections (hi·lo, lo·hi), the others for chains of hi·hi.  The tensor core truncates at every addition,
+    // and the large sums take one per 16 K-elements so instead of three: 32 x 768 x 3072 lies 1.6e-7 from fp64 instead of 2.7e-7
+    // (fp32 FFMA: 3.6e-7), at the same time.
+    constexpr int NACC = kAccCols / NB - 1, COLS = NB >= 32 ? NB / 2 : NB, EPI_WARPS = NB >= 32 ? 8 : 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cs = int(cluster_nctarank()), rank = int(cluster_ctarank());
     const int tile = blockIdx.x / cs, n0 = tile * BN;
@@ -199,13 +202,13 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, RowsParams p) {
                 if (leader) {
                     const uint64_t a = umma_desc_k_major_bytes<128>(smem_u32(s.w[st][0])), b = umma_desc_k_major_bytes<128>(smem_u32(s.x[i][0]));
                     constexpr uint64_t kALo = BN * BK * 2 / 16, kBLo = NB * BK * 2 / 16;
-                    const uint32_t acc = tmem + uint32_t(i % NACC) * NB;
+                    const uint32_t corr = tmem, acc = tmem + uint32_t(1 + i % NACC) * NB;
 #pragma unroll
                     for (int kk = 0; kk < BK / 16; kk++) {
                         const uint64_t adv = uint64_t((kk * 32) >> 4);
-                        umma_f16_ss<false>(acc, a + kALo + adv, b + adv, kIdesc, (i >= NACC || kk > 0) ? 1u : 0u);
-                        umma_f16_ss<false>(acc, a + adv, b + kBLo + adv, kIdesc, 1u);
-                        umma_f16_ss<false>(acc, a + adv, b + adv, kIdesc, 1u);
+                        umma_f16_ss<false>(corr, a + kALo + adv, b + adv, kIdesc, (i > 0 || kk > 0) ? 1u : 0u);
+                        umma_f16_ss<false>(corr, a + adv, b + kBLo + adv, kIdesc, 1u);
+                        umma_f16_ss<false>(acc, a + adv, b + adv, kIdesc, (i >= NACC || kk > 0) ? 1u : 0u);
                     }
                     umma_commit(&s.empty[st]);
                     if (i + 1 == ns) umma_commit(&s.done);
@@ -226,7 +229,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, RowsParams p) {
         if (!alive) give_up(abort_flag, p.status, kErrRowsDone);
         tc_fence_after();
         if (alive && warp < EPI_WARPS) {
-            const int nacc = min(ns, NACC);
+            const int nacc = 1 + min(ns, NACC);   // the corrections first
             for (int a = 0; a < nacc; a++) {
                 const uint32_t t = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(a * NB + mbase);
                 uint32_t d[COLS];

@@ -71,6 +71,24 @@ def test_rows_keep_their_precision_at_any_scale(built_lib, tmp_path):
     eng.close()
 
 
+# Distance from fp64 (2-norm).  Few rows: both factors to 22 bits and more with lo·lo dropped, 2^-23 together; and a running sum
+# that these shapes add to four times (one slab per accumulator), each time truncated by half an ulp, 2^-24, of a sum that is half of
+# the result on average, 2^-23.  The two are independent: sqrt(2) 2^-23.
+@pytest.mark.parametrize("M,N,K", [(1, 512, 512), (17, 640, 64), (32, 768, 768), (32, 768, 3072), (64, 1024, 256)])
+def test_distance_from_fp64(built_lib, tmp_path, M, N, K):
+    rng = np.random.default_rng(M + N + K)
+    w = _w(rng, N, K)
+    b = lowering.GraphBuilder(f"fp64_{M}_{N}_{K}")
+    x = b.input((M, K), wire.DT_F32)
+    b.output(b.op("Linear", [x, b.const(w), b.const(np.zeros(N, np.float32))], (M, N)))
+    _, eng = _engine(b, tmp_path)
+    xin = torch.randn(M, K, generator=torch.Generator().manual_seed(1))
+    want = xin.double() @ torch.from_numpy(w).double().T
+    got = eng.run([xin.cuda()])[0].cpu().double()
+    assert ((got - want).norm() / want.norm()).item() < 1.5 * 2.0 ** -23
+    eng.close()
+
+
 @pytest.mark.parametrize("M,D,F", [(65, 64, 256), (200, 768, 3072), (333, 136, 72)])
 @pytest.mark.parametrize("precision", ["auto", "bf16"])
 def test_activations_stay_in_split_form_between_nodes(built_lib, tmp_path, M, D, F, precision):
