@@ -974,7 +974,12 @@ int make_out_map(CUtensorMap* map, const F16GemmArgs& a, int planes) {
 // K-elements per accumulation chain.  Convolutions run 50 deep without normalisation: ResNet-50's logits lie 1.1e-5 from fp64 with
 // chains of 128 (5.7e-6 with 64; three TF32 products in chains of 64: 1.4e-5), and a chain of 64 drains at every slab
 // (128 images of 56 x 56, 64 channels, 3x3: 136 against 114 us).
-constexpr int kChunkKDense = 1024, kChunkKConv = 128, kChunkKRows = 256;
+// Tiles of up to 128 columns drain 32 or 64 sums per thread: chains of 256 cost them little (985 rows, 12 layers of 768: 1421 us with
+// either) except where K = 512 was one chain (1500 x 512 x 512, 16 layers: 121.4 -> 124.8 us), and the tensor core truncates at
+// every addition: those 16 layers lie 3.9e-7 from fp64 instead of 8.3e-7 (one TF32 product + two bf16 corrections: 6.9e-7).  Wide
+// tiles hold 96 or 128 sums and serve products whose error the other arithmetic of a transformer layer covers (8192 x 768 x 3072:
+// 3.6e-6; the TF32 arithmetic 5.0e-6).
+constexpr int kChunkKDense = 1024, kChunkKNarrow = 256, kChunkKConv = 128, kChunkKRows = 256;
 
 // Times in microseconds as measured on B200 inside a chain of launches: `slab` per 64-deep K-slab of a tile, `gap` what every
 // tile adds (its epilogue runs under the next tile's products), `drain` the exposed epilogue of the last one.
@@ -1081,7 +1086,7 @@ static F16Plan plan_launch(int64_t M, int64_t N, int64_t K, F16Form form, bool l
                              form == F16Form::kImages ? kImageVariants : (form == F16Form::kBf16 ? kBf16Variants : kVariants), &ts, &r.workers);
     if (r.variant < 0) return r;
     const Variant& var = kVariants[r.variant];
-    const int64_t chunk_k = lim.chunk_k > 0 ? lim.chunk_k : (form == F16Form::kImages ? kChunkKConv : kChunkKDense);
+    const int64_t chunk_k = lim.chunk_k > 0 ? lim.chunk_k : (form == F16Form::kImages ? kChunkKConv : (form == F16Form::kRows && var.bn <= 128 ? kChunkKNarrow : kChunkKDense));
     r.chunk_slabs = int(std::max<int64_t>(1, chunk_k / BK));
     r.epilogue_warps = r.variant == 0 && K <= int64_t(r.chunk_slabs) * BK && (form == F16Form::kImages || (form == F16Form::kBf16 && ts.parts == 1 && !lean)) ? 16 : 8;
     const int64_t ctas = ts.tail * ts.parts * (var.pair ? 2 : 1);
