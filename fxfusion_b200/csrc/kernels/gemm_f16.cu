@@ -978,8 +978,9 @@ int make_out_map(CUtensorMap* map, const F16GemmArgs& a, int planes) {
 // either) except where K = 512 was one chain (1500 x 512 x 512, 16 layers: 121.4 -> 124.8 us), and the tensor core truncates at
 // every addition: those 16 layers lie 3.9e-7 from fp64 instead of 8.3e-7 (one TF32 product + two bf16 corrections: 6.9e-7).  Wide
 // tiles hold 96 or 128 sums and serve products whose error the other arithmetic of a transformer layer covers (8192 x 768 x 3072:
-// 3.6e-6; the TF32 arithmetic 5.0e-6).
-constexpr int kChunkKDense = 1024, kChunkKNarrow = 256, kChunkKConv = 128, kChunkKRows = 256;
+// 3.6e-6; the TF32 arithmetic 5.0e-6).  Few rows against a streamed weight ran in fp32 FFMA before: chains of 128 leave GPT-2-small
+// over 40 positions 7.0e-7 from fp64 (1.1e-6 with 256; fp32 7.9e-7), at 628 instead of 624 us.
+constexpr int kChunkKDense = 1024, kChunkKNarrow = 256, kChunkKConv = 128, kChunkKRows = 128;
 
 // Times in microseconds as measured on B200 inside a chain of launches: `slab` per 64-deep K-slab of a tile, `gap` what every
 // tile adds (its epilogue runs under the next tile's products), `drain` the exposed epilogue of the last one.
