@@ -749,6 +749,9 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             }
             for (auto& n : e->nodes) {
                 if (n.op != FXF_OP_SIZE || n.folded || n.out.size() != 1 || !sole_tensor(n.out[0])) continue;
+                if (n.in.empty() || n.params.ints.empty() || e->reg[n.out[0]].dtype != FXF_I64) continue;   // (the kernel reports these)
+                const int rank = e->reg[n.in[0]].rank;
+                if (n.params.ints[0] < -rank || n.params.ints[0] >= rank) continue;
                 bool used = false;
                 for (auto& r : e->nodes)
                     for (auto id : r.in) used = used || (id == n.out[0] && r.view_of < 0);

@@ -394,3 +394,22 @@ def test_filters_that_are_not_constants(built_lib, tmp_path):
         assert ok, info
     assert eng.device_status() == 0
     eng.close()
+
+
+@pytest.mark.parametrize("dim,refused", [(1, False), (-2, False), (3, True), (-4, True)])
+def test_size_that_nothing_needs_is_still_checked(built_lib, tmp_path, dim, refused):
+    """A Size read only by the Narrow of a constant launches nothing, and is refused as before where its dimension does not exist."""
+    b = lowering.GraphBuilder(f"size_{dim}")
+    x = b.input((2, 5, 8), wire.DT_F32)
+    y = b.op("Relu", [x], (2, 5, 8))
+    size = b.op("Size", [y], (), wire.DT_I64, ints=[dim])
+    table = np.random.default_rng(0).standard_normal((1, 9, 8), dtype=np.float32)
+    b.output(b.op("Add", [y, b.op("Narrow", [b.const(table), size], (1, 5, 8), ints=[1, 0, -1])], (2, 5, 8)))
+    if refused:
+        with pytest.raises(RuntimeError, match="size: dim out of range"):
+            _engine(b, tmp_path)
+        return
+    graph, eng = _engine(b, tmp_path)
+    xin = torch.randn(2, 5, 8)
+    assert torch.equal(eng.run([xin.cuda()])[0].cpu(), GraphOracle(graph).run([xin])[0])
+    eng.close()
