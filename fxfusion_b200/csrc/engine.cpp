@@ -899,6 +899,8 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             if (escapes[t] || meta[t].kind != kActivation || producer[t] != int(pi) || n_readers[t] == 0 || !arena_range(t, &lo, &hi) || !on_16_bytes(t)) continue;
             const bool norm = P.op == FXF_OP_LAYER_NORM || P.op == FXF_OP_ADD_LAYER_NORM;   // (only its vector kernel writes split form)
             if (norm && !std::all_of(P.in.begin(), P.in.end(), on_16_bytes)) continue;
+            // fp32 rows may be normalised in place; the planes of one row lie where other rows still have to be read
+            if (std::any_of(P.in.begin(), P.in.end(), [&](uint32_t id) { return overlap(id, t); })) continue;
             if (numel(e->reg[P.out[0]]) != P.plan->split_rows * P.plan->split_cols || e->reg[P.out[0]].dtype != FXF_F32 || !is_contiguous(e->reg[P.out[0]])) continue;
             bool ok = true;
             for (size_t ri = 0; ri < e->nodes.size() && ok; ri++)

@@ -413,3 +413,30 @@ def test_size_that_nothing_needs_is_still_checked(built_lib, tmp_path, dim, refu
     xin = torch.randn(2, 5, 8)
     assert torch.equal(eng.run([xin.cuda()])[0].cpu(), GraphOracle(graph).run([xin])[0])
     eng.close()
+
+
+@pytest.mark.parametrize("op", ["LayerNorm", "AddLayerNorm"])
+def test_rows_normalised_in_place_stay_fp32(built_lib, tmp_path, op):
+    """A file may place a LayerNorm's result on its input.  Row by row that works in fp32; in split form the planes of a row would
+    cover rows that other blocks have not read yet."""
+    from fxfusion_b200.engine import ExecutionEngine
+    M, D = 3000, 128
+    rng = np.random.default_rng(5)
+    b = lowering.GraphBuilder(f"in_place_{op}")
+    x = b.op("Relu", [b.input((M, D), wire.DT_F32)], (M, D))
+    affine = [b.const(rng.standard_normal(D, dtype=np.float32)), b.const(rng.standard_normal(D, dtype=np.float32))]
+    ln = b.op(op, ([x] if op == "LayerNorm" else [x, b.input((M, D), wire.DT_F32)]) + affine, (M, D), ints=[1, D], floats=[1e-5])
+    b.output(b.op("Linear", [ln, b.const(_w(rng, 64, D)), b.const(np.zeros(64, np.float32))], (M, 64)))
+    graph = b.finish()
+    want_graph = graph.tensors[ln].offset
+    gen = torch.Generator().manual_seed(1)
+    xin = [torch.randn(M, D, generator=gen) for _ in range(1 if op == "LayerNorm" else 2)]
+    want = GraphOracle(graph).run(xin)[0]
+    graph.tensors[ln].offset = graph.tensors[x].offset
+    assert graph.tensors[ln].offset != want_graph
+    wire.dump(graph, tmp_path / "g.bin")
+    eng = ExecutionEngine(str(tmp_path / "g.bin"), "cuda:0")
+    assert "output in split form" not in eng.describe()
+    ok, info = compare_outputs(eng.run([t.cuda() for t in xin])[0].cpu(), want, atol=ATOL, rtol=RTOL)
+    assert ok, info
+    eng.close()
