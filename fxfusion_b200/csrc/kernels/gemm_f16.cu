@@ -934,6 +934,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     if (PAIR) cluster_sync_all();
     if (warp == kMmaWarp) {
         tc_fence_after();
+    let_copies_land(abort_flag);
         if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
         else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }

@@ -286,6 +286,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, RowsParams p) {
     tc_fence_before();
     if (cs > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     __syncthreads();
+    let_copies_land(abort_flag);
     if (warp == kMmaWarp) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kAccCols) : "memory");

@@ -76,6 +76,16 @@ __device__ __forceinline__ void give_up(volatile int* abort_flag, int* status, i
     }
 }
 
+// Teardown, behind the block's barrier.  A CTA that gave up may still have loads on their way into its shared memory, requested just
+// before another warp's wait ran out: they land within microseconds, and nobody leaves (or frees tensor memory) before.
+constexpr unsigned long long kLandingNs = 1000000ull;
+__device__ __forceinline__ void let_copies_land(volatile int* abort_flag) {
+    if (!*abort_flag) return;
+    const unsigned long long t0 = global_ns();
+    while (global_ns() - t0 < kLandingNs) __nanosleep(1000);
+    __syncwarp();
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar))
