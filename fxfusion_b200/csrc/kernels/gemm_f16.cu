@@ -975,13 +975,15 @@ int make_out_map(CUtensorMap* map, const F16GemmArgs& a, int planes) {
 // K-elements per accumulation chain.  Convolutions run 50 deep without normalisation: ResNet-50's logits lie 1.1e-5 from fp64 with
 // chains of 128 (5.7e-6 with 64; three TF32 products in chains of 64: 1.4e-5), and a chain of 64 drains at every slab
 // (128 images of 56 x 56, 64 channels, 3x3: 136 against 114 us).
-// Tiles of up to 128 columns drain 32 or 64 sums per thread: chains of 256 cost them little (985 rows, 12 layers of 768: 1421 us with
-// either) except where K = 512 was one chain (1500 x 512 x 512, 16 layers: 121.4 -> 124.8 us), and the tensor core truncates at
-// every addition: those 16 layers lie 3.9e-7 from fp64 instead of 8.3e-7 (one TF32 product + two bf16 corrections: 6.9e-7).  Wide
-// tiles hold 96 or 128 sums and serve products whose error the other arithmetic of a transformer layer covers (8192 x 768 x 3072:
-// 3.6e-6; the TF32 arithmetic 5.0e-6).  Few rows against a streamed weight ran in fp32 FFMA before: chains of 128 leave GPT-2-small
-// over 40 positions 7.0e-7 from fp64 (1.1e-6 with 256; fp32 7.9e-7), at 628 instead of 624 us.
-constexpr int kChunkKDense = 1024, kChunkKNarrow = 256, kChunkKConv = 128, kChunkKRows = 128;
+// The tensor core truncates at every addition, so chains bound the error.  Tiles of up to 64 columns drain 32 sums per thread at most:
+// chains of 256 cost them nothing (us per launch in a chain, 256 against 1024: 1800 x 512 x 512 8.75 and 8.98; 16 layers of an MLP over
+// 1500 rows 125 and 123), and those 16 layers lie 3.9e-7 from fp64 instead of 8.3e-7 (one TF32 product + two bf16 corrections:
+// 6.9e-7).  At 128 columns 512 is the shortest chain that costs little (8192 x 768 x 768 29.1 / 26.9 / 26.6 us with 256 / 512 / 1024,
+// 16384 x 1024 x 512 52.2 / 47.2 / 46.9; 14 layers of 1024 over 1565 rows 9.2e-7, 1.16e-6 with 1024, TF32 9.7e-7).  Wider tiles hold
+// 96 or 128 sums and serve products whose error the rest of a transformer layer covers (8192 x 768 x 3072: 3.6e-6; TF32 5.0e-6).
+// Few rows against a streamed weight ran in fp32 FFMA before: chains of 128 leave GPT-2-small over 40 positions 7.0e-7 from fp64
+// (1.1e-6 with 256; fp32 7.9e-7), at 628 instead of 624 us.
+constexpr int kChunkKDense = 1024, kChunkK128 = 512, kChunkKNarrow = 256, kChunkKConv = 128, kChunkKRows = 128;
 
 // Times in microseconds as measured on B200 inside a chain of launches: `slab` per 64-deep K-slab of a tile, `gap` what every
 // tile adds (its epilogue runs under the next tile's products), `drain` the exposed epilogue of the last one.
@@ -1088,7 +1090,7 @@ static F16Plan plan_launch(int64_t M, int64_t N, int64_t K, F16Form form, bool l
                              form == F16Form::kImages ? kImageVariants : (form == F16Form::kBf16 ? kBf16Variants : kVariants), &ts, &r.workers);
     if (r.variant < 0) return r;
     const Variant& var = kVariants[r.variant];
-    const int64_t chunk_k = lim.chunk_k > 0 ? lim.chunk_k : (form == F16Form::kImages ? kChunkKConv : (form == F16Form::kRows && var.bn <= 128 ? kChunkKNarrow : kChunkKDense));
+    const int64_t chunk_k = lim.chunk_k > 0 ? lim.chunk_k : (form == F16Form::kImages ? kChunkKConv : (form != F16Form::kRows || var.bn > 128 ? kChunkKDense : (var.bn > 64 ? kChunkK128 : kChunkKNarrow)));
     r.chunk_slabs = int(std::max<int64_t>(1, chunk_k / BK));
     r.epilogue_warps = r.variant == 0 && K <= int64_t(r.chunk_slabs) * BK && (form == F16Form::kImages || (form == F16Form::kBf16 && ts.parts == 1 && !lean)) ? 16 : 8;
     const int64_t ctas = ts.tail * ts.parts * (var.pair ? 2 : 1);
