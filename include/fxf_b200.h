@@ -60,13 +60,25 @@ typedef struct FxfTensor {
 
 /* GEMM arithmetic used by Linear / LinearRelu / FeedForward / MHA projections. */
 enum {
-    FXF_GEMM_AUTO = 0,      /* fp32-grade on the tensor cores where the shape allows it (FXF_GEMM_TF32_BF16X2 for dense layers
-                               whose K is a multiple of 8, FXF_GEMM_TF32X3 otherwise and for convolutions), else fp32 SIMT */
+    FXF_GEMM_AUTO = 0,      /* fp32-grade on the tensor cores where the shape allows it, else fp32 SIMT.  One GPU, constant
+                               weights, K >= 16 and K % 8 == 0, and convolutions between channels-last images: operands in
+                               split form, x * s = hi + lo as two fp16 planes with a power of two s per row (images: per
+                               image), and hi*hi + hi*lo + lo*hi as fp16 products with fp32 accumulation.  An element keeps 22
+                               bits down to 2^-17 of its row's bound, and an absolute error of at most 2^-39 of that bound
+                               below it; the bound is the row's largest magnitude, or for the result of a product max|x| *
+                               max ||w||_1 + max|b| (an image: over all its channels and pixels).  Ordinary networks do not
+                               notice; where columns of one row, or channels of one image, lie further apart than that and the
+                               next weights scale the small ones up again, take FXF_GEMM_TF32_BF16X2, FXF_GEMM_TF32X3 or
+                               FXF_GEMM_FP32_SIMT, which keep an exponent per element.  Tensor parallelism and the remaining
+                               shapes: FXF_GEMM_TF32_BF16X2 where K is a multiple of 8, FXF_GEMM_TF32X3 otherwise */
     FXF_GEMM_FP32_SIMT = 1, /* fp32 FFMA tiles only */
     FXF_GEMM_TF32X3 = 2,    /* tcgen05 kind::tf32 with hi/lo operand split (fp32-grade result) */
     FXF_GEMM_BF16 = 3,      /* optional reduced-precision mode: weights and activations rounded to bf16 for the tensor-core
-                               products (one product per logical product), fp32 accumulation and fp32 tensors everywhere
-                               else; results within about 1e-2 relative of the fp32 path, decode tokens may differ */
+                               products (one product per logical product; up to 64 rows they run as in FXF_GEMM_AUTO), fp32
+                               accumulation and fp32 tensors everywhere else; results within about 1e-2 relative of the fp32
+                               path, decode tokens may differ.  For convolutional networks FXF_GEMM_AUTO is the faster mode:
+                               this one still converts activations inside the product (ResNet-50 at batch 256 17.2 against
+                               9.4 ms, at batch 1 3.1 against 0.46 ms) */
     FXF_GEMM_TF32_BF16X2 = 4 /* fp32-grade like FXF_GEMM_TF32X3 (x = x_hi + x_lo, w = w_hi + w_lo): the main product
                                x_hi*w_hi in TF32, both correction products bf16(x_lo)*bf16(w_hi) and bf16(x)*bf16(w_lo) as
                                bf16 tensor-core products with fp32 accumulation.  The corrections are 2^-11 of a product, so
@@ -88,8 +100,10 @@ typedef struct FxfEngineOptions {
     int32_t p2p_end_budget_ms;     /* wait budget of its second peer barrier (0 = 2000) */
     int32_t p2p_grid;              /* blocks of the peer exchange kernels, 1..128 (0 = 128); must agree on all ranks */
     int32_t tc_chunk_k;            /* K-elements per tensor-core accumulation chain before the partial sums are added in fp32
-                                      by CUDA cores (0 = 1024 for dense layers, 64 for convolutions); larger = fewer
-                                      drains, more truncation bias per chain (about 4e-8 of the result's scale per element) */
+                                      by CUDA cores (0: dense layers 1024, on operands in split form 512 in tiles of 128 and
+                                      256 in tiles of fewer columns; convolutions 128 on images in split form, else 64; up to 64 rows the kernels keep
+                                      their own chains of 64 to 192); larger = fewer drains, more truncation bias per chain
+                                      (about 3e-9 of the result per element) */
     int32_t tc_pair;               /* 0: the widest tensor-core GEMM tiles (256 columns) are computed by pairs of CTAs
                                       (tcgen05 cta_group::2: 256-row tiles, each CTA stages half of the weight tile);
                                       1: never */
@@ -229,8 +243,9 @@ FXF_API int fxf_kernel_invoke(int op_code, const FxfTensor* reg, int n_reg,
                       const int64_t* ints, int n_ints, const float* floats, int n_floats,
                       void* scratch, int64_t scratch_bytes, int gemm_mode, void* stream);
 
-/* Name of the GEMM kernel variant the dispatch rule picks for out[M,N] = x[M,K] . w[N,K]^T in an engine with `sm_count`
- * SMs (0 = 148): "tcgen05-tf32x3-128x<width>-<where A is read from>", "tcgen05-bf16-...", or one of the fp32 FFMA
+/* Name of the kernel variant that serves out[M,N] = x[M,K] . w[N,K]^T in an engine with `sm_count` SMs (0 = 148) where its
+ * operands are not in split form (tensor parallelism, explicit arithmetic modes, weights that are not constants; what a
+ * node of an engine runs on stands in fxf_engine_describe): "tcgen05-tf32x3-128x<width>-<where A is read from>", "tcgen05-bf16-...", or one of the fp32 FFMA
  * kernels ("simt128x128", "simt64x64", "simt32x32", "skinny32x8").  Pure host code (no counterpart in the reference, whose
  * CUDA linear kernel has one 32x32 tile); tests use it to make sure every variant is exercised. */
 FXF_API int fxf_gemm_variant(int64_t M, int64_t N, int64_t K, int gemm_mode, int sm_count, char* out, size_t out_bytes);
@@ -262,8 +277,7 @@ FXF_API int fxf_decode_static(fxf_engine* e, int64_t* tokens_io, int initial_len
 /* The same loop and the same tokens, for a graph whose last node is the Linear that produces output 0
  * ([B,T,D] -> [B,T,V], the vocabulary projection): each step runs every node but that one, then evaluates
  * the projection only on row current_len-1 of each sequence — the only row the loop reads
- * (inference.py:38-40, `logits[:, current_len - 1, :]`) — into a [B,V] buffer inside the engine, in fp32
- * FFMA arithmetic.  Output 0 of the engine is NOT updated by this call; no counterpart in the reference,
+ * (inference.py:38-40, `logits[:, current_len - 1, :]`) — into a [B,V] buffer inside the engine.  Output 0 of the engine is NOT updated by this call; no counterpart in the reference,
  * whose loop always runs the whole graph.  fxf_engine_supports_last_row tells whether the graph qualifies. */
 FXF_API int fxf_engine_supports_last_row(const fxf_engine* e);
 /* Incremental ("KV cache") greedy decode, which the reference names as future work (README.md:183).  `e` runs a

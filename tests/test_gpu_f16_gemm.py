@@ -440,3 +440,48 @@ def test_rows_normalised_in_place_stay_fp32(built_lib, tmp_path, op):
     ok, info = compare_outputs(eng.run([t.cuda() for t in xin])[0].cpu(), want, atol=ATOL, rtol=RTOL)
     assert ok, info
     eng.close()
+
+
+@pytest.mark.parametrize("precision", ["auto", "fp32_tf32_bf16x2"])
+@pytest.mark.parametrize("form", ["rows", "few rows", "images"])
+def test_dynamic_range_inside_a_row_and_an_image(built_lib, tmp_path, form, precision):
+    """Columns of a row (channels of an image) from 1 down to 2^-44 of the largest, each scaled back up by the next product.  In split
+    form an element has 22 bits or an absolute error of 2^-39 of its row's (image's) bound, whichever is coarser, where the bound is
+    max|x| * max ||w||_1 + max|b|; the TF32 arithmetic keeps an exponent per element."""
+    C, size = 48, 16
+    rng = np.random.default_rng(9)
+    shrink = 2.0 ** -np.arange(C, dtype=np.float32)
+    shrink[shrink < 2.0 ** -44] = 2.0 ** -44
+    # weights of one sign on inputs that a ReLU made: no column is small by cancellation
+    w1 = (np.abs(rng.standard_normal((C, 64), dtype=np.float32)) * shrink[:, None]).astype(np.float32)
+    w2 = np.diag(1.0 / shrink).astype(np.float32)
+    zero = np.zeros(C, np.float32)
+    gen = torch.Generator().manual_seed(1)
+    b = lowering.GraphBuilder(f"range_{form.split()[0]}_{precision}")
+    if form == "images":
+        N, gb = 3, [1, 1, 1, 256, 1, 1]
+        x = b.input((N, 3, 2 * size, 2 * size), wire.DT_F32)
+        conv = lambda op, t, w, bias, k, s, p: b.op(op, [t, b.const(w), b.const(bias)], (N, w.shape[0], size, size), ints=[s, s, p, p, 1, 1, 1] + gb)
+        y = conv("Conv2dRelu", x, (rng.standard_normal((64, 3, 7, 7)) / 12).astype(np.float32), rng.standard_normal(64, dtype=np.float32), 7, 2, 3)
+        h = conv("Conv2dRelu", y, w1.reshape(C, 64, 1, 1), zero, 1, 1, 0)
+        out = conv("Conv2d", h, w2.reshape(C, C, 1, 1), zero, 1, 1, 0)
+        b.output(b.op("AvgPool2d", [out], (N, C, size, size), ints=[1, 1, 1, 1, 0, 0, 0] + gb))
+        xin = torch.randn(N, 3, 2 * size, 2 * size, generator=gen)
+    else:
+        M = 300 if form == "rows" else 40
+        x = b.input((M, 64), wire.DT_F32)
+        y = b.op("Relu", [x], (M, 64))
+        h = b.op("LinearRelu", [y, b.const(w1), b.const(zero)], (M, C))
+        b.output(b.op("Linear", [h, b.const(w2), b.const(zero)], (M, C)))
+        xin = torch.randn(M, 64, generator=gen)
+    graph, eng = _engine(b, tmp_path, precision=precision)
+    oracle = GraphOracle(graph)
+    want = oracle.run([xin])[0].double()
+    bound = oracle.reg[y].abs().max().item() * np.abs(w1).sum(1).max()
+    got = eng.run([xin.cuda()])[0].cpu().double()
+    dims = (0, 2, 3) if form == "images" else (0,)
+    err, top = (got - want).abs().amax(dim=dims), want.abs().amax(dim=dims)
+    lost = 2.0 ** -39 * bound / torch.from_numpy(shrink).double() if precision == "auto" else torch.zeros(C, dtype=torch.float64)
+    assert (err <= 4e-6 * top + lost).all(), (err / top, lost)
+    assert (err[:20] <= 4e-6 * top[:20]).all()   # to 2^-19 of the largest nothing shows
+    eng.close()
