@@ -5,7 +5,9 @@
 // Split form.  A row r of an fp32 matrix is stored as two fp16 planes and one power of two:
 //     x[r,k] * s_r = hi[r,k] + lo[r,k],   s_r a power of two with max_k |x[r,k]| * s_r <= 2^15,
 // hi = fp16(x * s_r), lo = fp16(x * s_r - hi): 22 significant bits for every element down to 2^-17 of the row's bound and an
-// absolute error of 2^-40 of that bound below it.  An fp16 significand has the 11 bits of TF32, so
+// absolute error of at most 2^-39 of that bound below it (the TF32 kernels keep an exponent per element: a caller whose columns
+// span more than that chooses them).  The bound is the row's maximum where the producer holds the row; a product's epilogue only
+// knows max|x| * max ||w||_1 + max|b|, 2^6 to 2^8 times as much in the models here, and images share one scale over all channels.  An fp16 significand has the 11 bits of TF32, so
 //     x·w = (hi·hi + hi·lo + lo·hi) / (s_x s_w)
 // drops the same 2^-22 term as three TF32 products (and less than one TF32 product + two bf16 corrections, whose corrections
 // are rounded at 2^-19), but a kind::f16 instruction covers K = 16 where a kind::tf32 instruction covers 8: three
@@ -18,8 +20,9 @@
 //     |y[r,j]| <= amax_r * max_j ||w_j||_1 + max_j |b_j|
 // (amax_r = max_k |x[r,k]|, kept beside the planes).  Anything else goes through split_rows_kernel first.
 //
-// Structure: persistent, 384 threads, one CTA per SM.  Warps 0-7 epilogue, warp 8 TMA producer, warp 9 MMA issuer (10 and 11
-// complete the warpgroup that setmaxnreg takes registers from: a wide tile's epilogue holds 128 running sums); nothing
+// Structure: persistent, one CTA per SM of 384 threads: warps 0-7 epilogue, warp 8 TMA producer, warp 9 MMA issuer (10 and 11
+// complete the warpgroup that setmaxnreg takes registers from: a wide tile's epilogue holds 128 running sums), or 640 with sixteen
+// epilogue warps (units of a single chain, see below).  Nothing
 // touches an operand between TMA and the tensor core, so K-slabs are 64 deep (128-byte rows, one 3-D TMA load brings both
 // planes of a tile).  PAIR: two CTAs of a cluster share a 256-row tile (cta_group::2), each staging half of the weight tile.
 // Accumulation runs in chains of `chunk_slabs` K-slabs into one of two TMEM accumulators; the epilogue warps drain finished
@@ -197,7 +200,7 @@ __device__ __forceinline__ void drain_chunk(uint32_t tacc, float (&sum)[HALF]) {
 
 // EW epilogue warps: eight, or sixteen for units of a single chain, which need no registers for sums.  Those are short products
 // (K <= 128) bound by the epilogue, where a scheduler with two of its warps issues an instruction every other cycle:
-// 128 images of 56 x 56, 64 -> 256 channels with residual 215 -> 178 us (7.7 TB/s would take 120).
+// 128 images of 56 x 56, 64 -> 256 channels with residual 215 -> 178 us (its bytes take 141 at 6.55 TB/s).
 template <int BN, int STAGES, bool PAIR, int NPL, bool IMG, int EW>
 __global__ void __launch_bounds__(EW * 32 + 128, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_r, F16Params p) {
@@ -931,10 +934,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     // ---------------- teardown ----------------
     tc_fence_before();
     __syncthreads();
+    let_copies_land(abort_flag);
     if (PAIR) cluster_sync_all();
     if (warp == kMmaWarp) {
         tc_fence_after();
-    let_copies_land(abort_flag);
         if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
         else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }

@@ -1,5 +1,6 @@
 // Tensor-core GEMM for sm_100a:  out[M,N] = act(x[M,K] · w[N,K]^T + bias[N])  with fp32-grade
-// accuracy from three TF32 products per logical product ("3xTF32").
+// accuracy from three TF32 products per logical product ("3xTF32"), or one TF32 product and two bf16 corrections.  Serves tensor
+// parallelism, the explicit arithmetic modes and shapes without a split form; the default products of one GPU are in gemm_f16.cu.
 //
 // The contraction behind Linear / LinearRelu / FeedForward / the MHA projections (reference:
 // torch::linear, csrc/kernels/cpu/linear.cpp:11, feedforward.cpp:13, mha.cpp:22,51; the
@@ -929,8 +930,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     // ---------------- teardown (every thread arrives here, whatever happened above) ----------------
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (PAIR) cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still touch its memory
     let_copies_land(abort_flag);
+    if (PAIR) cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still touch its memory
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");

@@ -152,8 +152,9 @@ inline void apply_fusion(ExecCtx& ctx, Args& g, bool partial) {
     g.relu = g.relu || ctx.fuse.relu;
     ctx.fuse.consumed = true;
 }
+// out = w[idx] * scale + rows, which repeat
+int launch_embedding_scale_add(const FxfTensor& idx, const FxfTensor& w, float scale, const FxfTensor& rows, const FxfTensor& out, ExecCtx& ctx);
 // out = act(out + residual) over n contiguous floats: the fallback when a GEMM without a fused epilogue ran
-int launch_embedding_scale_add(const FxfTensor& idx, const FxfTensor& w, float scale, const FxfTensor& rows, const FxfTensor& out, ExecCtx& ctx);   // out = w[idx] * scale + rows, which repeat
 int launch_residual_epilogue(float* out, const float* residual, int64_t n, bool relu, ExecCtx& ctx);
 
 struct NodePlan {
