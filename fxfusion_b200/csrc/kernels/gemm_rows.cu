@@ -352,7 +352,10 @@ int clusters_resident(int cs, int* out) {
     cfg.dynamicSmemBytes = r.smem;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    FXF_CUDA(cudaOccupancyMaxActiveClusters(out, r.kernel, &cfg));
+    if (cudaOccupancyMaxActiveClusters(out, r.kernel, &cfg) != cudaSuccess) {   // a size this device does not launch at all
+        (void)cudaGetLastError();
+        *out = 0;
+    }
     if (slot != nullptr) slot->store(*out + 1, std::memory_order_relaxed);
     return 0;
 }
