@@ -71,7 +71,8 @@ int launch_gemm(const GemmArgs& a, ExecCtx& ctx) {
         if (launch_gemm(plain, ctx)) return 1;
         return launch_residual_epilogue(a.out, a.residual, a.M * a.N, a.relu, ctx);
     }
-    FXF_CHECK(ctx.gemm_mode != FXF_GEMM_TF32X3, "gemm: FXF_GEMM_TF32X3 was requested but the shape M=%lld N=%lld K=%lld (or its alignment) is not supported by the tensor-core kernel",
+    const bool live_weight = a.w_hi == nullptr && gemm_tc_shape_ok(a.M, a.N, a.K);   // not a constant: nothing was converted
+    FXF_CHECK(ctx.gemm_mode != FXF_GEMM_TF32X3 || live_weight, "gemm: FXF_GEMM_TF32X3 was requested but the shape M=%lld N=%lld K=%lld (or its alignment) is not supported by the tensor-core kernel",
               (long long)a.M, (long long)a.N, (long long)a.K);
     return launch_gemm_simt(a, ctx);
 }
