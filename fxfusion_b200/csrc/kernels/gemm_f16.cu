@@ -944,16 +944,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 }
 
 // ---- host side -------------------------------------------------------------------------------------
-// [planes][rows][cols] 16-bit elements, `ld` elements between rows and `plane` between planes; box = 64 columns x box_rows x all planes
 int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int64_t plane, int planes, int box_rows) {
-    const auto fn = encode_tiled_fn();
-    FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
-    cuuint64_t dims[3] = {cuuint64_t(cols), cuuint64_t(rows), cuuint64_t(planes)};
-    cuuint64_t strides[2] = {cuuint64_t(ld) * 2, cuuint64_t(planes > 1 ? plane : rows * ld) * 2};
-    cuuint32_t box[3] = {cuuint32_t(BK), cuuint32_t(box_rows), cuuint32_t(planes)};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult r = encode_planes(map, base, rows, cols, ld, plane, planes, BK, box_rows);
     FXF_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (f16) failed with code %d (rows %lld cols %lld planes %d)", int(r), (long long)rows, (long long)cols, planes);
     return 0;
 }

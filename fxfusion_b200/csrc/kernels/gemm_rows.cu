@@ -293,19 +293,6 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, RowsParams p) {
     }
 }
 
-int make_weight_map(CUtensorMap* map, const SplitMat& w, int64_t rows, int64_t cols) {
-    const auto fn = encode_tiled_fn();
-    FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
-    cuuint64_t dims[3] = {cuuint64_t(cols), cuuint64_t(rows), 2};
-    cuuint64_t strides[2] = {cuuint64_t(cols) * 2, cuuint64_t(w.plane) * 2};
-    cuuint32_t box[3] = {BK, BN, 2};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<uint16_t*>(w.planes), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    FXF_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (rows) failed with code %d", int(r));
-    return 0;
-}
-
 // The instances: rows of x per CTA, K-slabs per CTA that fit without refilling the rings, CTAs per SM (two slabs take 70-100 KB of
 // shared memory: two CTAs share an SM, or one stands beside one of the kernel before it).
 using RowsKernel = void (*)(const CUtensorMap, RowsParams);
@@ -404,7 +391,8 @@ int launch_gemm_rows(const F16GemmArgs& a, const float* x, int64_t ldx, ExecCtx&
     FXF_CHECK(gemm_rows_ok(a.M, a.N, a.K) && !a.bf16 && a.w.planes && a.out && (x != nullptr || a.x.planes != nullptr), "few-row GEMM: unsupported operands");
     FXF_CHECK(x == nullptr || (aligned16(x) && ldx % 4 == 0), "few-row GEMM: unaligned rows");
     CUtensorMap map;
-    if (make_weight_map(&map, a.w, a.N, a.K)) return 1;
+    const CUresult r = encode_planes(&map, a.w.planes, a.N, a.K, a.K, a.w.plane, 2, BK, BN);
+    FXF_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (rows) failed with code %d", int(r));
     RowsParams p{};
     p.x = x; p.ldx = ldx;
     if (x == nullptr) {

@@ -429,5 +429,18 @@ inline auto encode_tiled_fn() {
     return fn;
 }
 
+// [planes][rows][cols] 16-bit elements, `ld` elements between rows and `plane` between planes; box = box_cols (128 bytes, swizzled)
+// x box_rows x all planes
+inline CUresult encode_planes(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int64_t plane, int planes, int box_cols, int box_rows) {
+    const auto fn = encode_tiled_fn();
+    if (fn == nullptr) return CUDA_ERROR_NOT_SUPPORTED;
+    cuuint64_t dims[3] = {cuuint64_t(cols), cuuint64_t(rows), cuuint64_t(planes)};
+    cuuint64_t strides[2] = {cuuint64_t(ld) * 2, cuuint64_t(planes > 1 ? plane : rows * ld) * 2};
+    cuuint32_t box[3] = {cuuint32_t(box_cols), cuuint32_t(box_rows), cuuint32_t(planes)};
+    cuuint32_t estr[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
+
 }  // namespace sm100
 }  // namespace fxf
