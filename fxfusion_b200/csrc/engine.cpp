@@ -994,9 +994,12 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
             const int64_t D = x.rank >= 1 ? x.shape[x.rank - 1] : 0;
             auto plain = [&](uint32_t id, int64_t n) { return e->reg[id].dtype == FXF_F32 && is_contiguous(e->reg[id]) && numel(e->reg[id]) == n && on_16_bytes(id); };
             if (D < 1 || P.params.ints[1] != D || y.rank < 1 || y.shape[y.rank - 1] != D || !plain(P.in[0], numel(y)) || !plain(P.in[1], D) || !plain(P.in[2], D)) continue;
-            // its rows are read while the product's results are written
-            bool clash = R.fuse_out >= 0 && overlap(P.in[0], uint32_t(R.fuse_out));
-            for (uint32_t id : R.out) clash = clash || overlap(P.in[0], id);
+            // its rows, gamma and beta are read while the product's results are written; to the planner they died at the LayerNorm
+            bool clash = false;
+            for (size_t k = 0; k < 3; k++) {
+                clash = clash || (R.fuse_out >= 0 && overlap(P.in[k], uint32_t(R.fuse_out)));
+                for (uint32_t id : R.out) clash = clash || overlap(P.in[k], id);
+            }
             if (clash) continue;
             R.norm_of = int(pi);
             P.folded = true;

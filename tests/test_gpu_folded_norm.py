@@ -70,3 +70,40 @@ def test_not_folded(built_lib, tmp_path, why):
         ok, info = compare_outputs(g, w, atol=2e-5, rtol=1e-4)
         assert ok, info
     eng.close()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1024, 512), (8, 256, 1024), (64, 32, 1024)])
+@pytest.mark.parametrize("after", ["Relu", "residual"])
+@pytest.mark.parametrize("kept", [False, True])
+def test_computed_gamma_and_beta(built_lib, tmp_path, M, N, K, after, kept):
+    """Gamma and beta that the graph computes die at the LayerNorm, and the planner gives their place to what the product behind it writes: a folded
+    LayerNorm would read them meanwhile.  Where they live on (`kept`), it is folded and reads what the launches before it wrote."""
+    from fxfusion_b200.engine import ExecutionEngine
+    rng = np.random.default_rng(N)
+    b = lowering.GraphBuilder(f"computed_{M}_{N}_{K}")
+    x, r, gin, bin_ = b.input((M, K), wire.DT_F32), b.input((M, N), wire.DT_F32), b.input((K,), wire.DT_F32), b.input((K,), wire.DT_F32)
+    gamma, beta = b.op("Relu", [gin], (K,)), b.op("Relu", [bin_], (K,))
+    y = b.op("LayerNorm", [x, gamma, beta], (M, K), ints=[1, K], floats=[1e-5])
+    w = [b.const((rng.standard_normal((N, K)) / math.sqrt(K)).astype(np.float32)), b.const(rng.standard_normal(N, dtype=np.float32))]
+    z = b.op("Linear", [y, *w], (M, N)) if after == "residual" else b.op("LinearRelu", [y, *w], (M, N))
+    z2 = b.op("Add", [z, r], (M, N)) if after == "residual" else z
+    b.output(b.op("Relu", [z2], (M, N)))
+    if kept:
+        b.output(b.op("Add", [gamma, beta], (K,)))
+    graph = b.finish()
+    place = lambda v: (graph.tensors[v].offset, graph.tensors[v].offset + graph.tensors[v].size_bytes)
+    below = [v for v in (gamma, beta) for o in (z, z2) if place(v)[0] < place(o)[1] and place(o)[0] < place(v)[1]]
+    assert bool(below) == (not kept)
+    path = tmp_path / "g.bin"
+    wire.dump(graph, path)
+    eng = ExecutionEngine(str(path), "cuda:0")
+    gen = torch.Generator().manual_seed(M)
+    for _ in range(3):   # (every forward has a gamma and a beta of its own)
+        ins = [torch.randn(M, K, generator=gen), torch.randn(M, N, generator=gen), torch.randn(K, generator=gen) + 1, torch.randn(K, generator=gen)]
+        for got, want in zip(eng.run([t.cuda() for t in ins]), GraphOracle(graph).run(ins)):
+            ok, info = compare_outputs(got.cpu(), want, atol=5e-5, rtol=2e-4)
+            assert ok, info
+    kernels = [q["kernel"] for q in eng.profile_launches()]
+    assert ("LayerNorm" in kernels) == (not kept), kernels
+    assert eng.device_status() == 0
+    eng.close()
