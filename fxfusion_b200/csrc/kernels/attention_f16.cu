@@ -289,10 +289,10 @@ attn_f16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 const uint32_t* src = row_bits + (__ffs(rem) - 1) * (BKEY / 32);
                 uint32_t keep[CH];
                 if constexpr (CH == 2) {
-                    const uint2 k2 = __ldg(reinterpret_cast<const uint2*>(src));
+                    const uint2 k2 = *reinterpret_cast<const uint2*>(src);
                     keep[0] = k2.x; keep[CH - 1] = k2.y;
                 } else {
-                    keep[0] = __ldg(src);
+                    keep[0] = *src;
                 }
                 const bool whole = warp_all((keep[0] & keep[CH - 1]) == 0xffffffffu);
                 if (alive && !warp_all(mbar_wait(&s.bar_s, t & 1, abort_flag))) { give_up(abort_flag, p.status, kErrAttnF16S); alive = false; }

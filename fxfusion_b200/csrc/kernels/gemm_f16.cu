@@ -184,7 +184,7 @@ template <int N>
 struct Words { uint32_t w[N]; };
 // 32 bytes of global memory at once: a whole sector per lane, so that lanes may own rows
 __device__ __forceinline__ void load32(const void* p, Words<8>& r) {
-    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7]) : "l"(p));
 }
 __device__ __forceinline__ void store32(void* p, const Words<8>& r) {
@@ -463,8 +463,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             const int image = IMG ? int(unsigned(grow) / p.im.rpi) : 0;
             const int64_t sx = IMG ? image : grow * p.x_inv_stride;
             const int so_at = IMG ? image : grow;   // where the row's scales stand
-            const float ri = (row_ok && p.x_inv != nullptr) ? __ldg(p.x_inv + sx) : 1.f;
-            const float res_inv = (IMG && p.im.res != nullptr && row_ok) ? __ldg(p.im.res_inv + image) : 0.f;
+            const float ri = (row_ok && p.x_inv != nullptr) ? p.x_inv[sx] : 1.f;
+            const float res_inv = (IMG && p.im.res != nullptr && row_ok) ? p.im.res_inv[image] : 0.f;
             const float row_bias = (p.swap && row_ok && p.bias != nullptr) ? __ldg(p.bias + grow) : 0.f;
             float rscale = 1.f, rinv = 0.f;
             __half2 rmax = __half2half2(__ushort_as_half(0));   // largest |hi| of the row so far
@@ -473,9 +473,9 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 split_cap_scale(p.so_cap, p.w_bound, rscale, rinv);
             } else if (NPL == 2 && p.so != nullptr && !writes_partial && row_ok) {
                 float am = 0.f;
-                for (int j = 0; j < p.x_parts; j++) am = fmaxf(am, __ldg(p.x_amax + sx * p.x_parts + j));
+                for (int j = 0; j < p.x_parts; j++) am = fmaxf(am, p.x_amax[sx * p.x_parts + j]);
                 float bound = fmaf(am, __ldg(p.w_bound), __ldg(p.w_bound + 1));
-                if (IMG && p.im.res != nullptr) bound += __ldg(p.im.res_amax + image);
+                if (IMG && p.im.res != nullptr) bound += p.im.res_amax[image];
                 split_scale(bound, rscale, rinv);
                 if (part == 0 && tn == 0 && (!IMG || unsigned(grow) == unsigned(image) * p.im.rpi)) p.so_inv[so_at] = rinv;
             }
@@ -506,7 +506,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 __syncwarp();
                 for (int j = lane; j < COLS; j += 32) {
                     const int c = col_base + j;
-                    cinv[j] = (p.w_inv && c < N) ? __ldg(p.w_inv + c * p.w_inv_stride) : 1.f;
+                    cinv[j] = (p.w_inv && c < N) ? p.w_inv[c * p.w_inv_stride] : 1.f;
                     cbias[j] = (p.bias && !p.swap && c < N) ? __ldg(p.bias + c) : 0.f;
                 }
                 __syncwarp();

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_lanes_kernel(LanesParams p) 
     auto fetch_bias = [&]() {
 #pragma unroll
         for (int i = 0; i < PER; i++)
-            if (row[i] >= 0 && p.bias) bi[i] = __ldg(p.bias + col[i]);
+            if (row[i] >= 0 && p.bias) bi[i] = p.bias[col[i]];
     };
 #pragma unroll
     for (int i = 0; i < PER; i++) {
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_lanes_kernel(LanesParams p) 
             for (int i = 0; i < NV; i++) {
                 const int c = lane + 32 * i;
                 if (c < k4) {
-                    const float4 g = __ldg(reinterpret_cast<const float4*>(p.gamma) + c), b = __ldg(reinterpret_cast<const float4*>(p.beta) + c);
+                    const float4 g = *(reinterpret_cast<const float4*>(p.gamma) + c), b = *(reinterpret_cast<const float4*>(p.beta) + c);
                     *reinterpret_cast<float4*>(xs + size_t(r) * K + c * 4) =
                         make_float4((v[i].x * rstd + shift) * g.x + b.x, (v[i].y * rstd + shift) * g.y + b.y, (v[i].z * rstd + shift) * g.z + b.z, (v[i].w * rstd + shift) * g.w + b.w);
                 }

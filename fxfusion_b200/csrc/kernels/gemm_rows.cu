@@ -196,7 +196,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, RowsParams p) {
                         v[q][i] = *reinterpret_cast<const float4*>(p.x + (m0 + r) * p.ldx + k);
                     } else {
                         const uint2 h = *reinterpret_cast<const uint2*>(p.x_planes + (m0 + r) * p.ld_planes + k), l = *reinterpret_cast<const uint2*>(p.x_planes + p.x_plane + (m0 + r) * p.ld_planes + k);
-                        const float inv = __ldg(p.x_inv + (m0 + r) * p.x_inv_stride);
+                        const float inv = p.x_inv[(m0 + r) * p.x_inv_stride];
                         const float2 h0 = __half22float2(*reinterpret_cast<const __half2*>(&h.x)), h1 = __half22float2(*reinterpret_cast<const __half2*>(&h.y));
                         const float2 l0 = __half22float2(*reinterpret_cast<const __half2*>(&l.x)), l1 = __half22float2(*reinterpret_cast<const __half2*>(&l.y));
                         v[q][i] = make_float4((h0.x + l0.x) * inv, (h0.y + l0.y) * inv, (h1.x + l1.x) * inv, (h1.y + l1.y) * inv);
@@ -214,8 +214,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, RowsParams p) {
             for (int i = 0; i < V; i++) {
                 const int at = i * 128 + lane * 4, k = kb + at;
                 in[i] = at < ns * BK && k < p.K;
-                g[i] = in[i] ? __ldg(reinterpret_cast<const float4*>(p.gamma + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                bt[i] = in[i] ? __ldg(reinterpret_cast<const float4*>(p.beta + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                g[i] = in[i] ? *reinterpret_cast<const float4*>(p.gamma + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                bt[i] = in[i] ? *reinterpret_cast<const float4*>(p.beta + k) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             float t[ROWS], mean[ROWS], rstd[ROWS];
 #pragma unroll

@@ -754,7 +754,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                     bool bad = false;
 #pragma unroll
                     for (int d = 0; d < 32; d++) {
-                        const float v = sum[hh * 32 + d] + (p.bias ? __ldg(p.bias + c0 + d) : 0.f);
+                        const float v = sum[hh * 32 + d] + (p.bias ? p.bias[c0 + d] : 0.f);
                         bad = bad || (v - v != 0.f);   // NaN or infinity
                         if (ok) dst[int64_t(d) * p.vt_T] = v;
                     }
@@ -774,7 +774,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
                     for (int j = 0; j < HALF; j++) {
                         const int64_t c = col_base + j;
-                        sum[j] += c < p.N ? __ldg(p.bias + c) : 0.f;   // the same address in every lane: one broadcast load
+                        sum[j] += c < p.N ? p.bias[c] : 0.f;   // the same address in every lane: one broadcast load
                     }
                 }
                 if (p.relu) {
@@ -885,7 +885,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                     // consecutive columns
                     const int cl = lane & 15, r2 = lane >> 4;
                     const bool col_ok = col + cl < p.N;
-                    const float b = (p.bias && col_ok) ? __ldg(p.bias + col + cl) : 0.f;
+                    const float b = (p.bias && col_ok) ? p.bias[col + cl] : 0.f;
                     if (!p.cv.enabled && !adds_partials && p.residual == nullptr) {
                         // dense rows without extras: affine addresses, independent iterations (the stores of consecutive rows pipeline)
                         const int64_t grow = int64_t(tm) * BM + row0 + r2;

@@ -42,8 +42,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) layernorm_warp_kernel(con
 #pragma unroll
             for (int i = 0; i < NV; i++) {
                 int c = lane + 32 * i;
-                gs[i] = c < n4 ? w[c] : make_float4(0.f, 0.f, 0.f, 0.f);
-                bs[i] = c < n4 ? b[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+                gs[i] = c < n4 ? sm100::load_in_order(w + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                bs[i] = c < n4 ? sm100::load_in_order(b + c) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
     };

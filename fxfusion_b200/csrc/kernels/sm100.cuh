@@ -103,11 +103,21 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
 }
 // Programmatic dependent launch: everything the kernels before this one in the stream wrote is visible after the wait; the
 // launch signal lets the next kernel become resident (its own wait still holds it back until this one has finished).
+// What the launches before may write is read behind the wait with plain loads: a kernel that is resident meanwhile must not call it read-only
+// for its whole life (__ldg, ld.global.nc).
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep() {   // first statement of a kernel with nothing to do ahead of its inputs
     grid_dep_launch();
     grid_dep_wait();
+}
+
+// A load that stays on its side of grid_dep_wait() even where the pointer is __restrict__, which would let the compiler merge the loads of a
+// branch ahead of the wait and of one behind it.
+__device__ __forceinline__ float4 load_in_order(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
 }
 
 __device__ __forceinline__ float max_keep_nan(float v, float floor_at) {

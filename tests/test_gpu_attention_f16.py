@@ -93,3 +93,51 @@ def test_masked_keys_do_not_move_a_bit(built_lib, tmp_path):
     b = eng.run([x.cuda(), mask.cuda()])[0].cpu()
     assert torch.equal(a[:, :100], b[:, :100]) and not torch.equal(a[:, 100:], b[:, 100:])
     eng.close()
+
+
+@pytest.mark.parametrize("cross", [False, True])
+@pytest.mark.parametrize("r", [1.0, 16.0, 1024.0, 3e5])
+@pytest.mark.parametrize("what", ["thirds", "heads", "columns"])
+def test_uneven_sizes(built_lib, tmp_path, what, r, cross):
+    """Q's weights divided and K's multiplied by the same factors, which leaves the function as it is: all of them by r, or by r in one head and 1 / r
+    in the next, or every column by a factor of its own up to r.  Against fp64: Q, K and V keep 22 bits of what they add to a score, sum |q_d k_d| / 8
+    is about 5 here, so a score is off by 5 * 2^-21 at most and a probability by that much of itself; 2^-18 covers it and the sums in fp32."""
+    from fxfusion_b200.engine import ExecutionEngine
+    B, T, Tk, D, H = 1, 130, 200, 384, 6
+    rng = np.random.default_rng(11)
+    f = {"thirds": np.full(D, r), "heads": np.repeat(r ** np.where(np.arange(H) % 2, -1.0, 1.0), 64), "columns": r ** rng.uniform(-1, 1, D)}[what].astype(np.float32)
+    wq, wk, wv, wo = (rng.standard_normal((D, D)) / math.sqrt(D) for _ in range(4))
+    bq, bk, bv, bo = (0.1 * rng.standard_normal(D) for _ in range(4))
+    wq, bq, wk, bk = wq / f[:, None], bq / f, wk * f[:, None], bk * f
+    w = [t.astype(np.float32) for t in (wq, wk, wv, wo)]
+    bias = [t.astype(np.float32) for t in (bq, bk, bv, bo)]
+    b = lowering.GraphBuilder(f"uneven_{what}_{r}")
+    one, zero = b.const(np.ones(D, np.float32)), b.const(np.zeros(D, np.float32))
+    norm = lambda v, L: b.op("LayerNorm", [v, one, zero], (B, L, D), ints=[1, D], floats=[1e-5])
+    x = b.input((B, T, D), wire.DT_F32)
+    if cross:
+        mem = b.input((B, Tk, D), wire.DT_F32)
+        m = b.input((1, 1, T, Tk), wire.DT_BOOL)
+        b.output(b.op("CrossMHA", [norm(x, T), norm(mem, Tk), m, b.const(w[0]), b.const(bias[0]), b.const(np.concatenate(w[1:3])), b.const(np.concatenate(bias[1:3])), b.const(w[3]),
+                                   b.const(bias[3])], (B, T, D), ints=[H, 64, D, 2 * D], floats=[8.0]))
+    else:
+        Tk = T
+        m = b.input((1, 1, T, T), wire.DT_BOOL)
+        b.output(b.op("MHA", [norm(x, T), m, b.const(np.concatenate(w[:3])), b.const(np.concatenate(bias[:3])), b.const(w[3]), b.const(bias[3])], (B, T, D), ints=[H, 64, D, 3 * D], floats=[8.0]))
+    path = tmp_path / "g.bin"
+    wire.dump(b.finish(), path)
+    eng = ExecutionEngine(str(path), "cuda:0")
+    gen = torch.Generator().manual_seed(5)
+    xin, min_ = torch.randn(B, T, D, generator=gen), torch.randn(B, Tk, D, generator=gen)
+    mask = torch.ones(1, 1, T, Tk, dtype=torch.bool).tril(Tk - T)
+    got = eng.run([xin.cuda(), min_.cuda(), mask.cuda()] if cross else [xin.cuda(), mask.cuda()])[0].cpu().double()
+    ln = lambda t: torch.nn.functional.layer_norm(t.double(), (D,), eps=1e-5)
+    rows = ln(min_) if cross else ln(xin)
+    d = lambda a: torch.from_numpy(a).double()
+    heads = lambda t, i: (t @ d(w[i]).T + d(bias[i])).view(B, -1, H, 64).transpose(1, 2)
+    s = (heads(ln(xin), 0) @ heads(rows, 1).transpose(-1, -2) / 8.0).masked_fill(~mask, float("-inf"))
+    want = (torch.softmax(s, -1) @ heads(rows, 2)).transpose(1, 2).reshape(B, T, D) @ d(w[3]).T + d(bias[3])
+    assert ((got - want).norm() / want.norm()).item() < 2.0 ** -18
+    assert any("attention_f16x3" in q["kernel"] for q in eng.profile_launches())
+    assert eng.device_status() == 0
+    eng.close()
