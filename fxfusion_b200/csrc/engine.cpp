@@ -974,6 +974,7 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
                 const size_t at = P.op == FXF_OP_LAYER_NORM ? 1 : 2;
                 if (P.in.size() > at + 1) m.cap = 1.001f * (std::sqrt(float(D)) * largest(P.in[at], D) + largest(P.in[at + 1], D));
                 if (!std::isfinite(m.cap)) m.cap = 0.f;
+                if (m.cap > 0.f) { m.gamma = int(P.in[at]); m.beta = int(P.in[at + 1]); }
             }
             for (uint32_t id = 0; id < n_tensors; id++)
                 if (root(id) == t) e->splits[id] = m;

@@ -1,8 +1,8 @@
 // Tensor-core attention core for head_dim 64 on operands that are already in split form (gemm_f16.cu):
 //     ctx = softmax(mask_fill(Q·K^T / scale_divisor)) · V        per (batch, head)
-// Q, K and V are two fp16 planes each, written by the epilogue of their projection under ONE power-of-two scale for all rows
-// (F16GemmArgs::split_cap), so both contractions are three kind::f16 products (hi·lo, lo·hi, hi·hi) on tiles that nothing
-// touches between TMA and tensor core.  V needs no transposed copy: as the B operand of P·V it is read with the head columns
+// Q, K and V are two fp16 planes each, written by the epilogue of their projection under a power-of-two scale per column
+// (attention_scales_kernel: a pair of columns of Q and K has the same product of scales throughout a head), so both contractions are
+// three kind::f16 products (hi·lo, lo·hi, hi·hi) on tiles that nothing touches between TMA and tensor core.  V needs no transposed copy: as the B operand of P·V it is read with the head columns
 // contiguous (MN-major).  Semantics are those of attention.cu and attention_tc.cu (which serves the other arithmetic modes, rows
 // whose size is not bounded by a LayerNorm, few rows and more than kMaxKeys keys): -inf where mask == 0, fully masked rows give NaN,
 // masked keys still enter P·V with weight 0, and a block of keys is skipped only when every mask byte of it is 0 for all 128
@@ -57,6 +57,7 @@ struct alignas(1024) AttnF16Smem {
     uint16_t q[2][BQ * HD];
     uint16_t k[2][BKEY * HD];
     uint16_t v[2 * BQ * HD];       // both planes of a block's V, later the context [quarter of the rows][plane]
+    float vf[8][36];               // per softmax warp: the factors of its 32 columns, and AttnScales::ctx_inv
     float exch[2][2][BQ];          // row statistics exchanged between the two threads of a row, by block parity
     uint64_t bar_q, bar_k, bar_v, bar_s, bar_p, bar_o, bar_free;   // bar_free: the staged context has been read, V may be loaded
     uint32_t tmem_base;
@@ -71,9 +72,8 @@ struct AttnF16Params {
     int B, T, Tk, H, q_tiles, units;
     int q_col, k_col, v_col;
     int64_t ld_ctx;
-    float scale_divisor;
-    float q_cap, kv_cap;           // scales: see split_cap_scale
-    const float *q_bound, *kv_bound;
+    const float *score_inv, *v_factor, *ctx_inv;   // AttnScales; v_factor: v_ctx where split is 2, v_inv otherwise
+    float score_scale;             // log2(e) / scale_divisor
     int split;                     // the context leaves by TMA: 2: as two fp16 planes, 1: as bf16; 0: fp32 in ctx
     float* so_inv;
     int* status;
@@ -267,19 +267,17 @@ attn_f16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         const int row = quarter * 32 + lane;
         const uint32_t lane_base = uint32_t(quarter * 32) << 16;
         const uint32_t scol = tmem + lane_base + uint32_t(half * (BKEY / 2)), ocol = tmem + lane_base + kColO + uint32_t(half * 32);
-        float c, kv_inv;
-        {
-            float scale, q_inv;
-            split_cap_scale(p.q_cap, p.q_bound, scale, q_inv);
-            split_cap_scale(p.kv_cap, p.kv_bound, scale, kv_inv);
-            // scores in the log2 domain; kept away from 0 and infinity, where -inf * c would not be -inf
-            c = fminf(fmaxf(q_inv * kv_inv * (kLog2e / p.scale_divisor), 1.2e-38f), 3.0e38f);
-        }
         bool alive = true;   // warp-uniform; a warp that gave up keeps walking the loop so that pair_sync() stays matched
         uint32_t t = 0;
         Unit u;
         for (int r = 0; unit_of(r, u); r++) {
             const int b = u.b, h = u.h, qi = u.q0 + row;
+            // on their way while the keys are walked (a round trip to L2 behind them costs 0.4 us where a CTA has one unit)
+            auto fetch = [](float* dst, const float* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); };
+            fetch(&s.vf[warp - kSoftWarp0][lane], p.v_factor + h * HD + half * 32 + lane);
+            if (lane == 0) fetch(&s.vf[warp - kSoftWarp0][32], p.ctx_inv);
+            // scores in the log2 domain; kept away from 0 and infinity, where -inf * c would not be -inf
+            const float c = fminf(fmaxf(p.score_inv[h] * p.score_scale, 1.2e-38f), 3.0e38f);
             const uint32_t* row_bits = p.bits + b * p.bit_sb + h * p.bit_sh + int64_t(min(qi, T - 1)) * p.bit_sq + half * CH;
             float o[32];
 #pragma unroll
@@ -374,34 +372,38 @@ attn_f16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             s.exch[t & 1][half][row] = l_run;
             pair_sync(quarter);
             const float l_tot = s.exch[t & 1][0][row] + s.exch[t & 1][1][row];
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
             if (alive) {   // a fully masked row has o = 0 and l = 0: 0 * inf = NaN, as the reference softmax gives
                 const float inv_l = 1.0f / l_tot;
+                const float4* vf = reinterpret_cast<const float4*>(s.vf[warp - kSoftWarp0]);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const float4 f = vf[j];
+                    o[4 * j] *= inv_l * f.x; o[4 * j + 1] *= inv_l * f.y; o[4 * j + 2] *= inv_l * f.z; o[4 * j + 3] *= inv_l * f.w;
+                }
                 if (p.split == 0) {
                     if (qi < T) {
                         float* dst = p.ctx + (int64_t(b) * T + qi) * p.ld_ctx + int64_t(h) * HD + half * 32;
-                        const float f = inv_l * kv_inv;
 #pragma unroll
-                        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(o[j] * f, o[j + 1] * f, o[j + 2] * f, o[j + 3] * f);
+                        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
                     }
                 } else {
                     // Staged where V was (every P·V is done), 32 rows per quarter and plane, and stored by TMA, which leaves out the rows behind the
                     // last: sixteen bytes per lane and row kept the load / store unit busy for 4000 cycles.
                     char* stage = reinterpret_cast<char*>(s.v) + quarter * 8192 + lane * 128;
-                    if (p.split == 2) {   // a convex combination of V rows fits their scale, which no masked row can move
-                        if (h == 0 && half == 0 && qi < T) p.so_inv[int64_t(b) * T + qi] = kv_inv;
+                    if (p.split == 2) {   // a convex combination of V rows fits the scale of V's largest column, which no masked row can move
+                        if (h == 0 && half == 0 && qi < T) p.so_inv[int64_t(b) * T + qi] = s.vf[warp - kSoftWarp0][32];
 #pragma unroll
                         for (int j = 0; j < 4; j++) {
                             uint4 hi, lo;
 #pragma unroll
-                            for (int e = 0; e < 4; e++) split_f16x2(o[8 * j + 2 * e] * inv_l, o[8 * j + 2 * e + 1] * inv_l, (&hi.x)[e], (&lo.x)[e]);
+                            for (int e = 0; e < 4; e++) split_f16x2(o[8 * j + 2 * e], o[8 * j + 2 * e + 1], (&hi.x)[e], (&lo.x)[e]);
                             const int at = ((half * 4 + j) ^ (lane & 7)) << 4;
                             *reinterpret_cast<uint4*>(stage + at) = hi;
                             *reinterpret_cast<uint4*>(stage + 4096 + at) = lo;
                         }
                     } else {
-                        const float f = inv_l * kv_inv;
-#pragma unroll
-                        for (int j = 0; j < 32; j++) o[j] *= f;
 #pragma unroll
                         for (int j = 0; j < 4; j++)
                             *reinterpret_cast<uint4*>(stage + (((half * 4 + j) ^ (lane & 7)) << 4)) =
@@ -529,7 +531,7 @@ int launch_attention_f16(const AttnArgs& a, const AttnSplit& sp, ExecCtx& ctx) {
     const int Tk = a.kv ? a.Tk : a.T;
     const int64_t ldk = a.kv ? a.ld_kv : a.ld_qkv;
     FXF_CHECK(attention_f16_ok(a.T, Tk, a.hd, a.scale_divisor) && sp.q && sp.kv && aligned16(sp.q) && aligned16(sp.kv) && sp.q_plane % 8 == 0 && sp.kv_plane % 8 == 0 && a.ld_qkv % 8 == 0 &&
-                  ldk % 8 == 0 && (a.q_off | a.k_off | a.v_off) % 8 == 0 && a.ld_ctx % 8 == 0 && sp.q_cap > 0.f && sp.kv_cap > 0.f && sp.q_bound && sp.kv_bound && sp.mask != nullptr && sp.mask->bits != nullptr && int64_t(a.B) * a.H * ((a.T + BQ - 1) / BQ) < (1 << 30),
+                  ldk % 8 == 0 && (a.q_off | a.k_off | a.v_off) % 8 == 0 && a.ld_ctx % 8 == 0 && sp.scales != nullptr && sp.mask != nullptr && sp.mask->bits != nullptr && int64_t(a.B) * a.H * ((a.T + BQ - 1) / BQ) < (1 << 30),
               "attention (split form): unsupported operands");
     FXF_CHECK(a.split_ctx.planes == nullptr || (aligned16(a.split_ctx.planes) && (a.split_ctx.plane * 2) % 16 == 0 && (a.split_bf16 || a.split_ctx.inv)), "attention: a context in split form needs 16-byte rows");
     AttnF16Params p{};
@@ -539,9 +541,10 @@ int launch_attention_f16(const AttnArgs& a, const AttnSplit& sp, ExecCtx& ctx) {
     p.bad = mb.bad;
     p.ctx = a.ctx; p.B = a.B; p.T = a.T; p.Tk = Tk; p.H = a.H; p.ld_ctx = a.ld_ctx;
     p.q_col = int(a.q_off); p.k_col = int(a.k_off); p.v_col = int(a.v_off);
-    p.scale_divisor = a.scale_divisor;
-    p.q_cap = sp.q_cap; p.kv_cap = sp.kv_cap; p.q_bound = sp.q_bound; p.kv_bound = sp.kv_bound;
     p.split = a.split_ctx.planes == nullptr ? 0 : (a.split_bf16 ? 1 : 2);
+    p.score_inv = sp.scales->score_inv; p.ctx_inv = sp.scales->ctx_inv;
+    p.v_factor = p.split == 2 ? sp.scales->v_ctx : sp.scales->v_inv;
+    p.score_scale = kLog2e / a.scale_divisor;
     p.so_inv = a.split_ctx.inv;
     p.status = ctx.status;
     tag_launch(ctx, "attention_f16x3_tcgen05", 4.0 * double(a.B) * a.H * double(a.T) * Tk * a.hd,

@@ -128,7 +128,7 @@ struct F16Params {
     int64_t so_plane;
     float *so_inv, *so_amax;
     int so_parts;
-    float so_cap;                 // > 0: one scale for all rows, two fp16 planes (F16GemmArgs::split_cap)
+    int so_cols;                  // columns come scaled, two fp16 planes (F16GemmArgs::col_inv)
     uint32_t* so_bad;
     int bad_rows, bad_block;
     const float *x_amax, *w_bound;
@@ -469,9 +469,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             float rscale = 1.f, rinv = 0.f;
             __half2 rmax = __half2half2(__ushort_as_half(0));   // largest |hi| of the row so far
             auto larger = [](__half2 a, __half2 b) { return larger_half2<IMG>(a, b); };
-            if (!IMG && p.so_cap > 0.f) {
-                split_cap_scale(p.so_cap, p.w_bound, rscale, rinv);
-            } else if (NPL == 2 && p.so != nullptr && !writes_partial && row_ok) {
+            if (NPL == 2 && p.so != nullptr && (IMG || !p.so_cols) && !writes_partial && row_ok) {
                 float am = 0.f;
                 for (int j = 0; j < p.x_parts; j++) am = fmaxf(am, p.x_amax[sx * p.x_parts + j]);
                 float bound = fmaf(am, __ldg(p.w_bound), __ldg(p.w_bound + 1));
@@ -917,7 +915,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll
                         for (int j = 0; j < 4; j++)
                             *reinterpret_cast<float4*>(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                    } else if (NPL == 1 && !(p.so_cap > 0.f)) {
+                    } else if (NPL == 1 && !p.so_cols) {
 #pragma unroll
                         for (int j = 0; j < 2; j++)
                             *reinterpret_cast<uint4*>(stage + lane * 32 + ((j ^ ((lane >> 2) & 1)) << 4)) =
@@ -1024,7 +1022,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 if (p.so == nullptr) {
                     all_groups([&](int g, float (&v)[16]) { finish_fast(g, v, std::integral_constant<int, 0>()); });
                 } else if constexpr (NPL == 1) {
-                    if (p.so_cap > 0.f) all_groups([&](int g, float (&v)[16]) { finish_fast(g, v, std::integral_constant<int, 2>()); });
+                    if (p.so_cols) all_groups([&](int g, float (&v)[16]) { finish_fast(g, v, std::integral_constant<int, 2>()); });
                     else all_groups([&](int g, float (&v)[16]) { finish_fast(g, v, std::integral_constant<int, 1>()); });
                 } else {
                     all_groups([&](int g, float (&v)[16]) { finish_fast(g, v, std::integral_constant<int, 2>()); });
@@ -1034,7 +1032,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             } else {
                 all_groups(finish);
             }
-            if (!IMG && p.so_cap > 0.f) {
+            if (!IMG && p.so_cols) {
                 if (row_ok && !writes_partial && p.so_bad != nullptr && !(__low2float(rmax) <= 65504.f && __high2float(rmax) <= 65504.f))
                     atomicOr(p.so_bad + grow / p.bad_rows, 1u << (grow % p.bad_rows / p.bad_block));
             } else if (NPL == 2 && p.so != nullptr && !writes_partial) {
@@ -1081,7 +1079,7 @@ int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int
 
 // the result as the epilogue stores it: boxes of 32 rows x 16 columns, fp32 (64-byte rows) or split form (32-byte rows, all planes)
 int make_out_map(CUtensorMap* map, const F16GemmArgs& a, int planes) {
-    if (a.split_cap > 0.f) planes = 2;
+    if (a.col_inv != nullptr) planes = 2;
     const auto fn = encode_tiled_fn();
     FXF_CHECK(fn != nullptr, "cuTensorMapEncodeTiled is not available from the CUDA driver");
     const bool split = a.split_out.planes != nullptr;
@@ -1294,7 +1292,7 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     const bool split = a.split_out.planes != nullptr;
     FXF_CHECK(split || a.out != nullptr, "f16 GEMM: no output");
     FXF_CHECK(!split || (a.N % 8 == 0 && a.residual == nullptr && a.vt_out == nullptr), "f16 GEMM: a split output needs N %% 8 == 0 and no residual");
-    FXF_CHECK(!(a.split_cap > 0.f) || (split && im == nullptr && a.w.bound != nullptr && a.bad_rows > 0 && a.bad_block > 0), "f16 GEMM: one scale for all rows needs a split output and the bound of w");
+    FXF_CHECK(a.col_inv == nullptr || (split && im == nullptr && a.col_bias != nullptr && a.bad_rows > 0 && a.bad_block > 0), "f16 GEMM: scaled columns are those of a split output");
     const bool tma_out = split || (a.ldo % 4 == 0 && aligned16(a.out) && (a.residual == nullptr || aligned16(a.residual)));
     const bool lean = !split && !tma_out && a.residual == nullptr;
     const F16Form form = im != nullptr ? F16Form::kImages : (a.bf16 ? F16Form::kBf16 : F16Form::kRows);
@@ -1312,8 +1310,8 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     const Variant& var = kVariants[v];
     const int rows = var.pair ? 2 * BM : BM;
     F16Params p{};
-    p.bias = a.bias; p.residual = a.residual; p.out = a.out;
-    p.x_inv = a.bf16 ? nullptr : a.x.inv; p.w_inv = a.bf16 ? nullptr : a.w.inv;
+    p.bias = a.col_inv != nullptr ? a.col_bias : a.bias; p.residual = a.residual; p.out = a.out;
+    p.x_inv = a.bf16 ? nullptr : a.x.inv; p.w_inv = a.col_inv != nullptr ? a.col_inv : (a.bf16 ? nullptr : a.w.inv);
     p.x_inv_stride = a.x.inv_stride;
     p.w_inv_stride = 1;
     p.M = a.M; p.N = a.N; p.K = a.K; p.ldo = split ? a.N : a.ldo;
@@ -1334,10 +1332,10 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     if (split) {
         p.so = a.split_out.planes; p.so_plane = a.split_out.plane; p.so_inv = a.split_out.inv; p.so_amax = a.split_out.amax;
         p.so_parts = plan.epilogue_warps / 4 * p.tiles_n;
-        p.so_cap = a.split_cap; p.so_bad = a.split_bad; p.bad_rows = a.bad_rows; p.bad_block = a.bad_block;
+        p.so_cols = a.col_inv != nullptr ? 1 : 0; p.so_bad = a.split_bad; p.bad_rows = a.bad_rows; p.bad_block = a.bad_block;
         if (a.split_out.parts_out) *a.split_out.parts_out = p.so_parts;
         p.x_amax = a.x.amax; p.x_parts = a.x.parts; p.w_bound = a.w.bound;
-        FXF_CHECK(a.bf16 || a.split_cap > 0.f || (p.so_inv && p.so_amax && p.x_amax && p.w_bound), "f16 GEMM: a split output needs the row bounds of x and w");
+        FXF_CHECK(a.bf16 || a.col_inv != nullptr || (p.so_inv && p.so_amax && p.x_amax && p.w_bound), "f16 GEMM: a split output needs the row bounds of x and w");
     }
     if (a.vt_out != nullptr) {
         p.vt_out = a.vt_out; p.vt_flags = a.vt_flags; p.vt_col0 = a.vt_col0; p.vt_T = a.vt_T; p.vt_heads = a.vt_heads; p.vt_n32 = a.vt_n32;

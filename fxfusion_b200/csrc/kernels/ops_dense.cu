@@ -100,7 +100,6 @@ struct Slice {
     bool bf16 = false;              // bf16 mode: one bf16 copy instead (hi points to it, lo stays NULL)
     bool mixed = false;             // mixed mode: hi = TF32 high part (fp32), lo -> bf16(w - hi)
     bool f16 = false;               // operand of the f16 GEMM instead: split form (gemm_f16.cu), or its bf16 plane in bf16 mode
-    bool bounded = false;           // its bound is wanted in bf16 mode too
     bool drop = false;              // replaced by "no bias" (rank != 0 of a row-parallel product)
     size_t off_copy = 0, off_split = 0;  // byte offsets inside the plan's persistent memory
     const float *ptr = nullptr, *hi = nullptr, *lo = nullptr;  // resolved by prepare()
@@ -117,6 +116,11 @@ struct DensePlan : NodePlan {
     int64_t M = 0, heads_local = 0, head0 = 0, n_local = 0, col_off = 0;
     size_t cache_off = 0;   // CachedMHA: byte offset of the K/V cache inside the persistent memory
     bool prepared = false;
+    int64_t H_scales = 0;   // > 0: attention that may run on Q, K and V in split form
+    size_t off_scales = 0;
+    AttnScales scales;
+    bool scaled = false;    // it will: `scales` are there
+    bool uneven = false;    // it will not: its columns differ too much in size
     bool bf16_mode = false;   // set by the plan builders from the engine's GEMM mode
     bool mixed_mode = false;  // likewise: FXF_GEMM_TF32_BF16X2
 
@@ -132,7 +136,7 @@ struct DensePlan : NodePlan {
         x.f16 = true;
         x.bf16 = as_bf16;
         x.off_split = persist_bytes;
-        persist_bytes += round_up(size_t(x.elems()) * (as_bf16 ? 2 : 4), 256) + (as_bf16 && !x.bounded ? 1 : 2) * round_up(size_t(x.rows()) * 4, 256) + 256;   // planes, scales, L1 norms, bound
+        persist_bytes += round_up(size_t(x.elems()) * (as_bf16 ? 2 : 4), 256) + (as_bf16 ? 1 : 2) * round_up(size_t(x.rows()) * 4, 256) + 256;   // planes, scales, L1 norms, bound
     }
     void reserve(Slice& x, bool want_split) {
         if (x.drop) return;
@@ -147,6 +151,42 @@ struct DensePlan : NodePlan {
             x.off_split = persist_bytes;
             persist_bytes += round_up(x.bf16 ? size_t(x.elems()) * 2 : size_t(2) * size_t(x.elems()) * sizeof(float), 256);
         }
+    }
+    // MHA and CrossMHA: room for the scales of Q, K and V (AttnScales) behind what the weights take
+    void reserve_scales(int64_t heads) {
+        H_scales = heads;
+        off_scales = persist_bytes;
+        persist_bytes += round_up(size_t(11 * 64 * heads + heads + 2) * sizeof(float), 256);
+    }
+    // Where the rows of every projection come in split form from a LayerNorm.  Run once per engine, which waits for it anyway.
+    int prepare_scales(Registry& reg, const TensorIds& in, ExecCtx& ctx) {
+        const SplitMat *x = split_of(ctx, in[0]), *m = mask_rows_from & 2u ? split_of(ctx, in[1]) : x;
+        if (x == nullptr || m == nullptr || !(x->cap > 0.f) || !(m->cap > 0.f) || x->gamma < 0 || m->gamma < 0) return 0;
+        const int wk = mask_rows_from & 2u ? 2 : 0;
+        if (!s[0].f16 || !s[wk].f16 || s[1].drop) return 0;
+        const int64_t n = 64 * H_scales, k0 = wk == 0 ? n : 0;   // the first of K's rows in its weight
+        float* f = reinterpret_cast<float*>(static_cast<char*>(persist) + off_scales);
+        float* bound = f;
+        auto values = [&](int id) { return static_cast<const float*>(reg[uint32_t(id)].ptr); };
+        if (launch_column_bounds(s[0].ptr, s[0].rows(), s[0].ncol, values(x->gamma), values(x->beta), s[1].ptr, bound, ctx)) return 1;
+        if (wk != 0 && launch_column_bounds(s[wk].ptr, s[wk].rows(), s[wk].ncol, values(m->gamma), values(m->beta), s[wk + 1].ptr, bound + n, ctx)) return 1;
+        scales.bound = bound;
+        scales.col_inv = f + 3 * n; scales.col_bias = f + 6 * n;
+        scales.v_inv = f + 9 * n; scales.v_ctx = f + 10 * n;
+        scales.score_inv = f + 11 * n; scales.ctx_inv = scales.score_inv + H_scales;
+        scales.unusable = reinterpret_cast<int*>(scales.ctx_inv + 1);
+        scales.q_winv = s[0].bf16 ? nullptr : s[0].mat.inv;
+        scales.kv_winv = s[wk].bf16 ? nullptr : s[wk].mat.inv + k0;
+        scales.q_bias = s[1].ptr; scales.kv_bias = s[wk + 1].ptr + k0;
+        scales.H = int(H_scales);
+        FXF_CUDA(cudaMemsetAsync(scales.unusable, 0, sizeof(int), ctx.stream));
+        if (launch_attention_scales(scales, ctx)) return 1;
+        int unusable = 1;
+        FXF_CUDA(cudaMemcpyAsync(&unusable, scales.unusable, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
+        FXF_CUDA(cudaStreamSynchronize(ctx.stream));
+        scaled = unusable == 0;
+        uneven = !scaled;
+        return 0;
     }
     int prepare(Registry& reg, const TensorIds& in, const TensorIds&, const Params&, ExecCtx& ctx) override {
         for (int i = 0; i < n; i++) {
@@ -175,7 +215,7 @@ struct DensePlan : NodePlan {
                 o.plane = x.elems();
                 o.inv = reinterpret_cast<float*>(base + round_up(size_t(x.elems()) * (x.bf16 ? 2 : 4), 256));
                 float* bound = reinterpret_cast<float*>(reinterpret_cast<char*>(o.inv) + round_up(size_t(x.rows()) * 4, 256));
-                if (launch_split_rows(x.ptr, x.ncol, x.rows(), x.ncol, x.bf16, o, x.bf16 && !x.bounded ? nullptr : x.l1(bound), ctx)) return 1;
+                if (launch_split_rows(x.ptr, x.ncol, x.rows(), x.ncol, x.bf16, o, x.bf16 ? nullptr : x.l1(bound), ctx)) return 1;
                 x.mat = SplitMat{};
                 x.mat.planes = o.planes; x.mat.plane = o.plane; x.mat.inv = o.inv; x.mat.bound = bound;
             }
@@ -198,10 +238,11 @@ struct DensePlan : NodePlan {
             }
         }
         for (int i = 0; i + 1 < n; i++)   // a weight's bias follows it
-            if (s[i].f16 && (!s[i].bf16 || s[i].bounded)) {
+            if (s[i].f16 && !s[i].bf16) {
                 float* bound = const_cast<float*>(s[i].mat.bound);
                 if (launch_weight_bound(s[i].l1(bound), s[i].rows(), s[i + 1].drop ? nullptr : s[i + 1].ptr, s[i + 1].rows(), bound, ctx)) return 1;
             }
+        if (H_scales > 0 && prepare_scales(reg, in, ctx)) return 1;
         prepared = true;
         return 0;
     }
@@ -220,8 +261,7 @@ bool want_f16(const PlanEnv& env, int64_t M, int64_t N, int64_t K) {
 }
 // A weight's bias is the input after it.  Both have to be constants for split form: its conversion happens at build time and
 // includes a bound of the bias, and the few-row kernel reads both ahead of the end of the kernel before it.
-void reserve_weight(DensePlan& p, Slice& w, const TensorIds& in, const PlanEnv& env, int64_t M, int64_t N, int64_t K, bool bounded = false) {
-    w.bounded = bounded;
+void reserve_weight(DensePlan& p, Slice& w, const TensorIds& in, const PlanEnv& env, int64_t M, int64_t N, int64_t K) {
     const bool constant = env.is_constant(in[size_t(w.input)]);
     if (constant && env.is_constant(in[size_t(w.input) + 1]) && want_f16(env, M, N, K)) p.reserve_f16(w, p.bf16_mode && M > kFewRows);
     else p.reserve(w, constant && want_tc(env, M, N, K));
@@ -529,16 +569,14 @@ SplitMat context_in_split_form(AttnArgs& a, const Slice& wv, const Slice& wo, co
     return m;
 }
 
-// A projection whose result only the attention core reads leaves it in split form under one scale for all rows, where its own rows
-// come so from a LayerNorm, which caps them.
-bool projects_in_split_form(const Slice& w, const SplitMat* rows, int64_t M) {
-    return w.f16 && M > kFewRows && rows != nullptr && rows->cap > 0.f && w.mat.bound != nullptr && w.rows() % 16 == 0 && (!w.bf16 || w.bounded);
-}
-// rows_per: rows per batch; block: rows per bit of `bad`
-void into_split_form(F16GemmArgs& f, const Slice& w, const SplitMat& rows, float* dst, int64_t M, uint32_t* bad, int64_t rows_per, int block) {
+// A projection whose result only the attention core reads leaves it in split form, where its own rows come so from a LayerNorm, which bounds
+// what each column can hold (DensePlan::prepare_scales).  first: of the columns of Q, K and V; rows_per: rows per batch; block:
+// rows per bit of `bad`
+void into_split_form(F16GemmArgs& f, const DensePlan& pl, const Slice& w, int64_t first, float* dst, int64_t M, uint32_t* bad, int64_t rows_per, int block) {
     f.split_out.planes = reinterpret_cast<uint16_t*>(dst);
     f.split_out.plane = M * w.rows();
-    f.split_cap = rows.cap;
+    f.col_inv = pl.scales.col_inv + first;
+    f.col_bias = pl.scales.col_bias + first;
     f.split_bad = bad;
     f.bad_rows = int(rows_per);
     f.bad_block = block;
@@ -587,16 +625,15 @@ int k_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const Params
 
     bool v_transposed = false;
     const SplitMat* xs = split_of(ctx, in[0]);
-    const bool split_qkv = ctx.mask_bits.bits != nullptr && have_vt && Hl == H && attention_f16_ok(T, T, hd, p.floats[0]) && projects_in_split_form(pl->s[0], xs, M);
+    const bool split_qkv = ctx.mask_bits.bits != nullptr && have_vt && Hl == H && attention_f16_ok(T, T, hd, p.floats[0]) && pl->scaled && xs != nullptr;
     AttnSplit sp;
     sp.mask = &ctx.mask_bits;
     if (split_qkv) {
         F16GemmArgs f;
-        into_split_form(f, pl->s[0], *xs, qkv, M, ctx.mask_bits.bad, T, attention_f16_block(T));
+        into_split_form(f, *pl, pl->s[0], 0, qkv, M, ctx.mask_bits.bad, T, attention_f16_block(T));
         sp.q = sp.kv = f.split_out.planes;
         sp.q_plane = sp.kv_plane = f.split_out.plane;
-        sp.q_cap = sp.kv_cap = xs->cap;
-        sp.q_bound = sp.kv_bound = pl->s[0].mat.bound;
+        sp.scales = &pl->scales;
         if (f16_product(pl->s[0], &pl->s[1], nullptr, D, xs, nullptr, M, QKVl, false, false, area, ctx, &f)) return 1;
     } else if (pl->s[0].f16) {
         F16GemmArgs f;
@@ -639,7 +676,7 @@ int k_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const Params
         cs = context_in_split_form(a, pl->s[0], pl->s[2], xs, cx, area, M, D);
         if (launch_attention_f16(a, sp, ctx)) return 1;
     } else if (have_vt && attention_tc_supported(a, ctx.gemm_mode)) {
-        cs = context_in_split_form(a, pl->s[0], pl->s[2], xs, cx, area, M, D);
+        cs = context_in_split_form(a, pl->s[0], pl->s[2], pl->uneven ? nullptr : xs, cx, area, M, D);
         if (launch_attention_tc(a, vt, ctx, v_transposed)) return 1;
     } else {
         FXF_CHECK(!v_transposed, "mha: the projection wrote V transposed but the tensor-core attention kernel cannot run");
@@ -685,7 +722,7 @@ std::unique_ptr<NodePlan> plan_mha(const Registry& reg, const TensorIds& in, con
     } else if (env.tp_size > 1) {
         pl->variant = "replicated ";
     }
-    reserve_weight(*pl, s_wq, in, env, M, 3 * Dl, D, hd == 64);
+    reserve_weight(*pl, s_wq, in, env, M, 3 * Dl, D);
     pl->reserve(s_bq, false);
     reserve_weight(*pl, s_wo, in, env, M, D, Dl);
     pl->reserve(s_bo, false);
@@ -695,6 +732,7 @@ std::unique_ptr<NodePlan> plan_mha(const Registry& reg, const TensorIds& in, con
     if (s_wq.f16) pl->takes_split = takes_split_rows(env, M, 3 * Dl) ? 1 : 0;
     pl->takes_norm = takes_norm(env, s_wq, M, 3 * Dl, D);
     if (n == 1 && s_wq.f16 && M > kFewRows && p.floats.size() >= 1 && attention_f16_ok(T, T, hd, p.floats[0])) {
+        pl->reserve_scales(Hl);
         pl->mask_input = 1;
         pl->mask_B = B; pl->mask_T = T; pl->mask_Tk = T;
         pl->mask_rows_from = 1u;
@@ -763,7 +801,7 @@ int k_cross_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const 
     F16GemmArgs vt_args;
     bool v_transposed = false;
     const SplitMat *xs = split_of(ctx, in[0]), *ms_rows = split_of(ctx, in[1]);
-    const bool split_qkv = ctx.mask_bits.bits != nullptr && have_vt && Hl == H && attention_f16_ok(Tq, Tk, hd, p.floats[0]) && projects_in_split_form(pl->s[0], xs, Mq) && projects_in_split_form(pl->s[2], ms_rows, Mk);
+    const bool split_qkv = ctx.mask_bits.bits != nullptr && have_vt && Hl == H && attention_f16_ok(Tq, Tk, hd, p.floats[0]) && pl->scaled && xs != nullptr && ms_rows != nullptr;
     if (!split_qkv && pl->s[2].f16 && have_vt && hd == 64 && Mk > kFewRows && Tk >= 16 && Tk <= 4096) {
         F16GemmArgs& f = vt_args;
         f.M = Mk; f.N = 2 * Dl; f.K = D;
@@ -786,10 +824,11 @@ int k_cross_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const 
     sp.mask = &ctx.mask_bits;
     if (split_qkv) {
         F16GemmArgs fq, fkv;
-        into_split_form(fq, pl->s[0], *xs, q, Mq, nullptr, 1, 1);   // (nobody asks whether Q is finite)
-        into_split_form(fkv, pl->s[2], *ms_rows, kv, Mk, ctx.mask_bits.bad, Tk, attention_f16_block(Tk));
-        sp.q = fq.split_out.planes; sp.q_plane = fq.split_out.plane; sp.q_cap = xs->cap; sp.q_bound = pl->s[0].mat.bound;
-        sp.kv = fkv.split_out.planes; sp.kv_plane = fkv.split_out.plane; sp.kv_cap = ms_rows->cap; sp.kv_bound = pl->s[2].mat.bound;
+        into_split_form(fq, *pl, pl->s[0], 0, q, Mq, nullptr, 1, 1);   // (nobody asks whether Q is finite)
+        into_split_form(fkv, *pl, pl->s[2], Dl, kv, Mk, ctx.mask_bits.bad, Tk, attention_f16_block(Tk));
+        sp.q = fq.split_out.planes; sp.q_plane = fq.split_out.plane;
+        sp.kv = fkv.split_out.planes; sp.kv_plane = fkv.split_out.plane;
+        sp.scales = &pl->scales;
         if (f16_product(pl->s[0], &pl->s[1], nullptr, D, xs, nullptr, Mq, Dl, false, false, area, ctx, &fq)) return 1;
         if (f16_product(pl->s[2], &pl->s[3], nullptr, D, ms_rows, nullptr, Mk, 2 * Dl, false, false, area, ctx, &fkv)) return 1;
     } else {
@@ -813,7 +852,7 @@ int k_cross_mha(Registry& reg, const TensorIds& in, const TensorIds& out, const 
             cs = context_in_split_form(a, pl->s[2], pl->s[4], ms_rows, cx, area, Mq, D);
             if (launch_attention_f16(a, sp, ctx)) return 1;
         } else if (have_vt && attention_tc_supported(a, ctx.gemm_mode)) {
-            cs = context_in_split_form(a, pl->s[2], pl->s[4], ms_rows, cx, area, Mq, D);
+            cs = context_in_split_form(a, pl->s[2], pl->s[4], pl->uneven ? nullptr : ms_rows, cx, area, Mq, D);
             if (launch_attention_tc(a, vt, ctx, v_transposed)) return 1;
         } else {
             FXF_CHECK(!v_transposed, "cross_mha: the projection wrote V transposed but the tensor-core attention kernel cannot run");
@@ -867,9 +906,9 @@ std::unique_ptr<NodePlan> plan_cross_mha(const Registry& reg, const TensorIds& i
     } else if (env.tp_size > 1) {
         pl->variant = "replicated ";
     }
-    reserve_weight(*pl, s_wq, in, env, Mq, Dl, D, hd == 64);
+    reserve_weight(*pl, s_wq, in, env, Mq, Dl, D);
     pl->reserve(s_bq, false);
-    reserve_weight(*pl, s_wkv, in, env, Mk, 2 * Dl, D, hd == 64);
+    reserve_weight(*pl, s_wkv, in, env, Mk, 2 * Dl, D);
     pl->reserve(s_bkv, false);
     reserve_weight(*pl, s_wo, in, env, Mq, D, Dl);
     pl->reserve(s_bo, false);
@@ -878,6 +917,7 @@ std::unique_ptr<NodePlan> plan_cross_mha(const Registry& reg, const TensorIds& i
     if (s_wq.f16 || s_wkv.f16 || s_wo.f16) pl->scratch_bytes += split_area_bytes(std::max(Mq, Mk), D);
     pl->takes_split = (s_wq.f16 && takes_split_rows(env, Mq, Dl) ? 1u : 0u) | (s_wkv.f16 && takes_split_rows(env, Mk, 2 * Dl) ? 2u : 0u);
     if (n == 1 && s_wq.f16 && s_wkv.f16 && Mq > kFewRows && Mk > kFewRows && p.floats.size() >= 1 && attention_f16_ok(Tq, Tk, hd, p.floats[0])) {
+        pl->reserve_scales(Hl);
         pl->mask_input = 2;
         pl->mask_B = B; pl->mask_T = Tq; pl->mask_Tk = Tk;
         pl->mask_rows_from = 3u;

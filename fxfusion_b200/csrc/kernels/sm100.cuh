@@ -135,8 +135,6 @@ __device__ __forceinline__ void split_scale(float bound, float& scale, float& in
     scale = __int_as_float((268 - e) << 23);
     inv = __int_as_float((e - 14) << 23);
 }
-// One scale for all rows of a product, from |x| <= cap: bound = {largest L1 norm of a weight row, largest |bias|} (SplitMat::cap, bound).
-__device__ __forceinline__ void split_cap_scale(float cap, const float* bound, float& scale, float& inv) { split_scale(fmaf(cap, __ldg(bound), __ldg(bound + 1)) * 1.001f, scale, inv); }
 __device__ __forceinline__ void split_f16x2(float x, float y, uint32_t& hi, uint32_t& lo) {
     const __half2 h = __floats2half2_rn(x, y);
     const float2 f = __half22float2(h);

@@ -90,6 +90,7 @@ struct SplitMat {
     const float* amax = nullptr;        // activations: max_k |x[r,k]| as `parts` partial maxima per row
     int parts = 1;
     float cap = 0.f;                    // activations: no |x| exceeds it whatever the input (normalised rows); 0: unknown
+    int gamma = -1, beta = -1;          // with a cap: the tensors (constants) that a LayerNorm multiplied and shifted the rows with
     const float* bound = nullptr;       // weights: {max_j ||w_j||_1, max_j |b_j|}
 };
 struct SplitOut {
@@ -382,10 +383,10 @@ struct F16GemmArgs {
     NormInput norm;                     // few-row products (x as fp32 rows): gamma != NULL: the rows are normalised first
     float* out = nullptr;               // fp32 result, or
     SplitOut split_out;                 // the result in split form (pitch N)
-    // > 0: ONE scale for all rows of the split result, from |x| <= split_cap and w.bound (split_cap_scale); two fp16 planes in the bf16
-    // mode too.  No scales or maxima are written.  Where a value of row r is NaN or infinite, bit r % bad_rows / bad_block of
-    // split_bad[r / bad_rows] is set.
-    float split_cap = 0.f;
+    // != NULL: the columns of the split result come scaled, 1 / scale of a row of w times the column's factor in col_inv, the bias times it in
+    // col_bias (which stand for w.inv and bias); two fp16 planes in the bf16 mode too.  No scales or maxima of rows are written.  Where a
+    // value of row r is NaN or infinite, bit r % bad_rows / bad_block of split_bad[r / bad_rows] is set.
+    const float *col_inv = nullptr, *col_bias = nullptr;
     uint32_t* split_bad = nullptr;
     int bad_rows = 1, bad_block = 1;
     int64_t M = 0, N = 0, K = 0, ldo = 0;
@@ -437,6 +438,20 @@ int gemm_f16_split_parts(int64_t N);    // partial maxima per row a split output
 // kernels/split_form.cu.  l1_out (weights): the L1 norm of each row; bound = {largest of them, largest |bias|} (SplitMat::bound).
 int launch_split_rows(const float* x, int64_t ld, int64_t M, int64_t K, bool bf16, const SplitOut& out, float* l1_out, ExecCtx& ctx);
 int launch_weight_bound(const float* l1, int64_t rows, const float* bias, int64_t n, float* bound, ExecCtx& ctx);
+// bound[n]: no |w_n · x + bias_n| exceeds it, x a row that a LayerNorm of width K with this gamma and beta has written
+int launch_column_bounds(const float* w, int64_t rows, int64_t K, const float* gamma, const float* beta, const float* bias, float* bound, ExecCtx& ctx);
+// The scales of Q, K and V in split form (kernels/attention_f16.cu), H heads of 64 columns: a power of two for each column of each.
+// Arrays of 3 * 64 * H: Q's columns, K's, V's.  w_inv: 1 / scale of the weights' rows (NULL: 1), for Q, and for K and V.
+struct AttnScales {
+    const float *bound = nullptr, *q_winv = nullptr, *kv_winv = nullptr, *q_bias = nullptr, *kv_bias = nullptr;
+    float *col_inv = nullptr, *col_bias = nullptr;   // F16GemmArgs
+    float *score_inv = nullptr;                      // [H]: 1 / (scale of Q times scale of K), the same for all columns of a head
+    float *v_inv = nullptr, *v_ctx = nullptr;        // [64 * H]: 1 / scale of V's columns; the same times the one scale of a context in split form
+    float* ctx_inv = nullptr;                        // 1 / the latter
+    int* unusable = nullptr;                         // set where a column's size is beyond what scales can serve
+    int H = 0;
+};
+int launch_attention_scales(const AttnScales& s, ExecCtx& ctx);
 // M <= 64 rows in fp32 FFMA (kernels/gemm_lanes.cu): w as the graph has it; of `a` the sizes, bias, residual, output and ReLU count
 bool gemm_lanes_better(int64_t M, int64_t N, int64_t K, int sm_count);   // than the kernels on split form
 int launch_gemm_lanes(const F16GemmArgs& a, const float* w, const float* x, int64_t ldx, ExecCtx& ctx);
@@ -553,14 +568,13 @@ int tp_all_gather(const void* send, void* recv, int64_t bytes, ExecCtx& ctx);
 // tcgen05 path (head_dim 64): needs 6*B*T*H*64 floats of scratch for the split, per-head operand copies
 bool attention_tc_supported(const AttnArgs& a, int gemm_mode);
 size_t attention_tc_scratch_bytes(int64_t B, int64_t T, int64_t H);
-// Attention on Q, K and V in split form under one scale each (kernels/attention_f16.cu).  The fields of AttnArgs name the layout
-// (ld_qkv, ld_kv, offsets in elements of a plane; kv != NULL marks cross-attention), these the data: the scale of Q follows from
-// q_cap and q_bound (split_cap_scale), of K and V from kv_cap and kv_bound.  The projections have put what is not finite into mask->bad.
+// Attention on Q, K and V in split form, a scale per column (kernels/attention_f16.cu).  The fields of AttnArgs name the layout
+// (ld_qkv, ld_kv, offsets in elements of a plane; kv != NULL marks cross-attention), these the data.  The projections have put what is
+// not finite into mask->bad.
 struct AttnSplit {
     const uint16_t *q = nullptr, *kv = nullptr;
     int64_t q_plane = 0, kv_plane = 0;
-    float q_cap = 0.f, kv_cap = 0.f;
-    const float *q_bound = nullptr, *kv_bound = nullptr;
+    const AttnScales* scales = nullptr;
     const MaskBits* mask = nullptr;
 };
 int attention_f16_block(int64_t Tk);   // keys per block

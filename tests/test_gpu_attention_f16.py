@@ -96,8 +96,7 @@ def test_masked_keys_do_not_move_a_bit(built_lib, tmp_path):
 
 
 @pytest.mark.parametrize("cross", [False, True])
-@pytest.mark.parametrize("r", [1.0, 16.0, 1024.0, 3e5])
-@pytest.mark.parametrize("what", ["thirds", "heads", "columns"])
+@pytest.mark.parametrize("what,r", [(w, r) for w in ("thirds", "heads", "columns") for r in (1.0, 16.0, 1024.0, 3e5)] + [("thirds", 1e21)])
 def test_uneven_sizes(built_lib, tmp_path, what, r, cross):
     """Q's weights divided and K's multiplied by the same factors, which leaves the function as it is: all of them by r, or by r in one head and 1 / r
     in the next, or every column by a factor of its own up to r.  Against fp64: Q, K and V keep 22 bits of what they add to a score, sum |q_d k_d| / 8
@@ -137,7 +136,10 @@ def test_uneven_sizes(built_lib, tmp_path, what, r, cross):
     heads = lambda t, i: (t @ d(w[i]).T + d(bias[i])).view(B, -1, H, 64).transpose(1, 2)
     s = (heads(ln(xin), 0) @ heads(rows, 1).transpose(-1, -2) / 8.0).masked_fill(~mask, float("-inf"))
     want = (torch.softmax(s, -1) @ heads(rows, 2)).transpose(1, 2).reshape(B, T, D) @ d(w[3]).T + d(bias[3])
-    assert ((got - want).norm() / want.norm()).item() < 2.0 ** -18
-    assert any("attention_f16x3" in q["kernel"] for q in eng.profile_launches())
+    # (what scales of fp16 pairs cannot serve runs on the kernel for fp32 rows, whose 19 bits count here as 22 do above: 2^-15)
+    beyond = r > 1e20
+    assert ((got - want).norm() / want.norm()).item() < 2.0 ** (-15 if beyond else -18)
+    kernels = [q["kernel"] for q in eng.profile_launches()]
+    assert any(("attention_tf32" if beyond else "attention_f16x3") in k for k in kernels), kernels
     assert eng.device_status() == 0
     eng.close()
