@@ -1286,6 +1286,15 @@ static int clusters_resident(int cs, int* out) {
     return 0;
 }
 
+// The launch of a product whose tiles are cut inside clusters, by the width of its tiles and the number of parts
+static const char* cut_tag(bool images, int bn, int parts) {
+#define FXF_CUT(name, bn) {name "_" #bn "_cut2", name "_" #bn "_cut3", name "_" #bn "_cut4", name "_" #bn "_cut5", name "_" #bn "_cut6", name "_" #bn "_cut7", name "_" #bn "_cut8"}
+    static const char* const names[2][3][kMaxClusterK - 1] = {{FXF_CUT("gemm_f16x3_tcgen05", 32), FXF_CUT("gemm_f16x3_tcgen05", 64), FXF_CUT("gemm_f16x3_tcgen05", 128)},
+                                                              {FXF_CUT("conv2d_f16x3_tcgen05", 32), FXF_CUT("conv2d_f16x3_tcgen05", 64), FXF_CUT("conv2d_f16x3_tcgen05", 128)}};
+#undef FXF_CUT
+    return names[images ? 1 : 0][bn == 32 ? 0 : (bn == 64 ? 1 : 2)][parts - 2];
+}
+
 static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorMap* im2col, const char* tag, double flops, ExecCtx& ctx) {
     FXF_CHECK(gemm_f16_shape_ok(a.M, a.N, a.K) && a.x.planes && a.w.planes && aligned16(a.x.planes) && aligned16(a.w.planes) && (a.x.plane * 2) % 16 == 0,
               "f16 GEMM: unsupported operands (M=%lld N=%lld K=%lld)", (long long)a.M, (long long)a.N, (long long)a.K);
@@ -1340,7 +1349,7 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     if (a.vt_out != nullptr) {
         p.vt_out = a.vt_out; p.vt_flags = a.vt_flags; p.vt_col0 = a.vt_col0; p.vt_T = a.vt_T; p.vt_heads = a.vt_heads; p.vt_n32 = a.vt_n32;
     }
-    tag_launch(ctx, tag, flops, 4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.N) + double(a.M) * a.N));
+    tag_launch(ctx, plan.cluster > 1 ? cut_tag(im != nullptr, var.bn, plan.cluster) : tag, flops, 4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.N) + double(a.M) * a.N));
     if (a.bf16) {
         switch (v) {
             case 0:
