@@ -1284,7 +1284,10 @@ int fxf_engine_describe(const fxf_engine* e, char* out, size_t out_bytes) {
             os << " +exchange(residual " << n.xchg_res << ") -> x " << n.xchg_x << (n.xchg_x >= 0 ? (n.xchg_replicate_x ? " [all rows on every rank]" : " [own rows]") : "")
                << " y " << n.xchg_y;
         if (n.splits) os << " output in split form";
-        if (n.folded) os << " folded into an earlier node";
+        if (n.mask_off != 0 && n.plan->scaled) os << " on Q, K and V in split form";
+        if (n.norm_of >= 0) os << " +LayerNorm(node " << n.norm_of << ")";
+        const bool norm_later = n.folded && std::any_of(e->nodes.begin(), e->nodes.end(), [&](const Node& r) { return r.norm_of == int(i); });
+        if (n.folded) os << (norm_later ? " folded into a later node" : " folded into an earlier node");
         os << "\n";
     }
     std::string s = os.str();

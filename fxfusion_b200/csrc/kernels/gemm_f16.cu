@@ -1245,6 +1245,9 @@ static F16Plan plan_launch(int64_t M, int64_t N, int64_t K, F16Form form, bool l
 }
 F16Plan gemm_f16_plan(int64_t M, int64_t N, int64_t K, F16Form form, const F16Limits& lim) { return plan_launch(M, N, K, form, false, false, 0, lim); }
 
+// One round of the widest single-CTA tiles at most: more tiles than SMs are more than a round.
+bool gemm_f16_may_cut(int64_t M, int64_t N, int sm_count) { return (M + BM - 1) / BM * ((N + 127) / 128) < sm_count; }
+
 std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, int sm_count) {
     const int v = pick_variant(M, N, K, sm_count, true, true, false, 0, bf16 ? kBf16Variants : kVariants, nullptr, nullptr);
     if (v < 0) return "none";
@@ -1309,7 +1312,7 @@ static int launch_f16(const F16GemmArgs& a, const ImageGeom* im, const CUtensorM
     lim.sm_count = ctx.sm_count; lim.pairs = ctx.tc_pair != 1; lim.chunk_k = ctx.tc_chunk_k;
     if (ctx.gemm_ws != nullptr && ctx.gemm_flags != nullptr) { lim.ws_bytes = ctx.gemm_ws_bytes; lim.flag_count = ctx.gemm_flag_count; }
     int clusters[kMaxClusterK + 1] = {};
-    if (!a.bf16 && (a.M + BM - 1) / BM * ((a.N + 127) / 128) < ctx.sm_count)   // (more tiles than SMs: more than a round)
+    if (!a.bf16 && gemm_f16_may_cut(a.M, a.N, ctx.sm_count))
         for (int cs = 2; cs <= kMaxClusterK; cs++)
             if (clusters_resident(cs, &clusters[cs])) return 1;
     lim.clusters = clusters;

@@ -119,8 +119,7 @@ struct DensePlan : NodePlan {
     int64_t H_scales = 0;   // > 0: attention that may run on Q, K and V in split form
     size_t off_scales = 0;
     AttnScales scales;
-    bool scaled = false;    // it will: `scales` are there
-    bool uneven = false;    // it will not: its columns differ too much in size
+    bool uneven = false;    // its columns differ too much in size for that
     bool bf16_mode = false;   // set by the plan builders from the engine's GEMM mode
     bool mixed_mode = false;  // likewise: FXF_GEMM_TF32_BF16X2
 
@@ -279,7 +278,8 @@ std::string variant_of(const PlanEnv& env, const Slice& w, int64_t M, int64_t N,
     std::string v = gemm_variant_name(g, w.f16 || w.split ? env.gemm_mode : FXF_GEMM_FP32_SIMT, env.sm_count, env.tc_pairs);
     if (!w.f16) return v;
     const bool lanes = M <= kFewRows && !gemm_rows_streams(M, N, env.sm_count) && gemm_lanes_better(M, N, K, env.sm_count);
-    return v + " (split operands: tcgen05-" + (M > kFewRows ? gemm_f16_variant_name(M, N, K, w.bf16, env.sm_count) : std::string(takes_split_rows(env, M, N) ? "f16x3-stream128" : "f16x3-rows128")) + (lanes ? "; at this number of rows ffma-lanes)" : ")");
+    const bool may_cut = M > kFewRows && !w.bf16 && gemm_f16_may_cut(M, N, env.sm_count);
+    return v + " (split operands: tcgen05-" + (M > kFewRows ? gemm_f16_variant_name(M, N, K, w.bf16, env.sm_count) : std::string(takes_split_rows(env, M, N) ? "f16x3-stream128" : "f16x3-rows128")) + (lanes ? "; at this number of rows ffma-lanes)" : (may_cut ? "; or narrower tiles, cut along K inside clusters: the launch decides and is named so)" : ")"));
 }
 
 // Room for an activation matrix that has to be split before its product: planes, scales, row maxima.

@@ -190,6 +190,7 @@ struct NodePlan {
     int mask_input = -1;
     int64_t mask_B = 0, mask_T = 0, mask_Tk = 0;
     uint32_t mask_rows_from = 0;   // the inputs that have to arrive in split form for that, a bit each
+    bool scaled = false;           // found by prepare(): Q, K and V have scales, the node runs so wherever the engine keeps the mask's bits
     bool images = false;        // decided by the engine before prepare(): the node runs on them
     size_t scratch_bytes = 0;   // shared scratch wanted at execute time
     size_t persist_bytes = 0;   // memory that must survive across runs (e.g. re-laid-out weights)
@@ -413,7 +414,8 @@ int launch_conv_f16(const ConvF16Args& a, ExecCtx& ctx);
 bool gemm_f16_shape_ok(int64_t M, int64_t N, int64_t K);
 bool gemm_f16_vt_ok(const F16GemmArgs& a, const ExecCtx& ctx);
 int launch_gemm_f16(const F16GemmArgs& a, ExecCtx& ctx);
-std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, int sm_count);
+std::string gemm_f16_variant_name(int64_t M, int64_t N, int64_t K, bool bf16, int sm_count);   // of tiles that are not cut inside clusters
+bool gemm_f16_may_cut(int64_t M, int64_t N, int sm_count);   // the launch asks the device how many clusters it holds, and may cut
 // How a product in split form is launched, and what it uses of the K-split workspace (host side, no device needed).
 enum class F16Form { kRows, kBf16, kImages };
 struct F16Limits {

@@ -252,7 +252,7 @@ FXF_API int fxf_gemm_variant(int64_t M, int64_t N, int64_t K, int gemm_mode, int
 
 /* What a product on operands in split form (FXF_GEMM_AUTO, FXF_GEMM_BF16; images = 1: a convolution, M pixels by N output
  * channels by K) writes of the engine's workspace for tiles cut along K — partial tiles in bytes, ready flags — and how much
- * of each an engine with `sm_count` SMs (0 = 148) keeps.  tc_chunk_k as in FxfEngineOptions.  Pure host code, for tests. */
+ * of each an engine with `sm_count` SMs (0 = 148) keeps.  Tiles that a launch cuts inside clusters instead use none of it.  tc_chunk_k as in FxfEngineOptions.  Pure host code, for tests. */
 FXF_API int fxf_gemm_workspace(int64_t M, int64_t N, int64_t K, int gemm_mode, int images, int tc_chunk_k, int sm_count,
                                int64_t* bytes, int64_t* bytes_kept, int64_t* flags, int64_t* flags_kept);
 

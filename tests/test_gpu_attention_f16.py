@@ -139,6 +139,7 @@ def test_uneven_sizes(built_lib, tmp_path, what, r, cross):
     # (what scales of fp16 pairs cannot serve runs on the kernel for fp32 rows, whose 19 bits count here as 22 do above: 2^-15)
     beyond = r > 1e20
     assert ((got - want).norm() / want.norm()).item() < 2.0 ** (-15 if beyond else -18)
+    assert ("on Q, K and V in split form" in eng.describe()) != beyond, eng.describe()
     kernels = [q["kernel"] for q in eng.profile_launches()]
     assert any(("attention_tf32" if beyond else "attention_f16x3") in k for k in kernels), kernels
     assert eng.device_status() == 0

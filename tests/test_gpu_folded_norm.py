@@ -40,7 +40,20 @@ def test_folded(built_lib, tmp_path, M, N, K, op):
     xin = (torch.randn(M, K, generator=gen) + 2) * torch.logspace(-1, 3, M).reshape(M, 1)   # rows of very different size, away from zero
     got, want, kernels, eng = _run(b, tmp_path, [xin])
     assert "LayerNorm" not in kernels, kernels
+    lines = eng.describe().splitlines()[-3:]
+    assert lines[0].endswith("folded into a later node") and "+LayerNorm(node 0)" in lines[1], lines
     ok, info = compare_outputs(got[0], want[0], atol=5e-5, rtol=2e-4)
+    assert ok, info
+    # a row without variance is beta whatever its value; a row with a NaN or an infinity is NaN and no other is touched
+    xin[0] = 0.5
+    if M > 2:
+        xin[1, K // 2], xin[2, 0] = float("nan"), float("inf")
+    got, want = eng.run([xin.cuda()])[0].cpu(), GraphOracle(str(tmp_path / "g.bin")).run([xin])[0]
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.isnan(want).any() == (M > 2)
+    # a mean off by an ulp leaves 0.5 * 2^-24 / sqrt(1e-5) = 1e-5 in every element of the constant row: at most ten times that behind the products
+    ok, info = compare_outputs(got[0], want[0], atol=1.5e-4, rtol=2e-4)
+    assert ok, info
+    ok, info = compare_outputs(got[3:], want[3:], atol=5e-5, rtol=2e-4)
     assert ok, info
     eng.close()
 
