@@ -37,7 +37,7 @@ namespace {
 using namespace sm100;
 
 constexpr int HD = 64, BQ = 128, kThreads = 320, kSoftWarp0 = 2;
-constexpr int kMaxKeys = 2048;   // key blocks are tracked in one 32-bit word (32 x 64 at least)
+constexpr int kMaxKeys = 2048;   // 16 blocks of 128; the words that track key blocks have room for 32, but more has not been measured against attention_tc.cu
 constexpr float kLog2e = 1.4426950408889634f;
 enum : int { kErrAttnF16Load = 151, kErrAttnF16S = 152, kErrAttnF16P = 153, kErrAttnF16O = 154 };
 
