@@ -211,7 +211,7 @@ LanesPlan plan(int64_t M, int64_t N, int64_t K, int sm_count) {
             for (int c : {1, 2, 4, 8}) {
                 const int64_t cb = int64_t(cg) * c, ctas = (N + cb - 1) / cb * ((M + r - 1) / r);
                 const size_t smem = size_t(cb + r) * size_t(K) * 4;
-                if (smem > kSmemLimit) continue;
+                if (smem > kSmemLimit || ctas > 2 * sm_count) continue;
                 const double per_sm = double((ctas + sm_count - 1) / sm_count), fill = std::min(1.0, double(ctas) / sm_count), k = double(K) / cycles;
                 const double us = 1.7 + per_sm * (std::max(1.6 * r * double(cb) * k / 128, 0.8 * cg * (r + c) * k * 4 / 128) + (2.1 * r + 0.4 * double(cb)) * k * 4 / 50) + 0.4 * r * c / 64 + 0.25 * fill + (cg < kWarps ? 0.08 : 0.0);
                 if (best.kernel == nullptr || us < best.us) {
@@ -228,7 +228,12 @@ LanesPlan plan(int64_t M, int64_t N, int64_t K, int sm_count) {
 // Against gemm_rows.cu, whose time in the same chains is 2.45 us + 1.15 per 1000 of K + 0.3 per 1000 of N + 0.062 per row from 9 on (within
 // 15 %; the modelled minimum above is 5 to 15 % below what its tile measures).  us per launch, that kernel and this one:  1 row: 512 x 512 3.3, 2.0; 3072 x 768 4.9, 2.9; 768 x 3072 6.1, 3.5;  8 rows: 512 x 512 3.3, 2.9;
 // 768 x 3072 6.2, 5.7;  32 rows: 256 x 256 4.9, 2.8; 512 x 512 4.6, 3.7; 768 x 768 5.1, 4.6; but 2304 x 768 6.7, 6.7 and 768 x 3072 7.1, 16.0.
+// Neither formula knows what a CTA pays for its outputs, nor that a narrow product's clusters grow with K, so they count only inside what has been
+// measured (42 shapes of 16 to 18000 columns, K 16 to 4096, 12 numbers of rows from 1 to 64).  Beyond it this kernel took, against the other, per launch:  1 row
+// 16000 x 64 +0.3 us; 8 rows 16000 x 64 +3.3, 128 x 2048 +0.8, 1024 x 4096 +3.4; 9 rows 5000 x 32 +2.6; 16 rows 256 x 2048 +1.0; 32 rows 3000 x 32 +0.9; 33 rows 2048 x 128
+// +0.9; 64 rows 704 x 704 and 1500 x 16 +1.2 and, with a CTA per output column as the model would have it, 16000 x 64 +26.
 bool gemm_lanes_better(int64_t M, int64_t N, int64_t K, int sm_count) {
+    if (M <= 8 ? N > 64 * int64_t(sm_count) || (M > 4 && K > 1408) : N > 3072 || M * N > 67000 || K > 1024 || M * N * K > 30000000) return false;
     const LanesPlan pl = plan(M, N, K, sm_count);
     return pl.kernel != nullptr && 1.13 * pl.us < 2.45 + 0.00115 * double(K) + 0.0003 * double(N) + 0.062 * double(std::max<int64_t>(M - 8, 0));
 }

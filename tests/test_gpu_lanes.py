@@ -42,3 +42,25 @@ def test_against_fp64(built_lib, tmp_path, M, N, K):
     assert all(q["kernel"] == "gemm_lanes_ffma" for q in eng.profile_launches())
     assert eng.device_status() == 0
     eng.close()
+
+
+# On either side of what the rule was measured for (rows, columns, K)
+@pytest.mark.parametrize("M,N,K,lanes", [(1, 9472, 64, True), (1, 9473, 64, False), (1, 16000, 64, False), (8, 9000, 64, True), (8, 64, 1408, True), (8, 64, 1416, False), (4, 64, 1416, True),
+                                         (9, 3072, 32, True), (9, 3073, 32, False), (9, 64, 1032, False), (32, 3000, 32, False), (64, 704, 704, False), (64, 16000, 64, False)])
+def test_dispatch(built_lib, tmp_path, M, N, K, lanes):
+    from fxfusion_b200.engine import ExecutionEngine
+    rng = np.random.default_rng(M + N + K)
+    w, bias = (rng.standard_normal((N, K)) / math.sqrt(K)).astype(np.float32), rng.standard_normal(N, dtype=np.float32)
+    b = lowering.GraphBuilder(f"rule_{M}_{N}_{K}")
+    x = b.input((M, K), wire.DT_F32)
+    b.output(b.op("Relu", [b.op("LinearRelu", [x, b.const(w), b.const(bias)], (M, N))], (M, N)))
+    path = tmp_path / "g.bin"
+    wire.dump(b.finish(), path)
+    eng = ExecutionEngine(str(path), "cuda:0")
+    xin = torch.randn(M, K, generator=torch.Generator().manual_seed(K))
+    got = eng.run([xin.cuda()])[0].cpu().double()
+    want = torch.relu(xin.double() @ torch.from_numpy(w).double().T + torch.from_numpy(bias).double())
+    assert ((got - want).norm() / want.norm()).item() < 2.0 ** -20   # 22 bits of each factor, at most K / 16 truncated additions
+    assert [q["kernel"] for q in eng.profile_launches()][0].startswith("gemm_lanes_ffma" if lanes else "gemm_f16x3"), eng.describe()
+    assert eng.device_status() == 0
+    eng.close()
