@@ -1140,7 +1140,8 @@ TailSplit plan_tail(int64_t tiles, int num_k, const Variant& v, int workers, boo
     // One round, cut inside clusters: the partial blocks are added through distributed shared memory in 1.8 us whatever their number (through L2,
     // flag by flag, it takes 3 to 8), and the more SMs the clusters take, and the more the launch before them does (`before`, its share), the later they start, up to 3 us each.
     // From wait to end, through L2 and so: 512 x 256 x 1024 8.1 and 5.0 us; one image of 14 x 14, 256 channels, 3x3 10.4 and 6.2; 7 x 7, 512 channels
-    // 14.5 and 11.
+    // 14.5 and 11.  Every pick against the same launch without clusters, pairs of products in a chain, 18 shapes of 32 to 3072 columns x 11 numbers of
+    // rows from 65 to 1000: from +0.4 us (65 x 64 x 512) to -46 (128 x 32 x 8192, whose partial tiles otherwise wait for one another in L2).
     if (clusters != nullptr && !v.pair && rounds == 0)
         for (int s = 2; s <= kMaxClusterK && s <= num_k; s++) {
             if (tiles > clusters[s]) continue;
@@ -1196,7 +1197,8 @@ int gemm_f16_split_parts(int64_t N) { return int((N + 31) / 32) * 2; }
 static int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, bool pairs, bool k_split, bool vt, int64_t vt_col0, const Variant* table, TailSplit* out_ts, int* out_workers,
                         const int* clusters = nullptr, bool images = false) {
     const int num_k = int((K + BK - 1) / BK);
-    // what wrote x[M, K] had about a CTA per 128 x 64 of it (images: K counts every tap, and the maps that are cut are small)
+    // An assumption about a launch that is not known here: what wrote x[M, K] had about a CTA per 128 x 64 of it (images: K counts every tap, and the maps
+    // that are cut are small).  Off by all of it, it is 3 us for one variant against another.
     const double before = images ? 0.0 : std::min(1.0, double((M + BM - 1) / BM) * num_k / sm_count);
     int best = -1;
     double best_us = 0;
