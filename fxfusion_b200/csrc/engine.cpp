@@ -1076,6 +1076,8 @@ int build(fxf_engine* e, const uint8_t* bytes, size_t nbytes) {
         if (n.plan->prepare(e->reg, n.in, n.out, n.params, e->ctx)) return 1;
     }
     FXF_CUDA(cudaDeviceSynchronize());
+    for (auto& n : e->nodes)
+        if (n.plan->settle()) return 1;
     e->ctx.weights_settled = true;   // prepared and waited for: later kernels may read weights before their predecessors end
 
     // ---- warm-up run (validates every node's arguments), then capture ------------------------

@@ -157,7 +157,7 @@ struct DensePlan : NodePlan {
         off_scales = persist_bytes;
         persist_bytes += round_up(size_t(11 * 64 * heads + heads + 2) * sizeof(float), 256);
     }
-    // Where the rows of every projection come in split form from a LayerNorm.  Run once per engine, which waits for it anyway.
+    // Where the rows of every projection come in split form from a LayerNorm.
     int prepare_scales(Registry& reg, const TensorIds& in, ExecCtx& ctx) {
         const SplitMat *x = split_of(ctx, in[0]), *m = mask_rows_from & 2u ? split_of(ctx, in[1]) : x;
         if (x == nullptr || m == nullptr || !(x->cap > 0.f) || !(m->cap > 0.f) || x->gamma < 0 || m->gamma < 0) return 0;
@@ -179,10 +179,12 @@ struct DensePlan : NodePlan {
         scales.q_bias = s[1].ptr; scales.kv_bias = s[wk + 1].ptr + k0;
         scales.H = int(H_scales);
         FXF_CUDA(cudaMemsetAsync(scales.unusable, 0, sizeof(int), ctx.stream));
-        if (launch_attention_scales(scales, ctx)) return 1;
+        return launch_attention_scales(scales, ctx);
+    }
+    int settle() override {
+        if (scales.unusable == nullptr) return 0;
         int unusable = 1;
-        FXF_CUDA(cudaMemcpyAsync(&unusable, scales.unusable, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
-        FXF_CUDA(cudaStreamSynchronize(ctx.stream));
+        FXF_CUDA(cudaMemcpy(&unusable, scales.unusable, sizeof(int), cudaMemcpyDeviceToHost));
         scaled = unusable == 0;
         uneven = !scaled;
         return 0;

@@ -190,7 +190,7 @@ struct NodePlan {
     int mask_input = -1;
     int64_t mask_B = 0, mask_T = 0, mask_Tk = 0;
     uint32_t mask_rows_from = 0;   // the inputs that have to arrive in split form for that, a bit each
-    bool scaled = false;           // found by prepare(): Q, K and V have scales, the node runs so wherever the engine keeps the mask's bits
+    bool scaled = false;           // found by settle(): Q, K and V have scales, the node runs so wherever the engine keeps the mask's bits
     bool images = false;        // decided by the engine before prepare(): the node runs on them
     size_t scratch_bytes = 0;   // shared scratch wanted at execute time
     size_t persist_bytes = 0;   // memory that must survive across runs (e.g. re-laid-out weights)
@@ -200,6 +200,8 @@ struct NodePlan {
     bool tp_sharded = false;    // the node computes a partial result on each tensor-parallel rank (summed by an exchange)
     // Called once after device memory exists (constants uploaded).  May launch kernels.
     virtual int prepare(Registry&, const TensorIds&, const TensorIds&, const Params&, ExecCtx&) { return 0; }
+    // Called by the engine once all of that has run on the device.
+    virtual int settle() { return 0; }
 };
 
 // What a plan builder needs to know about the engine it plans for.
