@@ -7,7 +7,7 @@ import fxfusion_b200
 
 KERNELS = Path(fxfusion_b200.__file__).parent / "csrc" / "kernels"
 # prepared when the engine is built: bounds of weights, biases of weights in split form (constants of the graph)
-CONSTANT = {"p.w_bound", "p.w_bound + 1", "bound", "bound + 1", "p.v_bound", "p.v_bound + 1", "p.bias + c", "p.bias + grow"}
+CONSTANT = {"p.w_bound", "p.w_bound + 1", "p.v_bound", "p.v_bound + 1", "p.bias + c", "p.bias + grow"}
 
 
 def test_read_only_loads_are_of_constants():
